@@ -366,16 +366,25 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> Non
     _check(f(_ptr(src), _ptr(out), _ptr(rows), c_int(rows.numel()), c_int(row_bytes), _stream()), "gather_rows")
 
 
+def _sgemm_scratch(lib: ctypes.CDLL):
+    f = _fn(lib, "tkb_sgemm_tn_scratch")
+    f.restype, f.argtypes = ctypes.c_longlong, (c_int, c_int, c_int)
+    return f
+
+
 def sgemm_tn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FP32 FMA, fixed summation order)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (all 24 bits of both operands, fixed summation order whatever M)."""
     _need_cuda(a, w, out)
     M, K = a.shape
     N = w.shape[0]
     _need(w.shape[1] == K and out.shape == (M, N), "sgemm_tn: shapes")
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "sgemm_tn: float32 only")
     _need(a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1, "sgemm_tn: rows must be contiguous")
-    f = _fn(_libs.get("sgemm.cu"), "tkb_sgemm_tn_f32")
-    _check(f(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(a.stride(0) if M > 1 else K),
+    lib = _libs.get("sgemm.cu")
+    n_scratch = _sgemm_scratch(lib)(M, N, K)
+    scratch = torch.empty((n_scratch,), dtype=torch.float32, device=a.device) if n_scratch else None
+    f = _fn(lib, "tkb_sgemm_tn_f32")
+    _check(f(_ptr(a), _ptr(w), _ptr(out), _ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(a.stride(0) if M > 1 else K),
              c_int(w.stride(0) if N > 1 else K), c_int(out.stride(0) if M > 1 else N), _stream()), "sgemm_tn")
 
 
