@@ -1,0 +1,112 @@
+"""The recurrence in chunks of tokens against the token-by-token sums in float64 and against the walk: every form of the decays,
+requests around the length from which chunks are used and around whole chunks, decays of zero and below, decays that underflow,
+heads that share q and k, column slices, slots that are not written, and rows that only the walk takes."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def plain(q, k, v, a, c, skip, S):
+    """q, k [T, H, d], v [T, H, e], a [T, H, d or 1], c [T, H], S [H, d, e], all float64."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S = a[t][:, :, None] * S + c[t][:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+        out[t] = torch.einsum("hde,hd->he", S, q[t]) + skip[:, None] * v[t]
+    return out, S
+
+
+def problem(form, heads, groups, vdim, lens, seed):
+    g = torch.Generator().manual_seed(seed)
+    T, d = sum(lens), 128
+    p = dict(q=torch.randn(T, groups * d, generator=g), k=torch.randn(T, groups * d, generator=g), v=torch.randn(T, heads * vdim, generator=g),
+             dt_dec=None, decay_head=None, decay_vec=None, skip=None)
+    if form == "head":
+        dec = torch.rand(heads, generator=g) * 0.5 + 0.5
+        dec[0], dec[1 % heads] = 0.9995, -0.9
+        p["decay_head"], a, c = dec, dec.expand(T, heads)[:, :, None], torch.ones(T, heads)
+    elif form == "token":
+        c, dec = torch.rand(T, heads, generator=g) * 2, torch.rand(T, heads, generator=g)
+        dec[::37] = 0.0
+        dec[50:60] = 1e-9
+        p["dt_dec"], p["skip"], a = torch.cat([c, dec], 1), torch.randn(heads, generator=g), dec[:, :, None]
+    else:
+        f = torch.sigmoid(torch.randn(T, heads * d, generator=g) * 3) ** (1 / 16 if form == "channel" else 4)
+        f[::41] = 0.0
+        p["decay_vec"], a, c = f, f.view(T, heads, d), torch.ones(T, heads)
+    state = torch.randn(len(lens) + 1, heads * vdim * d + 4, generator=g)
+    ref, at = [], 0
+    for i, n in enumerate(lens):
+        r = slice(at, at + n)
+        rep = lambda x: x[r].double().view(n, groups, d).repeat_interleave(heads // groups, 1)  # noqa: E731
+        S = state[i, : heads * vdim * d].double().view(heads, vdim, d).transpose(1, 2)
+        skip = p["skip"].double() if p["skip"] is not None else torch.zeros(heads, dtype=torch.float64)
+        o, S = plain(rep(p["q"]), rep(p["k"]), p["v"][r].double().view(n, heads, vdim), a[r].double(), c[r].double(), skip, S)
+        ref.append((o.reshape(n, -1), S.transpose(1, 2).reshape(-1)))
+        at += n
+    return p, state, ref
+
+
+def run(p, state, lens, heads, groups, vdim, wide=4, write=True):
+    from tokasaurus_b200.kernels import ops
+
+    T = sum(lens)
+    both = torch.zeros(T, p["q"].shape[1] * 2 + p["v"].shape[1] + wide)  # q, k and v as column slices of one tensor
+    both[:, : p["q"].shape[1]], both[:, p["q"].shape[1]:2 * p["q"].shape[1]] = p["q"], p["k"]
+    both[:, 2 * p["q"].shape[1]:both.shape[1] - wide] = p["v"]
+    both = both.to(DEV)
+    n = p["q"].shape[1]
+    dev = lambda x: None if x is None else x.to(DEV)  # noqa: E731
+    st, out = state.to(DEV), torch.full((T, heads * vdim), 7.0, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    ops.decay_walk(both[:, :n], both[:, n:2 * n], both[:, 2 * n:both.shape[1] - wide], heads // groups, dev(p["dt_dec"]),
+                   dev(p["decay_head"]), dev(p["skip"]), st, out, i32(list(range(len(lens)))), i32(starts), i32(lens), len(lens),
+                   heads, 128, vdim, write, decay_vec=dev(p["decay_vec"]))
+    return out.cpu(), st.cpu()
+
+
+@pytest.mark.parametrize("form,heads,groups", [("head", 3, 3), ("token", 4, 2), ("channel", 2, 2), ("sharp", 2, 2)])
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("lens", [[192], [191, 192, 193], [1, 256, 5, 257, 383], [40, 700]])
+def test_chunks(form, heads, groups, vdim, lens, monkeypatch):
+    from tokasaurus_b200.kernels import ops
+
+    p, state, ref = problem(form, heads, groups, vdim, lens, 7 * sum(lens) + vdim)
+    out, st = run(p, state, lens, heads, groups, vdim)
+    monkeypatch.setattr(ops, "DECAY_CHUNKS_FROM", 1 << 30)
+    walked, wst = run(p, state, lens, heads, groups, vdim)
+    at, size = 0, heads * vdim * 128
+    rel = lambda x, y: float((x.double() - y).norm() / y.norm())  # noqa: E731
+    for i, n in enumerate(lens):
+        o, S = ref[i]
+        # a sum of some hundred float32 products, each exact to 2^-24 and rounded a few times on its way: 16 units in the last place
+        assert rel(out[at:at + n], o) < 16 * 2.0 ** -24 and rel(st[i, :size], S) < 16 * 2.0 ** -24
+        assert rel(out[at:at + n], o) < 1.5 * rel(walked[at:at + n], o) + 2.0 ** -24  # no less exact than the walk
+        if n < 192:
+            assert torch.equal(out[at:at + n], walked[at:at + n]) and torch.equal(st[i], wst[i])
+        at += n
+    assert torch.equal(st[:, size:], state[:, size:]) and torch.equal(st[-1], state[-1])  # nothing beside the requests' states
+    monkeypatch.undo()
+    again, kept = run(p, state, lens, heads, groups, vdim, write=False)
+    assert torch.equal(again, out) and torch.equal(kept, state)
+    odd, _ = run(p, state, lens, heads, groups, vdim, wide=3)  # strides that are no whole 16-byte pieces: the walk
+    assert torch.equal(odd, walked)
+
+
+def test_chunks_cut_into_steps():
+    """A request in portions: chunks, walk, chunks, walk; the state goes from one to the other."""
+    lens = [700]
+    p, state, ref = problem("channel", 2, 2, 128, lens, 3)
+    st, outs, at = state, [], 0
+    for n in (200, 100, 321, 79):
+        part = {k: (v[at:at + n] if v is not None and v.shape[0] == 700 else v) for k, v in p.items()}
+        out, st = run(part, st, [n], 2, 2, 128)
+        outs.append(out)
+        at += n
+    assert float((torch.cat(outs).double() - ref[0][0]).norm() / ref[0][0].norm()) < 16 * 2.0 ** -24

@@ -1,0 +1,622 @@
+// The recurrence of decay_recurrence.cu for requests that bring many tokens, in chunks of 64:
+//
+//     S_t = diag(a_t) S_(t-1) + (c_t k_t) v_t^T,        o_t = S_t^T q_t + D v_t
+//
+// (a_t one number a head and token, a constant a head, or a number for every key channel).  The walk over the tokens there is
+// a chain of one step a token; here what tokens of one chunk do to one another is products of matrices, and only the state
+// goes from chunk to chunk:
+//   chunk_states   a block a (chunk, head): what the chunk adds to the state, U = sum_s (decay from s to the chunk's end) c_s k_s v_s^T;
+//   chunk_scan     element by element over a request's chunks: the state each chunk starts from (in U's place), and the
+//                  state after the last one into the request's slot;
+//   chunk_outputs  a block a (chunk, head): o_t = (q_t decayed from the chunk's start) S_start + sum_s A[t][s] v_s with
+//                  A[t][s] = q_t . (decay from s to t) c_s k_s for s <= t.
+// No factor exceeds the decays' own products: one number a head is kept as a sum of logarithms in 64 bits, whose differences
+// are exact enough; a number a channel is kept as running products inside blocks of 16 tokens: A's blocks beside the diagonal
+// take q decayed from its block's start, k decayed to its block's end and the product of the blocks between, and A's diagonal
+// blocks are summed on the FP32 pipes with the product running along.  So nothing overflows, and what underflows is zero.
+//
+// Precision: every float32 operand of a product is cut into three bfloat16 numbers (x = h + m + l, all 24 bits) when it
+// comes into shared memory, and six products are kept (what is left out is below 2^-24 of a term).  The tensor instructions
+// (mma.sync m16n8k16) cut their sums off instead of rounding them, so a chain of the six for 16 terms starts from zero, the
+// small ones first, and its result is added to the float32 sum with an ordinary addition.
+//
+// What bounds it: instruction issue and, with one block an SM in chunk_outputs, the loads that open a block; then the states'
+// way through the L2 (64 KB a chunk and head, four times).  Operands are cut once a block and not once a warp that reads
+// them (cut from the fragments into tf32 halves, the kernels took 132 us where they take 108 now).  Chunks of 64: half the
+// states' traffic of 32, and the products inside a chunk are still a third of the work.
+// Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 147 us (358);
+// three requests of 3,001 tokens in all 158 (382) and 213 us (511); 64 heads of 128 x 64 on 8 groups 250 us (455).
+#include "common.cuh"
+
+using namespace tkb;
+
+namespace {
+
+constexpr int C = 64;            // tokens of a chunk
+constexpr int DIM = 128;         // key size
+constexpr int THREADS = 512;     // 16 warps, 4 x 4 over a block's result
+constexpr int PITCH = (DIM + 8) * 2;   // bytes of a staged row of 128 bfloat16 numbers: rows meet different banks
+constexpr int PLANE = C * PITCH;       // one of the three planes of 64 such rows
+constexpr int P_PITCH = (C + 8) * 2;   // ... of A's rows
+constexpr int P_PLANE = C * P_PITCH;
+constexpr int LDR = DIM + 4;           // floats of a staged float32 row
+
+struct Args {
+  const float *q, *k, *v, *fvec, *dt_dec, *decay_head, *skip;
+  float *state, *out, *states, *gains;  // states [chunks][heads][vdim][dim]; gains [chunks][heads] or [chunks][heads][dim]
+  const int *seq_slot, *seq_q_start, *seq_q_len;
+  long long slot_stride;
+  int q_stride, k_stride, v_stride, f_stride, qk_div, n_seqs, heads, least, write_state;
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ int chunks_of(const Args& p, int s) {
+  const int n = s < p.n_seqs ? p.seq_q_len[s] : 0;
+  return n >= p.least ? (n + C - 1) / C : 0;
+}
+// The request and the chunk of it that number `id` is (chunks are counted over the requests in order), by one warp.
+__device__ __forceinline__ bool find_chunk(const Args& p, int id, int& seq, int& chunk) {
+  const int lane = threadIdx.x & 31;
+  for (int s0 = 0, base = 0; s0 < p.n_seqs; s0 += 32) {
+    const int n = chunks_of(p, s0 + lane);
+    int upto = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, base + upto > id);
+    if (past) {
+      const int l = __ffs(past) - 1;
+      seq = s0 + l;
+      chunk = id - base - __shfl_sync(0xffffffffu, upto - n, l);
+      return true;
+    }
+    base += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
+// ------------------------------------------------- products of float32 operands on the bfloat16 tensor instructions
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack2(a, b);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  m = pack2(ra, rb);
+  l = pack2(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+}
+// Eight numbers into the three planes (p: 16-byte aligned place in the first).
+__device__ __forceinline__ void put8(unsigned char* p, int plane, const float4& x, const float4& y) {
+  uint4 h, m, l;
+  cut2(x.x, x.y, h.x, m.x, l.x);
+  cut2(x.z, x.w, h.y, m.y, l.y);
+  cut2(y.x, y.y, h.z, m.z, l.z);
+  cut2(y.z, y.w, h.w, m.w, l.w);
+  *reinterpret_cast<uint4*>(p) = h;
+  *reinterpret_cast<uint4*>(p + plane) = m;
+  *reinterpret_cast<uint4*>(p + 2 * plane) = l;
+}
+__device__ __forceinline__ void put1(unsigned char* p, int plane, float x) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(x);
+  const float r = x - __bfloat162float(h);
+  const __nv_bfloat16 m = __float2bfloat16_rn(r);
+  *reinterpret_cast<__nv_bfloat16*>(p) = h;
+  *reinterpret_cast<__nv_bfloat16*>(p + plane) = m;
+  *reinterpret_cast<__nv_bfloat16*>(p + 2 * plane) = __float2bfloat16_rn(r - __bfloat162float(m));
+}
+template <bool TRANS> __device__ __forceinline__ void ldmat(uint32_t (&r)[4], uint32_t addr) {
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// acc += A B over 16 k's; A [16 MT x 16] and B [16 x 8 NT] in planes.  A_ROW: A lies [m][k], else [k][m]; B_ROW: B lies [n][k],
+// else [k][n].  a, b: shared-memory addresses of the first plane's element (0, 0).
+template <int MT, int NT, bool A_ROW, bool B_ROW>
+__device__ __forceinline__ void step16(float (&acc)[MT][NT][4], uint32_t a, int a_pitch, int a_plane, uint32_t b, int b_pitch, int b_plane) {
+  static_assert(NT % 2 == 0, "column tiles come in pairs");
+  const int lane = threadIdx.x & 31;
+  a += A_ROW ? (lane & 15) * a_pitch + (lane >> 4) * 16 : ((lane & 7) + ((lane >> 4) & 1) * 8) * a_pitch + ((lane >> 3) & 1) * 16;
+  b += B_ROW ? ((lane & 7) + ((lane >> 4) & 1) * 8) * b_pitch + ((lane >> 3) & 1) * 16
+             : ((lane & 7) + ((lane >> 3) & 1) * 8) * b_pitch + ((lane >> 4) & 1) * 16;
+  uint32_t fa[MT][3][4], fb[NT / 2][3][4];
+#pragma unroll
+  for (int w = 0; w < 3; w++) {
+#pragma unroll
+    for (int i = 0; i < MT; i++) ldmat<!A_ROW>(fa[i][w], a + w * a_plane + i * (A_ROW ? 16 * a_pitch : 32));
+#pragma unroll
+    for (int j = 0; j < NT / 2; j++) ldmat<!B_ROW>(fb[j][w], b + w * b_plane + j * (B_ROW ? 16 * b_pitch : 32));
+  }
+  float x[MT][NT][4];
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) x[i][j][e] = 0.f;
+  constexpr int WA[6] = {1, 0, 2, 0, 1, 0}, WB[6] = {1, 2, 0, 1, 0, 0};
+#pragma unroll
+  for (int w = 0; w < 6; w++)
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int j = 0; j < NT; j++) mma16(x[i][j], fa[i][WA[w]], fb[j / 2][WB[w]][(j & 1) * 2], fb[j / 2][WB[w]][(j & 1) * 2 + 1]);
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[i][j][e] += x[i][j][e];
+}
+template <int MT, int NT> __device__ __forceinline__ void zero(float (&acc)[MT][NT][4]) {
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
+}
+
+// A thread's pieces of 8 numbers of ROWS float32 rows of COLS: fetched into registers (rows from nt on: zeros), later cut
+// into planes.
+template <int ROWS, int COLS> struct Pieces {
+  static constexpr int N = ROWS * COLS / 8 / THREADS;
+  static_assert(ROWS * COLS / 8 % THREADS == 0, "whole pieces for every thread");
+  float4 x[N][2];
+  __device__ __forceinline__ void fetch(const float* src, int stride, int nt) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const int e = threadIdx.x + i * THREADS, r = e / (COLS / 8), c = (e % (COLS / 8)) * 8;
+      x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < nt) {
+        const float4* p = reinterpret_cast<const float4*>(src + (size_t)r * stride + c);
+        x[i][0] = p[0];
+        x[i][1] = p[1];
+      }
+    }
+  }
+  __device__ __forceinline__ void scale(const float* by) {  // a factor a row
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const float f = by[(threadIdx.x + i * THREADS) / (COLS / 8)];
+#pragma unroll
+      for (int u = 0; u < 2; u++) x[i][u].x *= f, x[i][u].y *= f, x[i][u].z *= f, x[i][u].w *= f;
+    }
+  }
+  __device__ __forceinline__ void put(unsigned char* planes, int pitch, int plane) const {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const int e = threadIdx.x + i * THREADS;
+      put8(planes + (e / (COLS / 8)) * pitch + (e % (COLS / 8)) * 16, plane, x[i][0], x[i][1]);
+    }
+  }
+  __device__ __forceinline__ void put_floats(float* dst, int ld) const {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const int e = threadIdx.x + i * THREADS;
+      float4* p = reinterpret_cast<float4*>(dst + (e / (COLS / 8)) * ld + (e % (COLS / 8)) * 8);
+      p[0] = x[i][0];
+      p[1] = x[i][1];
+    }
+  }
+};
+
+// One decay a token: sums of log |a| up to and with token t, and how many of them are negative (two warps).
+__device__ __forceinline__ void log_sums(const Args& p, int head, int row0, int nt, double* logs, int* negs, float* scale) {
+  const int t = threadIdx.x;
+  double x = 0.0;
+  int neg = 0;
+  if (t < C) {
+    float a = 1.f, c = 1.f;
+    if (t < nt) {
+      if (p.dt_dec) {
+        c = p.dt_dec[(size_t)(row0 + t) * 2 * p.heads + head];
+        a = p.dt_dec[(size_t)(row0 + t) * 2 * p.heads + p.heads + head];
+      } else {
+        a = p.decay_head[head];
+      }
+    }
+    scale[t] = c;
+    neg = a < 0.f;
+    x = a == 0.f ? -1e5 : log(fabs((double)a));  // (a decay of zero: e^-100000 is zero, and differences stay numbers)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, o);
+      const int m = __shfl_up_sync(0xffffffffu, neg, o);
+      if ((t & 31) >= o) x += y, neg += m;
+    }
+    logs[t] = x;
+    negs[t] = neg;
+  }
+  __syncthreads();
+  if (t >= 32 && t < C) logs[t] = x + logs[31], negs[t] = neg + negs[31];
+  __syncthreads();
+}
+// The product of the decays of tokens s + 1 .. t (s = -1: from the chunk's start).
+__device__ __forceinline__ float decay_between(const double* logs, const int* negs, int s, int t) {
+  const double from = s < 0 ? 0.0 : logs[s];
+  const float f = expf((float)(logs[t] - from));
+  return (negs[t] - (s < 0 ? 0 : negs[s])) & 1 ? -f : f;
+}
+
+// ------------------------------------------------------------------------------------------------ what a chunk adds
+template <int VDIM, bool VEC>
+__global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int V_PITCH = (VDIM + 8) * 2, V_PLANE = C * V_PITCH;
+  unsigned char* kp = smem;              // k's planes
+  unsigned char* vp = kp + 3 * PLANE;    // v's
+  __shared__ double logs[C];
+  __shared__ float scale[C], blocks[4][DIM];
+  __shared__ int negs[C], where[2];
+  trigger_dependents();
+  grid_dependency_wait();
+  const int id = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    int s = -1, c = 0;
+    if (!find_chunk(p, id, s, c)) s = -1;
+    if (lane == 0) where[0] = s, where[1] = c;
+  }
+  __syncthreads();
+  const int seq = where[0];
+  if (seq < 0) return;
+  const int nt = min(C, p.seq_q_len[seq] - where[1] * C), row0 = p.seq_q_start[seq] + where[1] * C;
+  const size_t at = (size_t)id * p.heads + head;
+  Pieces<C, VDIM> v;
+  v.fetch(p.v + (size_t)row0 * p.v_stride + (size_t)head * VDIM, p.v_stride, nt);
+  if (VEC) {
+    // a thread one channel of 16 tokens: k decayed to the chunk's end
+    const int d = tid & (DIM - 1), blk = tid >> 7;
+    const float* kc = p.k + (size_t)(row0 + blk * 16) * p.k_stride + head * DIM + d;
+    const float* fc = p.fvec + (size_t)(row0 + blk * 16) * p.f_stride + head * DIM + d;
+    float k[16], f[16], run = 1.f;
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+      const bool there = blk * 16 + s < nt;
+      k[s] = there ? kc[(size_t)s * p.k_stride] : 0.f;
+      f[s] = there ? fc[(size_t)s * p.f_stride] : 1.f;
+    }
+#pragma unroll
+    for (int s = 0; s < 16; s++) run *= f[s];
+    blocks[blk][d] = run;
+    __syncthreads();
+    run = 1.f;
+    for (int b = 3; b > blk; b--) run *= blocks[b][d];
+#pragma unroll
+    for (int s = 15; s >= 0; s--) {
+      put1(kp + (blk * 16 + s) * PITCH + 2 * d, PLANE, k[s] * run);
+      run *= f[s];
+    }
+    if (blk == 0) p.gains[at * DIM + d] = run;
+  } else {
+    Pieces<C, DIM> k;
+    k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
+    log_sums(p, head, row0, nt, logs, negs, scale);
+    if (tid < C) scale[tid] *= decay_between(logs, negs, tid, nt - 1);
+    if (tid == 0) p.gains[at] = decay_between(logs, negs, -1, nt - 1);
+    __syncthreads();
+    k.scale(scale);  // (rows from nt on are zeros; their factors are finite: no decays follow them)
+    k.put(kp, PITCH, PLANE);
+  }
+  v.put(vp, V_PITCH, V_PLANE);
+  __syncthreads();
+  constexpr int MT = VDIM / 64;
+  const int m0 = (warp >> 2) * (VDIM / 4), n0 = (warp & 3) * 32;
+  float acc[MT][4][4];
+  zero(acc);
+  for (int s = 0; s < nt; s += 16)
+    step16<MT, 4, false, false>(acc, smem_addr(vp) + s * V_PITCH + 2 * m0, V_PITCH, V_PLANE, smem_addr(kp) + s * PITCH + 2 * n0, PITCH, PLANE);
+  float* u = p.states + at * VDIM * DIM;
+  const int g = lane >> 2, t2 = (lane & 3) * 2;
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      float* o = u + (size_t)(m0 + 16 * i + g) * DIM + n0 + 8 * j + t2;
+      *reinterpret_cast<float2*>(o) = make_float2(acc[i][j][0], acc[i][j][1]);
+      *reinterpret_cast<float2*>(o + 8 * DIM) = make_float2(acc[i][j][2], acc[i][j][3]);
+    }
+}
+
+// --------------------------------------------------------------------------------- the state every chunk starts from
+template <int VDIM, bool VEC>
+__global__ void __launch_bounds__(256) chunk_scan_kernel(Args p) {
+  trigger_dependents();
+  grid_dependency_wait();
+  const int seq = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
+  const int n = chunks_of(p, seq);
+  if (n == 0) return;
+  int first = 0;  // the request's first chunk: those of the requests before it
+  for (int s0 = 0; s0 < seq; s0 += 32) first += s0 + lane < seq ? chunks_of(p, s0 + lane) : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+  const int e = (blockIdx.z * 256 + threadIdx.x) * 4;  // (VDIM * DIM is a multiple of 1,024)
+  float* st = p.state + (size_t)p.seq_slot[seq] * p.slot_stride + (size_t)head * VDIM * DIM + e;
+  float4 S = *reinterpret_cast<const float4*>(st);
+  constexpr int AHEAD = 4;
+  float4 u[AHEAD];
+  auto place = [&](int c) { return (size_t)(first + c) * p.heads + head; };
+#pragma unroll
+  for (int i = 0; i < AHEAD; i++)
+    if (i < n) u[i] = *reinterpret_cast<const float4*>(p.states + place(i) * VDIM * DIM + e);
+  for (int c0 = 0; c0 < n; c0 += AHEAD) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++) {
+      const int c = c0 + i;
+      if (c >= n) break;
+      float4 a;
+      if (VEC) {
+        a = *reinterpret_cast<const float4*>(p.gains + place(c) * DIM + (e & (DIM - 1)));
+      } else {
+        a.x = a.y = a.z = a.w = p.gains[place(c)];
+      }
+      const float4 x = u[i];
+      float* slot = p.states + place(c) * VDIM * DIM + e;
+      if (c + AHEAD < n) u[i] = *reinterpret_cast<const float4*>(p.states + place(c + AHEAD) * VDIM * DIM + e);
+      *reinterpret_cast<float4*>(slot) = S;
+      S.x = fmaf(a.x, S.x, x.x);
+      S.y = fmaf(a.y, S.y, x.y);
+      S.z = fmaf(a.z, S.z, x.z);
+      S.w = fmaf(a.w, S.w, x.w);
+    }
+  }
+  if (p.write_state) *reinterpret_cast<float4*>(st) = S;
+}
+
+// ------------------------------------------------------------------------------------------------------ the outputs
+// Sums of four values over a warp's lanes; value i comes out in the lanes with (lane >> 3) == i.
+__device__ __forceinline__ float sum4(const float (&x)[4], int lane) {
+  const bool up = lane & 16;
+  float a = up ? x[2] : x[0], b = up ? x[3] : x[1];
+  a += __shfl_xor_sync(0xffffffffu, up ? x[0] : x[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, up ? x[1] : x[3], 16);
+  const bool mid = lane & 8;
+  float s = (mid ? b : a) + __shfl_xor_sync(0xffffffffu, mid ? a : b, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+// Shared memory of chunk_outputs (bytes): q's planes, whose place v's take in the end | k's planes and, with a decay a
+// channel, those of q's rows decayed from further back; then the state's planes | A's planes.  With a decay a channel q, k
+// and the decays first stand in the first two places as float32 rows.
+constexpr int OFF_K = 3 * PLANE, OFF_FAR = 6 * PLANE, OFF_P = OFF_K + 3 * DIM * PITCH, OUT_SMEM = OFF_P + 3 * P_PLANE;
+constexpr int FAR_PLANE = 48 * PITCH;  // q of the third and fourth blocks from one block further back, then of the fourth from two
+static_assert(3 * C * LDR * 4 <= 6 * PLANE && OFF_FAR + 3 * FAR_PLANE <= OFF_P, "places");
+
+template <int VDIM, bool VEC>
+__global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int V_PITCH = (VDIM + 8) * 2, V_PLANE = C * V_PITCH;
+  __shared__ double logs[C];
+  __shared__ float scale[C], blocks[4][DIM];
+  __shared__ int negs[C], where[2];
+  trigger_dependents();
+  grid_dependency_wait();
+  const int id = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    int s = -1, c = 0;
+    if (!find_chunk(p, id, s, c)) s = -1;
+    if (lane == 0) where[0] = s, where[1] = c;
+  }
+  __syncthreads();
+  const int seq = where[0];
+  if (seq < 0) return;
+  const int nt = min(C, p.seq_q_len[seq] - where[1] * C), row0 = p.seq_q_start[seq] + where[1] * C;
+  const size_t at = (size_t)id * p.heads + head;
+  const int wm = warp >> 2, wn = warp & 3, g = lane >> 2, t2 = (lane & 3) * 2;
+  const uint32_t q_at = smem_addr(smem), k_at = q_at + OFF_K, p_at = q_at + OFF_P;
+  unsigned char* pp = smem + OFF_P;
+  Pieces<VDIM, DIM> state;
+  // put two neighbouring elements of A
+  auto put_p = [&](int t, int s, float x, float y) {
+    uint32_t h, m, l;
+    cut2(x, y, h, m, l);
+    unsigned char* o = pp + t * P_PITCH + 2 * s;
+    *reinterpret_cast<uint32_t*>(o) = h;
+    *reinterpret_cast<uint32_t*>(o + P_PLANE) = m;
+    *reinterpret_cast<uint32_t*>(o + 2 * P_PLANE) = l;
+  };
+  float qd[16];  // VEC: a channel of 16 of q's rows, decayed from their block's start
+  const int d = tid & (DIM - 1), blk = tid >> 7;
+  {
+    Pieces<C, DIM> q, k;
+    q.fetch(p.q + (size_t)row0 * p.q_stride + (head / p.qk_div) * DIM, p.q_stride, nt);
+    k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
+    if (VEC) {
+      float* qs = reinterpret_cast<float*>(smem);
+      float* ks = qs + C * LDR;
+      float* fs = ks + C * LDR;
+      Pieces<C, DIM> f;
+      f.fetch(p.fvec + (size_t)row0 * p.f_stride + head * DIM, p.f_stride, nt);
+      q.put_floats(qs, LDR);
+      k.put_floats(ks, LDR);
+      f.put_floats(fs, LDR);
+      __syncthreads();
+      // A's diagonal blocks: four warps a block of 16 tokens, a warp four of its tokens (34 products in all for each warp);
+      // a lane four channels
+      const float4* k4 = reinterpret_cast<const float4*>(ks) + lane;
+      const float4* f4 = reinterpret_cast<const float4*>(fs) + lane;
+      for (int r = 0; r < 4; r++) {
+        const int in = r == 0 ? wn : r == 1 ? 7 - wn : r == 2 ? 8 + wn : 15 - wn;
+        const int t = wm * 16 + in;
+        float4 w = reinterpret_cast<const float4*>(qs + t * LDR)[lane];
+        for (int s0 = in; s0 >= 0; s0 -= 4) {
+          float x[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int s = wm * 16 + s0 - u;
+            x[u] = 0.f;
+            if (s0 - u >= 0) {
+              const float4 kk = k4[s * (LDR / 4)], ff = f4[s * (LDR / 4)];
+              x[u] = fmaf(w.x, kk.x, fmaf(w.y, kk.y, fmaf(w.z, kk.z, w.w * kk.w)));
+              w.x *= ff.x, w.y *= ff.y, w.z *= ff.z, w.w *= ff.w;
+            }
+          }
+          const float sum = sum4(x, lane);
+          const int u = lane >> 3;
+          if ((lane & 7) == 0 && s0 - u >= 0) put1(pp + t * P_PITCH + 2 * (wm * 16 + s0 - u), P_PLANE, sum);
+        }
+        for (int s = wm * 16 + in + 1 + lane; s < wm * 16 + 16; s += 32) put1(pp + t * P_PITCH + 2 * s, P_PLANE, 0.f);
+      }
+      // a thread one channel of 16 tokens: q decayed from its block's start, k to its block's end, the block's product
+      float kd[16], ff[16], run = 1.f;
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const int row = blk * 16 + t;
+        ff[t] = row < nt ? fs[row * LDR + d] : 1.f;
+        run *= ff[t];
+        qd[t] = qs[row * LDR + d] * run;
+      }
+      blocks[blk][d] = run;
+      run = 1.f;
+#pragma unroll
+      for (int t = 15; t >= 0; t--) {
+        kd[t] = ks[(blk * 16 + t) * LDR + d] * run;
+        run *= ff[t];
+      }
+      __syncthreads();  // the float32 rows have been read
+      const float one = blk >= 2 ? blocks[blk - 1][d] : 0.f, two = blk == 3 ? one * blocks[1][d] : 0.f;
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        put1(smem + (blk * 16 + t) * PITCH + 2 * d, PLANE, qd[t]);
+        put1(smem + OFF_K + (blk * 16 + t) * PITCH + 2 * d, PLANE, kd[t]);
+        if (blk >= 2) put1(smem + OFF_FAR + ((blk - 2) * 16 + t) * PITCH + 2 * d, FAR_PLANE, qd[t] * one);
+        if (blk == 3) put1(smem + OFF_FAR + (32 + t) * PITCH + 2 * d, FAR_PLANE, qd[t] * two);
+      }
+    } else {
+      log_sums(p, head, row0, nt, logs, negs, scale);
+      q.put(smem, PITCH, PLANE);
+      k.put(smem + OFF_K, PITCH, PLANE);
+    }
+  }
+  __syncthreads();
+  state.fetch(p.states + at * VDIM * DIM, DIM, VDIM);
+  if (VEC ? wn < wm : wn <= wm) {  // A's blocks below (and, with one decay a token, on) the diagonal
+    float acc[1][2][4];
+    zero(acc);
+    uint32_t a = q_at + wm * 16 * PITCH;
+    int plane = PLANE;
+    if (VEC && wm - wn >= 2) a = q_at + OFF_FAR + (wm - wn == 3 ? 32 : (wm - 2) * 16) * PITCH, plane = FAR_PLANE;
+#pragma unroll 2
+    for (int kk = 0; kk < DIM; kk += 16)
+      step16<1, 2, true, true>(acc, a + 2 * kk, PITCH, plane, k_at + wn * 16 * PITCH + 2 * kk, PITCH, PLANE);
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int t = wm * 16 + g + 8 * h, s = wn * 16 + 8 * j + t2;
+        float x = acc[0][j][2 * h], y = acc[0][j][2 * h + 1];
+        if (!VEC) {
+          x = s <= t && t < nt ? x * (scale[s] * decay_between(logs, negs, s, t)) : 0.f;
+          y = s + 1 <= t && t < nt ? y * (scale[s + 1] * decay_between(logs, negs, s + 1, t)) : 0.f;
+        }
+        put_p(t, s, x, y);
+      }
+  }
+  __syncthreads();  // k's planes have been read
+  state.put(smem + OFF_K, PITCH, DIM * PITCH);
+  if (VEC && blk > 0) {  // q decayed from the chunk's start
+    float run = 1.f;
+    for (int c = 0; c < blk; c++) run *= blocks[c][d];
+#pragma unroll
+    for (int t = 0; t < 16; t++) put1(smem + (blk * 16 + t) * PITCH + 2 * d, PLANE, qd[t] * run);
+  }
+  Pieces<C, VDIM> v;
+  v.fetch(p.v + (size_t)row0 * p.v_stride + (size_t)head * VDIM, p.v_stride, nt);
+  __syncthreads();
+  constexpr int NT = VDIM / 32;
+  const int n0 = wn * (VDIM / 4);
+  float acc[1][NT][4];
+  zero(acc);
+#pragma unroll 2
+  for (int kk = 0; kk < DIM; kk += 16)
+    step16<1, NT, true, true>(acc, q_at + wm * 16 * PITCH + 2 * kk, PITCH, PLANE, k_at + n0 * PITCH + 2 * kk, PITCH, DIM * PITCH);
+  const int t0 = wm * 16 + g;
+  if (!VEC) {
+    const float f0 = decay_between(logs, negs, -1, t0), f1 = decay_between(logs, negs, -1, t0 + 8);
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[0][j][e] *= e < 2 ? f0 : f1;
+  }
+  __syncthreads();  // q's planes have been read
+  v.put(smem, V_PITCH, V_PLANE);
+  __syncthreads();
+  for (int s = 0; s < 16 * (wm + 1); s += 16)
+    step16<1, NT, true, false>(acc, p_at + wm * 16 * P_PITCH + 2 * s, P_PITCH, P_PLANE, q_at + s * V_PITCH + 2 * n0, V_PITCH, V_PLANE);
+  const float d_skip = p.skip ? p.skip[head] : 0.f;
+  const size_t row = (size_t)p.heads * VDIM;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int t = t0 + 8 * h;
+    if (t >= nt) continue;
+    float* o = p.out + (size_t)(row0 + t) * row + (size_t)head * VDIM + n0 + t2;
+    const float* vrow = p.v + (size_t)(row0 + t) * p.v_stride + (size_t)head * VDIM + n0 + t2;
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      float2 x = make_float2(acc[0][j][2 * h], acc[0][j][2 * h + 1]);
+      if (p.skip) {
+        const float2 vv = *reinterpret_cast<const float2*>(vrow + 8 * j);
+        x.x = fmaf(d_skip, vv.x, x.x);
+        x.y = fmaf(d_skip, vv.y, x.y);
+      }
+      *reinterpret_cast<float2*>(o + 8 * j) = x;
+    }
+  }
+}
+
+template <int VDIM, bool VEC>
+int chunks_launch(const Args& p, int max_chunks, cudaStream_t st) {
+  constexpr size_t smem1 = 3 * PLANE + 3 * C * (VDIM + 8) * 2, smem3 = OUT_SMEM;
+  static bool attr_done = false;
+  if (!attr_done) {
+    cudaError_t e = cudaFuncSetAttribute(chunk_states_kernel<VDIM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(chunk_outputs_kernel<VDIM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
+    if (e != cudaSuccess) return (int)e;
+    attr_done = true;
+  }
+  int rc = launch_pdl(chunk_states_kernel<VDIM, VEC>, dim3(max_chunks, p.heads), dim3(THREADS), smem1, st, p);
+  if (rc) return rc;
+  rc = launch_pdl(chunk_scan_kernel<VDIM, VEC>, dim3(p.n_seqs, p.heads, VDIM * DIM / 1024), dim3(256), 0, st, p);
+  if (rc) return rc;
+  return launch_pdl(chunk_outputs_kernel<VDIM, VEC>, dim3(max_chunks, p.heads), dim3(THREADS), smem3, st, p);
+}
+
+}  // namespace
+
+// For the requests that bring at least `least` tokens (the others are left alone).  Arguments as in tkb_decay_walk; dim is
+// 128, vdim 64 or 128; q, k, v, fvec rows and their strides, state and slot_stride in whole 16-byte pieces.  states:
+// float32 [max_chunks][heads][vdim][128], gains: float32 [max_chunks][heads] (fvec: [max_chunks][heads][128]) are scratch;
+// max_chunks: at least the requests' tokens in chunks of 64, each request rounded up.
+TKB_EXPORT int tkb_decay_chunks(const float* q, int q_stride, const float* k, int k_stride, int qk_div, const float* fvec,
+                                int f_stride, const float* v, int v_stride, const float* dt_dec, const float* decay_head,
+                                const float* skip, float* state, long long slot_stride, float* out, const int* seq_slot,
+                                const int* seq_q_start, const int* seq_q_len, int n_seqs, int heads, int dim, int vdim,
+                                int write_state, int least, float* states, float* gains, int max_chunks, void* st_) {
+  if (n_seqs <= 0 || max_chunks <= 0) return 0;
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (dim != DIM || (vdim != 64 && vdim != 128) || heads <= 0 || heads > 65535 || qk_div <= 0 || least < 1) return -2;
+  if ((q_stride | k_stride | v_stride | (fvec ? f_stride : 0)) % 4 || slot_stride % 4 || !al(q) || !al(k) || !al(v) ||
+      (fvec && !al(fvec)) || !al(state) || !al(states) || !al(gains))
+    return -2;
+  if (fvec != nullptr && (dt_dec != nullptr || decay_head != nullptr || qk_div != 1)) return -2;
+  const Args p = {q, k, v, fvec, dt_dec, decay_head, skip, state, out, states, gains, seq_slot, seq_q_start, seq_q_len,
+                  slot_stride, q_stride, k_stride, v_stride, f_stride, qk_div, n_seqs, heads, least, write_state};
+  cudaStream_t st = (cudaStream_t)st_;
+  if (fvec) return vdim == 64 ? chunks_launch<64, true>(p, max_chunks, st) : chunks_launch<128, true>(p, max_chunks, st);
+  return vdim == 64 ? chunks_launch<64, false>(p, max_chunks, st) : chunks_launch<128, false>(p, max_chunks, st);
+}

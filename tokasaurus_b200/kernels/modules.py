@@ -31,7 +31,9 @@ def family_modules() -> list[tuple[str, dict | None]]:
     distance or behind a convolution, the gated recurrence a channel), at one or two sets of compile-time sizes each: the build
     check compiles these; a model compiles the sizes it needs (``Part.kernel_modules``)."""
     return [("post_norm.cu", None), ("decay_recurrence.cu", {"TKB_DR_LANES": 32, "TKB_DR_DPT": 4}),
-            ("decay_recurrence.cu", {"TKB_DR_LANES": 16, "TKB_DR_DPT": 8}), ("decay_recurrence.cu", {"TKB_DR_LANES": 8, "TKB_DR_DPT": 16}), ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 64}),
+            ("decay_recurrence.cu", {"TKB_DR_LANES": 16, "TKB_DR_DPT": 8}), ("decay_recurrence.cu", {"TKB_DR_LANES": 8, "TKB_DR_DPT": 16}),
+            ("decay_chunks.cu", None), ("attention_sink.cu", {"TKB_QK": 64, "TKB_VD": 64}),
+            ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 128}), ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 64}),
             ("attention_sink.cu", {"TKB_QK": 24, "TKB_VD": 40}), ("attention_sink.cu", {"TKB_QK": 64, "TKB_VD": 64, "TKB_SIGMOID": 1}),
             ("norm_conv.cu", None), ("moe.cu", None), ("recurrence.cu", {"TKB_REC_DPT": 16, "TKB_REC_CPT": 1}),
             ("recurrence.cu", {"TKB_REC_DPT": 3, "TKB_REC_CPT": 2}), ("latent_attention.cu", {"TKB_LAT_RANK": 192}),

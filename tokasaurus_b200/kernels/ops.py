@@ -1357,6 +1357,18 @@ def decay_walk_modules(dim: int, vdim: int) -> list[dict]:
     return out
 
 
+# Tokens of a request from which the recurrence goes in chunks of DECAY_CHUNK.  Measured on B200, 4 to 16 heads of
+# 128 x 128: the walk takes 12 us for 64 tokens, 22 for 128 and 0.15 us for each more; the chunk kernels 26 us for one chunk
+# as for two, 108 us for 2,048 tokens of 16 heads (the walk 300), and 35 and 147 us with a decay vector (11 and 358).
+DECAY_CHUNK = 64
+DECAY_CHUNKS_FROM = 192
+
+
+def decay_chunk_modules(dim: int, vdim: int) -> tuple:
+    """The kernel module for long requests, if heads of this size have one."""
+    return (("decay_chunks.cu", None),) if dim == 128 and vdim in (64, 128) else ()
+
+
 def _walk_defines(dim: int, vdim: int, columns: int, single: bool, device) -> dict:
     """Which build walks ``columns`` state columns (requests x heads x vdim).  Single tokens: 8 threads a column, each
     with several 16-byte loads of the state in flight (the time is the state's trip through memory).  Portions: the
@@ -1437,13 +1449,30 @@ def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: 
     _need(ones_out is None or (decay_vec is None and ones_out.dtype == torch.float32 and ones_out.is_contiguous()
                                and tuple(ones_out.shape) == (T, heads)), "decay_walk: ones_out float32 [T, heads]")
     _need(out.dtype == torch.float32 and out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "decay_walk: out float32 [T, heads * vdim]")
+    below = 0
+    rows = [q, k, v] + ([decay_vec] if decay_vec is not None else [])
+    if (ones_out is None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and decay_chunk_modules(dim, vdim)
+            and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in rows)
+            and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0):
+        # requests that bring many tokens; the walk below then leaves them alone.  Which requests these are is read on the
+        # device: a step graph is replayed for other lengths.
+        below = DECAY_CHUNKS_FROM
+        chunks = T // DECAY_CHUNK + min(n_seqs, T // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
+        states = torch.empty((chunks, heads, vdim, dim), dtype=torch.float32, device=q.device)
+        gains = torch.empty((chunks, heads, dim if decay_vec is not None else 1), dtype=torch.float32, device=q.device)
+        _check(_fn(_libs.get("decay_chunks.cu"), "tkb_decay_chunks")(
+            _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),
+            c_int(decay_vec.stride(0) if decay_vec is not None else 0), _ptr(v), c_int(v.stride(0)),
+            _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
+            _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
+            c_int(1 if write_state else 0), c_int(below), _ptr(states), _ptr(gains), c_int(chunks), _stream()), "decay_chunks")
     defines = _walk_defines(dim, vdim, n_seqs * heads * vall, T == n_seqs, q.device)
     _check(_fn(_libs.get("decay_recurrence.cu", **defines), "tkb_decay_walk")(
         _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),
         c_int(decay_vec.stride(0) if decay_vec is not None else 0), _ptr(v), c_int(v.stride(0)),
         _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
         _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(T), c_int(heads), c_int(dim), c_int(vdim),
-        c_int(1 if write_state else 0), _ptr(ones_out), _stream()), "decay_walk")
+        c_int(1 if write_state else 0), _ptr(ones_out), c_int(below), _stream()), "decay_walk")
 
 
 def memory_gates(proj: torch.Tensor, i_off: int, f_off: int, i_bias: torch.Tensor, f_bias: torch.Tensor, cap: float,

@@ -94,7 +94,8 @@ class DecayedLinearAttention(Mixer):
                 WeightSpec(n["o"], (self.width, H * e)), WeightSpec(n["norm"], (H * e,), role="vector"))
 
     def kernel_modules(self, dtype):
-        return tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + (("post_norm.cu", None),)
+        return (tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + ops.decay_chunk_modules(self.dim, self.vdim)
+                + (("post_norm.cu", None),))
 
     def cache_need(self):
         return StateNeed((self.n_heads * self.vdim * self.dim,), "float32")  # S^T: [head][value][key channel]
@@ -160,7 +161,8 @@ class GatedLinearAttention(Mixer):
                 WeightSpec(n["o"], (self.width, H * e)))
 
     def kernel_modules(self, dtype):
-        return tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + (("post_norm.cu", None),)
+        return (tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + ops.decay_chunk_modules(self.dim, self.vdim)
+                + (("post_norm.cu", None),))
 
     def cache_need(self):
         return StateNeed((self.n_heads * self.vdim * self.dim,), "float32")  # S^T: [head][value][key channel]
@@ -232,7 +234,8 @@ class Retention(Mixer):
                 WeightSpec(n["o"], (self.width, H * e)))
 
     def kernel_modules(self, dtype):
-        return tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + (("post_norm.cu", None),)
+        return (tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + ops.decay_chunk_modules(self.dim, self.vdim)
+                + (("post_norm.cu", None),))
 
     def cache_need(self):
         return StateNeed((self.n_heads * self.vdim * self.dim,), "float32")  # S^T: [head][value][key channel]

@@ -53,7 +53,8 @@ class SelectiveStateSpace(Mixer):
                 WeightSpec(n["o"], (self.width, self.inner)))
 
     def kernel_modules(self, dtype):
-        return tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + (("post_norm.cu", None),)
+        return (tuple(("decay_recurrence.cu", d) for d in self.walk_builds) + ops.decay_chunk_modules(self.state, self.vdim)
+                + (("post_norm.cu", None),))
 
     def cache_need(self):
         # [S^T of every head: heads x vdim x state | the convolution's last taps - 1 inputs: (taps - 1) x channels]
