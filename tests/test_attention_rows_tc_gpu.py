@@ -1,0 +1,158 @@
+"""Prompt portions over cached rows on the tcgen05 kernel against float64 sums: latent rows and [k | v] rows, groups of heads that
+do and do not divide a block's 128 rows, portions behind cached tokens, windows and chunks that start inside a tile, pages that
+come as TMA boxes and pages that are gathered, scores far beyond the cap, factors below zero, sinks, gates and sigmoid weights."""
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+class Problem:
+    """Requests with cached rows (the step's own among them) on shuffled pages; what no request owns is no number."""
+
+    def __init__(self, row, nkv, ps, lens, new, seed):
+        g = torch.Generator().manual_seed(seed)
+        pages = [-(-n // ps) for n in lens]
+        n_pages = sum(pages) + 3
+        perm = torch.randperm(n_pages, generator=g).tolist()
+        cache = torch.full((n_pages, nkv, ps, row), math.nan)
+        self.rows, table, indptr = [], [], [0]
+        for n, np_ in zip(lens, pages):
+            mine = [perm.pop() for _ in range(np_)]
+            rows = torch.randn(n, nkv, row, generator=g).bfloat16().float()
+            for j in range(n):
+                cache[mine[j // ps], :, j % ps] = rows[j]
+            table += mine
+            indptr.append(len(table))
+            self.rows.append(rows.to(DEV))
+        self.cache, self.lens, self.new, self.nkv, self.ps = cache.bfloat16().to(DEV), lens, new, nkv, ps
+        self.start = [sum(new[:i]) for i in range(len(new))]
+        self.T = sum(new)
+        self.tables = dict(seq_q_start=i32(self.start), seq_q_len=i32(new), seq_kv_len=i32(lens), page_indptr=i32(indptr), page_ids=i32(table))
+        self.g = g
+
+    def want(self, q, kd, v0, vd, heads, scale, window=0, chunk=0, cap=0.0, sinks=None, head_scale=None, head_bias=None, sigmoid=False):
+        out = torch.zeros(self.T, heads, vd, dtype=torch.float64, device=DEV)
+        group = heads // self.nkv
+        for s, (n, L) in enumerate(zip(self.new, self.lens)):
+            r = self.rows[s].double()
+            k, v = (x.repeat_interleave(group, 1) for x in (r[..., :kd], r[..., v0:v0 + vd]))
+            qq = q[self.start[s]:self.start[s] + n].double().view(n, heads, kd)
+            y = torch.einsum("thd,shd->hts", qq, k) * scale
+            if head_scale is not None:
+                y = y * head_scale.double()[:, None, None]
+            if cap:
+                y = cap * torch.tanh(y / cap)
+            if head_bias is not None:
+                y = y + head_bias.double()[:, None, None]
+            i = torch.arange(L - n, L, device=DEV)[:, None]
+            j = torch.arange(L, device=DEV)[None, :]
+            see = j <= i
+            if window:
+                see &= j > i - window
+            if chunk:
+                see &= j >= i - i % chunk
+            if sigmoid:
+                w = torch.sigmoid(y) * see
+            else:
+                y = y.masked_fill(~see, -math.inf)
+                top = y.amax(-1, keepdim=True)
+                if sinks is not None:
+                    top = torch.maximum(top, sinks.double()[:, None, None])
+                w = torch.exp(y - top)
+                den = w.sum(-1, keepdim=True) + (torch.exp(sinks.double()[:, None, None] - top) if sinks is not None else 0)
+                w = w / den
+            out[self.start[s]:self.start[s] + n] = torch.einsum("hts,shv->thv", w, v)
+        return out
+
+
+def check(got, want, several, magnitude):
+    """Weights are rounded to bfloat16 for their product with the values and the result once more: 2^-9 of the sum of
+    |weight value|, which is at most ``magnitude``, and 2^-9 of the result, doubled for what the score loses."""
+    err = (got.double() - want)[several].abs()
+    assert err.max() <= 2.0 ** -7 * magnitude, (float(err.max()), magnitude)
+    assert err.norm() <= 6e-3 * want[several].norm()
+
+
+@pytest.mark.parametrize("row,vd,heads", [(256, 192, 16), (256, 192, 32), (256, 128, 5), (128, 64, 128), (192, 96, 1)])
+@pytest.mark.parametrize("window,ps", [(0, 16), (100, 16), (64, 128), (300, 12)])
+def test_latent_rows(row, vd, heads, window, ps):
+    from tokasaurus_b200.kernels import ops
+
+    (module,) = ops.rows_tc_modules(row, row, 0, vd, False)
+    p = Problem(row, 1, ps, [37, 200, 1, 449], [37, 71, 1, 130], heads + window)
+    q = torch.randn(p.T, heads * row, generator=p.g).bfloat16().to(DEV)
+    out = torch.full((p.T, heads * row), 7.0, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    scale = 1 / math.sqrt(row)
+    ops.attn_rows_tc(module, q, out, row, p.cache, **p.tables, n_seqs=4, n_heads=heads, n_kv_heads=1, page_size=ps, scale=scale,
+                     window=window, status=status)
+    want = p.want(q, row, 0, vd, heads, scale, window)
+    several = torch.ones(p.T, dtype=torch.bool, device=DEV)
+    several[p.start[2]] = False
+    got = out.view(p.T, heads, row)
+    assert int(status) == 0
+    check(got[..., :vd], want, several, 4.5)
+    assert (got[..., vd:] == 7).all() and (got[~several] == 7).all()  # nothing beside the values, nothing of a single token
+
+
+@pytest.mark.parametrize("dim,vdim,heads,nkv", [(64, 64, 8, 2), (128, 128, 4, 4), (128, 64, 6, 2)])
+@pytest.mark.parametrize("window,chunk,ps", [(0, 0, 16), (100, 0, 16), (65, 0, 4), (0, 96, 16)])
+@pytest.mark.parametrize("form", ["plain", "capped", "far", "heads", "sigmoid"])
+def test_key_value_rows(dim, vdim, heads, nkv, window, chunk, ps, form):
+    from tokasaurus_b200.kernels import ops
+
+    p = Problem(dim + vdim, nkv, ps, [300, 64, 1, 129], [172, 64, 1, 2], dim + vdim + window + len(form))
+    q = torch.randn(p.T, heads * dim, generator=p.g).bfloat16().to(DEV)
+    scale = dim ** -0.5
+    opt = {}
+    vec = lambda f: f(torch.randn(heads, generator=p.g)).to(DEV)  # noqa: E731
+    if form == "capped":  # scores well within the cap: the polynomial; with sinks and an output gate
+        opt = dict(softcap=50.0, sinks=vec(lambda x: 3 * x))
+    if form == "far":  # scores many times the cap
+        opt, scale = dict(softcap=4.0, sinks=vec(lambda x: x)), scale * 8
+    if form == "heads":
+        opt = dict(head_scale=vec(lambda x: x), head_bias=vec(lambda x: x), softcap=6.0)
+    if form == "sigmoid":
+        opt = dict(head_bias=vec(lambda x: x), sigmoid=True)
+    gate = torch.randn(p.T, heads, generator=p.g).to(DEV) if form == "capped" else None
+    out = torch.full((p.T, heads * vdim), 7.0, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    (module,) = ops.sink_rows_tc_modules(dim, vdim)
+    ops.attn_rows_tc(module, q, out, vdim, p.cache, **p.tables, n_seqs=4, n_heads=heads, n_kv_heads=nkv, page_size=ps, scale=scale,
+                     window=window, status=status, chunk=chunk, gate=gate, out_scale=0.5, **opt)
+    names = dict(softcap="cap")
+    want = 0.5 * p.want(q, dim, dim, vdim, heads, scale, window, chunk, **{names.get(k, k): v for k, v in opt.items()})
+    if gate is not None:
+        want = want * torch.sigmoid(gate.double())[..., None]
+    several = torch.ones(p.T, dtype=torch.bool, device=DEV)
+    several[p.start[2]] = False
+    assert int(status) == 0
+    keys = min(300, window or 300, chunk or 300)
+    check(out.view(p.T, heads, vdim), want, several, 2.5 * (0.5 * keys ** 0.5 if form == "sigmoid" else 1.0) * (2 if form == "sigmoid" else 1))
+    assert (out.view(p.T, heads, vdim)[~several] == 7).all()
+
+
+def test_the_step_takes_it():
+    """``attn_sink_tc``: portions on this kernel, single tokens on theirs; forms that it does not have stay where they were."""
+    from tokasaurus_b200.kernels import ops
+
+    p = Problem(128, 2, 16, [300, 64, 90], [172, 64, 1], 5)
+    q = torch.randn(p.T, 8 * 64, generator=p.g).bfloat16().to(DEV)
+    sinks = torch.randn(8, generator=p.g).to(DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = torch.empty(p.T, 8 * 64, dtype=torch.bfloat16, device=DEV)
+    ops.attn_sink_tc(q, out, p.cache, **p.tables, n_seqs=3, sinks=sinks, n_heads=8, n_kv_heads=2, dim=64, vdim=64, page_size=16,
+                     scale=0.125, softcap=30.0, window=100, status=status)
+    want = p.want(q, 64, 64, 64, 8, 0.125, 100, 0, 30.0, sinks)
+    check(out.view(p.T, 8, 64), want, torch.ones(p.T, dtype=torch.bool, device=DEV), 2.5)
+    assert ops.sink_rows_tc_modules(64, 64, maps=2) == ops.sink_rows_tc_modules(64, 64, distance=True) == ()
+    assert ops.sink_rows_tc_modules(64, 64, keep_first=4) == ops.sink_rows_tc_modules(48, 64) == ops.sink_rows_tc_modules(64, 256) == ()

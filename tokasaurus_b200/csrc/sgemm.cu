@@ -179,20 +179,6 @@ __device__ __forceinline__ void fetch8(const float* __restrict__ p, int left, fl
   }
 }
 
-// The tensor instruction and its commit as a whole warp calls them: one lane is elected, and the operands stay where the
-// warp's common values live (called by one lane in a branch of its own, the 24 of a chunk took 1,390 cycles to issue, 560 so).
-__device__ __forceinline__ void umma_warp(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void commit_warp(uint64_t* bar) {
-  asm volatile(
-      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar)) : "memory");
-}
-
 __device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ w, int K) {
   float acc = 0.f;
   for (int k = 0; k < K; k++) acc = fmaf(a[k], w[k], acc);

@@ -40,7 +40,11 @@ def family_modules() -> list[tuple[str, dict | None]]:
             ("attention_mma.cu", {"TKB_HD": 256}), ("attention_sink.cu", {"TKB_QK": 64, "TKB_VD": 128, "TKB_MAPS": 2}),
             ("attention_sink.cu", {"TKB_QK": 24, "TKB_VD": 40, "TKB_MAPS": 2}), ("gated_recurrence.cu", None),
             ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 128, "TKB_DIST": 1}),
-            ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 128, "TKB_TAPS": 4})]
+            ("attention_sink.cu", {"TKB_QK": 128, "TKB_VD": 128, "TKB_TAPS": 4}),
+            ("attention_rows_tc.cu", {"TKB_ROW": 256, "TKB_KD": 256, "TKB_V0": 0, "TKB_VD": 192}),
+            ("attention_rows_tc.cu", {"TKB_ROW": 128, "TKB_KD": 64, "TKB_V0": 64, "TKB_VD": 64, "TKB_CAP": 1}),
+            ("attention_rows_tc.cu", {"TKB_ROW": 192, "TKB_KD": 128, "TKB_V0": 128, "TKB_VD": 64, "TKB_CAP": 1}),
+            ("attention_rows_tc.cu", {"TKB_ROW": 256, "TKB_KD": 128, "TKB_V0": 128, "TKB_VD": 128, "TKB_CAP": 1})]
 
 
 def optional_modules(head_dim: int) -> list[tuple[str, dict | None]]:

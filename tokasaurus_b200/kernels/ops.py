@@ -1596,6 +1596,43 @@ def silu_cols(x: torch.Tensor, ncols: int, defines: dict) -> None:
 
 
 # ---------------------------------------------------------------------------------------------
+# Prompt portions over cached rows that hold key and value, on the tcgen05 tensor cores (csrc/attention_rows_tc.cu)
+def rows_tc_modules(row: int, kd: int, v0: int, vd: int, capped: bool) -> tuple:
+    """The kernel module for rows of ``row`` values whose first ``kd`` are the key and whose ``vd`` from ``v0`` on are the
+    value, if one can be built for these sizes (64-column blocks, tensor memory for two shares of the output)."""
+    if row % 64 or kd % 64 or v0 % 64 or vd % 32 or not (0 < vd <= 192 and row <= 256 and 0 < kd <= row and v0 + vd <= row):
+        return ()
+    d = dict(TKB_ROW=row, TKB_KD=kd, TKB_V0=v0, TKB_VD=vd)
+    if capped:
+        d["TKB_CAP"] = 1
+    return (("attention_rows_tc.cu", d),)
+
+
+def attn_rows_tc(module: tuple, q: torch.Tensor, out: torch.Tensor, out_head: int, cache: torch.Tensor, seq_q_start: torch.Tensor,
+                 seq_q_len: torch.Tensor, seq_kv_len: torch.Tensor, page_indptr: torch.Tensor, page_ids: torch.Tensor, n_seqs: int,
+                 n_heads: int, n_kv_heads: int, page_size: int, scale: float, window: int | None, status: torch.Tensor,
+                 softcap: float = 0.0, chunk: int = 0, sinks: torch.Tensor | None = None, head_scale: torch.Tensor | None = None,
+                 head_bias: torch.Tensor | None = None, sigmoid: bool = False, gate: torch.Tensor | None = None,
+                 out_scale: float = 1.0) -> None:
+    """Attention of the requests that bring several tokens over cached rows [pages, kv heads, page size, row]; ``module``: an
+    element of ``rows_tc_modules``.  q [T, heads * kd]; head h's values go to columns h * out_head .. of out's rows."""
+    _need_cuda(q, out, cache, seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids, sinks, status, head_scale, head_bias, gate)
+    d = module[1]
+    T = q.shape[0]
+    _need(q.dtype == out.dtype == cache.dtype == torch.bfloat16 and q.is_contiguous() and q.shape[1] == n_heads * d["TKB_KD"],
+          "attn_rows_tc: bfloat16, q [T, heads * key size]")
+    _need(cache.is_contiguous() and tuple(cache.shape[1:]) == (n_kv_heads, page_size, d["TKB_ROW"]), "attn_rows_tc: cache rows")
+    _need(out.dim() == 2 and out.shape[0] == T and out.stride(1) == 1 and out.shape[1] >= (n_heads - 1) * out_head + d["TKB_VD"]
+          and (gate is None or (gate.dtype == torch.float32 and tuple(gate.shape) == (T, n_heads))), "attn_rows_tc: out and gate")
+    _check(_fn(_libs.get(module[0], **d), "tkb_attn_rows_tc")(
+        _ptr(q), _ptr(out), _ptr(cache), c_int(cache.shape[0]), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len),
+        _ptr(page_indptr), _ptr(page_ids), c_int(n_seqs), c_int(T), c_int(n_heads), c_int(n_kv_heads), c_int(page_size),
+        c_float(scale), c_float(softcap), c_int(window or 0), c_int(chunk), _ptr(sinks), _ptr(head_scale), _ptr(head_bias),
+        c_int(1 if sigmoid else 0), _ptr(gate), c_int(_row_stride(gate) if gate is not None else 0), c_float(out_scale),
+        ctypes.c_longlong(_row_stride(out)), c_int(out_head), _ptr(status), _stream()), "attn_rows_tc")
+
+
+# ---------------------------------------------------------------------------------------------
 # Attention with a score cap and a sink, keys and values of different sizes (csrc/attention_sink.cu)
 def sink_attention_defines(dim: int, vdim: int, sigmoid: bool = False, maps: int = 1, distance: bool = False,
                            taps: int = 0) -> dict:
@@ -1615,6 +1652,11 @@ def sink_attention_defines(dim: int, vdim: int, sigmoid: bool = False, maps: int
         _need(0 < taps <= 16, f"sink attention: one to sixteen taps, not {taps}")
         d["TKB_TAPS"] = taps
     return d
+
+
+def sink_rows_tc_modules(dim: int, vdim: int, maps: int = 1, distance: bool = False, keep_first: int = 0) -> tuple:
+    """The tcgen05 kernel module for prompt portions over rows [k | v], where it has the form."""
+    return rows_tc_modules(dim + vdim, dim, dim, vdim, True) if maps == 1 and not distance and not keep_first else ()
 
 
 def _sink_lib(dim, vdim, sigmoid=False, maps=1, distance=False, taps=0):
@@ -1796,6 +1838,19 @@ def attn_sink_tc(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, seq_q_
         if splits > 1:
             part = torch.empty((n_seqs * n_heads * maps * splits * (vdim + 2),), dtype=torch.float32, device=q.device)
     gate_args = _sink_gate(gate, T, n_heads, maps, "attn_sink_tc")
+    # portions on the tcgen05 kernel where it has the form: one map, no bias by distance, no kept first positions, head sizes of
+    # whole 64-column blocks, an output that takes 16-byte stores, up to 128 heads a kv head (measured on B200, 4,001 tokens of
+    # 32 heads of 64 + 64, window 1,024, capped: 224 us on mma.sync, 111 us there)
+    module = sink_rows_tc_modules(dim, vdim, maps, head_slope is not None, keep_first if window else 0)
+    by_rows = (portions and bool(module) and n_heads // n_kv_heads <= 128 and _row_stride(out) % 8 == 0
+               and all(t.data_ptr() % 16 == 0 for t in (q, out, cache)))
+    if by_rows:
+        attn_rows_tc(module[0], q, out, vdim, cache, seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids, n_seqs, n_heads,
+                     n_kv_heads, page_size, scale, window, status, softcap or 0.0, chunk or 0, sinks, head_scale, head_bias,
+                     sigmoid, gate, out_scale)
+        portions = False
+        if not singles:
+            return
     _check(_fn(_sink_lib(dim, vdim, sigmoid, maps, head_slope is not None, taps), "tkb_attn_sink_tc_bf16")(
         _ptr(q), _ptr(out), _ptr(cache), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(page_indptr),
         _ptr(page_ids), c_int(T), c_int(n_seqs), c_int(1 if portions else 0), c_int(1 if singles else 0), _ptr(sinks),

@@ -36,8 +36,9 @@ class LatentAttention(AttentionPlanning, Mixer):
     """In bfloat16, when the cached row (rank + rot values) is a multiple of 16 values and at most 256, the attention
     runs on the framework's tensor-core kernels for grouped queries: the rows are at once the keys (all rank + rot
     values) and the values (the kernel's output beyond the first rank values is not used) of ONE key/value head that
-    every query head reads, single tokens through the split-key kernel and portions through the tiled one, planned
-    on the host like ``PagedAttention``'s.  Otherwise (float32, other sizes, only some rows wanted) the FP32-pipe
+    every query head reads, single tokens through the split-key kernel, planned on the host like ``PagedAttention``'s, and
+    portions through the tcgen05 kernel for rows (rows of whole 64-column blocks, latents of at most 192 values) or the tiled
+    ``mma.sync`` one.  Otherwise (float32, other sizes, only some rows wanted) the FP32-pipe
     kernel of csrc/latent_attention.cu serves every token."""
 
     graph_safe = True
@@ -109,7 +110,12 @@ class LatentAttention(AttentionPlanning, Mixer):
         mods = [("latent_attention.cu", {"TKB_LAT_RANK": self.kv_rank})]
         if dtype == "bfloat16" and self._rows_fit_tensor_cores():
             mods.append(("attention_mma.cu", {"TKB_HD": self.head_dim}))
+            mods += self._rows_tc()
         return tuple(mods)
+
+    def _rows_tc(self) -> tuple:
+        """The tcgen05 kernel module for portions, where there is one for these sizes (else the mma.sync kernel serves)."""
+        return ops.rows_tc_modules(self.head_dim, self.head_dim, 0, self.kv_rank, False) if self.n_heads <= 128 else ()
 
     def cache_need(self):
         return PagedCacheNeed(1, self.kv_rank + self.rot_dim, self.cache_window, planes=1)
@@ -215,7 +221,10 @@ class LatentAttention(AttentionPlanning, Mixer):
                                 plan["items"], c[0:1], items_cap, plan["dec_seqs"], plan["dec_item_start"], c[1:2],
                                 dec_cap, attn, H, 1, Dk, cache.page_size, self.scale, self.window,
                                 item_entry=plan["item_entry"], tma=bool(counts[5]), status=ctx.status)
-        if tiles_cap:
+        if tiles_cap and self._rows_tc():
+            ops.attn_rows_tc(self._rows_tc()[0], q2, attn, Dk, rows, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, tables.indptr,
+                             tables.page_ids, ctx.n_seqs, H, 1, cache.page_size, self.scale, self.window, ctx.status)
+        elif tiles_cap:
             ops.attn_prefill_mma(q2, attn, rows, rows, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, tables.indptr,
                                  tables.page_ids, plan["tiles"], c[2:3], tiles_cap, H, 1, Dk, cache.page_size, self.scale,
                                  self.window, ctx.status)

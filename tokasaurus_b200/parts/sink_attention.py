@@ -165,7 +165,9 @@ class SinkAttention(Mixer):
         return self.bias_names[:(2 if self.values_are_keys else 3) if self.own_kv else 1]
 
     def kernel_modules(self, dtype):
-        return (("attention_sink.cu", self.defines),)
+        tc = ops.sink_rows_tc_modules(self.dim, self.vdim, self.maps, self.distance_bias is not None,
+                                      self.keep_first if self.window else 0)
+        return (("attention_sink.cu", self.defines),) + (tc if dtype == "bfloat16" else ())
 
     def _conv_columns(self) -> int:
         H, G, M = self.n_heads, self.n_kv_heads, self.maps
