@@ -22,8 +22,10 @@
 //
 // What bounds it: the softmax threads (at 64 + 64: 64 scores a thread and tile, an exponential each and a polynomial for the
 // cap in place of an exponential and a reciprocal, of which the special function unit does four a cycle and scheduler).
-// Measured on B200: 2,048 tokens of 16 heads over latent rows of 192 + 64, window 1,024: 302 us on mma.sync, 67 us here; two
-// prompts of 4,001 tokens, 32 heads of 64 + 64 on 8, window 1,024, capped: 224 us, 111 us here.
+// Measured on B200: 2,048 tokens of 16 heads over latent rows of 192 + 64, window 1,024: 302 us on mma.sync, 51 us here (67 with three stages and the page
+// lookups behind the wait for a stage); two
+// prompts of 4,001 tokens, 32 heads of 64 + 64 on 8, window 1,024, capped: 224 us, 96 us here (111 with the cap's arithmetic
+// one score at a time).
 #include "tcgen05.cuh"
 
 #if !defined(TKB_ROW) || !defined(TKB_KD) || !defined(TKB_V0) || !defined(TKB_VD)
@@ -43,7 +45,7 @@ static_assert(KD <= ROW && V0 + VD <= ROW && ROW <= 256, "key and value lie in t
 constexpr int ATOMS = ROW / 64;          // 64-column (128-byte) blocks of a row
 constexpr int BM = 128;                  // rows of scores a block
 constexpr int BKV = 64;                  // keys a tile
-constexpr int STAGES = 3;
+constexpr int STAGES = ROW > 128 ? 4 : 3;  // (128: two blocks an SM)
 constexpr int THREADS = 384;
 constexpr int ATOM_BYTES = BKV * 128;
 constexpr int TILE_BYTES = ATOMS * ATOM_BYTES;
@@ -56,7 +58,7 @@ constexpr int BLOCKS = TMEM_COLS == 256 && SMEM_BYTES <= 110 * 1024 ? 2 : 1;  //
 constexpr float NEG_BIG = -1.0e30f;
 constexpr float REF_SLACK = 16.f;        // a row's reference moves when a score tops it by more than this (log2)
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr float SMALL_CAP = 0.5f;        // scores up to this share of the cap go through the polynomial
+constexpr float SMALL_CAP = 0.4f;        // scores up to this share of the cap go through the polynomial
 
 struct Args {
   const bf16* q;
@@ -159,17 +161,35 @@ struct ScoreMap {
   float k1, c0;  // plain: d k1 + c0
   float kx, cap; // capped: cap tanh(d kx) + c0, cap in units of log2 (0: plain)
 };
-__device__ __forceinline__ float tanh_small(float x) {  // the odd series; 9e-7 of x off at 0.5
-  const float u = x * x;
-  float p = fmaf(u, -1382.f / 155925.f, 62.f / 2835.f);
-  p = fmaf(u, p, -17.f / 315.f);
-  p = fmaf(u, p, 2.f / 15.f);
-  p = fmaf(u, p, -1.f / 3.f);
-  return fmaf(x * u, p, x);
-}
 __device__ __forceinline__ float tanh_any(float x) { return fmaf(fast_rcp(fast_exp2(x * (2.f * LOG2E)) + 1.f), -2.f, 1.f); }
 __device__ __forceinline__ float score(float d, const ScoreMap& m) {
   return TKB_CAP && m.cap > 0.f ? fmaf(tanh_any(d * m.kx), m.cap, m.c0) : fmaf(d, m.k1, m.c0);
+}
+
+// Two neighbouring scores at a time.
+struct Pair {
+  unsigned long long v;
+};
+__device__ __forceinline__ Pair pair(float a, float b) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+  return p;
+}
+__device__ __forceinline__ void unpair(const Pair& p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+__device__ __forceinline__ Pair operator*(const Pair& a, const Pair& b) {
+  Pair p;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
+  return p;
+}
+__device__ __forceinline__ Pair operator+(const Pair& a, const Pair& b) {
+  Pair p;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
+  return p;
+}
+__device__ __forceinline__ Pair fma2(const Pair& a, const Pair& b, const Pair& c) {
+  Pair p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return p;
 }
 
 // The largest and (TKB_CAP) smallest of one thread's 64 products in tensor memory that its row sees.
@@ -202,8 +222,15 @@ __device__ __forceinline__ void row_range(uint32_t s_addr, int lo, uint32_t span
 // row: bfloat16 into the row's place of the swizzled P tile; returns the row's sum.
 template <int MODE, bool MASKED>
 __device__ __forceinline__ float row_exp(uint32_t s_addr, unsigned char* prow, int r, int lo, uint32_t span, const ScoreMap& m, float ref) {
-  float s0 = 0.f, s1 = 0.f;
+  Pair sum = pair(0.f, 0.f);
   const float c = m.c0 - ref;
+  const Pair k1 = pair(m.k1, m.k1), c2 = pair(c, c);
+  // cap tanh(x) = d k1 (1 + v (a1 + v (a2 + v (a3 + v a4)))) with v = d^2: the odd series with kx^2, ... in its coefficients (x up
+  // to 0.4: 9e-7 of the score off, what rcp and ex2 of the other form leave of a score of the cap's size)
+  const float q = m.kx * m.kx;
+  const Pair a1 = pair(q * (-1.f / 3.f), q * (-1.f / 3.f)), a2 = pair(q * q * (2.f / 15.f), q * q * (2.f / 15.f)),
+             a3 = pair(q * q * q * (-17.f / 315.f), q * q * q * (-17.f / 315.f)),
+             a4 = pair(q * q * q * q * (62.f / 2835.f), q * q * q * q * (62.f / 2835.f)), one = pair(1.f, 1.f);
 #pragma unroll 1
   for (int c0 = 0; c0 < BKV; c0 += 32) {
     uint32_t v[32];
@@ -212,20 +239,21 @@ __device__ __forceinline__ float row_exp(uint32_t s_addr, unsigned char* prow, i
     uint32_t pk[16];
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
-      float p[2];
+      float p[2], y[2];
+      const Pair d = pair(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+      if (MODE == 0) unpair(fma2(d, k1, c2), y[0], y[1]);
+      if (MODE == 1) {
+        const Pair vv = d * d;
+        unpair(fma2(d * k1, fma2(vv, fma2(vv, fma2(vv, fma2(vv, a4, a3), a2), a1), one), c2), y[0], y[1]);
+      }
 #pragma unroll
       for (int u = 0; u < 2; u++) {
-        const float d = __uint_as_float(v[i + u]);
-        float y;
-        if (MODE == 0) y = fmaf(d, m.k1, c);
-        if (MODE == 1) y = fmaf(tanh_small(d * m.kx), m.cap, c);
-        if (MODE == 2) y = fmaf(tanh_any(d * m.kx), m.cap, c);
-        if (MODE == 3) p[u] = fast_rcp(fast_exp2(-score(d, m)) + 1.f);
-        else p[u] = fast_exp2(y);
+        if (MODE == 2) y[u] = fmaf(tanh_any(__uint_as_float(v[i + u]) * m.kx), m.cap, c);
+        if (MODE == 3) p[u] = fast_rcp(fast_exp2(-score(__uint_as_float(v[i + u]), m)) + 1.f);
+        else p[u] = fast_exp2(y[u]);
         if (MASKED && (uint32_t)(c0 + i + u - lo) > span) p[u] = 0.f;
       }
-      s0 += p[0];
-      s1 += p[1];
+      sum = sum + pair(p[0], p[1]);
       pk[i >> 1] = pack_bf16(p[0], p[1]);
     }
     const int cbase = c0 >> 3;  // 32 keys = four 16-byte chunks of this row
@@ -234,6 +262,8 @@ __device__ __forceinline__ float row_exp(uint32_t s_addr, unsigned char* prow, i
       *reinterpret_cast<uint4*>(prow + (((cbase + cc) ^ (r & 7)) << 4)) =
           make_uint4(pk[4 * cc], pk[4 * cc + 1], pk[4 * cc + 2], pk[4 * cc + 3]);
   }
+  float s0, s1;
+  unpair(sum, s0, s1);
   return s0 + s1;
 }
 
@@ -243,7 +273,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
   __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], s_full[2], p_full[2], pv_done[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int failed, where[2];
-  __shared__ float part_ref[2][BM], part_l[2][BM];
   trigger_dependents();
   grid_dependency_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -330,20 +359,25 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
   if (warp == 8) {
     // ---------------- loader
     bool ok = true, bad_page = false;
+    const int boxes = a.tma_rows > 0 ? BKV / a.tma_rows : 1;
     for (int j = 0; j < n_tiles; j++) {
       const int b = j % STAGES;
       const int key_base = k_begin + j * BKV;
-      if (j >= STAGES && !mbar_wait_idle(&empty[b], ((j / STAGES) - 1) & 1)) { ok = false; break; }
-      if (a.tma_rows > 0 && key_base + BKV <= kv_len) {
+      const bool by_tma = a.tma_rows > 0 && key_base + BKV <= kv_len;
+      // the rows of the tile's boxes, looked up before the wait: a lane the box (lane % boxes) of the atoms lane / boxes, ...
+      // (an id beyond the pool becomes -1: a negative row is outside the tensor map and reads as zeros)
+      int row = 0;
+      if (by_tma) {
+        const int key = key_base + (lane % boxes) * a.tma_rows;
+        row = (checked_page(__ldg(table + (key >> ps_shift)), a.num_pages, bad_page) * a.nkv + kvh) * a.ps + (key & (a.ps - 1));
+      }
+      if (j >= STAGES && !mbar_wait(&empty[b], ((j / STAGES) - 1) & 1)) { ok = false; break; }
+      if (by_tma) {
         // every key of the tile exists: per 64-column block one box per page (or per 64 slots of a larger page)
         if (lane == 0) mbar_expect_tx(&full[b], TILE_BYTES);
         __syncwarp();
-        const int boxes = BKV / a.tma_rows;
-        for (int i = lane; i < boxes * ATOMS; i += 32) {
+        for (int i = lane; i < boxes * ATOMS; i += 32) {  // (boxes divides 32: i % boxes is the lane's own)
           const int atom = i / boxes, bx = i - atom * boxes;
-          const int key = key_base + bx * a.tma_rows;
-          // an id beyond the pool becomes -1: a negative row is outside the tensor map and reads as zeros
-          const int row = (checked_page(__ldg(table + (key >> ps_shift)), a.num_pages, bad_page) * a.nkv + kvh) * a.ps + (key & (a.ps - 1));
           tma_load_2d(ring + b * TILE_BYTES + atom * ATOM_BYTES + bx * a.tma_rows * 128, &map, &full[b], atom * 64, row);
         }
       } else {
@@ -474,19 +508,20 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
     }
     if (ok && i > 0) ok = mbar_wait(&pv_done[hh], (i - 1) & 1);
     if (!ok) failed = 1;
-    part_ref[hh][r] = ref;
-    part_l[hh][r] = l;
+    float2* parts = reinterpret_cast<float2*>(sP);  // a half's P tile has been read by its last product
+    parts[hh * (P_BYTES / 8) + r] = make_float2(ref, l);
     tcgen05_fence_before();
     asm volatile("bar.sync 1, 256;" ::: "memory");
     tcgen05_fence_after();
     if (!failed) {
       // the halves together: each takes every other 32 columns of the row
-      const float ra = part_ref[0][r], rb = part_ref[1][r];
+      const float2 pa = parts[r], pb = parts[P_BYTES / 8 + r];
+      const float ra = pa.x, rb = pb.x;
       const bool sink = TKB_CAP && a.sinks != nullptr && live;
       const float rs = sink ? a.sinks[head] * LOG2E : NEG_BIG;
       const float top = fmaxf(fmaxf(ra, rb), rs);
       const float fa = fast_exp2(ra - top), fb = fast_exp2(rb - top);
-      float sum = part_l[0][r] * fa + part_l[1][r] * fb + (sink ? fast_exp2(rs - top) : 0.f);
+      float sum = pa.y * fa + pb.y * fb + (sink ? fast_exp2(rs - top) : 0.f);
       float inv = a.out_scale / (TKB_CAP && a.sigmoid ? 1.f : sum);
       if (TKB_CAP && a.gate != nullptr && live) inv *= 1.f / (1.f + expf(-a.gate[(size_t)(t0 + tok) * a.gate_stride + head]));
       const float wa = fa * inv, wb = fb * inv;

@@ -1840,7 +1840,7 @@ def attn_sink_tc(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, seq_q_
     gate_args = _sink_gate(gate, T, n_heads, maps, "attn_sink_tc")
     # portions on the tcgen05 kernel where it has the form: one map, no bias by distance, no kept first positions, head sizes of
     # whole 64-column blocks, an output that takes 16-byte stores, up to 128 heads a kv head (measured on B200, 4,001 tokens of
-    # 32 heads of 64 + 64, window 1,024, capped: 224 us on mma.sync, 111 us there)
+    # 32 heads of 64 + 64, window 1,024, capped: 224 us on mma.sync, 96 us there)
     module = sink_rows_tc_modules(dim, vdim, maps, head_slope is not None, keep_first if window else 0)
     by_rows = (portions and bool(module) and n_heads // n_kv_heads <= 128 and _row_stride(out) % 8 == 0
                and all(t.data_ptr() % 16 == 0 for t in (q, out, cache)))
