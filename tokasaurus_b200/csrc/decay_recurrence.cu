@@ -125,11 +125,27 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 // SiLU in place on `ncols` columns of float32 rows (the projections of a mixer whose q, k and v pass through it): done
 // once for all tokens, not by every block that walks over them.
-__global__ void silu_cols_kernel(float* __restrict__ x, int stride, int ncols) {
+// VEC: 16-byte pieces, four of a thread's in flight together (2,048 rows of 6,144 columns: 24 us value by value, 17 so).
+template <bool VEC>
+__global__ void __launch_bounds__(512) silu_cols_kernel(float* __restrict__ x, int stride, int ncols) {
   trigger_dependents();
   grid_dependency_wait();
   float* row = x + (size_t)blockIdx.x * stride;
-  for (int c = threadIdx.x; c < ncols; c += blockDim.x) row[c] = silu_f(row[c]);
+  if (VEC) {
+    float4* p = reinterpret_cast<float4*>(row);
+    const int n = ncols >> 2;
+    for (int c0 = threadIdx.x; c0 < n; c0 += 4 * blockDim.x) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (c0 + i * blockDim.x < n) v[i] = p[c0 + i * blockDim.x];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (c0 + i * blockDim.x < n) p[c0 + i * blockDim.x] = make_float4(silu_f(v[i].x), silu_f(v[i].y), silu_f(v[i].z), silu_f(v[i].w));
+    }
+  } else {
+    for (int c = threadIdx.x; c < ncols; c += blockDim.x) row[c] = silu_f(row[c]);
+  }
 }
 
 // Shared memory of the walk, per buffer: q and k rows of QROW floats as they lie in memory (lane L reads the 16-byte
@@ -423,7 +439,9 @@ TKB_EXPORT int tkb_silu_cols(float* x, int stride, int ncols, int rows, void* st
   if (rows <= 0 || ncols <= 0) return 0;
   int threads = 32;
   while (threads < ncols / 4 && threads < 512) threads <<= 1;
-  return launch_pdl(silu_cols_kernel, dim3(rows), dim3(threads), 0, (cudaStream_t)st, x, stride, ncols);
+  const bool vec = ncols % 4 == 0 && stride % 4 == 0 && ((uintptr_t)x & 15) == 0;
+  return launch_pdl(vec ? silu_cols_kernel<true> : silu_cols_kernel<false>, dim3(rows), dim3(threads), 0, (cudaStream_t)st, x, stride,
+                    ncols);
 }
 
 namespace {
