@@ -22,10 +22,9 @@
 //
 // What bounds it: the softmax threads (at 64 + 64: 64 scores a thread and tile, an exponential each and a polynomial for the
 // cap in place of an exponential and a reciprocal, of which the special function unit does four a cycle and scheduler).
-// Measured on B200: 2,048 tokens of 16 heads over latent rows of 192 + 64, window 1,024: 302 us on mma.sync, 51 us here (67 with three stages and the page
-// lookups behind the wait for a stage); two
-// prompts of 4,001 tokens, 32 heads of 64 + 64 on 8, window 1,024, capped: 224 us, 96 us here (111 with the cap's arithmetic
-// one score at a time).
+// Measured on B200: 2,048 tokens of 16 heads over latent rows of 192 + 64, window 1,024: 302 us on mma.sync, 51 us here (67
+// with three stages and the page lookups behind the wait for a stage); two prompts of 4,001 tokens, 32 heads of 64 + 64 on 8,
+// window 1,024, capped: 224 us, 96 us here (111 with the cap's arithmetic one score at a time).
 #include "tcgen05.cuh"
 
 #if !defined(TKB_ROW) || !defined(TKB_KD) || !defined(TKB_V0) || !defined(TKB_VD)
