@@ -108,6 +108,15 @@ __device__ __forceinline__ void put1(unsigned char* p, int plane, float x) {
   *reinterpret_cast<__nv_bfloat16*>(p + plane) = m;
   *reinterpret_cast<__nv_bfloat16*>(p + 2 * plane) = __float2bfloat16_rn(r - __bfloat162float(m));
 }
+// Two neighbouring numbers.
+__device__ __forceinline__ void put2(unsigned char* p, int plane, float x, float y) {
+  uint32_t h, m, l;
+  cut2(x, y, h, m, l);
+  *reinterpret_cast<uint32_t*>(p) = h;
+  *reinterpret_cast<uint32_t*>(p + plane) = m;
+  *reinterpret_cast<uint32_t*>(p + 2 * plane) = l;
+}
+__device__ __forceinline__ float2 operator*(const float2& a, const float2& b) { return make_float2(a.x * b.x, a.y * b.y); }
 template <bool TRANS> __device__ __forceinline__ void ldmat(uint32_t (&r)[4], uint32_t addr) {
   if (TRANS)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -213,7 +222,11 @@ template <int ROWS, int COLS> struct Pieces {
 };
 
 // One decay a token: sums of log |a| up to and with token t, and how many of them are negative (two warps).
-__device__ __forceinline__ void log_sums(const Args& p, int head, int row0, int nt, double* logs, int* negs, float* scale) {
+// The sums leave as two floats each: differences of these are as exact as those of the 64-bit sums to within a rounding of
+// the difference itself, at a fraction of the cost (64-bit arithmetic for A's 4,096 factors took 4,000 cycles a block).
+__device__ __forceinline__ void log_sums(const Args& p, int head, int row0, int nt, float2* logs, int* negs, float* scale) {
+  __shared__ double first_half;
+  __shared__ int first_negs;
   const int t = threadIdx.x;
   double x = 0.0;
   int neg = 0;
@@ -236,17 +249,21 @@ __device__ __forceinline__ void log_sums(const Args& p, int head, int row0, int 
       const int m = __shfl_up_sync(0xffffffffu, neg, o);
       if ((t & 31) >= o) x += y, neg += m;
     }
-    logs[t] = x;
+    if (t == 31) first_half = x, first_negs = neg;
+  }
+  __syncthreads();
+  if (t < C) {
+    if (t >= 32) x += first_half, neg += first_negs;
+    const float hi = (float)x;
+    logs[t] = make_float2(hi, (float)(x - (double)hi));
     negs[t] = neg;
   }
   __syncthreads();
-  if (t >= 32 && t < C) logs[t] = x + logs[31], negs[t] = neg + negs[31];
-  __syncthreads();
 }
 // The product of the decays of tokens s + 1 .. t (s = -1: from the chunk's start).
-__device__ __forceinline__ float decay_between(const double* logs, const int* negs, int s, int t) {
-  const double from = s < 0 ? 0.0 : logs[s];
-  const float f = expf((float)(logs[t] - from));
+__device__ __forceinline__ float decay_between(const float2* logs, const int* negs, int s, int t) {
+  const float2 from = s < 0 ? make_float2(0.f, 0.f) : logs[s], to = logs[t];
+  const float f = expf((to.x - from.x) + (to.y - from.y));
   return (negs[t] - (s < 0 ? 0 : negs[s])) & 1 ? -f : f;
 }
 
@@ -257,8 +274,8 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
   constexpr int V_PITCH = (VDIM + 8) * 2, V_PLANE = C * V_PITCH;
   unsigned char* kp = smem;              // k's planes
   unsigned char* vp = kp + 3 * PLANE;    // v's
-  __shared__ double logs[C];
-  __shared__ float scale[C], blocks[4][DIM];
+  __shared__ float2 logs[C];
+  __shared__ float scale[C], eighths[8][DIM];
   __shared__ int negs[C], where[2];
   trigger_dependents();
   grid_dependency_wait();
@@ -276,29 +293,30 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
   Pieces<C, VDIM> v;
   v.fetch(p.v + (size_t)row0 * p.v_stride + (size_t)head * VDIM, p.v_stride, nt);
   if (VEC) {
-    // a thread one channel of 16 tokens: k decayed to the chunk's end
-    const int d = tid & (DIM - 1), blk = tid >> 7;
-    const float* kc = p.k + (size_t)(row0 + blk * 16) * p.k_stride + head * DIM + d;
-    const float* fc = p.fvec + (size_t)(row0 + blk * 16) * p.f_stride + head * DIM + d;
-    float k[16], f[16], run = 1.f;
+    // a thread two channels of 8 tokens: k decayed to the chunk's end
+    const int d = (tid & 63) * 2, part = tid >> 6;
+    const float* kc = p.k + (size_t)(row0 + part * 8) * p.k_stride + head * DIM + d;
+    const float* fc = p.fvec + (size_t)(row0 + part * 8) * p.f_stride + head * DIM + d;
+    float2 k[8], f[8], run = make_float2(1.f, 1.f);
 #pragma unroll
-    for (int s = 0; s < 16; s++) {
-      const bool there = blk * 16 + s < nt;
-      k[s] = there ? kc[(size_t)s * p.k_stride] : 0.f;
-      f[s] = there ? fc[(size_t)s * p.f_stride] : 1.f;
+    for (int s = 0; s < 8; s++) {
+      const bool there = part * 8 + s < nt;
+      k[s] = there ? *reinterpret_cast<const float2*>(kc + (size_t)s * p.k_stride) : make_float2(0.f, 0.f);
+      f[s] = there ? *reinterpret_cast<const float2*>(fc + (size_t)s * p.f_stride) : make_float2(1.f, 1.f);
     }
 #pragma unroll
-    for (int s = 0; s < 16; s++) run *= f[s];
-    blocks[blk][d] = run;
+    for (int s = 0; s < 8; s++) run = run * f[s];
+    *reinterpret_cast<float2*>(&eighths[part][d]) = run;
     __syncthreads();
-    run = 1.f;
-    for (int b = 3; b > blk; b--) run *= blocks[b][d];
+    run = make_float2(1.f, 1.f);
+    for (int b = 7; b > part; b--) run = run * *reinterpret_cast<const float2*>(&eighths[b][d]);
 #pragma unroll
-    for (int s = 15; s >= 0; s--) {
-      put1(kp + (blk * 16 + s) * PITCH + 2 * d, PLANE, k[s] * run);
-      run *= f[s];
+    for (int s = 7; s >= 0; s--) {
+      const float2 x = k[s] * run;
+      put2(kp + (part * 8 + s) * PITCH + 2 * d, PLANE, x.x, x.y);
+      run = run * f[s];
     }
-    if (blk == 0) p.gains[at * DIM + d] = run;
+    if (part == 0) *reinterpret_cast<float2*>(p.gains + at * DIM + d) = run;
   } else {
     Pieces<C, DIM> k;
     k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
@@ -400,8 +418,8 @@ template <int VDIM, bool VEC>
 __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int V_PITCH = (VDIM + 8) * 2, V_PLANE = C * V_PITCH;
-  __shared__ double logs[C];
-  __shared__ float scale[C], blocks[4][DIM];
+  __shared__ float2 logs[C];
+  __shared__ float scale[C], eighths[8][DIM];
   __shared__ int negs[C], where[2];
   trigger_dependents();
   grid_dependency_wait();
@@ -420,17 +438,10 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
   const uint32_t q_at = smem_addr(smem), k_at = q_at + OFF_K, p_at = q_at + OFF_P;
   unsigned char* pp = smem + OFF_P;
   Pieces<VDIM, DIM> state;
-  // put two neighbouring elements of A
-  auto put_p = [&](int t, int s, float x, float y) {
-    uint32_t h, m, l;
-    cut2(x, y, h, m, l);
-    unsigned char* o = pp + t * P_PITCH + 2 * s;
-    *reinterpret_cast<uint32_t*>(o) = h;
-    *reinterpret_cast<uint32_t*>(o + P_PLANE) = m;
-    *reinterpret_cast<uint32_t*>(o + 2 * P_PLANE) = l;
-  };
-  float qd[16];  // VEC: a channel of 16 of q's rows, decayed from their block's start
-  const int d = tid & (DIM - 1), blk = tid >> 7;
+  auto put_p = [&](int t, int s, float x, float y) { put2(pp + t * P_PITCH + 2 * s, P_PLANE, x, y); };  // two elements of A
+  float2 qd[8];  // VEC: two channels of 8 of q's rows, decayed from their block of 16's start
+  const int d = (tid & 63) * 2, part = tid >> 6, blk = part >> 1;
+  auto eighth = [&](int i) { return *reinterpret_cast<const float2*>(&eighths[i][d]); };
   {
     Pieces<C, DIM> q, k;
     q.fetch(p.q + (size_t)row0 * p.q_stride + (head / p.qk_div) * DIM, p.q_stride, nt);
@@ -471,30 +482,37 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
         }
         for (int s = wm * 16 + in + 1 + lane; s < wm * 16 + 16; s += 32) put1(pp + t * P_PITCH + 2 * s, P_PLANE, 0.f);
       }
-      // a thread one channel of 16 tokens: q decayed from its block's start, k to its block's end, the block's product
-      float kd[16], ff[16], run = 1.f;
+      // a thread two channels of 8 tokens: q decayed from its block of 16's start, k to its block's end
+      float2 kd[8], ff[8], run = make_float2(1.f, 1.f);
 #pragma unroll
-      for (int t = 0; t < 16; t++) {
-        const int row = blk * 16 + t;
-        ff[t] = row < nt ? fs[row * LDR + d] : 1.f;
-        run *= ff[t];
-        qd[t] = qs[row * LDR + d] * run;
+      for (int t = 0; t < 8; t++) {
+        const int row = part * 8 + t;
+        ff[t] = row < nt ? *reinterpret_cast<const float2*>(fs + row * LDR + d) : make_float2(1.f, 1.f);
+        run = run * ff[t];
+        qd[t] = *reinterpret_cast<const float2*>(qs + row * LDR + d) * run;
       }
-      blocks[blk][d] = run;
-      run = 1.f;
+      *reinterpret_cast<float2*>(&eighths[part][d]) = run;
+      run = make_float2(1.f, 1.f);
 #pragma unroll
-      for (int t = 15; t >= 0; t--) {
-        kd[t] = ks[(blk * 16 + t) * LDR + d] * run;
-        run *= ff[t];
+      for (int t = 7; t >= 0; t--) {
+        kd[t] = *reinterpret_cast<const float2*>(ks + (part * 8 + t) * LDR + d) * run;
+        run = run * ff[t];
       }
       __syncthreads();  // the float32 rows have been read
-      const float one = blk >= 2 ? blocks[blk - 1][d] : 0.f, two = blk == 3 ? one * blocks[1][d] : 0.f;
+      const float2 before = part & 1 ? eighth(part - 1) : make_float2(1.f, 1.f);  // the rest of the block on either side
+      const float2 behind = part & 1 ? make_float2(1.f, 1.f) : eighth(part + 1);
+      const float2 none = make_float2(0.f, 0.f);
+      const float2 one = blk >= 2 ? eighth(2 * blk - 2) * eighth(2 * blk - 1) : none;  // the block ahead, the two ahead
+      const float2 two = blk == 3 ? one * (eighth(2) * eighth(3)) : none;
 #pragma unroll
-      for (int t = 0; t < 16; t++) {
-        put1(smem + (blk * 16 + t) * PITCH + 2 * d, PLANE, qd[t]);
-        put1(smem + OFF_K + (blk * 16 + t) * PITCH + 2 * d, PLANE, kd[t]);
-        if (blk >= 2) put1(smem + OFF_FAR + ((blk - 2) * 16 + t) * PITCH + 2 * d, FAR_PLANE, qd[t] * one);
-        if (blk == 3) put1(smem + OFF_FAR + (32 + t) * PITCH + 2 * d, FAR_PLANE, qd[t] * two);
+      for (int t = 0; t < 8; t++) {
+        const int at16 = (part & 1) * 8 + t, row = part * 8 + t;
+        qd[t] = qd[t] * before;
+        put2(smem + row * PITCH + 2 * d, PLANE, qd[t].x, qd[t].y);
+        const float2 kk = kd[t] * behind;
+        put2(smem + OFF_K + row * PITCH + 2 * d, PLANE, kk.x, kk.y);
+        if (blk >= 2) put2(smem + OFF_FAR + ((blk - 2) * 16 + at16) * PITCH + 2 * d, FAR_PLANE, qd[t].x * one.x, qd[t].y * one.y);
+        if (blk == 3) put2(smem + OFF_FAR + (32 + at16) * PITCH + 2 * d, FAR_PLANE, qd[t].x * two.x, qd[t].y * two.y);
       }
     } else {
       log_sums(p, head, row0, nt, logs, negs, scale);
@@ -529,10 +547,10 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
   __syncthreads();  // k's planes have been read
   state.put(smem + OFF_K, PITCH, DIM * PITCH);
   if (VEC && blk > 0) {  // q decayed from the chunk's start
-    float run = 1.f;
-    for (int c = 0; c < blk; c++) run *= blocks[c][d];
+    float2 run = make_float2(1.f, 1.f);
+    for (int c = 0; c < 2 * blk; c++) run = run * eighth(c);
 #pragma unroll
-    for (int t = 0; t < 16; t++) put1(smem + (blk * 16 + t) * PITCH + 2 * d, PLANE, qd[t] * run);
+    for (int t = 0; t < 8; t++) put2(smem + (part * 8 + t) * PITCH + 2 * d, PLANE, qd[t].x * run.x, qd[t].y * run.y);
   }
   Pieces<C, VDIM> v;
   v.fetch(p.v + (size_t)row0 * p.v_stride + (size_t)head * VDIM, p.v_stride, nt);
