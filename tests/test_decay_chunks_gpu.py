@@ -110,3 +110,44 @@ def test_chunks_cut_into_steps():
         outs.append(out)
         at += n
     assert float((torch.cat(outs).double() - ref[0][0]).norm() / ref[0][0].norm()) < 16 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vdim,heads,lens", [(128, 2, [192, 1, 259]), (64, 3, [700, 191]), (128, 160, [200, 193])])
+def test_chunks_of_the_forgetting_recurrence(dtype, vdim, heads, lens, monkeypatch):
+    """S_t = diag(f) S + (1 - f) v^T with its gates and norm: chunks against the walk and float64; many heads too, for which the
+    walk alone would not have split its gates from its sums."""
+    from tokasaurus_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(heads)
+    T, d = sum(lens), 128
+    qfv = torch.randn(T, heads * (2 * d + vdim), generator=g)
+    fb, low = torch.randn(heads * d, generator=g), torch.rand(heads * d, generator=g) * 0.95
+    nw = torch.rand(vdim, generator=g) + 0.5
+    state = torch.randn(len(lens) + 1, heads, vdim, d, generator=g)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+
+    def run():
+        st, out = state.to(DEV), torch.empty(T, heads * vdim, dtype=dtype, device=DEV)
+        ops.gated_recurrence(qfv.to(DEV), st, fb.to(DEV), low.to(DEV), nw.to(DEV), out, i32(list(range(len(lens)))), i32(starts), i32(lens),
+                             len(lens), heads, d, vdim, 1e-5)
+        return out.double().cpu(), st.double().cpu()
+
+    out, st = run()
+    monkeypatch.setattr(ops, "DECAY_CHUNKS_FROM", 1 << 30)
+    walked, wst = run()
+    x = qfv.double().to(DEV)
+    q = x[:, :heads * d] * torch.sigmoid(x[:, :heads * d])
+    f = low.double().to(DEV) + (1 - low.double().to(DEV)) * torch.sigmoid(x[:, heads * d:2 * heads * d] + fb.double().to(DEV))
+    q, f, v = q.view(T, heads, d), f.view(T, heads, d), x[:, 2 * heads * d:].reshape(T, heads, vdim)
+    for i, n in enumerate(lens):
+        r = slice(starts[i], starts[i] + n)
+        o, S = plain(q[r], 1 - f[r], v[r], f[r], torch.ones(n, heads, dtype=torch.float64, device=DEV),
+                     torch.zeros(heads, dtype=torch.float64, device=DEV), state[i].double().to(DEV).transpose(1, 2))
+        o = (o * torch.rsqrt(o.pow(2).mean(-1, keepdim=True) + 1e-5) * nw.double().to(DEV)).reshape(n, -1).cpu()
+        S = S.transpose(1, 2).cpu()
+        rel = lambda a, b: float((a - b).norm() / b.norm())  # noqa: E731
+        bound = 16 * 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -8
+        assert rel(out[r], o) < bound and rel(st[i], S) < 16 * 2.0 ** -24
+        assert rel(out[r], o) < 1.5 * rel(walked[r], o) + 2.0 ** -24 and rel(st[i], S) < 1.5 * rel(wst[i], S) + 2.0 ** -24
+    assert torch.equal(st[-1].float(), state[-1])

@@ -2,7 +2,7 @@
 //
 //     S_t = diag(a_t) S_(t-1) + (c_t k_t) v_t^T,        o_t = S_t^T q_t + D v_t
 //
-// (a_t one number a head and token, a constant a head, or a number for every key channel).  The walk over the tokens there is
+// (a_t one number a head and token, a constant a head, or a number for every key channel; k may be 1 - a).  The walk over the tokens there is
 // a chain of one step a token; here what tokens of one chunk do to one another is products of matrices, and only the state
 // goes from chunk to chunk:
 //   chunk_states   a block a (chunk, head): what the chunk adds to the state, U = sum_s (decay from s to the chunk's end) c_s k_s v_s^T;
@@ -195,6 +195,17 @@ template <int ROWS, int COLS> struct Pieces {
       }
     }
   }
+  __device__ __forceinline__ void one_minus(const Pieces& f, int nt) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const bool there = (threadIdx.x + i * THREADS) / (COLS / 8) < nt;
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const float4 a = f.x[i][u];
+        x[i][u] = there ? make_float4(1.f - a.x, 1.f - a.y, 1.f - a.z, 1.f - a.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
   __device__ __forceinline__ void scale(const float* by) {  // a factor a row
 #pragma unroll
     for (int i = 0; i < N; i++) {
@@ -301,8 +312,9 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
 #pragma unroll
     for (int s = 0; s < 8; s++) {
       const bool there = part * 8 + s < nt;
-      k[s] = there ? *reinterpret_cast<const float2*>(kc + (size_t)s * p.k_stride) : make_float2(0.f, 0.f);
       f[s] = there ? *reinterpret_cast<const float2*>(fc + (size_t)s * p.f_stride) : make_float2(1.f, 1.f);
+      if (p.k != nullptr) k[s] = there ? *reinterpret_cast<const float2*>(kc + (size_t)s * p.k_stride) : make_float2(0.f, 0.f);
+      else k[s] = make_float2(1.f - f[s].x, 1.f - f[s].y);  // (0 where no token is)
     }
 #pragma unroll
     for (int s = 0; s < 8; s++) run = run * f[s];
@@ -445,13 +457,14 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
   {
     Pieces<C, DIM> q, k;
     q.fetch(p.q + (size_t)row0 * p.q_stride + (head / p.qk_div) * DIM, p.q_stride, nt);
-    k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
+    if (!VEC || p.k != nullptr) k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
     if (VEC) {
       float* qs = reinterpret_cast<float*>(smem);
       float* ks = qs + C * LDR;
       float* fs = ks + C * LDR;
       Pieces<C, DIM> f;
       f.fetch(p.fvec + (size_t)row0 * p.f_stride + head * DIM, p.f_stride, nt);
+      if (p.k == nullptr) k.one_minus(f, nt);
       q.put_floats(qs, LDR);
       k.put_floats(ks, LDR);
       f.put_floats(fs, LDR);
@@ -616,7 +629,8 @@ int chunks_launch(const Args& p, int max_chunks, cudaStream_t st) {
 
 }  // namespace
 
-// For the requests that bring at least `least` tokens (the others are left alone).  Arguments as in tkb_decay_walk; dim is
+// For the requests that bring at least `least` tokens (the others are left alone).  Arguments as in tkb_decay_walk; k null (only
+// with fvec): k = 1 - f, what a gate that forgets leaves room for (recurrence.cu); dim is
 // 128, vdim 64 or 128; q, k, v, fvec rows and their strides, state and slot_stride in whole 16-byte pieces.  states:
 // float32 [max_chunks][heads][vdim][128], gains: float32 [max_chunks][heads] (fvec: [max_chunks][heads][128]) are scratch;
 // max_chunks: at least the requests' tokens in chunks of 64, each request rounded up.
@@ -632,6 +646,7 @@ TKB_EXPORT int tkb_decay_chunks(const float* q, int q_stride, const float* k, in
       (fvec && !al(fvec)) || !al(state) || !al(states) || !al(gains))
     return -2;
   if (fvec != nullptr && (dt_dec != nullptr || decay_head != nullptr || qk_div != 1)) return -2;
+  if (k == nullptr && fvec == nullptr) return -2;
   const Args p = {q, k, v, fvec, dt_dec, decay_head, skip, state, out, states, gains, seq_slot, seq_q_start, seq_q_len,
                   slot_stride, q_stride, k_stride, v_stride, f_stride, qk_div, n_seqs, heads, least, write_state};
   cudaStream_t st = (cudaStream_t)st_;

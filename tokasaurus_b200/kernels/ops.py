@@ -874,9 +874,23 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
     _need(out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "gated_recurrence: out [T, heads * vdim]")
     f = _fn(_libs.get("recurrence.cu", **recurrence_defines(dim, vdim)), f"tkb_gated_recurrence_{_suffix(out.dtype)}")
     raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=qfv.device) if (split_heads and T > n_seqs) else None
-    _check(f(_ptr(qfv), c_int(qfv.stride(0)), _ptr(state), _ptr(f_bias), _ptr(low), _ptr(norm_w), _ptr(out),
-             _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(T), c_int(heads), c_int(dim),
-             c_int(vdim), c_float(eps), c_int(1 if write_state else 0), _ptr(raw), _stream()), "gated_recurrence")
+    # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the gates and the norm
+    by_chunks = (raw is not None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and bool(decay_chunk_modules(dim, vdim))
+                 and qfv.stride(0) % 4 == 0 and qfv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0)
+
+    def run(phase: int, below: int) -> None:
+        _check(f(_ptr(qfv), c_int(qfv.stride(0)), _ptr(state), _ptr(f_bias), _ptr(low), _ptr(norm_w), _ptr(out),
+                 _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(T), c_int(heads), c_int(dim),
+                 c_int(vdim), c_float(eps), c_int(1 if write_state else 0), _ptr(raw), c_int(below), c_int(phase), _stream()),
+               "gated_recurrence")
+
+    if not by_chunks:
+        return run(0, 0)
+    run(1, DECAY_CHUNKS_FROM)
+    decay = qfv[:, heads * dim:2 * heads * dim]
+    _decay_chunks(qfv[:, :heads * dim], None, qfv[:, 2 * heads * dim:], 1, None, None, decay, None, state.view(state.shape[0], -1), raw,
+                  seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state)
+    run(2, 0)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -1417,6 +1431,22 @@ def ssm_prep(proj: torch.Tensor, xbc_off: int, channels: int, conv_w: torch.Tens
         _ptr(dt_bias), _ptr(a_log), _ptr(dt_dec), c_int(1 if write_state else 0), _stream()), "ssm_prep")
 
 
+def _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
+                  heads, dim, vdim, write_state) -> None:
+    """The recurrence of ``decay_walk`` for the requests that bring at least ``DECAY_CHUNKS_FROM`` tokens, in chunks (the caller
+    has checked the operands).  ``k`` None: 1 - decay_vec."""
+    T = q.shape[0]
+    chunks = T // DECAY_CHUNK + min(n_seqs, T // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
+    states = torch.empty((chunks, heads, vdim, dim), dtype=torch.float32, device=q.device)
+    gains = torch.empty((chunks, heads, dim if decay_vec is not None else 1), dtype=torch.float32, device=q.device)
+    stride = lambda t: c_int(t.stride(0) if t is not None else 0)  # noqa: E731
+    _check(_fn(_libs.get("decay_chunks.cu"), "tkb_decay_chunks")(
+        _ptr(q), stride(q), _ptr(k), stride(k), c_int(heads_per_qk), _ptr(decay_vec), stride(decay_vec), _ptr(v), stride(v),
+        _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
+        _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
+        c_int(1 if write_state else 0), c_int(DECAY_CHUNKS_FROM), _ptr(states), _ptr(gains), c_int(chunks), _stream()), "decay_chunks")
+
+
 def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: int, dt_dec: torch.Tensor | None,
                decay_head: torch.Tensor | None, skip: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor,
                seq_slot: torch.Tensor, seq_q_start: torch.Tensor, seq_q_len: torch.Tensor, n_seqs: int, heads: int,
@@ -1457,15 +1487,8 @@ def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: 
         # requests that bring many tokens; the walk below then leaves them alone.  Which requests these are is read on the
         # device: a step graph is replayed for other lengths.
         below = DECAY_CHUNKS_FROM
-        chunks = T // DECAY_CHUNK + min(n_seqs, T // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
-        states = torch.empty((chunks, heads, vdim, dim), dtype=torch.float32, device=q.device)
-        gains = torch.empty((chunks, heads, dim if decay_vec is not None else 1), dtype=torch.float32, device=q.device)
-        _check(_fn(_libs.get("decay_chunks.cu"), "tkb_decay_chunks")(
-            _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),
-            c_int(decay_vec.stride(0) if decay_vec is not None else 0), _ptr(v), c_int(v.stride(0)),
-            _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
-            _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
-            c_int(1 if write_state else 0), c_int(below), _ptr(states), _ptr(gains), c_int(chunks), _stream()), "decay_chunks")
+        _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
+                      heads, dim, vdim, write_state)
     defines = _walk_defines(dim, vdim, n_seqs * heads * vall, T == n_seqs, q.device)
     _check(_fn(_libs.get("decay_recurrence.cu", **defines), "tkb_decay_walk")(
         _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),

@@ -39,7 +39,7 @@ class GatedLinearRecurrence(Mixer):
         )
 
     def kernel_modules(self, dtype):
-        return (("recurrence.cu", ops.recurrence_defines(self.dim, self.vdim)),)
+        return (("recurrence.cu", ops.recurrence_defines(self.dim, self.vdim)),) + ops.decay_chunk_modules(self.dim, self.vdim)
 
     def cache_need(self):
         return StateNeed((self.n_heads, self.vdim, self.dim), "float32")  # S transposed: [head][value][key channel]
