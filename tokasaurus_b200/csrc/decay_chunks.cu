@@ -24,8 +24,8 @@
 // way through the L2 (64 KB a chunk and head, four times).  Operands are cut once a block and not once a warp that reads
 // them (cut from the fragments into tf32 halves, the kernels took 132 us where they take 108 now).  Chunks of 64: half the
 // states' traffic of 32, and the products inside a chunk are still a third of the work.
-// Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 147 us (358);
-// three requests of 3,001 tokens in all 158 (382) and 213 us (511); 64 heads of 128 x 64 on 8 groups 250 us (455).
+// Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 137 us (358);
+// three requests of 3,001 tokens in all 159 (383) and 200 us (513); 64 heads of 128 x 64 on 8 groups 242 us (455).
 #include "common.cuh"
 
 using namespace tkb;

@@ -316,23 +316,27 @@ __global__ void moe_order_kernel(const int* __restrict__ top_idx, int n_pairs, i
 }
 
 // dst[p] = src[src_token[p]] (zeros where src_token[p] < 0): the step's rows in the order of the experts' spans; and, if
-// asked, place_scale[p] = pair_scale[order[p]] (0 at the padding, where order holds nothing).
-template <typename T>
+// asked, place_scale[p] = pair_scale[order[p]] (0 at the padding, where order holds nothing).  Of every `tile` places only the
+// first tile_rows are made (a step of few tokens never fills more of a tile: 16 tokens on 16 tiles of 128 took 13 us, most of
+// it for zeros).  VEC: rows in 16-byte pieces.
+template <typename T, bool VEC>
 __global__ void moe_gather_kernel(const T* __restrict__ src, const int* __restrict__ src_token, T* __restrict__ dst,
                                   int H, const int* __restrict__ order, const float* __restrict__ pair_scale,
-                                  float* __restrict__ place_scale) {
+                                  float* __restrict__ place_scale, int tile, int tile_rows) {
   trigger_dependents();
   grid_dependency_wait();
-  const int p = blockIdx.x;
+  const int p = blockIdx.x / tile_rows * tile + blockIdx.x % tile_rows;
   const int t = src_token[p];
   if (place_scale != nullptr && threadIdx.x == 0) place_scale[p] = t >= 0 ? pair_scale[order[p]] : 0.f;
   T* d = dst + (size_t)p * H;
-  if (t < 0) {
-    for (int i = threadIdx.x; i < H; i += blockDim.x) d[i] = from_float<T>(0.f);
-    return;
+  const T* r = src + (size_t)max(t, 0) * H;
+  if (VEC) {
+    const int n = H * (int)sizeof(T) / 16;
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      reinterpret_cast<uint4*>(d)[i] = t >= 0 ? reinterpret_cast<const uint4*>(r)[i] : make_uint4(0u, 0u, 0u, 0u);
+  } else {
+    for (int i = threadIdx.x; i < H; i += blockDim.x) d[i] = t >= 0 ? r[i] : from_float<T>(0.f);
   }
-  const T* r = src + (size_t)t * H;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) d[i] = r[i];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -794,11 +798,15 @@ TKB_EXPORT int tkb_moe_order(const int* top_idx, int n_pairs, int E, int top, in
                                     H, top, shared_gate, (cudaStream_t)st);                                            \
   }                                                                                                                    \
   TKB_EXPORT int tkb_moe_gather_##SUF(const void* src, const int* src_token, void* dst, int n_places, int H,           \
-                                      const int* order, const float* pair_scale, float* place_scale, void* st) {       \
+                                      const int* order, const float* pair_scale, float* place_scale, int tile,         \
+                                      int tile_rows, void* st) {                                                       \
     if (n_places <= 0) return 0;                                                                                       \
     if (place_scale != nullptr && (order == nullptr || pair_scale == nullptr)) return -2;                              \
-    return launch_pdl(moe_gather_kernel<T>, dim3(n_places), dim3(H >= 1024 ? 256 : 128), 0, (cudaStream_t)st,          \
-                      (const T*)src, src_token, (T*)dst, H, order, pair_scale, place_scale);                           \
+    if (tile <= 0 || tile_rows <= 0 || tile_rows > tile || n_places % tile) return -2;                                 \
+    const bool vec = (H * sizeof(T)) % 16 == 0 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0;                       \
+    return launch_pdl(vec ? moe_gather_kernel<T, true> : moe_gather_kernel<T, false>,                                  \
+                      dim3(n_places / tile * tile_rows), dim3(H >= 1024 ? 256 : 128), 0, (cudaStream_t)st,             \
+                      (const T*)src, src_token, (T*)dst, H, order, pair_scale, place_scale, tile, tile_rows);          \
   }
 
 TKB_MOE_EXPORTS(f32, float)

@@ -5,7 +5,7 @@ from __future__ import annotations
 
 # every precision: embedding, norms, rotary + cache write, activation, row gather; sampling
 SHARED = [("elementwise.cu", None), ("sampling.cu", None)]
-# float32: the FP32-FMA product; attention on the FP32 pipes (per head size, below)
+# float32: the true 32-bit product; attention on the FP32 pipes (per head size, below)
 FLOAT32 = [("sgemm.cu", None)]
 # bfloat16: small-batch products (mma.sync and tcgen05), the tcgen05 product for many rows
 BFLOAT16 = [("linear_smallm.cu", None), ("gemm_tcgen05.cu", None), ("gemm_tcgen05_decode.cu", None)]

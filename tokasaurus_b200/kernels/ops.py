@@ -1105,9 +1105,10 @@ def moe_order(top_idx: torch.Tensor, n_experts: int, offsets: torch.Tensor, orde
 
 
 def moe_gather(src: torch.Tensor, src_token: torch.Tensor, out: torch.Tensor, order: torch.Tensor | None = None,
-               pair_scale: torch.Tensor | None = None, place_scale: torch.Tensor | None = None) -> None:
+               pair_scale: torch.Tensor | None = None, place_scale: torch.Tensor | None = None, tile: int = 1,
+               tile_rows: int = 1) -> None:
     """out[p] = src[src_token[p]], zeros where src_token[p] < 0.  ``place_scale`` float32 [places]: receives
-    pair_scale[order[p]] (0 at the padding)."""
+    pair_scale[order[p]] (0 at the padding).  Of every ``tile`` places only the first ``tile_rows`` are made."""
     _need_cuda(src, src_token, out, order, pair_scale, place_scale)
     _need(place_scale is None or (order is not None and pair_scale is not None and pair_scale.dtype == torch.float32
                                   and place_scale.dtype == torch.float32 and place_scale.numel() == out.shape[0]
@@ -1116,18 +1117,19 @@ def moe_gather(src: torch.Tensor, src_token: torch.Tensor, out: torch.Tensor, or
           and src_token.dtype == torch.int32 and src_token.numel() == out.shape[0], "moe_gather: shapes")
     f = _fn(_libs.get("moe.cu"), f"tkb_moe_gather_{_suffix(src.dtype)}")
     _check(f(_ptr(src), _ptr(src_token), _ptr(out), c_int(out.shape[0]), c_int(src.shape[1]), _ptr(order), _ptr(pair_scale),
-             _ptr(place_scale), _stream()), "moe_gather")
+             _ptr(place_scale), c_int(tile), c_int(tile_rows), _stream()), "moe_gather")
 
 
 def gemm_tcgen05_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, status: torch.Tensor,
                          gated: bool = False, act: str | None = None, clamp: tuple[float, float] | None = None,
-                         row_scale: torch.Tensor | None = None) -> torch.Tensor:
+                         row_scale: torch.Tensor | None = None, tile_rows: int = 128) -> torch.Tensor:
     """Row tile i (128 rows) of a[M, K] times the weights w[tile_group[i]] of w [groups, N, K], bfloat16 on the tcgen05
     tensor cores; tiles with tile_group[i] < 0 are left out (their rows of the result are not written).
     ``gated``: every group's rows interleave gate and up (``interleave_gate_up``); the result is [M, N / 2].
     ``act`` (ungated): an activation of every result in the epilogue (``UNGATED_ACTS``).  ``clamp`` = (limit, alpha), with ``gated``:
     the clamped unit g * sigmoid(alpha g) * (u + 1), g = min(gate, limit), u = clamp(up, -limit, limit), in the SiLU's
-    place.  ``row_scale`` float32 [M] (``gated``, no ``clamp``): row i of ``a`` counts row_scale[i] times."""
+    place.  ``row_scale`` float32 [M] (``gated``, no ``clamp``): row i of ``a`` counts row_scale[i] times.
+    ``tile_rows`` (a multiple of 8): of every row tile only the first so many rows are read and written."""
     _need_cuda(a, w, tile_group, status, row_scale)
     _need(row_scale is None or (gated and clamp is None and row_scale.dtype == torch.float32 and row_scale.numel() >= a.shape[0]),
           "gemm_tcgen05_grouped: row_scale float32 [M], with the SiLU-gated form")
@@ -1142,12 +1144,13 @@ def gemm_tcgen05_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Ten
         _need(gated and clamp[0] > 0, "gemm_tcgen05_grouped: the clamped unit is a gated form with a positive limit")
         _check(_fn(_libs.get("gemm_tcgen05.cu"), "tkb_gemm_tcgen05_grouped_clamped_bf16")(
             _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(K), _ptr(out), c_int(out.stride(0)), c_int(M), c_int(N), c_int(K),
-            c_float(clamp[0]), c_float(clamp[1]), _ptr(tile_group), c_int(G), _ptr(status), _stream()), "gemm_tcgen05_grouped")
+            c_float(clamp[0]), c_float(clamp[1]), _ptr(tile_group), c_int(G), c_int(tile_rows), _ptr(status), _stream()),
+            "gemm_tcgen05_grouped")
         return out
     _check(_fn(_libs.get("gemm_tcgen05.cu"), "tkb_gemm_tcgen05_grouped_bf16")(
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(K), _ptr(out), c_int(out.stride(0)), c_int(M), c_int(N), c_int(K),
-        c_int(1 if gated else (UNGATED_ACTS[act] if act else 0)), _ptr(tile_group), c_int(G), _ptr(row_scale), _ptr(status), _stream()),
-        "gemm_tcgen05_grouped")
+        c_int(1 if gated else (UNGATED_ACTS[act] if act else 0)), _ptr(tile_group), c_int(G), _ptr(row_scale), c_int(tile_rows),
+        _ptr(status), _stream()), "gemm_tcgen05_grouped")
     return out
 
 
@@ -1373,7 +1376,8 @@ def decay_walk_modules(dim: int, vdim: int) -> list[dict]:
 
 # Tokens of a request from which the recurrence goes in chunks of DECAY_CHUNK.  Measured on B200, 4 to 16 heads of
 # 128 x 128: the walk takes 12 us for 64 tokens, 22 for 128 and 0.15 us for each more; the chunk kernels 26 us for one chunk
-# as for two, 108 us for 2,048 tokens of 16 heads (the walk 300), and 35 and 147 us with a decay vector (11 and 358).
+# as for two (192 tokens: 27 us, the walk 31), 108 us for 2,048 tokens of 16 heads (300), and 34 and 137 us with a decay
+# vector (192 tokens: 37 for the walk; 358).
 DECAY_CHUNK = 64
 DECAY_CHUNKS_FROM = 192
 

@@ -333,7 +333,7 @@ class PagedAttention(AttentionPlanning, Mixer):
                                 item_entry=plan["row_item_entry"], tma=bool(counts[6]), status=ctx.status)
             return project(attn, self.w_o)
         if plan is None or out_rows is not None:
-            # float32, or only some rows are wanted: the FP32-pipe kernel, one warp per (row, head)
+            # float32, or only some rows are wanted: the FP32-pipe kernel
             n_rows = T if out_rows is None else out_rows.numel()
             attn = torch.empty((n_rows, nh * hd), dtype=h.dtype, device=h.device)
             ops.attn_paged(qkv, qkv.shape[1], attn, cache.k, cache.v, ctx.token_seq, ctx.positions, tables.indptr,

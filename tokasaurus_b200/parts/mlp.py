@@ -345,17 +345,21 @@ class RoutedExperts(FeedForward):
             # products on the tcgen05 tensor cores, each row tile with its own expert's weights
             tile = 128
             n_tiles = (T * top) // tile + E
+            # a router's choices differ, so an expert has at most one row of each token (a table's may not): with few tokens
+            # the rest of its tile is nobody's
+            tile_rows = min(tile, -(-(T * top if self.by_token else T) // 8) * 8)
             order = torch.empty((n_tiles * tile,), dtype=torch.int32, device=dev)
             src_token = torch.empty((n_tiles * tile,), dtype=torch.int32, device=dev)
             tile_group = torch.empty((n_tiles,), dtype=torch.int32, device=dev)
             ops.moe_order(top_idx, E, offsets, order, place_of, pad=tile, tile_group=tile_group, src_token=src_token)
             placed = torch.empty((n_tiles * tile, self.width), dtype=h.dtype, device=dev)
             scale = torch.empty((n_tiles * tile,), dtype=torch.float32, device=dev) if self.weigh_input else None
-            ops.moe_gather(h, src_token, placed, order if self.weigh_input else None, top_w if self.weigh_input else None, scale)
+            ops.moe_gather(h, src_token, placed, order if self.weigh_input else None, top_w if self.weigh_input else None, scale,
+                           tile, tile_rows)
             status = ctx.status if ctx is not None else torch.zeros(1, dtype=torch.int32, device=dev)
             act = ops.gemm_tcgen05_grouped(placed, self.w_gate_up_tc, tile_group, status, gated=self.act is None, act=self.act,
-                                           clamp=self.clamp, row_scale=scale)
-            y = ops.gemm_tcgen05_grouped(act, self.w_down, tile_group, status)
+                                           clamp=self.clamp, row_scale=scale, tile_rows=tile_rows)
+            y = ops.gemm_tcgen05_grouped(act, self.w_down, tile_group, status, tile_rows=tile_rows)
             ops.moe_combine(y, place_of, top_w, shared, out, shared_gate, weigh=not self.weigh_input)
             return out
         order = torch.empty((T * top,), dtype=torch.int32, device=dev)
