@@ -151,3 +151,92 @@ def test_chunks_of_the_forgetting_recurrence(dtype, vdim, heads, lens, monkeypat
         assert rel(out[r], o) < bound and rel(st[i], S) < 16 * 2.0 ** -24
         assert rel(out[r], o) < 1.5 * rel(walked[r], o) + 2.0 ** -24 and rel(st[i], S) < 1.5 * rel(wst[i], S) + 2.0 ** -24
     assert torch.equal(st[-1].float(), state[-1])
+
+
+NOT_FINITE = [("v", float("inf")), ("v", float("nan")), ("v", 3.4e38), ("k", float("-inf")), ("q", float("nan")), ("decay", float("nan")),
+              ("state", float("inf"))]
+
+
+@pytest.mark.parametrize("form,heads,groups,what,value", [
+    (form, heads, groups, what, value) for form, heads, groups in (("head", 2, 1), ("token", 2, 2), ("channel", 2, 2))
+    for what, value in NOT_FINITE if (form, what) != ("head", "decay")])  # (a constant a head has no token of its own)
+@pytest.mark.parametrize("vdim", [64, 128])
+def test_chunks_not_finite(form, heads, groups, vdim, what, value, monkeypatch):
+    """One number that is not finite (or whose first bfloat16 is not): tokens ahead of it do not see it, those behind have what
+    the walk gives them, and other requests and heads have the bits of a clean run."""
+    from tokasaurus_b200.kernels import ops
+
+    lens, hit, size = [200, 300, 260], 200 + 137, heads * vdim * 128  # the second request's third chunk, inside a block of 16
+    p, state, ref = problem(form, heads, groups, vdim, lens, 11 + vdim)
+    if form != "head":
+        for name in ("dt_dec", "decay_vec"):  # (decays of zero would bury what is looked for)
+            if p[name] is not None:
+                p[name] = p[name].clamp(min=0.3)
+    clean, cst = run(p, state, lens, heads, groups, vdim)
+    head = heads - 1
+    col = {"v": head * vdim + 5, "k": (groups - 1) * 128 + 3, "q": (groups - 1) * 128 + 3}
+    bad, bstate = dict(p), state.clone()
+    if what == "state":
+        bstate[1, head * vdim * 128 + 77], hit = value, 200
+    elif what == "decay":
+        name = "dt_dec" if form == "token" else "decay_vec"
+        bad[name] = p[name].clone()
+        bad[name][hit, heads + head if form == "token" else head * 128 + 3] = value
+    else:
+        bad[what] = p[what].clone()
+        bad[what][hit, col[what]] = value
+    out, st = run(bad, bstate, lens, heads, groups, vdim)
+    monkeypatch.setattr(ops, "DECAY_CHUNKS_FROM", 1 << 30)
+    walked, wst = run(bad, bstate, lens, heads, groups, vdim)
+    one = slice(head * vdim, (head + 1) * vdim)
+    others = torch.ones(heads * vdim, dtype=torch.bool)
+    others[one if groups > 1 or what in ("v", "state") else slice(None)] = False  # (heads that share q and k share their numbers)
+    chunk0 = 200 + (hit - 200) // 64 * 64
+    assert torch.equal(out[:chunk0], clean[:chunk0]) and torch.equal(out[500:], clean[500:])
+    assert torch.equal(out[:, others], clean[:, others])
+    near = lambda x, y: float((x.double() - y.double()).norm()) <= 16 * 2.0 ** -24 * float(y.double().norm())  # noqa: E731
+    assert out[chunk0:hit].isfinite().all() and near(out[chunk0:hit], clean[chunk0:hit])
+    assert (~walked[hit:500, one].isfinite()).any() or value == 3.4e38
+    for got, want in ((out[hit:500], walked[hit:500]), (st[1], wst[1])):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[got.isinf()], want[want.isinf()])
+        assert torch.equal(got.isinf(), want.isinf())
+        fine = want.isfinite()
+        assert near(got[fine], want[fine])
+    assert torch.equal(st[0], cst[0]) and torch.equal(st[2:], cst[2:])
+    monkeypatch.undo()
+    assert torch.equal(run(bad, bstate, lens, heads, groups, vdim, write=False)[0].nan_to_num(), out.nan_to_num())
+
+
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_chunks_of_the_forgetting_recurrence_not_finite(vdim, value, monkeypatch):
+    """The same behind gates: a value that is not finite, in the middle of a block of 16 tokens."""
+    from tokasaurus_b200.kernels import ops
+
+    heads, d, lens, hit = 2, 128, [250, 1, 200], 101
+    g = torch.Generator().manual_seed(vdim)
+    T, starts = sum(lens), [0, 250, 251]
+    qfv = torch.randn(T, heads * (2 * d + vdim), generator=g)
+    fb, low = torch.randn(heads * d, generator=g), torch.rand(heads * d, generator=g) * 0.95
+    nw = torch.rand(vdim, generator=g) + 0.5
+    state = torch.randn(len(lens), heads, vdim, d, generator=g)
+
+    def run(x):
+        st, out = state.to(DEV), torch.empty(T, heads * vdim, device=DEV)
+        ops.gated_recurrence(x.to(DEV), st, fb.to(DEV), low.to(DEV), nw.to(DEV), out, i32([0, 1, 2]), i32(starts), i32(lens), len(lens), heads, d,
+                             vdim, 1e-5)
+        return out.cpu(), st.cpu()
+
+    clean, cst = run(qfv)
+    x = qfv.clone()
+    x[hit, 2 * heads * d + vdim + 9] = value  # the second head's
+    out, st = run(x)
+    monkeypatch.setattr(ops, "DECAY_CHUNKS_FROM", 1 << 30)
+    walked, wst = run(x)
+    near = lambda a, b: float((a.double() - b.double()).norm()) <= 64 * 2.0 ** -24 * float(b.double().norm())  # noqa: E731
+    assert torch.equal(out[:64], clean[:64]) and torch.equal(out[250:], clean[250:]) and torch.equal(out[:, :vdim], clean[:, :vdim])
+    assert out[64:hit].isfinite().all() and near(out[64:hit], clean[64:hit]) and torch.equal(st[1:], cst[1:])
+    for got, want in ((out[hit:250], walked[hit:250]), (st[0], wst[0])):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        fine = want.isfinite()
+        assert near(got[fine], want[fine])

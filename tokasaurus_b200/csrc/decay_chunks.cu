@@ -10,6 +10,7 @@
 //                  state after the last one into the request's slot;
 //   chunk_outputs  a block a (chunk, head): o_t = (q_t decayed from the chunk's start) S_start + sum_s A[t][s] v_s with
 //                  A[t][s] = q_t . (decay from s to t) c_s k_s for s <= t.
+// What is not finite, and what overflows on the way, is the walk's (decay_chunks.cuh).
 // No factor exceeds the decays' own products: one number a head is kept as a sum of logarithms in 64 bits, whose differences
 // are exact enough; a number a channel is kept as running products inside blocks of 16 tokens: A's blocks beside the diagonal
 // take q decayed from its block's start, k decayed to its block's end and the product of the blocks between, and A's diagonal
@@ -26,13 +27,13 @@
 // states' traffic of 32, and the products inside a chunk are still a third of the work.
 // Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 137 us (358);
 // three requests of 3,001 tokens in all 159 (383) and 200 us (513); 64 heads of 128 x 64 on 8 groups 242 us (455).
-#include "common.cuh"
+#include "decay_chunks.cuh"
 
 using namespace tkb;
 
 namespace {
 
-constexpr int C = 64;            // tokens of a chunk
+constexpr int C = DECAY_CHUNK;
 constexpr int DIM = 128;         // key size
 constexpr int THREADS = 512;     // 16 warps, 4 x 4 over a block's result
 constexpr int PITCH = (DIM + 8) * 2;   // bytes of a staged row of 128 bfloat16 numbers: rows meet different banks
@@ -44,6 +45,7 @@ constexpr int LDR = DIM + 4;           // floats of a staged float32 row
 struct Args {
   const float *q, *k, *v, *fvec, *dt_dec, *decay_head, *skip;
   float *state, *out, *states, *gains;  // states [chunks][heads][vdim][dim]; gains [chunks][heads] or [chunks][heads][dim]
+  int* bad;                             // [chunks][heads]: something of the chunk is not finite (decay_chunks.cuh)
   const int *seq_slot, *seq_q_start, *seq_q_len;
   long long slot_stride;
   int q_stride, k_stride, v_stride, f_stride, qk_div, n_seqs, heads, least, write_state;
@@ -52,9 +54,10 @@ struct Args {
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ int chunks_of(const Args& p, int s) {
-  const int n = s < p.n_seqs ? p.seq_q_len[s] : 0;
-  return n >= p.least ? (n + C - 1) / C : 0;
+  return s < p.n_seqs ? decay_chunks_of(p.seq_q_len[s], p.least) : 0;
 }
+// Zero, or a NaN once something that is not finite came by.
+__device__ __forceinline__ void watch(float& w, float x) { w = fmaf(x, 0.f, w); }
 // The request and the chunk of it that number `id` is (chunks are counted over the requests in order), by one warp.
 __device__ __forceinline__ bool find_chunk(const Args& p, int id, int& seq, int& chunk) {
   const int lane = threadIdx.x & 31;
@@ -301,6 +304,7 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
   if (seq < 0) return;
   const int nt = min(C, p.seq_q_len[seq] - where[1] * C), row0 = p.seq_q_start[seq] + where[1] * C;
   const size_t at = (size_t)id * p.heads + head;
+  float odd = 0.f;
   Pieces<C, VDIM> v;
   v.fetch(p.v + (size_t)row0 * p.v_stride + (size_t)head * VDIM, p.v_stride, nt);
   if (VEC) {
@@ -328,13 +332,21 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
       put2(kp + (part * 8 + s) * PITCH + 2 * d, PLANE, x.x, x.y);
       run = run * f[s];
     }
-    if (part == 0) *reinterpret_cast<float2*>(p.gains + at * DIM + d) = run;
+    if (part == 0) {
+      *reinterpret_cast<float2*>(p.gains + at * DIM + d) = run;
+      watch(odd, run.x);
+      watch(odd, run.y);
+    }
   } else {
     Pieces<C, DIM> k;
     k.fetch(p.k + (size_t)row0 * p.k_stride + (head / p.qk_div) * DIM, p.k_stride, nt);
     log_sums(p, head, row0, nt, logs, negs, scale);
     if (tid < C) scale[tid] *= decay_between(logs, negs, tid, nt - 1);
-    if (tid == 0) p.gains[at] = decay_between(logs, negs, -1, nt - 1);
+    if (tid == 0) {
+      const float gain = decay_between(logs, negs, -1, nt - 1);
+      p.gains[at] = gain;
+      watch(odd, gain);
+    }
     __syncthreads();
     k.scale(scale);  // (rows from nt on are zeros; their factors are finite: no decays follow them)
     k.put(kp, PITCH, PLANE);
@@ -356,7 +368,11 @@ __global__ void __launch_bounds__(THREADS) chunk_states_kernel(Args p) {
       float* o = u + (size_t)(m0 + 16 * i + g) * DIM + n0 + 8 * j + t2;
       *reinterpret_cast<float2*>(o) = make_float2(acc[i][j][0], acc[i][j][1]);
       *reinterpret_cast<float2*>(o + 8 * DIM) = make_float2(acc[i][j][2], acc[i][j][3]);
+#pragma unroll
+      for (int e = 0; e < 4; e++) watch(odd, acc[i][j][e]);
     }
+  const int bad = __syncthreads_or(odd != 0.f);  // (a NaN is not zero)
+  if (tid == 0) p.bad[at] = bad;
 }
 
 // --------------------------------------------------------------------------------- the state every chunk starts from
@@ -364,13 +380,10 @@ template <int VDIM, bool VEC>
 __global__ void __launch_bounds__(256) chunk_scan_kernel(Args p) {
   trigger_dependents();
   grid_dependency_wait();
-  const int seq = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
+  const int seq = blockIdx.x, head = blockIdx.y;
   const int n = chunks_of(p, seq);
   if (n == 0) return;
-  int first = 0;  // the request's first chunk: those of the requests before it
-  for (int s0 = 0; s0 < seq; s0 += 32) first += s0 + lane < seq ? chunks_of(p, s0 + lane) : 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+  const int first = decay_first_chunk(p.seq_q_len, seq, p.least);
   const int e = (blockIdx.z * 256 + threadIdx.x) * 4;  // (VDIM * DIM is a multiple of 1,024)
   float* st = p.state + (size_t)p.seq_slot[seq] * p.slot_stride + (size_t)head * VDIM * DIM + e;
   float4 S = *reinterpret_cast<const float4*>(st);
@@ -402,6 +415,12 @@ __global__ void __launch_bounds__(256) chunk_scan_kernel(Args p) {
     }
   }
   if (p.write_state) *reinterpret_cast<float4*>(st) = S;
+  float odd = 0.f;
+  watch(odd, S.x);
+  watch(odd, S.y);
+  watch(odd, S.z);
+  watch(odd, S.w);
+  if (odd != 0.f) p.bad[place(n - 1)] = 1;
 }
 
 // ------------------------------------------------------------------------------------------------------ the outputs
@@ -590,6 +609,7 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
     step16<1, NT, true, false>(acc, p_at + wm * 16 * P_PITCH + 2 * s, P_PITCH, P_PLANE, q_at + s * V_PITCH + 2 * n0, V_PITCH, V_PLANE);
   const float d_skip = p.skip ? p.skip[head] : 0.f;
   const size_t row = (size_t)p.heads * VDIM;
+  float odd = 0.f;
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const int t = t0 + 8 * h;
@@ -605,8 +625,11 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
         x.y = fmaf(d_skip, vv.y, x.y);
       }
       *reinterpret_cast<float2*>(o + 8 * j) = x;
+      watch(odd, x.x);
+      watch(odd, x.y);
     }
   }
+  if (__syncthreads_or(odd != 0.f) && tid == 0) p.bad[at] = 1;
 }
 
 template <int VDIM, bool VEC>
@@ -632,13 +655,15 @@ int chunks_launch(const Args& p, int max_chunks, cudaStream_t st) {
 // For the requests that bring at least `least` tokens (the others are left alone).  Arguments as in tkb_decay_walk; k null (only
 // with fvec): k = 1 - f, what a gate that forgets leaves room for (recurrence.cu); dim is
 // 128, vdim 64 or 128; q, k, v, fvec rows and their strides, state and slot_stride in whole 16-byte pieces.  states:
-// float32 [max_chunks][heads][vdim][128], gains: float32 [max_chunks][heads] (fvec: [max_chunks][heads][128]) are scratch;
+// float32 [max_chunks][heads][vdim][128], gains: float32 [max_chunks][heads] (fvec: [max_chunks][heads][128]) are scratch; bad:
+// int32 [max_chunks][heads], the chunks that the walk is to do over again (with states; see decay_chunks.cuh);
 // max_chunks: at least the requests' tokens in chunks of 64, each request rounded up.
 TKB_EXPORT int tkb_decay_chunks(const float* q, int q_stride, const float* k, int k_stride, int qk_div, const float* fvec,
                                 int f_stride, const float* v, int v_stride, const float* dt_dec, const float* decay_head,
                                 const float* skip, float* state, long long slot_stride, float* out, const int* seq_slot,
                                 const int* seq_q_start, const int* seq_q_len, int n_seqs, int heads, int dim, int vdim,
-                                int write_state, int least, float* states, float* gains, int max_chunks, void* st_) {
+                                int write_state, int least, float* states, float* gains, int* bad, int max_chunks,
+                                void* st_) {
   if (n_seqs <= 0 || max_chunks <= 0) return 0;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (dim != DIM || (vdim != 64 && vdim != 128) || heads <= 0 || heads > 65535 || qk_div <= 0 || least < 1) return -2;
@@ -647,7 +672,7 @@ TKB_EXPORT int tkb_decay_chunks(const float* q, int q_stride, const float* k, in
     return -2;
   if (fvec != nullptr && (dt_dec != nullptr || decay_head != nullptr || qk_div != 1)) return -2;
   if (k == nullptr && fvec == nullptr) return -2;
-  const Args p = {q, k, v, fvec, dt_dec, decay_head, skip, state, out, states, gains, seq_slot, seq_q_start, seq_q_len,
+  const Args p = {q, k, v, fvec, dt_dec, decay_head, skip, state, out, states, gains, bad, seq_slot, seq_q_start, seq_q_len,
                   slot_stride, q_stride, k_stride, v_stride, f_stride, qk_div, n_seqs, heads, least, write_state};
   cudaStream_t st = (cudaStream_t)st_;
   if (fvec) return vdim == 64 ? chunks_launch<64, true>(p, max_chunks, st) : chunks_launch<128, true>(p, max_chunks, st);

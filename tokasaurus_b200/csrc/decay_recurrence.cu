@@ -35,7 +35,7 @@
 //
 // Compile with -DTKB_DR_LANES=<threads that share a column: the power of two from 8 to 32 nearest above dim / 4> and
 // -DTKB_DR_DPT=<dims a lane: 4 * ceil(dim / (4 * lanes))>.
-#include "common.cuh"
+#include "decay_chunks.cuh"
 #include <limits.h>
 
 #ifndef TKB_DR_DPT
@@ -165,7 +165,7 @@ decay_walk_kernel(const float* __restrict__ q, int q_stride, const float* __rest
                   long long slot_stride, float* __restrict__ out, const int* __restrict__ seq_slot,
                   const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dim, int vdim,
                   int write_state, int cols_per_block, int vec_qk, int vec_v, int vec_s, int chunk,
-                  float* __restrict__ ones_out, int below) {
+                  float* __restrict__ ones_out, ChunkMarks marks) {
   extern __shared__ __align__(16) float smem[];
   const int cols = min(cols_per_block, vdim) + (ONES ? 1 : 0);
   const int cols4 = (cols + 3) & ~3;
@@ -174,9 +174,10 @@ decay_walk_kernel(const float* __restrict__ q, int q_stride, const float* __rest
   float* os = smem + 2 * buf_floats;  // the lanes' shares of a chunk's outputs: [cols][LANES][chunk + 1]
   const int orow = chunk + 1;         // (one float of padding: the lanes of a column write different banks)
   const int s = blockIdx.x, head = blockIdx.y;
-  const int n = seq_q_len[s];
-  if (n <= 0 || n >= below) return;
-  const int start = seq_q_start[s];
+  grid_dependency_wait();
+  int n = seq_q_len[s], start = seq_q_start[s];
+  const float* from = nullptr;
+  if (ONES ? n <= 0 : !walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from)) return;
   const int tid = threadIdx.x, lane = tid & (LANES - 1);
   const int col_begin = blockIdx.z * cols_per_block;
   const int v_end = min(vdim, col_begin + cols_per_block);
@@ -189,15 +190,15 @@ decay_walk_kernel(const float* __restrict__ q, int q_stride, const float* __rest
   // dims beyond `dim` of the last lanes are read: zero the buffers once if there are any (the copies never touch them)
   if (dim < LANES * DPT)
     for (int idx = tid; idx < 2 * buf_floats; idx += blockDim.x) smem[idx] = 0.f;
-  grid_dependency_wait();
   float* st = state + (size_t)seq_slot[s] * slot_stride + (size_t)head * (vdim + (ONES ? 1 : 0)) * dim;
+  if (from == nullptr) from = st;
 
   float S[DPT];
   if (vec_s) {
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
       const int d = 4 * (lane + LANES * (i >> 2));
-      const float4 x = (j < col_end && d < dim) ? *reinterpret_cast<const float4*>(st + (size_t)j * dim + d)
+      const float4 x = (j < col_end && d < dim) ? *reinterpret_cast<const float4*>(from + (size_t)j * dim + d)
                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
       S[i] = x.x; S[i + 1] = x.y; S[i + 2] = x.z; S[i + 3] = x.w;
     }
@@ -205,7 +206,7 @@ decay_walk_kernel(const float* __restrict__ q, int q_stride, const float* __rest
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
       const int d = 4 * (lane + LANES * (i >> 2)) + (i & 3);
-      S[i] = (j < col_end && d < dim) ? st[(size_t)j * dim + d] : 0.f;
+      S[i] = (j < col_end && d < dim) ? from[(size_t)j * dim + d] : 0.f;
     }
   }
   const float* qh = q + (size_t)(head / qk_div) * dim;
@@ -364,7 +365,7 @@ int walk_launch(const float* q, int q_stride, const float* k, int k_stride, int 
                 const float* v, int v_stride,
                 const float* dt_dec, const float* decay_head, const float* skip, float* state, long long slot_stride,
                 float* out, const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
-                int heads, int dim, int vdim, int write_state, float* ones_out, int below, cudaStream_t st) {
+                int heads, int dim, int vdim, int write_state, float* ones_out, const ChunkMarks& marks, cudaStream_t st) {
   if (n_seqs <= 0 || n_tokens <= 0) return 0;
   if (dim <= 0 || dim > DPT * LANES || vdim <= 0 || heads <= 0 || qk_div <= 0) return -2;
   if (heads > 65535) return -3;
@@ -397,7 +398,7 @@ int walk_launch(const float* q, int q_stride, const float* k, int k_stride, int 
   // part of the GPU (measured: 0.84 ms instead of 0.36 ms for 2,048 tokens of 16 heads).
   kernel<<<dim3(n_seqs, heads, splits), dim3(threads), smem, st>>>(
       q, q_stride, k, k_stride, qk_div, fvec, f_stride, v, v_stride, dt_dec, decay_head, skip, state, slot_stride, out,
-      seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state, cols_per_block, vec_qk, vec_v, vec_s, chunk, ones_out, below > 0 ? below : INT_MAX);
+      seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state, cols_per_block, vec_qk, vec_v, vec_s, chunk, ones_out, marks);
   return launch_status();
 }
 
@@ -423,16 +424,19 @@ TKB_EXPORT int tkb_ssm_prep(const float* proj, int stride, int xbc_off, int C, i
 // dt_dec: float32 [T, 2 * heads] (key scale, then decay) or null, then decay_head [heads] is the decay and the key
 // scale is 1; or fvec [T, heads * dim] (rows of f_stride floats): a decay for every key channel, key scale 1 (then
 // dt_dec and decay_head are null).  skip: [heads] or null.  ones_out: float32 [T, heads] or null; given, a head's state
-// holds one more column whose value is 1 at every token, and S^T q of that column goes there (not with fvec).  below: requests that bring
-// so many tokens or more are left alone (0: none are); decay_chunks.cu does them.
+// holds one more column whose value is 1 at every token, and S^T q of that column goes there (not with fvec).  bad, states, least: what
+// decay_chunks.cu left of the requests that bring at least `least` tokens (ChunkMarks; bad null: nothing went in chunks).
 TKB_EXPORT int tkb_decay_walk(const float* q, int q_stride, const float* k, int k_stride, int qk_div, const float* fvec,
                               int f_stride, const float* v, int v_stride, const float* dt_dec, const float* decay_head, const float* skip,
                               float* state, long long slot_stride, float* out, const int* seq_slot,
                               const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens, int heads, int dim,
-                              int vdim, int write_state, float* ones_out, int below, void* st) {
+                              int vdim, int write_state, float* ones_out, const int* bad, const float* states, int least,
+                              void* st) {
+  if (bad != nullptr && (states == nullptr || least < 1 || ones_out != nullptr)) return -2;
+  const ChunkMarks marks = {bad, states, bad != nullptr ? least : INT_MAX};
   if (fvec != nullptr && (dt_dec != nullptr || qk_div != 1 || ones_out != nullptr)) return -2;
   return walk_launch(q, q_stride, k, k_stride, qk_div, fvec, f_stride, v, v_stride, dt_dec, decay_head, skip, state, slot_stride, out,
-                     seq_slot, seq_q_start, seq_q_len, n_seqs, n_tokens, heads, dim, vdim, write_state, ones_out, below, (cudaStream_t)st);
+                     seq_slot, seq_q_start, seq_q_len, n_seqs, n_tokens, heads, dim, vdim, write_state, ones_out, marks, (cudaStream_t)st);
 }
 
 TKB_EXPORT int tkb_silu_cols(float* x, int stride, int ncols, int rows, void* st) {

@@ -15,7 +15,7 @@
 // that owns all columns of its head normalises them itself; with the columns of a head split over several blocks
 // (few requests with many tokens: the walk over the tokens is what takes the time, so it is spread over as many
 // SMs as there are) the raw outputs go to a float32 buffer and a second kernel normalises them.
-#include "common.cuh"
+#include "decay_chunks.cuh"
 #include <limits.h>
 
 #ifndef TKB_REC_DPT
@@ -58,7 +58,7 @@ gated_recurrence_kernel(const float* __restrict__ qfv, int row_stride, float* __
                         const float* __restrict__ f_bias, const float* __restrict__ low,
                         const float* __restrict__ norm_w, T* __restrict__ out, const int* __restrict__ seq_slot,
                         const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dim,
-                        int vdim, float eps, int write_state, int cols_per_block, float* __restrict__ raw_out, int below) {
+                        int vdim, float eps, int write_state, int cols_per_block, float* __restrict__ raw_out, ChunkMarks marks) {
   extern __shared__ float smem[];
   float* qs = smem;                 // [CHUNK][dim]
   float* fs = qs + CHUNK * dim;     // [CHUNK][dim]
@@ -67,15 +67,16 @@ gated_recurrence_kernel(const float* __restrict__ qfv, int row_stride, float* __
   trigger_dependents();
   grid_dependency_wait();
   const int s = blockIdx.x, head = blockIdx.y;
-  const int n = seq_q_len[s];
-  if (n <= 0 || n >= below) return;
-  const int start = seq_q_start[s];
+  int n = seq_q_len[s], start = seq_q_start[s];
+  const float* from = nullptr;
+  if (PREGATED ? !walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from) : n <= 0) return;
   const int tid = threadIdx.x, lane = tid & (LANES - 1);
   const int cols_per_pass = blockDim.x / LANES;
   const int col_begin = blockIdx.z * cols_per_block;
   const int col_end = min(vdim, col_begin + cols_per_block);
   const int col0 = col_begin + tid / LANES;
   float* st = state + ((size_t)seq_slot[s] * heads + head) * (size_t)vdim * dim;
+  if (from == nullptr) from = st;
 
   float S[CPT][DPT];
 #pragma unroll
@@ -84,7 +85,7 @@ gated_recurrence_kernel(const float* __restrict__ qfv, int row_stride, float* __
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
       const int d = lane + LANES * i;
-      S[c][i] = (j < col_end && d < dim) ? st[(size_t)j * dim + d] : 0.f;
+      S[c][i] = (j < col_end && d < dim) ? from[(size_t)j * dim + d] : 0.f;
     }
   }
   const float* q_raw = qfv + (size_t)head * dim;
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS_MAX)
 gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, float* __restrict__ state,
                               const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
                               const int* __restrict__ seq_q_len, int heads, int dim, int vdim, int write_state,
-                              int cols_per_block, float* __restrict__ raw_out, int below) {
+                              int cols_per_block, float* __restrict__ raw_out, ChunkMarks marks) {
   extern __shared__ __align__(16) float smem[];
   // A thread's state values: with DPT a multiple of 4 the DPT consecutive dims lane * DPT ..., so that its gates
   // come out of shared memory as 16-byte vectors (a quarter of the loads); each thread's stretch of a row is
@@ -204,9 +205,9 @@ gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, flo
   trigger_dependents();
   grid_dependency_wait();
   const int s = blockIdx.x, head = blockIdx.y;
-  const int n = seq_q_len[s];
-  if (n <= 0 || n >= below) return;
-  const int start = seq_q_start[s];
+  int n = seq_q_len[s], start = seq_q_start[s];
+  const float* from = nullptr;
+  if (!walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from)) return;
   const int tid = threadIdx.x, lane = tid & (LANES - 1);
   const int cols_per_pass = blockDim.x / LANES;
   const int col_begin = blockIdx.z * cols_per_block;
@@ -214,6 +215,7 @@ gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, flo
   const int ncols = col_end - col_begin;
   const int col0 = tid / LANES;  // within the block's columns
   float* st = state + ((size_t)seq_slot[s] * heads + head) * (size_t)vdim * dim;
+  if (from == nullptr) from = st;
   float S[CPT][DPT];
 #pragma unroll
   for (int c = 0; c < CPT; c++) {
@@ -221,7 +223,7 @@ gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, flo
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
       const int d = VEC ? lane * DPT + i : lane + LANES * i;
-      S[c][i] = (j < ncols && d < dim) ? st[(size_t)(col_begin + j) * dim + d] : 0.f;
+      S[c][i] = (j < ncols && d < dim) ? from[(size_t)(col_begin + j) * dim + d] : 0.f;
     }
   }
   const float* q_src = qfv + (size_t)head * dim;
@@ -339,7 +341,7 @@ __global__ void head_rmsnorm_kernel(const float* __restrict__ raw, const float* 
 template <typename T>
 int launch(float* qfv, int row_stride, float* state, const float* f_bias, const float* low, const float* norm_w,
            void* out, const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
-           int heads, int dim, int vdim, float eps, int write_state, float* raw, int below, int phase, cudaStream_t st) {
+           int heads, int dim, int vdim, float eps, int write_state, float* raw, const ChunkMarks& marks, int phase, cudaStream_t st) {
   if (n_seqs <= 0) return 0;
   if (heads <= 0 || dim <= 0 || vdim <= 0 || dim > LANES * DPT || heads > 65535) return -2;
   // columns a block: all of the head's, unless the requests and heads alone leave SMs idle and a buffer for raw
@@ -362,18 +364,17 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
     cudaFuncSetAttribute(gated_recurrence_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
   const int rows = n_tokens * heads;
-  if (phase == 2)
-    return launch_pdl(head_rmsnorm_kernel<T>, dim3((rows + 7) / 8), dim3(256), 0, st, (const float*)raw, norm_w, (T*)out, rows, vdim, eps);
-  if (below > 0 && raw == nullptr) return -2;
-  float* raw_out = split > 1 || below > 0 ? raw : nullptr;
-  const int under = below > 0 ? below : INT_MAX;
+  if (phase != 0 && raw == nullptr) return -2;
+  float* raw_out = split > 1 || phase != 0 ? raw : nullptr;
   if (raw_out == nullptr)
     return launch_pdl(gated_recurrence_kernel<T, false>, dim3(n_seqs, heads, 1), dim3(threads), smem, st,
                       (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start,
-                      seq_q_len, heads, dim, vdim, eps, write_state, cols_per_block, raw_out, under);
-  int rc = launch_pdl(recurrence_gates_kernel, dim3(n_tokens), dim3(heads * dim >= 1024 ? 256 : 128), 0, st, qfv,
-                      row_stride, f_bias, low, heads * dim);
-  if (rc != 0) return rc;
+                      seq_q_len, heads, dim, vdim, eps, write_state, cols_per_block, raw_out, marks);
+  int rc = 0;
+  if (phase != 2)
+    rc = launch_pdl(recurrence_gates_kernel, dim3(n_tokens), dim3(heads * dim >= 1024 ? 256 : 128), 0, st, qfv, row_stride, f_bias,
+                    low, heads * dim);
+  if (rc != 0 || phase == 1) return rc;
   const bool by_16 = dim % 4 == 0 && vdim % 4 == 0 && row_stride % 4 == 0 && (((uintptr_t)qfv) & 15) == 0;
   constexpr int SPLIT_SP = (DPT % 4 == 0) ? DPT + (((DPT / 4) % 2 == 0) ? 4 : 0) : DPT;  // as in the kernel
   const size_t smem_split = (size_t)CHUNK * (2 * (2 * LANES * SPLIT_SP + cols_per_block) + cols_per_block) * sizeof(float);
@@ -382,13 +383,13 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
       cudaFuncSetAttribute(gated_recurrence_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split);
     rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
                     (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
-                    cols_per_block, raw_out, under);
+                    cols_per_block, raw_out, marks);
   } else {
     rc = launch_pdl(gated_recurrence_kernel<T, true>, dim3(n_seqs, heads, split), dim3(threads), smem, st,
                     (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start, seq_q_len,
-                    heads, dim, vdim, eps, write_state, cols_per_block, raw_out, under);
+                    heads, dim, vdim, eps, write_state, cols_per_block, raw_out, marks);
   }
-  if (rc != 0 || phase == 1) return rc;
+  if (rc != 0) return rc;
   return launch_pdl(head_rmsnorm_kernel<T>, dim3((rows + 7) / 8), dim3(256), 0, st, (const float*)raw_out, norm_w, (T*)out,
                     rows, vdim, eps);
 }
@@ -397,24 +398,26 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
 
 // qfv: float32 [tokens, row_stride]; state: float32 [slots, heads, vdim, dim]; out: [tokens, heads * vdim];
 // raw: float32 [tokens, heads * vdim] scratch for the split form, or null (every block then owns a whole head).
-// The split form turns the q and f columns of qfv into gates in place.  below: requests with so many tokens or more are left
-// to decay_chunks.cu (0: none; the split form, raw given), which reads the gates and fills raw.  phase 0: everything; 1: all but
-// the norm; 2: the norm.
+// The split form turns the q and f columns of qfv into gates in place.  phase 0: everything.  Where
+// decay_chunks.cu does the requests with at least `least` tokens (the split form, raw given), it runs between phase 1, the gates, and
+// phase 2, the walk over what it left (bad, states: ChunkMarks) and the norm.
 TKB_EXPORT int tkb_gated_recurrence_f32(float* qfv, int row_stride, float* state, const float* f_bias,
                                         const float* low, const float* norm_w, void* out, const int* seq_slot,
                                         const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
-                                        int heads, int dim, int vdim, float eps, int write_state, float* raw, int below,
-                                        int phase, void* st) {
+                                        int heads, int dim, int vdim, float eps, int write_state, float* raw, const int* bad,
+                                        const float* states, int least, int phase, void* st) {
   return launch<float>(qfv, row_stride, state, f_bias, low, norm_w, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
-                       n_tokens, heads, dim, vdim, eps, write_state, raw, below, phase, (cudaStream_t)st);
+                       n_tokens, heads, dim, vdim, eps, write_state, raw,
+                       {bad, states, bad != nullptr ? least : INT_MAX}, phase, (cudaStream_t)st);
 }
 TKB_EXPORT int tkb_gated_recurrence_bf16(float* qfv, int row_stride, float* state, const float* f_bias,
                                          const float* low, const float* norm_w, void* out, const int* seq_slot,
                                          const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
-                                         int heads, int dim, int vdim, float eps, int write_state, float* raw, int below,
-                                        int phase, void* st) {
+                                         int heads, int dim, int vdim, float eps, int write_state, float* raw, const int* bad,
+                                        const float* states, int least, int phase, void* st) {
   return launch<__nv_bfloat16>(qfv, row_stride, state, f_bias, low, norm_w, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
-                               n_tokens, heads, dim, vdim, eps, write_state, raw, below, phase, (cudaStream_t)st);
+                               n_tokens, heads, dim, vdim, eps, write_state, raw,
+                               {bad, states, bad != nullptr ? least : INT_MAX}, phase, (cudaStream_t)st);
 }
 TKB_EXPORT int tkb_gated_recurrence_dpt() { return DPT; }
 TKB_EXPORT int tkb_gated_recurrence_cpt() { return CPT; }

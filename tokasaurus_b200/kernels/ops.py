@@ -874,23 +874,23 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
     _need(out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "gated_recurrence: out [T, heads * vdim]")
     f = _fn(_libs.get("recurrence.cu", **recurrence_defines(dim, vdim)), f"tkb_gated_recurrence_{_suffix(out.dtype)}")
     raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=qfv.device) if (split_heads and T > n_seqs) else None
-    # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the gates and the norm
+    # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the gates and the walk over what is left
     by_chunks = (raw is not None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and bool(decay_chunk_modules(dim, vdim))
                  and qfv.stride(0) % 4 == 0 and qfv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0)
 
-    def run(phase: int, below: int) -> None:
+    def run(phase: int, marks: tuple) -> None:
         _check(f(_ptr(qfv), c_int(qfv.stride(0)), _ptr(state), _ptr(f_bias), _ptr(low), _ptr(norm_w), _ptr(out),
                  _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(T), c_int(heads), c_int(dim),
-                 c_int(vdim), c_float(eps), c_int(1 if write_state else 0), _ptr(raw), c_int(below), c_int(phase), _stream()),
+                 c_int(vdim), c_float(eps), c_int(1 if write_state else 0), _ptr(raw), *marks, c_int(phase), _stream()),
                "gated_recurrence")
 
     if not by_chunks:
-        return run(0, 0)
-    run(1, DECAY_CHUNKS_FROM)
+        return run(0, _NO_MARKS)
+    run(1, _NO_MARKS)
     decay = qfv[:, heads * dim:2 * heads * dim]
-    _decay_chunks(qfv[:, :heads * dim], None, qfv[:, 2 * heads * dim:], 1, None, None, decay, None, state.view(state.shape[0], -1), raw,
-                  seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state)
-    run(2, 0)
+    chunks = _decay_chunks(qfv[:, :heads * dim], None, qfv[:, 2 * heads * dim:], 1, None, None, decay, None, state.view(state.shape[0], -1),
+                           raw, seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state)
+    run(2, _marks(chunks))
 
 
 # ---------------------------------------------------------------------------------------------
@@ -1436,19 +1436,30 @@ def ssm_prep(proj: torch.Tensor, xbc_off: int, channels: int, conv_w: torch.Tens
 
 
 def _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
-                  heads, dim, vdim, write_state) -> None:
+                  heads, dim, vdim, write_state) -> tuple[torch.Tensor, torch.Tensor]:
     """The recurrence of ``decay_walk`` for the requests that bring at least ``DECAY_CHUNKS_FROM`` tokens, in chunks (the caller
-    has checked the operands).  ``k`` None: 1 - decay_vec."""
+    has checked the operands).  ``k`` None: 1 - decay_vec.  Returns what the walk that follows needs to do over again what was not
+    finite: the chunks' marks and the states they started from."""
     T = q.shape[0]
     chunks = T // DECAY_CHUNK + min(n_seqs, T // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
     states = torch.empty((chunks, heads, vdim, dim), dtype=torch.float32, device=q.device)
     gains = torch.empty((chunks, heads, dim if decay_vec is not None else 1), dtype=torch.float32, device=q.device)
+    bad = torch.empty((chunks, heads), dtype=torch.int32, device=q.device)
     stride = lambda t: c_int(t.stride(0) if t is not None else 0)  # noqa: E731
     _check(_fn(_libs.get("decay_chunks.cu"), "tkb_decay_chunks")(
         _ptr(q), stride(q), _ptr(k), stride(k), c_int(heads_per_qk), _ptr(decay_vec), stride(decay_vec), _ptr(v), stride(v),
         _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
         _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
-        c_int(1 if write_state else 0), c_int(DECAY_CHUNKS_FROM), _ptr(states), _ptr(gains), c_int(chunks), _stream()), "decay_chunks")
+        c_int(1 if write_state else 0), c_int(DECAY_CHUNKS_FROM), _ptr(states), _ptr(gains), _ptr(bad), c_int(chunks), _stream()),
+        "decay_chunks")
+    return bad, states
+
+
+_NO_MARKS = (c_void_p(0), c_void_p(0), c_int(0))  # the walk's arguments where nothing went in chunks
+
+
+def _marks(chunks: tuple[torch.Tensor, torch.Tensor]) -> tuple:
+    return _ptr(chunks[0]), _ptr(chunks[1]), c_int(DECAY_CHUNKS_FROM)
 
 
 def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: int, dt_dec: torch.Tensor | None,
@@ -1483,23 +1494,23 @@ def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: 
     _need(ones_out is None or (decay_vec is None and ones_out.dtype == torch.float32 and ones_out.is_contiguous()
                                and tuple(ones_out.shape) == (T, heads)), "decay_walk: ones_out float32 [T, heads]")
     _need(out.dtype == torch.float32 and out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "decay_walk: out float32 [T, heads * vdim]")
-    below = 0
+    chunks = None
     rows = [q, k, v] + ([decay_vec] if decay_vec is not None else [])
     if (ones_out is None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and decay_chunk_modules(dim, vdim)
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in rows)
             and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0):
-        # requests that bring many tokens; the walk below then leaves them alone.  Which requests these are is read on the
-        # device: a step graph is replayed for other lengths.
-        below = DECAY_CHUNKS_FROM
-        _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
-                      heads, dim, vdim, write_state)
+        # requests that bring many tokens; the walk below then leaves them alone, unless their numbers are not finite.  Which
+        # requests these are is read on the device: a step graph is replayed for other lengths.
+        chunks = _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len,
+                               n_seqs, heads, dim, vdim, write_state)
     defines = _walk_defines(dim, vdim, n_seqs * heads * vall, T == n_seqs, q.device)
     _check(_fn(_libs.get("decay_recurrence.cu", **defines), "tkb_decay_walk")(
         _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),
         c_int(decay_vec.stride(0) if decay_vec is not None else 0), _ptr(v), c_int(v.stride(0)),
         _ptr(dt_dec), _ptr(decay_head), _ptr(skip), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(out),
         _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(T), c_int(heads), c_int(dim), c_int(vdim),
-        c_int(1 if write_state else 0), _ptr(ones_out), c_int(below), _stream()), "decay_walk")
+        c_int(1 if write_state else 0), _ptr(ones_out),
+        *(_NO_MARKS if chunks is None else _marks(chunks)), _stream()), "decay_walk")
 
 
 def memory_gates(proj: torch.Tensor, i_off: int, f_off: int, i_bias: torch.Tensor, f_bias: torch.Tensor, cap: float,
