@@ -14,7 +14,7 @@
 //   memory, and every 128 terms both are read and added to a float32 register with ordinary additions.  Measured against 64
 //   bits the result is closer than an FMA chain's (normal numbers, K = 2,048 and 8,192: relative error 1.4e-7 and 1.5e-7).
 //   An element that does not come out finite (an infinity, a NaN or an overflow among its inputs: 0 times infinity in a cut
-//   form is not what it is uncut) is done once more as the FMA chain.
+//   form is not what it is uncut) is done once more as the FMA chain, by the warp that has it (redo).
 //   What bounds it: with many rows the tensor instructions (six products: a sixth of their rate is the bound) and their
 //   operands' way through shared memory, with few the weights' way from memory.  A block is 15 warps that fetch, cut and
 //   store (the next chunks on their way into registers meanwhile) and one that issues the tensor instructions; all 16 read
@@ -179,10 +179,76 @@ __device__ __forceinline__ void fetch8(const float* __restrict__ p, int left, fl
   }
 }
 
-__device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ w, int K) {
-  float acc = 0.f;
-  for (int k = 0; k < K; k++) acc = fmaf(a[k], w[k], acc);
-  return acc;
+// Results that did not come out finite, once more as FMA chains over K in index order.  A warp: o[i * ldo] (i below `tokens`) of the
+// lane's feature, whose weights are the row w, and of the token in row i of A.  G tokens at a time share a reading of the
+// weights, REDO_K numbers of which are on their way together.  Tokens that are finite in all of a warp's features are passed by,
+// and so are tokens with a NaN among their numbers: every result of theirs is NaN, and is there.
+// (One element after the other, a number of each row at a time, 500 rows of NaN took 69 ms where a clean product takes 0.26.)
+template <bool VEC, int G, int REDO_K>
+__device__ __forceinline__ void redo_chains(float (&acc)[G], const float* __restrict__ A, int lda, int rows, const float* __restrict__ w,
+                                            int K) {
+#pragma unroll
+  for (int i = 0; i < G; i++) acc[i] = 0.f;
+  int k = 0;
+  if (VEC) {
+    for (; k + REDO_K <= K; k += REDO_K) {
+      float4 x[REDO_K / 4];
+#pragma unroll
+      for (int u = 0; u < REDO_K / 4; u++) x[u] = __ldg(reinterpret_cast<const float4*>(w + k) + u);
+#pragma unroll
+      for (int u = 0; u < REDO_K / 4; u++)
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+          if (G > 1 && i >= rows) break;
+          const float4 a = __ldg(reinterpret_cast<const float4*>(A + (size_t)i * lda + k) + u);
+          acc[i] = fmaf(a.w, x[u].w, fmaf(a.z, x[u].z, fmaf(a.y, x[u].y, fmaf(a.x, x[u].x, acc[i]))));
+        }
+    }
+  }
+#pragma unroll 4
+  for (; k < K; k++) {
+    const float x = __ldg(w + k);
+#pragma unroll
+    for (int i = 0; i < G; i++)
+      if (G == 1 || i < rows) acc[i] = fmaf(__ldg(A + (size_t)i * lda + k), x, acc[i]);
+  }
+}
+template <int G, int REDO_K>
+__device__ __forceinline__ void redo(float* o, int ldo, int tokens, bool there, const float* __restrict__ A, int lda,
+                                  const float* __restrict__ w, int K, bool vec) {
+  for (int i0 = 0; i0 < tokens; i0 += G) {
+    const int rows = min(G, tokens - i0);
+    bool any = false;
+    for (int i = 0; i < rows; i++) {
+      if (!__any_sync(0xffffffffu, there && !isfinite(o[(size_t)(i0 + i) * ldo]))) continue;
+      bool nan = false;
+#pragma unroll 8
+      for (int k = threadIdx.x & 31; k < K; k += 32) nan |= isnan(A[(size_t)(i0 + i) * lda + k]);
+      any |= !__any_sync(0xffffffffu, nan);
+    }
+    if (!any) continue;
+    float acc[G];
+    if (vec) redo_chains<true, G, REDO_K>(acc, A + (size_t)i0 * lda, lda, rows, w, K);
+    else redo_chains<false, G, REDO_K>(acc, A + (size_t)i0 * lda, lda, rows, w, K);
+#pragma unroll
+    for (int i = 0; i < G; i++)
+      if (i < rows && there && !isfinite(o[(size_t)(i0 + i) * ldo])) o[(size_t)(i0 + i) * ldo] = acc[i];
+  }
+}
+
+// The same for a warp of sgemm_split_kernel (of sgemm_add_slices_kernel): out of line and with nothing from before it, so that these keep
+// their registers.
+template <int NT, bool VEC>
+__device__ __noinline__ void redo_tile(const float* __restrict__ A, const float* __restrict__ W, float* C, int M, int N, int K, int lda,
+                                       int ldw, int ldc) {
+  constexpr int CPT = SCfg<NT>::CPT;
+  const int n = blockIdx.x * 128 + (threadIdx.x & 127), m = blockIdx.y * NT + (threadIdx.x >> 7) * CPT;
+  redo<8, 32>(C + (size_t)m * ldc + n, ldc, min(CPT, M - m), n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, VEC);
+}
+__device__ __noinline__ void redo_row(const float* __restrict__ A, const float* __restrict__ W, float* C, int N, int K, int lda, int ldw,
+                                      int ldc, int vec) {
+  const int n = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
+  redo<1, 16>(C + (size_t)m * ldc + n, ldc, 1, n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, vec);
 }
 
 // out: C when a block does all slices (`slices_here`), else the slices' partial results [slice][M][N].
@@ -195,7 +261,7 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ volatile int failed;
+  __shared__ volatile int failed, odd;  // a wait ran out; some result is not finite
   unsigned char* planes = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.x * 128, m0 = blockIdx.y * NT;
@@ -213,7 +279,7 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], WARPS);
     }
-    failed = 0;
+    failed = odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   grid_dependency_wait();
@@ -263,9 +329,9 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
       for (int i = 0; i < CPT; i++) {
         const int m = m0 + (int)col0 + i;
         if (n < N && m < M) {
-          float x = first_slice ? acc[i] : o[(size_t)m * ldo] + acc[i];
-          if (last && !partial && !isfinite(x)) x = chain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+          const float x = first_slice ? acc[i] : o[(size_t)m * ldo] + acc[i];
           o[(size_t)m * ldo] = x;
+          if (last && !isfinite(x)) odd = 1;
         }
         acc[i] = 0.f;
       }
@@ -376,6 +442,7 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
   }
   tcgen05_fence_before();
   __syncthreads();
+  if (!partial && !failed && odd) redo_tile<NT, VEC>(A, W, out, M, N, K, lda, ldw, ldc);
   if (warp == 0) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Z::TMEM) : "memory");
@@ -383,21 +450,24 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
 }
 
 // C = the slices' results, added in order.
-__global__ void __launch_bounds__(256)
-sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict__ A, const float* __restrict__ W,
-                        float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int slices) {
+__global__ void __launch_bounds__(256, 6)
+sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict__ A, const float* __restrict__ W, float* C, int M, int N,
+                        int K, int lda, int ldw, int ldc, int slices, int vec) {
   trigger_dependents();
   grid_dependency_wait();
   const int m = blockIdx.y;
   const int n = blockIdx.x * 256 + threadIdx.x;
-  if (n >= N) return;
-  const float* p = part + (size_t)m * N + n;
-  const size_t stride = (size_t)M * N;
-  float v = p[0];
+  bool odd = false;
+  if (n < N) {
+    const float* p = part + (size_t)m * N + n;
+    const size_t stride = (size_t)M * N;
+    float v = p[0];
 #pragma unroll 8
-  for (int s = 1; s < slices; s++) v += p[s * stride];
-  if (!isfinite(v)) v = chain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
-  C[(size_t)m * ldc + n] = v;
+    for (int s = 1; s < slices; s++) v += p[s * stride];
+    C[(size_t)m * ldc + n] = v;
+    odd = !isfinite(v);
+  }
+  if (__any_sync(0xffffffffu, odd)) redo_row(A, W, C, N, K, lda, ldw, ldc, vec);
 }
 
 // Chunks of K a slice holds, by N and K alone: as many slices as bring the blocks of one row tile to the SMs' number.
@@ -428,7 +498,7 @@ int split_launch(const float* A, const float* W, float* C, float* part, int M, i
                       N, K, lda, ldw, ldc, per, 1, 1);
   if (rc) return rc;
   return launch_pdl(sgemm_add_slices_kernel, dim3((N + 255) / 256, M), dim3(256), 0, st, (const float*)part, A, W, C, M, N, K,
-                    lda, ldw, ldc, slices);
+                    lda, ldw, ldc, slices, (int)VEC);
 }
 
 // Token columns of an instruction: the fewest that hold all rows, at most 128.
