@@ -90,3 +90,28 @@ def test_split_product_not_finite_takes_no_age(M, N, K):
 
     clean = time(0, 0.0)
     assert time(M, math.nan) < 4 * clean and time(1, math.inf) < 60 * clean
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 256, 512), (300, 20000, 128)])  # slices, and all of K in a block
+def test_split_product_knows_the_step_s_status(M, N, K, monkeypatch):
+    """A wait that runs out is reported to the status word of the step that the thread is in, as by every kernel that waits."""
+    from tokasaurus_b200.kernels import ops
+
+    seen, real = [], ops._fn
+
+    def spy(lib, name):
+        f = real(lib, name)
+        return (lambda *a: seen.append(a[-2].value) or f(*a)) if name == "tkb_sgemm_tn_f32" else f
+
+    monkeypatch.setattr(ops, "_fn", spy)
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.linear(a, w)
+    with ops.reporting_to(status):
+        out = ops.linear(a, w)
+        with ops.reporting_to(None):
+            ops.linear(a, w)
+        ops.linear(a, w)
+    ops.linear(a, w)
+    assert seen == [None, status.data_ptr(), None, status.data_ptr(), None]
+    assert int(status) == 0 and torch.equal(out, ops.linear(a, w))

@@ -251,11 +251,14 @@ __device__ __noinline__ void redo_row(const float* __restrict__ A, const float* 
   redo<1, 16>(C + (size_t)m * ldc + n, ldc, 1, n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, vec);
 }
 
+// What a block leaves in the place of its results when one of its waits ran out (a NaN of its own: no arithmetic makes it).
+constexpr int LOST = 0x7fc0105e;
+
 // out: C when a block does all slices (`slices_here`), else the slices' partial results [slice][M][N].
 template <int NT, bool VEC>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N, int K,
-                   int lda, int ldw, int ldc, int per_slice, int slices_here, int partial) {
+                   int lda, int ldw, int ldc, int per_slice, int slices_here, int partial, int* __restrict__ status) {
   using Z = SCfg<NT>;
   constexpr int CPT = Z::CPT, AHEAD = Z::AHEAD, TASKS = Z::TASKS, STAGES = Z::STAGES;
   extern __shared__ unsigned char smem_raw[];
@@ -438,10 +441,11 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
   if (!ok) {  // a wait ran out: nothing that could be taken for a result stays behind
     failed = 1;
     for (int i = 0; i < CPT; i++)
-      if (n < N && m0 + (int)col0 + i < M) o[(size_t)(m0 + col0 + i) * ldo] = __int_as_float(0x7fc00000);
+      if (n < N && m0 + (int)col0 + i < M) o[(size_t)(m0 + col0 + i) * ldo] = __int_as_float(LOST);
   }
   tcgen05_fence_before();
   __syncthreads();
+  if (tid == 0 && failed && status != nullptr) atomicOr(status, TKB_STATUS_WAIT_TIMEOUT);
   if (!partial && !failed && odd) redo_tile<NT, VEC>(A, W, out, M, N, K, lda, ldw, ldc);
   if (warp == 0) {
     tcgen05_fence_after();
@@ -457,7 +461,7 @@ sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict_
   grid_dependency_wait();
   const int m = blockIdx.y;
   const int n = blockIdx.x * 256 + threadIdx.x;
-  bool odd = false;
+  bool odd = false, lost = false;
   if (n < N) {
     const float* p = part + (size_t)m * N + n;
     const size_t stride = (size_t)M * N;
@@ -466,8 +470,11 @@ sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict_
     for (int s = 1; s < slices; s++) v += p[s * stride];
     C[(size_t)m * ldc + n] = v;
     odd = !isfinite(v);
+    if (odd)
+      for (int s = 0; s < slices; s++) lost |= __float_as_int(p[s * stride]) == LOST;
   }
-  if (__any_sync(0xffffffffu, odd)) redo_row(A, W, C, N, K, lda, ldw, ldc, vec);
+  // (what a wait that ran out left stays a NaN: it has been reported, and is no number's doing)
+  if (__any_sync(0xffffffffu, odd) && !__any_sync(0xffffffffu, lost)) redo_row(A, W, C, N, K, lda, ldw, ldc, vec);
 }
 
 // Chunks of K a slice holds, by N and K alone: as many slices as bring the blocks of one row tile to the SMs' number.
@@ -481,7 +488,7 @@ int chunks_a_slice(int N, int K) {
 
 template <int NT, bool VEC>
 int split_launch(const float* A, const float* W, float* C, float* part, int M, int N, int K, int lda, int ldw, int ldc,
-                 cudaStream_t st) {
+                 int* status, cudaStream_t st) {
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(sgemm_split_kernel<NT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<NT>::SMEM);
@@ -493,9 +500,9 @@ int split_launch(const float* A, const float* W, float* C, float* part, int M, i
   const int tiles = (N + 127) / 128, rows = (M + NT - 1) / NT;
   if (part == nullptr)
     return launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, 1), block, (size_t)SCfg<NT>::SMEM, st, A, W, C, M, N, K,
-                      lda, ldw, ldc, per, slices, 0);
+                      lda, ldw, ldc, per, slices, 0, status);
   int rc = launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, slices), block, (size_t)SCfg<NT>::SMEM, st, A, W, part, M,
-                      N, K, lda, ldw, ldc, per, 1, 1);
+                      N, K, lda, ldw, ldc, per, 1, 1, status);
   if (rc) return rc;
   return launch_pdl(sgemm_add_slices_kernel, dim3((N + 255) / 256, M), dim3(256), 0, st, (const float*)part, A, W, C, M, N, K,
                     lda, ldw, ldc, slices, (int)VEC);
@@ -516,9 +523,10 @@ TKB_EXPORT long long tkb_sgemm_tn_scratch(int M, int N, int K) {
   return (long long)slices * M * N;
 }
 
-// scratch: as many float32 values as tkb_sgemm_tn_scratch says, or null where it says 0.
+// scratch: as many float32 values as tkb_sgemm_tn_scratch says, or null where it says 0.  status: the device status word that
+// a wait that runs out sets bit 4 of, or null; the results it would have brought are NaN.
 TKB_EXPORT int tkb_sgemm_tn_f32(const float* A, const float* W, float* C, float* scratch, int M, int N, int K, int lda,
-                                int ldw, int ldc, void* st_) {
+                                int ldw, int ldc, int* status, void* st_) {
   cudaStream_t st = (cudaStream_t)st_;
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return -2;
@@ -528,8 +536,8 @@ TKB_EXPORT int tkb_sgemm_tn_f32(const float* A, const float* W, float* C, float*
     if ((M + nt - 1) / nt > 65535) return -3;
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
 #define TKB_GO(NT)                                                                                                  \
-  return vec ? split_launch<NT, true>(A, W, C, scratch, M, N, K, lda, ldw, ldc, st)                                  \
-             : split_launch<NT, false>(A, W, C, scratch, M, N, K, lda, ldw, ldc, st);
+  return vec ? split_launch<NT, true>(A, W, C, scratch, M, N, K, lda, ldw, ldc, status, st)                                  \
+             : split_launch<NT, false>(A, W, C, scratch, M, N, K, lda, ldw, ldc, status, st);
     if (nt == 16) { TKB_GO(16) }
     if (nt == 32) { TKB_GO(32) }
     if (nt == 64) { TKB_GO(64) }

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 from ctypes import c_float, c_int, c_void_p
 
 import torch
@@ -366,6 +367,24 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> Non
     _check(f(_ptr(src), _ptr(out), _ptr(rows), c_int(rows.numel()), c_int(row_bytes), _stream()), "gather_rows")
 
 
+_step = threading.local()
+
+
+class reporting_to:
+    """``with reporting_to(status):`` kernels that this thread launches through a function without a status argument (the float32
+    product) report to this device status word."""
+
+    def __init__(self, status: torch.Tensor | None):
+        self.status = status
+
+    def __enter__(self) -> None:
+        self.before = getattr(_step, "status", None)
+        _step.status = self.status
+
+    def __exit__(self, *exc) -> None:
+        _step.status = self.before
+
+
 def _sgemm_scratch(lib: ctypes.CDLL):
     f = _fn(lib, "tkb_sgemm_tn_scratch")
     f.restype, f.argtypes = ctypes.c_longlong, (c_int, c_int, c_int)
@@ -385,7 +404,8 @@ def sgemm_tn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     scratch = torch.empty((n_scratch,), dtype=torch.float32, device=a.device) if n_scratch else None
     f = _fn(lib, "tkb_sgemm_tn_f32")
     _check(f(_ptr(a), _ptr(w), _ptr(out), _ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(a.stride(0) if M > 1 else K),
-             c_int(w.stride(0) if N > 1 else K), c_int(out.stride(0) if M > 1 else N), _stream()), "sgemm_tn")
+             c_int(w.stride(0) if N > 1 else K), c_int(out.stride(0) if M > 1 else N), _ptr(getattr(_step, "status", None)), _stream()),
+           "sgemm_tn")
 
 
 def attn_paged(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,

@@ -13,6 +13,7 @@ from typing import Sequence
 
 import torch
 
+from tokasaurus_b200.kernels import ops
 from tokasaurus_b200.parts.base import Part, WeightSpec
 
 
@@ -115,6 +116,10 @@ class DecoderModel(Part):
         """Run this step's tokens; return float32 logits [len(ctx.logit_rows), vocab].  If the context carries a list
         ``layer_outputs``, a copy of the residual stream after every layer call is appended to it (pending updates
         folded in), for looking at a model layer by layer."""
+        with ops.reporting_to(ctx.status):
+            return self._forward(ctx)
+
+    def _forward(self, ctx) -> torch.Tensor:
         stream = self.embedding.forward(ctx)
         taps = getattr(ctx, "layer_outputs", None)
         last = len(self.run_order) - 1
