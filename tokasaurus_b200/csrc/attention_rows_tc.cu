@@ -25,6 +25,7 @@
 // Measured on B200: 2,048 tokens of 16 heads over latent rows of 192 + 64, window 1,024: 302 us on mma.sync, 51 us here (67
 // with three stages and the page lookups behind the wait for a stage); two prompts of 4,001 tokens, 32 heads of 64 + 64 on 8,
 // window 1,024, capped: 224 us, 96 us here (111 with the cap's arithmetic one score at a time).
+#include "per_device.h"
 #include "tcgen05.cuh"
 
 #if !defined(TKB_ROW) || !defined(TKB_KD) || !defined(TKB_V0) || !defined(TKB_VD)
@@ -577,12 +578,8 @@ TKB_EXPORT int tkb_attn_rows_tc(const void* q, void* out, const void* cache, int
   const int tq = BM / (nh / nkv);
   const long long tiles = n_tokens / tq + (long long)n_seqs;  // no step of this shape has more
   if (tiles > 65535) return -3;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(attn_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  static SharedMemoryRequest shared_memory;
+  if (const int rc = shared_memory({{(const void*)attn_rows_tc_kernel, SMEM_BYTES}})) return rc;
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   int tma_rows = 0;

@@ -28,6 +28,7 @@
 // Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 137 us (358);
 // three requests of 3,001 tokens in all 159 (383) and 200 us (513); 64 heads of 128 x 64 on 8 groups 242 us (455).
 #include "decay_chunks.cuh"
+#include "per_device.h"
 
 using namespace tkb;
 
@@ -635,15 +636,10 @@ __global__ void __launch_bounds__(THREADS) chunk_outputs_kernel(Args p) {
 template <int VDIM, bool VEC>
 int chunks_launch(const Args& p, int max_chunks, cudaStream_t st) {
   constexpr size_t smem1 = 3 * PLANE + 3 * C * (VDIM + 8) * 2, smem3 = OUT_SMEM;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(chunk_states_kernel<VDIM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(chunk_outputs_kernel<VDIM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
-  int rc = launch_pdl(chunk_states_kernel<VDIM, VEC>, dim3(max_chunks, p.heads), dim3(THREADS), smem1, st, p);
+  static SharedMemoryRequest shared_memory;
+  int rc = shared_memory({{(const void*)chunk_states_kernel<VDIM, VEC>, (int)smem1}, {(const void*)chunk_outputs_kernel<VDIM, VEC>, (int)smem3}});
+  if (rc) return rc;
+  rc = launch_pdl(chunk_states_kernel<VDIM, VEC>, dim3(max_chunks, p.heads), dim3(THREADS), smem1, st, p);
   if (rc) return rc;
   rc = launch_pdl(chunk_scan_kernel<VDIM, VEC>, dim3(p.n_seqs, p.heads, VDIM * DIM / 1024), dim3(256), 0, st, p);
   if (rc) return rc;

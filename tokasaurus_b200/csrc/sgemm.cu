@@ -23,6 +23,7 @@
 //   With enough row tiles to fill the GPU a block does all slices and adds them in the same order.
 //   Measured on B200 (the whole product): 4 rows x 16,384 x 2,048 633 us on the FP32 pipes, 44 us here
 //   (3.1 TB/s of weights); 500 rows the same 1,390 us, 250 us here (134 TFLOP/s of float32 products; the FP32 pipes have 74).
+#include "per_device.h"
 #include "tcgen05.cuh"
 
 namespace {
@@ -489,19 +490,16 @@ int chunks_a_slice(int N, int K) {
 template <int NT, bool VEC>
 int split_launch(const float* A, const float* W, float* C, float* part, int M, int N, int K, int lda, int ldw, int ldc,
                  int* status, cudaStream_t st) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(sgemm_split_kernel<NT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<NT>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  static SharedMemoryRequest shared_memory;
+  int rc = shared_memory({{(const void*)sgemm_split_kernel<NT, VEC>, SCfg<NT>::SMEM}});
+  if (rc) return rc;
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
   const dim3 block(SPLIT_THREADS);
   const int tiles = (N + 127) / 128, rows = (M + NT - 1) / NT;
   if (part == nullptr)
     return launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, 1), block, (size_t)SCfg<NT>::SMEM, st, A, W, C, M, N, K,
                       lda, ldw, ldc, per, slices, 0, status);
-  int rc = launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, slices), block, (size_t)SCfg<NT>::SMEM, st, A, W, part, M,
+  rc = launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, slices), block, (size_t)SCfg<NT>::SMEM, st, A, W, part, M,
                       N, K, lda, ldw, ldc, per, 1, 1, status);
   if (rc) return rc;
   return launch_pdl(sgemm_add_slices_kernel, dim3((N + 255) / 256, M), dim3(256), 0, st, (const float*)part, A, W, C, M, N, K,
