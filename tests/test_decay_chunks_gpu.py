@@ -240,3 +240,28 @@ def test_chunks_of_the_forgetting_recurrence_not_finite(vdim, value, monkeypatch
         assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
         fine = want.isfinite()
         assert near(got[fine], want[fine])
+
+
+@pytest.mark.parametrize("form,heads,groups", [("head", 2, 1), ("token", 2, 2), ("channel", 2, 2)])
+@pytest.mark.parametrize("size", [1e-35, 1e-38, 1e27, 1e33])
+def test_chunks_far_from_one(form, heads, groups, size, monkeypatch):
+    """Values and states close to the smallest normal number, and so large that a cut number does not hold them: no less exact than the
+    walk."""
+    from tokasaurus_b200.kernels import ops
+
+    lens = [260]
+    p, state, _ = problem(form, heads, groups, 128, lens, 5)
+    p["v"], state = p["v"] * size, state * size
+    out, st = run(p, state, lens, heads, groups, 128)
+    monkeypatch.setattr(ops, "DECAY_CHUNKS_FROM", 1 << 30)
+    walked, wst = run(p, state, lens, heads, groups, 128)
+    # the walk at another size by a power of two, where nothing under- or overflows
+    up = 2.0 ** (100 if size < 1 else -100)
+    p["v"], big = p["v"] * up, state * up
+    ref, rst = run(p, big, lens, heads, groups, 128)
+    monkeypatch.undo()
+    n = heads * 128 * 128
+    for got, walk, want in ((out, walked, ref), (st[0, :n], wst[0, :n], rst[0, :n])):
+        want = want.double() / up
+        err = lambda x: float((x.double() - want).norm() / want.norm())  # noqa: E731
+        assert got.isfinite().all() and err(got) <= 1.5 * err(walk) + 16 * 2.0 ** -24

@@ -115,3 +115,19 @@ def test_split_product_knows_the_step_s_status(M, N, K, monkeypatch):
     ops.linear(a, w)
     assert seen == [None, status.data_ptr(), None, status.data_ptr(), None]
     assert int(status) == 0 and torch.equal(out, ops.linear(a, w))
+
+
+@pytest.mark.parametrize("M,N", [(3, 256), (130, 20000)])
+@pytest.mark.parametrize("small,large", [(1e-36, 1.0), (1e-40, 1e8), (1e-44, 1e14), (1e-30, 1e-6), (1e30, 1e4), (1e33, 1e-20), (1e-12, 1e12)])
+def test_split_product_far_from_one(M, N, small, large):
+    """All bits of numbers of every size: close to the smallest normal number, below it (where few bits are), and so large that they
+    do not fit the cut form."""
+    g = torch.Generator().manual_seed(9)
+    a = (torch.randn(M, 300, generator=g, dtype=torch.float64) * small).float().to(DEV)
+    w = (torch.randn(N, 300, generator=g, dtype=torch.float64) * large).float().to(DEV)
+    for x, y in ((a, w), (w[:200].contiguous(), torch.cat([a, a[:1].expand(200, -1)]).contiguous())):  # small tokens, then small weights
+        out = product(x, y)
+        want = x.double() @ y.double().T
+        # as for numbers around one, and half a unit of the smallest number for a result that is one
+        bound = 64 * 2.0 ** -24 * (x.abs().double() @ y.abs().double().T) + 2.0 ** -149
+        assert ((out.double() - want).abs() <= bound).all()

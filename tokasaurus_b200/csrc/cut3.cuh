@@ -1,0 +1,36 @@
+// A float32 number as three bfloat16 numbers, for products on the bfloat16 tensor instructions (sgemm.cu, decay_chunks.cu):
+//     x 2^24 = h + m + l, 8 bits each, rounded to nearest.
+// The power of two keeps all 24 bits of every number below 2^104, subnormal ones too: the lowest bit that a float32 number can have,
+// 2^-149, is 2^-125 here, and the pieces, all of which are multiples of it, are no subnormal numbers.  (Cut as they are, numbers
+// below 2^-109 lost bits of their third piece.)  From 2^104 on h is an infinity and a NaN follows: results that are not finite are
+// made again by other means.  Sums of products come back by CUT_BACK, in the fused multiply-add that takes them.
+#pragma once
+#include "common.cuh"
+
+namespace tkb {
+
+constexpr float CUT_SCALE = 16777216.f;                       // 2^24
+constexpr float CUT_BACK = 1.f / (CUT_SCALE * CUT_SCALE);     // 2^-48
+
+__device__ __forceinline__ uint32_t cut_pack(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// Two neighbouring numbers.
+__device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  a *= CUT_SCALE;
+  b *= CUT_SCALE;
+  h = cut_pack(a, b);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  m = cut_pack(ra, rb);
+  l = cut_pack(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+}
+// Eight numbers -> three 16-byte pieces.
+__device__ __forceinline__ void cut8(const float4& x, const float4& y, uint4& h, uint4& m, uint4& l) {
+  cut2(x.x, x.y, h.x, m.x, l.x);
+  cut2(x.z, x.w, h.y, m.y, l.y);
+  cut2(y.x, y.y, h.z, m.z, l.z);
+  cut2(y.z, y.w, h.w, m.w, l.w);
+}
+
+}  // namespace tkb

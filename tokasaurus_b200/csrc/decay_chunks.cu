@@ -16,7 +16,7 @@
 // take q decayed from its block's start, k decayed to its block's end and the product of the blocks between, and A's diagonal
 // blocks are summed on the FP32 pipes with the product running along.  So nothing overflows, and what underflows is zero.
 //
-// Precision: every float32 operand of a product is cut into three bfloat16 numbers (x = h + m + l, all 24 bits) when it
+// Precision: every float32 operand of a product is cut into three bfloat16 numbers (all 24 bits: cut3.cuh) when it
 // comes into shared memory, and six products are kept (what is left out is below 2^-24 of a term).  The tensor instructions
 // (mma.sync m16n8k16) cut their sums off instead of rounding them, so a chain of the six for 16 terms starts from zero, the
 // small ones first, and its result is added to the float32 sum with an ordinary addition.
@@ -27,6 +27,7 @@
 // states' traffic of 32, and the products inside a chunk are still a third of the work.
 // Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 137 us (358);
 // three requests of 3,001 tokens in all 159 (383) and 200 us (513); 64 heads of 128 x 64 on 8 groups 242 us (455).
+#include "cut3.cuh"
 #include "decay_chunks.cuh"
 #include "per_device.h"
 
@@ -83,28 +84,16 @@ __device__ __forceinline__ bool find_chunk(const Args& p, int id, int& seq, int&
 }
 
 // ------------------------------------------------- products of float32 operands on the bfloat16 tensor instructions
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-  h = pack2(a, b);
-  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-  m = pack2(ra, rb);
-  l = pack2(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
-}
 // Eight numbers into the three planes (p: 16-byte aligned place in the first).
 __device__ __forceinline__ void put8(unsigned char* p, int plane, const float4& x, const float4& y) {
   uint4 h, m, l;
-  cut2(x.x, x.y, h.x, m.x, l.x);
-  cut2(x.z, x.w, h.y, m.y, l.y);
-  cut2(y.x, y.y, h.z, m.z, l.z);
-  cut2(y.z, y.w, h.w, m.w, l.w);
+  cut8(x, y, h, m, l);
   *reinterpret_cast<uint4*>(p) = h;
   *reinterpret_cast<uint4*>(p + plane) = m;
   *reinterpret_cast<uint4*>(p + 2 * plane) = l;
 }
 __device__ __forceinline__ void put1(unsigned char* p, int plane, float x) {
+  x *= CUT_SCALE;
   const __nv_bfloat16 h = __float2bfloat16_rn(x);
   const float r = x - __bfloat162float(h);
   const __nv_bfloat16 m = __float2bfloat16_rn(r);
@@ -170,7 +159,7 @@ __device__ __forceinline__ void step16(float (&acc)[MT][NT][4], uint32_t a, int 
 #pragma unroll
     for (int j = 0; j < NT; j++)
 #pragma unroll
-      for (int e = 0; e < 4; e++) acc[i][j][e] += x[i][j][e];
+      for (int e = 0; e < 4; e++) acc[i][j][e] = fmaf(x[i][j][e], CUT_BACK, acc[i][j][e]);
 }
 template <int MT, int NT> __device__ __forceinline__ void zero(float (&acc)[MT][NT][4]) {
 #pragma unroll

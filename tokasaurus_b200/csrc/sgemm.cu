@@ -7,14 +7,14 @@
 // sgemm_tn_kernel (N or K below 128: matrices for which a block of the other kernel has next to nothing to do): the FP32
 //   pipes, each element one sequential FMA chain over K in index order.
 //
-// sgemm_split_kernel (everything else): the tensor cores with every float32 number cut into three bfloat16 numbers
-//   (x = h + m + l, 8 bits each, rounded to nearest: the three hold all 24 bits).  Of the nine products the six down to
+// sgemm_split_kernel (everything else): the tensor cores with every float32 number cut into three bfloat16 numbers, h, m and l, that
+//   hold all 24 bits (cut3.cuh).  Of the nine products the six down to
 //   2^-16 of the largest are kept (hh; hm, mh, mm, hl, lh); what is left out is below 2^-24 of a term.  The tensor cores' sums
 //   are not rounded to nearest, so they are kept short: hh and the five small ones have accumulators of their own in tensor
 //   memory, and every 128 terms both are read and added to a float32 register with ordinary additions.  Measured against 64
 //   bits the result is closer than an FMA chain's (normal numbers, K = 2,048 and 8,192: relative error 1.4e-7 and 1.5e-7).
-//   An element that does not come out finite (an infinity, a NaN or an overflow among its inputs: 0 times infinity in a cut
-//   form is not what it is uncut) is done once more as the FMA chain, by the warp that has it (redo).
+//   An element that does not come out finite (an infinity, a NaN or a number from 2^104 on among its inputs: 0 times infinity in a
+//   cut form is not what it is uncut; or a sum from 2^80 on) is done once more as the FMA chain, by the warp that has it (redo).
 //   What bounds it: with many rows the tensor instructions (six products: a sixth of their rate is the bound) and their
 //   operands' way through shared memory, with few the weights' way from memory.  A block is 15 warps that fetch, cut and
 //   store (the next chunks on their way into registers meanwhile) and one that issues the tensor instructions; all 16 read
@@ -24,6 +24,7 @@
 //   Measured on B200 (the whole product): 4 rows x 16,384 x 2,048 633 us on the FP32 pipes, 44 us here
 //   (3.1 TB/s of weights); 500 rows the same 1,390 us, 250 us here (134 TFLOP/s of float32 products; the FP32 pipes have 74).
 #include "per_device.h"
+#include "cut3.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -145,22 +146,6 @@ template <> __device__ __forceinline__ void tmem_read<32>(uint32_t a, float (&v)
   tmem_ld32(a, r);
 #pragma unroll
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
-
-// Eight numbers of a row -> three 16-byte pieces: x = h + m + l.
-__device__ __forceinline__ void cut8(const float4& x0, const float4& x1, uint4& h, uint4& m, uint4& l) {
-  const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-  uint32_t hh[4], mm[4], ll[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    hh[i] = pack_bf16(x[2 * i], x[2 * i + 1]);
-    const float r0 = x[2 * i] - __uint_as_float(hh[i] << 16), r1 = x[2 * i + 1] - __uint_as_float(hh[i] & 0xffff0000u);
-    mm[i] = pack_bf16(r0, r1);
-    ll[i] = pack_bf16(r0 - __uint_as_float(mm[i] << 16), r1 - __uint_as_float(mm[i] & 0xffff0000u));
-  }
-  h = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-  m = make_uint4(mm[0], mm[1], mm[2], mm[3]);
-  l = make_uint4(ll[0], ll[1], ll[2], ll[3]);
 }
 
 // Eight numbers from p on, of which `left` are there (p null: none).
@@ -320,10 +305,10 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     float v[CPT];
     tmem_read<CPT>(tmem_mine + buf * 2 * NT + NT, v);
 #pragma unroll
-    for (int i = 0; i < CPT; i++) acc[i] += v[i];
+    for (int i = 0; i < CPT; i++) acc[i] = fmaf(v[i], CUT_BACK, acc[i]);
     tmem_read<CPT>(tmem_mine + buf * 2 * NT, v);
 #pragma unroll
-    for (int i = 0; i < CPT; i++) acc[i] += v[i];
+    for (int i = 0; i < CPT; i++) acc[i] = fmaf(v[i], CUT_BACK, acc[i]);
     tcgen05_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(&acc_empty[buf]);
