@@ -49,3 +49,62 @@ def test_both_kernels_agree(dtype, hd, nh, nkv, window):
     last = 128 + 2 + 140 - 1
     keep = torch.arange(T, device=DEV) != last
     assert torch.equal(got[keep], out[keep]) and got[last].isnan().all()
+
+
+@pytest.mark.parametrize("hd,nh,nkv,window", [(64, 8, 2, None), (128, 6, 6, 200), (256, 10, 2, None)])
+@pytest.mark.parametrize("decoding,portion", [(5, 40), (1, 9), (70, 1100), (3, 2)])
+def test_requests_that_decode_beside_portions(hd, nh, nkv, window, decoding, portion):
+    """Steps of both: single tokens ahead of, between and behind portions, padding tokens at the end, more rows than a block scans at a
+    time, rows in another order; every row has the bits that it has alone."""
+    from tokasaurus_b200.kernels import ops
+
+    new = [portion] + [1] * decoding + [portion // 2 + 1, 1, 3]
+    lens = [n + 37 * (i % 11) * (n == 1) for i, n in enumerate(new)]
+    ps = 16
+    kc, vc, indptr, pages, K, V = make_paged(torch.float32, len(lens), lens, nkv, hd, ps, sum(-(-n // ps) for n in lens) + 2, seed=hd)
+    seq = [s for s, n in enumerate(new) for _ in range(n)]
+    pos = [lens[s] - n + i for s, n in enumerate(new) for i in range(n)]
+    token_seq, positions = i32(seq + [-1] * 5), i32(pos + [0] * 5)
+    T = len(seq)
+    q = torch.randn(T + 5, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(1)).to(DEV)
+
+    def run(rows, n):
+        out = torch.full((n, nh * hd), 9.0, device=DEV)
+        ops.attn_paged(q, q.shape[1], out, kc, vc, token_seq, positions, indptr, pages, rows, n, nh, nkv, hd, ps, 0.1, window)
+        return out
+
+    out = run(None, T + 5)
+    g = torch.Generator().manual_seed(2)
+    order = torch.randperm(T, generator=g).to(torch.int32)  # neighbours of other requests nearly everywhere
+    assert torch.equal(run(order.to(DEV), T), out[order.long().to(DEV)])
+    for t in [0, portion - 1, portion, portion + decoding - 1, T - 1, T - 4] + torch.randint(T, (6,), generator=g).tolist():
+        assert torch.equal(run(i32([t]), 1)[0], out[t])
+        want = plain_attention(q[t, : nh * hd].view(nh, hd).cpu(), K[seq[t]], V[seq[t]], pos[t], 0.1, window)
+        torch.testing.assert_close(out[t].view(nh, hd).cpu().double(), want, **tol(torch.float32), check_dtype=False)
+
+
+def test_requests_that_decode_do_not_wait_for_one_another():
+    """One kv head a head: 24 requests' contexts in one block were walked one after the other."""
+    from tokasaurus_b200.kernels import ops
+
+    nh, hd, ps, n, ctx, portion = 16, 128, 16, 24, 1500, 200
+    lens = [ctx] * n + [portion]
+    kc, vc, indptr, pages, _, _ = make_paged(torch.float32, n + 1, lens, nh, hd, ps, sum(-(-x // ps) for x in lens), seed=1)
+
+    def time(seqs, news):
+        seq = [s for s, k in zip(seqs, news) for _ in range(k)]
+        pos = [lens[s] - k + i for s, k in zip(seqs, news) for i in range(k)]
+        T = len(seq)
+        q, out = torch.randn(T, nh * hd, device=DEV), torch.empty(T, nh * hd, device=DEV)
+        args = (q, nh * hd, out, kc, vc, i32(seq), i32(pos), indptr, pages, None, T, nh, nh, hd, ps, 0.1, None)
+        ops.attn_paged(*args)
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        ev[0].record()
+        for _ in range(10):
+            ops.attn_paged(*args)
+        ev[1].record()
+        torch.cuda.synchronize()
+        return ev[0].elapsed_time(ev[1])
+
+    apart = time(range(n), [1] * n) + time([n], [portion])
+    assert time(range(n + 1), [1] * n + [portion]) < 2 * apart  # (was 12 times)

@@ -77,14 +77,20 @@ __device__ __forceinline__ float lane_sum(const float (&p)[TILES]) {
   return s;
 }
 
-// Steps of portions.  Grid: (blocks of `rows_a_block` rows, the last rows first; kv heads x head groups).
+// Row r's request (-1: padding), and whether r is its only row hereabouts: neither neighbour is of the same request.
+__device__ __forceinline__ int row_request(const int* token_seq, const int* rows, int r) { return token_seq[rows ? rows[r] : r]; }
+__device__ __forceinline__ bool lone_row(const int* token_seq, const int* rows, int r, int n_rows, int s) {
+  return (r == 0 || row_request(token_seq, rows, r - 1) != s) && (r + 1 == n_rows || row_request(token_seq, rows, r + 1) != s);
+}
+
+// Steps of portions.  skip_lone: the lone rows are the other kernel's.  Grid: (blocks of `rows_a_block` rows, the last rows first; kv heads x head groups).
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
 attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride, const T* __restrict__ kcache,
                  const T* __restrict__ vcache, const int* __restrict__ token_seq, const int* __restrict__ positions,
                  const int* __restrict__ page_indptr, const int* __restrict__ page_ids, const int* __restrict__ rows,
                  int n_rows, int nh, int nkv, int page_size, float scale_log2, int window, int num_pages,
-                 int* __restrict__ status, int rows_a_block, int heads_a_block) {
+                 int* __restrict__ status, int rows_a_block, int heads_a_block, int skip_lone) {
   extern __shared__ __align__(16) float smem[];
   float* qs = smem;                       // [PAIRS][HD]
   float* tile = qs + PAIRS * HD;          // [TILE][KROW]
@@ -101,7 +107,9 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
   const int nr = min(rows_a_block, n_rows - r0);
   for (int r = tid; r < PAIRS; r += ROW_THREADS) {
     const int t = r < nr ? (rows ? rows[r0 + r] : r0 + r) : 0;
-    row_seq[r] = r < nr ? token_seq[t] : -1;
+    int s = r < nr ? token_seq[t] : -1;
+    if (skip_lone && s >= 0 && lone_row(token_seq, rows, r0 + r, n_rows, s)) s = -1;
+    row_seq[r] = s;
     row_pos[r] = r < nr ? positions[t] : 0;
   }
   for (int i = tid; i < PAIRS * HD; i += ROW_THREADS) {
@@ -284,13 +292,41 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
   }
 }
 
-// Steps of single tokens.  Grid: (rows, kv heads x groups of four heads).
+// The `want`-th lone row (-1: there are fewer), by the whole block.
+__device__ __forceinline__ int find_lone_row(const int* token_seq, const int* rows, int n_rows, int want) {
+  __shared__ int counts[FEW_THREADS / 32], found;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) found = -1;
+  for (int r0 = 0; r0 < n_rows; r0 += FEW_THREADS) {
+    const int r = r0 + threadIdx.x, s = r < n_rows ? row_request(token_seq, rows, r) : -1;
+    const bool lone = s >= 0 && lone_row(token_seq, rows, r, n_rows, s);
+    const unsigned m = __ballot_sync(0xffffffffu, lone);
+    __syncthreads();
+    if (lane == 0) counts[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < FEW_THREADS / 32; w++) {
+      before += w < warp ? counts[w] : 0;
+      all += counts[w];
+    }
+    if (lone && before + __popc(m & ((1u << lane) - 1)) == want) found = r;
+    if (want < all) break;
+    want -= all;
+  }
+  __syncthreads();
+  const int r = found;
+  __syncthreads();
+  return r;
+}
+
+// Steps of single tokens, and (lone) the lone rows of a step that brings portions too.  Grid: (rows, kv heads x groups of four heads);
+// lone: (as many blocks as there are requests, which take turns, ...).
 template <typename T>
 __global__ void __launch_bounds__(FEW_THREADS)
 attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride, const T* __restrict__ kcache,
                 const T* __restrict__ vcache, const int* __restrict__ token_seq, const int* __restrict__ positions,
-                const int* __restrict__ page_indptr, const int* __restrict__ page_ids, const int* __restrict__ rows, int nh,
-                int nkv, int page_size, float scale_log2, int window, int num_pages, int* __restrict__ status) {
+                const int* __restrict__ page_indptr, const int* __restrict__ page_ids, const int* __restrict__ rows, int n_rows,
+                int nh, int nkv, int page_size, float scale_log2, int window, int num_pages, int* __restrict__ status, int lone) {
   __shared__ __align__(16) float qs[NQ][HD];
   __shared__ float sc[TEAMS][NQ][SEG];      // scores, then weights
   __shared__ float part[TEAMS][NQ][HD];     // a segment's sums
@@ -298,110 +334,115 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
   __shared__ long long offs[TEAMS][SEG];
   trigger_dependents();
   grid_dependency_wait();
-  const int t = rows ? rows[blockIdx.x] : blockIdx.x;
-  const int s = token_seq[t];
-  if (s < 0) return;
-  const int p = positions[t];
-  const int group = nh / nkv, splits = (group + NQ - 1) / NQ;
-  const int kvh = blockIdx.y / splits, h0 = kvh * group + (blockIdx.y % splits) * NQ;
-  const int heads = min(NQ, (kvh + 1) * group - h0);
-  const int tid = threadIdx.x, lane = tid & 31, team = tid >> 7, member = (tid >> 5) & 3;
-  const int* table = page_ids + page_indptr[s];
-  const int lo = window > 0 ? max(0, p - window + 1) : 0;
-  for (int i = tid; i < NQ * HD; i += FEW_THREADS) {
-    const int h = i / HD, d = i - h * HD;
-    qs[h][d] = h < heads ? to_float(q[(size_t)t * q_stride + (size_t)(h0 + h) * HD + d]) * scale_log2 : 0.f;
-  }
-  constexpr int MINE = (NQ * HD + FEW_THREADS - 1) / FEW_THREADS;  // output elements a thread merges
-  float M[MINE], L[MINE], O[MINE];
+  for (int turn = blockIdx.x;; turn += gridDim.x) {
+    const int row = lone ? find_lone_row(token_seq, rows, n_rows, turn) : turn;
+    if (row < 0) return;
+    const int t = rows ? rows[row] : row;
+    const int s = token_seq[t];
+    if (s < 0) return;
+    const int p = positions[t];
+    const int group = nh / nkv, splits = (group + NQ - 1) / NQ;
+    const int kvh = blockIdx.y / splits, h0 = kvh * group + (blockIdx.y % splits) * NQ;
+    const int heads = min(NQ, (kvh + 1) * group - h0);
+    const int tid = threadIdx.x, lane = tid & 31, team = tid >> 7, member = (tid >> 5) & 3;
+    const int* table = page_ids + page_indptr[s];
+    const int lo = window > 0 ? max(0, p - window + 1) : 0;
+    for (int i = tid; i < NQ * HD; i += FEW_THREADS) {
+      const int h = i / HD, d = i - h * HD;
+      qs[h][d] = h < heads ? to_float(q[(size_t)t * q_stride + (size_t)(h0 + h) * HD + d]) * scale_log2 : 0.f;
+    }
+    constexpr int MINE = (NQ * HD + FEW_THREADS - 1) / FEW_THREADS;  // output elements a thread merges
+    float M[MINE], L[MINE], O[MINE];
 #pragma unroll
-  for (int i = 0; i < MINE; i++) M[i] = -FLT_MAX, L[i] = 0.f, O[i] = 0.f;
+    for (int i = 0; i < MINE; i++) M[i] = -FLT_MAX, L[i] = 0.f, O[i] = 0.f;
 
-  for (int round = lo / SEG; round <= p / SEG; round += TEAMS) {
-    const int base = (round + team) * SEG;
-    {
-      const int j = tid & (SEG - 1), key = base + j;
-      const bool live = key >= lo && key <= p;
-      const long long at = live ? key_at(table, key, kvh, nkv, page_size, num_pages, status) : -1;
-      offs[team][j] = at;
-      __syncthreads();  // (the queries are in place; the round before has been merged)
-      float x[NQ] = {0.f, 0.f, 0.f, 0.f};
-      if (at >= 0) {
-        const T* k = kcache + at;
+    for (int round = lo / SEG; round <= p / SEG; round += TEAMS) {
+      const int base = (round + team) * SEG;
+      {
+        const int j = tid & (SEG - 1), key = base + j;
+        const bool live = key >= lo && key <= p;
+        const long long at = live ? key_at(table, key, kvh, nkv, page_size, num_pages, status) : -1;
+        offs[team][j] = at;
+        __syncthreads();  // (the queries are in place; the round before has been merged)
+        float x[NQ] = {0.f, 0.f, 0.f, 0.f};
+        if (at >= 0) {
+          const T* k = kcache + at;
 #pragma unroll 8
-        for (int i = 0; i < HD / 4; i++) {
-          const float4 kk = load4(k + 4 * i);
+          for (int i = 0; i < HD / 4; i++) {
+            const float4 kk = load4(k + 4 * i);
 #pragma unroll
-          for (int a = 0; a < NQ; a++) {
-            const float4 qq = *reinterpret_cast<const float4*>(&qs[a][4 * i]);
-            x[a] = fmaf(kk.x, qq.x, x[a]);
-            x[a] = fmaf(kk.y, qq.y, x[a]);
-            x[a] = fmaf(kk.z, qq.z, x[a]);
-            x[a] = fmaf(kk.w, qq.w, x[a]);
+            for (int a = 0; a < NQ; a++) {
+              const float4 qq = *reinterpret_cast<const float4*>(&qs[a][4 * i]);
+              x[a] = fmaf(kk.x, qq.x, x[a]);
+              x[a] = fmaf(kk.y, qq.y, x[a]);
+              x[a] = fmaf(kk.z, qq.z, x[a]);
+              x[a] = fmaf(kk.w, qq.w, x[a]);
+            }
           }
         }
+#pragma unroll
+        for (int a = 0; a < NQ; a++) sc[team][a][j] = at >= 0 ? x[a] : -FLT_MAX;
       }
+      __syncthreads();
+      if (member < heads) {  // a warp a head
+        float w[TILES];
 #pragma unroll
-      for (int a = 0; a < NQ; a++) sc[team][a][j] = at >= 0 ? x[a] : -FLT_MAX;
-    }
-    __syncthreads();
-    if (member < heads) {  // a warp a head
-      float w[TILES];
+        for (int u = 0; u < TILES; u++) w[u] = sc[team][member][u * TILE + lane];
+        float top = w[0];
 #pragma unroll
-      for (int u = 0; u < TILES; u++) w[u] = sc[team][member][u * TILE + lane];
-      float top = w[0];
+        for (int u = 1; u < TILES; u++) top = fmaxf(top, w[u]);
+        const float m = warp_max(fmaxf(top, -FLT_MAX));
 #pragma unroll
-      for (int u = 1; u < TILES; u++) top = fmaxf(top, w[u]);
-      const float m = warp_max(fmaxf(top, -FLT_MAX));
+        for (int u = 0; u < TILES; u++) {
+          w[u] = offs[team][u * TILE + lane] >= 0 ? exp2f(w[u] - m) : 0.f;
+          sc[team][member][u * TILE + lane] = w[u];
+        }
+        const float l = warp_sum(lane_sum(w));
+        __syncwarp();
+        float o[DPL];
 #pragma unroll
-      for (int u = 0; u < TILES; u++) {
-        w[u] = offs[team][u * TILE + lane] >= 0 ? exp2f(w[u] - m) : 0.f;
-        sc[team][member][u * TILE + lane] = w[u];
-      }
-      const float l = warp_sum(lane_sum(w));
-      __syncwarp();
-      float o[DPL];
-#pragma unroll
-      for (int i = 0; i < DPL; i++) o[i] = 0.f;
-      const int j0 = max(0, lo - base), j1 = min(SEG - 1, p - base);
+        for (int i = 0; i < DPL; i++) o[i] = 0.f;
+        const int j0 = max(0, lo - base), j1 = min(SEG - 1, p - base);
 #pragma unroll 16
-      for (int j = j0; j <= j1; j++) {
-        const long long at = offs[team][j];
-        const float pj = sc[team][member][j];
+        for (int j = j0; j <= j1; j++) {
+          const long long at = offs[team][j];
+          const float pj = sc[team][member][j];
 #pragma unroll
-        for (int i = 0; i < DPL; i++) {
-          const float v = at >= 0 && lane + 32 * i < HD ? to_float(vcache[at + lane + 32 * i]) : 0.f;
-          o[i] = fmaf(pj, v, o[i]);
+          for (int i = 0; i < DPL; i++) {
+            const float v = at >= 0 && lane + 32 * i < HD ? to_float(vcache[at + lane + 32 * i]) : 0.f;
+            o[i] = fmaf(pj, v, o[i]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < DPL; i++)
+          if (lane + 32 * i < HD) part[team][member][lane + 32 * i] = o[i];
+        if (lane == 0) {
+          seg_m[team][member] = m;
+          seg_l[team][member] = l;
         }
       }
+      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < DPL; i++)
-        if (lane + 32 * i < HD) part[team][member][lane + 32 * i] = o[i];
-      if (lane == 0) {
-        seg_m[team][member] = m;
-        seg_l[team][member] = l;
+      for (int i = 0; i < MINE; i++) {
+        const int e = tid + i * FEW_THREADS, h = e / HD, d = e - h * HD;
+        if (h >= heads) continue;
+        for (int u = 0; u < TEAMS; u++) {
+          const float l = seg_l[u][h];
+          if (l == 0.f) continue;  // no key of this segment
+          float keep, take;
+          merge_factors(M[i], L[i], seg_m[u][h], l, keep, take);
+          O[i] = fmaf(O[i], keep, part[u][h][d] * take);
+        }
       }
     }
-    __syncthreads();
 #pragma unroll
     for (int i = 0; i < MINE; i++) {
       const int e = tid + i * FEW_THREADS, h = e / HD, d = e - h * HD;
       if (h >= heads) continue;
-      for (int u = 0; u < TEAMS; u++) {
-        const float l = seg_l[u][h];
-        if (l == 0.f) continue;  // no key of this segment
-        float keep, take;
-        merge_factors(M[i], L[i], seg_m[u][h], l, keep, take);
-        O[i] = fmaf(O[i], keep, part[u][h][d] * take);
-      }
+      const float inv = L[i] == 0.f ? 0.f : 1.f / L[i];
+      out[(size_t)row * out_stride + (size_t)(h0 + h) * HD + d] = from_float<T>(O[i] * inv);
     }
-  }
-#pragma unroll
-  for (int i = 0; i < MINE; i++) {
-    const int e = tid + i * FEW_THREADS, h = e / HD, d = e - h * HD;
-    if (h >= heads) continue;
-    const float inv = L[i] == 0.f ? 0.f : 1.f / L[i];
-    out[(size_t)blockIdx.x * out_stride + (size_t)(h0 + h) * HD + d] = from_float<T>(O[i] * inv);
+    if (!lone) return;
   }
 }
 
@@ -415,13 +456,18 @@ int attn_launch(const void* q, int q_stride, void* out, int out_stride, const vo
   const int group = nh / nkv;
   const float scale_log2 = scale * 1.4426950408889634f;
   // Up to two rows a request: a block of its own for every row.  (Both kernels give the same bits, so the line may lie
-  // anywhere; blocks of several tokens pay from about four tokens of a request on.)
-  if (n_rows <= 2 * (long long)n_seqs) {
+  // anywhere; blocks of several tokens pay from about four tokens of a request on.)  More, of several requests: a block of its own
+  // for the rows that stand alone (requests that decode while prompts come in), and blocks of several rows for the others, which
+  // would otherwise walk the lone rows' contexts one after the other.  Measured on B200, a layer of 16 heads of 128, 24 requests
+  // that decode at contexts of up to 1,500 beside a portion of 200 tokens: @@ us with the lone rows in blocks of several.
+  const bool few = n_rows <= 2 * (long long)n_seqs, lone = !few && n_seqs > 1;
+  if (few || lone) {
     const long long y = (long long)nkv * ((group + NQ - 1) / NQ);
     if (y > 65535) return -3;
-    return launch_pdl(attn_few_kernel<T>, dim3(n_rows, (unsigned)y), dim3(FEW_THREADS), 0, st, (const T*)q, q_stride, (T*)out,
-                      out_stride, (const T*)kcache, (const T*)vcache, token_seq, positions, page_indptr, page_ids, rows, nh,
-                      nkv, page_size, scale_log2, window, num_pages, status);
+    const int rc = launch_pdl(attn_few_kernel<T>, dim3(few ? n_rows : n_seqs, (unsigned)y), dim3(FEW_THREADS), 0, st, (const T*)q,
+                              q_stride, (T*)out, out_stride, (const T*)kcache, (const T*)vcache, token_seq, positions, page_indptr,
+                              page_ids, rows, n_rows, nh, nkv, page_size, scale_log2, window, num_pages, status, lone ? 1 : 0);
+    if (rc != 0 || few) return rc;
   }
   const int heads_a_block = group < PAIRS ? group : PAIRS, rows_a_block = PAIRS / heads_a_block;
   const long long y = (long long)nkv * ((group + heads_a_block - 1) / heads_a_block);
@@ -434,7 +480,7 @@ int attn_launch(const void* q, int q_stride, void* out, int out_stride, const vo
   return launch_pdl(attn_rows_kernel<T>, dim3((n_rows + rows_a_block - 1) / rows_a_block, (unsigned)y), dim3(ROW_THREADS), smem,
                     st, (const T*)q, q_stride, (T*)out, out_stride, (const T*)kcache, (const T*)vcache, token_seq, positions,
                     page_indptr, page_ids, rows, n_rows, nh, nkv, page_size, scale_log2, window, num_pages, status,
-                    rows_a_block, heads_a_block);
+                    rows_a_block, heads_a_block, lone ? 1 : 0);
 }
 
 }  // namespace
