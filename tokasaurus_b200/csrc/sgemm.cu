@@ -231,14 +231,18 @@ __device__ __noinline__ void redo_tile(const float* __restrict__ A, const float*
   const int n = blockIdx.x * 128 + (threadIdx.x & 127), m = blockIdx.y * NT + (threadIdx.x >> 7) * CPT;
   redo<8, 32>(C + (size_t)m * ldc + n, ldc, min(CPT, M - m), n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, VEC);
 }
-__device__ __noinline__ void redo_row(const float* __restrict__ A, const float* __restrict__ W, float* C, int N, int K, int lda, int ldw,
-                                      int ldc, int vec) {
-  const int n = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
-  redo<1, 16>(C + (size_t)m * ldc + n, ldc, 1, n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, vec);
-}
-
 // What a block leaves in the place of its results when one of its waits ran out (a NaN of its own: no arithmetic makes it).
 constexpr int LOST = 0x7fc0105e;
+
+__device__ __noinline__ void redo_row(const float* __restrict__ part, const float* __restrict__ A, const float* __restrict__ W, float* C,
+                                      int M, int N, int K, int lda, int ldw, int ldc, int slices, int vec) {
+  const int n = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
+  // (what a wait that ran out left stays a NaN: it has been reported, and is no number's doing)
+  bool lost = false;
+  for (int s = 0; s < slices; s++) lost |= n < N && __float_as_int(part[((size_t)s * M + m) * N + n]) == LOST;
+  if (__any_sync(0xffffffffu, lost)) return;
+  redo<1, 16>(C + (size_t)m * ldc + n, ldc, 1, n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, vec);
+}
 
 // out: C when a block does all slices (`slices_here`), else the slices' partial results [slice][M][N].
 template <int NT, bool VEC>
@@ -378,23 +382,19 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     }
   } else {
     // ---------------- fetch, cut, store: pieces of 8 numbers, eight threads a row of the chunk
-    const float* src[TASKS];
-    uint32_t dst[TASKS];
+    // (a piece's place and where it goes are worked out where they are wanted: what is kept across the loop is short of registers)
     float4 x[AHEAD][TASKS][2];
-    const int seg = tid & 7, k0 = c_begin * CHUNK + seg * 8;
-#pragma unroll
-    for (int i = 0; i < TASKS; i++) {
-      const int r = (tid - 32 + i * CONVERTERS) >> 3;
-      src[i] = nullptr;
-      if (r < 128 && n0 + r < N) src[i] = W + (size_t)(n0 + r) * ldw + k0;
-      if (r >= 128 && r < 128 + NT && m0 + r - 128 < M) src[i] = A + (size_t)(m0 + r - 128) * lda + k0;
-      dst[i] = r < 128 + NT ? r * 128 + ((seg ^ (r & 7)) << 4) : 0xffffffffu;
-    }
+    const int seg = tid & 7, k0 = c_begin * CHUNK + seg * 8, r0 = (tid - 32) >> 3;
+    constexpr int ROWS = CONVERTERS / 8;  // rows between a thread's pieces
     auto fetch = [&](int c, int into) {
-      const int left = c < n_chunks ? K - k0 - c * CHUNK : 0;
+      const int k = k0 + c * CHUNK, left = c < n_chunks ? K - k : 0;
 #pragma unroll
-      for (int i = 0; i < TASKS; i++)
-        fetch8<VEC>(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
+      for (int i = 0; i < TASKS; i++) {
+        const int r = r0 + i * ROWS;
+        const bool is_w = r < 128, there = is_w ? n0 + r < N : r < 128 + NT && m0 + r - 128 < M;
+        const float* p = (is_w ? W + (size_t)(n0 + r) * ldw : A + (size_t)(m0 + r - 128) * lda) + k;
+        fetch8<VEC>(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
+      }
     };
 #pragma unroll
     for (int u = 0; u < AHEAD; u++) fetch(u, u);
@@ -408,12 +408,13 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
         unsigned char* st = planes + s * Z::STAGE;
 #pragma unroll
         for (int i = 0; i < TASKS; i++) {
-          if (dst[i] == 0xffffffffu) continue;
+          const int r = r0 + i * ROWS, dst = r * 128 + ((seg ^ (r & 7)) << 4);
+          if (r >= 128 + NT) continue;
           uint4 h, m, l;
           cut8(x[u][i][0], x[u][i][1], h, m, l);
-          *reinterpret_cast<uint4*>(st + dst[i]) = h;
-          *reinterpret_cast<uint4*>(st + dst[i] + Z::PLANE) = m;
-          *reinterpret_cast<uint4*>(st + dst[i] + 2 * Z::PLANE) = l;
+          *reinterpret_cast<uint4*>(st + dst) = h;
+          *reinterpret_cast<uint4*>(st + dst + Z::PLANE) = m;
+          *reinterpret_cast<uint4*>(st + dst + 2 * Z::PLANE) = l;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -447,7 +448,7 @@ sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict_
   grid_dependency_wait();
   const int m = blockIdx.y;
   const int n = blockIdx.x * 256 + threadIdx.x;
-  bool odd = false, lost = false;
+  bool odd = false;
   if (n < N) {
     const float* p = part + (size_t)m * N + n;
     const size_t stride = (size_t)M * N;
@@ -456,11 +457,8 @@ sgemm_add_slices_kernel(const float* __restrict__ part, const float* __restrict_
     for (int s = 1; s < slices; s++) v += p[s * stride];
     C[(size_t)m * ldc + n] = v;
     odd = !isfinite(v);
-    if (odd)
-      for (int s = 0; s < slices; s++) lost |= __float_as_int(p[s * stride]) == LOST;
   }
-  // (what a wait that ran out left stays a NaN: it has been reported, and is no number's doing)
-  if (__any_sync(0xffffffffu, odd) && !__any_sync(0xffffffffu, lost)) redo_row(A, W, C, N, K, lda, ldw, ldc, vec);
+  if (__any_sync(0xffffffffu, odd)) redo_row(part, A, W, C, M, N, K, lda, ldw, ldc, slices, vec);
 }
 
 // Chunks of K a slice holds, by N and K alone: as many slices as bring the blocks of one row tile to the SMs' number.
