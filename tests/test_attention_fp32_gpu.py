@@ -108,3 +108,20 @@ def test_requests_that_decode_do_not_wait_for_one_another():
 
     apart = time(range(n), [1] * n) + time([n], [portion])
     assert time(range(n + 1), [1] * n + [portion]) < 2 * apart  # (was 12 times)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 8, 2), (256, 10, 2), (16, 40, 1)])
+@pytest.mark.parametrize("new,pad", [([1, 1], 2), ([1, 9, 1], 5), ([40], 24), ([200, 1, 2], 53)])
+def test_rows_of_padding_tokens_are_zero(dtype, hd, nh, nkv, new, pad):
+    """A step graph's padding tokens: memory that nobody wrote (here NaN) does not go into the products behind."""
+    from tokasaurus_b200.kernels import ops
+
+    kc, vc, indptr, pages, _, _ = make_paged(dtype, len(new), new, nkv, hd, 16, 40, seed=1)
+    seq = [s for s, n in enumerate(new) for _ in range(n)]
+    token_seq, positions = i32(seq + [-1] * pad), i32([i for n in new for i in range(n)] + [0] * pad)
+    T = len(seq)
+    q = torch.randn(T + pad, nh * hd, generator=torch.Generator().manual_seed(1)).to(dtype).to(DEV)
+    out = torch.full((T + pad, nh * hd), math.nan, dtype=dtype, device=DEV)
+    ops.attn_paged(q, q.shape[1], out, kc, vc, token_seq, positions, indptr, pages, None, T + pad, nh, nkv, hd, 16, 0.1, None)
+    assert (out[T:] == 0).all() and out[:T].isfinite().all()

@@ -83,7 +83,10 @@ __device__ __forceinline__ bool lone_row(const int* token_seq, const int* rows, 
   return (r == 0 || row_request(token_seq, rows, r - 1) != s) && (r + 1 == n_rows || row_request(token_seq, rows, r + 1) != s);
 }
 
-// Steps of portions.  skip_lone: the lone rows are the other kernel's.  Grid: (blocks of `rows_a_block` rows, the last rows first; kv heads x head groups).
+constexpr int LONE = INT_MIN;  // in the place of a lone row's request
+
+// Steps of portions.  skip_lone: the lone rows are the other kernel's.  Grid: (blocks of `rows_a_block` rows, the last rows first;
+// kv heads x head groups).
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
 attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride, const T* __restrict__ kcache,
@@ -105,10 +108,12 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
   const int heads = min(heads_a_block, (kvh + 1) * group - h0);
   const int r0 = (gridDim.x - 1 - blockIdx.x) * rows_a_block;
   const int nr = min(rows_a_block, n_rows - r0);
+  bool padding = false;
   for (int r = tid; r < PAIRS; r += ROW_THREADS) {
     const int t = r < nr ? (rows ? rows[r0 + r] : r0 + r) : 0;
     int s = r < nr ? token_seq[t] : -1;
-    if (skip_lone && s >= 0 && lone_row(token_seq, rows, r0 + r, n_rows, s)) s = -1;
+    padding |= r < nr && s < 0;
+    if (skip_lone && s >= 0 && lone_row(token_seq, rows, r0 + r, n_rows, s)) s = LONE;
     row_seq[r] = s;
     row_pos[r] = r < nr ? positions[t] : 0;
   }
@@ -121,7 +126,12 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
     }
     qs[i] = v;
   }
-  __syncthreads();
+  if (__syncthreads_or(padding)) {  // a step graph's padding: zeros, which the products behind take for any other row
+    for (int i = tid; i < nr * heads * HD; i += ROW_THREADS) {
+      const int r = i / (heads * HD), c = i - r * heads * HD;
+      if (row_seq[r] < 0 && row_seq[r] != LONE) out[(size_t)(r0 + r) * out_stride + (size_t)h0 * HD + c] = from_float<T>(0.f);
+    }
+  }
 
   // rows of one request at a time (nearly always all of a block's)
   for (int first = 0; first < nr; first++) {
@@ -339,12 +349,15 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
     if (row < 0) return;
     const int t = rows ? rows[row] : row;
     const int s = token_seq[t];
-    if (s < 0) return;
-    const int p = positions[t];
     const int group = nh / nkv, splits = (group + NQ - 1) / NQ;
     const int kvh = blockIdx.y / splits, h0 = kvh * group + (blockIdx.y % splits) * NQ;
     const int heads = min(NQ, (kvh + 1) * group - h0);
     const int tid = threadIdx.x, lane = tid & 31, team = tid >> 7, member = (tid >> 5) & 3;
+    if (s < 0) {  // a step graph's padding: zeros, which the products behind take for any other row
+      for (int i = tid; i < heads * HD; i += FEW_THREADS) out[(size_t)row * out_stride + (size_t)h0 * HD + i] = from_float<T>(0.f);
+      return;
+    }
+    const int p = positions[t];
     const int* table = page_ids + page_indptr[s];
     const int lo = window > 0 ? max(0, p - window + 1) : 0;
     for (int i = tid; i < NQ * HD; i += FEW_THREADS) {
@@ -486,7 +499,8 @@ int attn_launch(const void* q, int q_stride, void* out, int out_stride, const vo
 }  // namespace
 
 // q: [tokens, q_stride] with head h at column h*HD; out: [n_rows, out_stride].  `rows` (nullable)
-// names the tokens whose output is wanted; row r of `out` belongs to token rows[r].  n_seqs: requests in the step (or any
+// names the tokens whose output is wanted; row r of `out` belongs to token rows[r] (zeros for a padding token, whose request is
+// below zero).  n_seqs: requests in the step (or any
 // number: it only chooses between two kernels with the same results).  num_pages, status: a page id
 // beyond the pool sets the status flag and its keys count for nothing (num_pages <= 0: not checked).
 TKB_EXPORT int tkb_attn_paged_simt_f32(const void* q, int q_stride, void* out, int out_stride, const void* kcache,
