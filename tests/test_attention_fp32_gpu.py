@@ -125,3 +125,31 @@ def test_rows_of_padding_tokens_are_zero(dtype, hd, nh, nkv, new, pad):
     out = torch.full((T + pad, nh * hd), math.nan, dtype=dtype, device=DEV)
     ops.attn_paged(q, q.shape[1], out, kc, vc, token_seq, positions, indptr, pages, None, T + pad, nh, nkv, hd, 16, 0.1, None)
     assert (out[T:] == 0).all() and out[:T].isfinite().all()
+
+
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 8, 2), (256, 10, 2)])
+@pytest.mark.parametrize("rows", [1, 40])
+def test_scores_that_are_all_minus_infinity(hd, nh, nkv, rows):
+    """A softmax over nothing but minus infinities is 0 / 0, as it is in float64; one score that is a number takes all the weight,
+    and keys on pages that were given back count for nothing."""
+    from tokasaurus_b200.kernels import ops
+
+    L, ps = 300, 16
+    kc, vc, indptr, pages, K, V = make_paged(torch.float32, 1, [L], nkv, hd, ps, 30, seed=2)
+    kc[:, :, :, 3] = 1e30
+    q = torch.randn(rows, nh * hd, generator=torch.Generator().manual_seed(1)).to(DEV)
+    q.view(rows, nh, hd)[:, 0, 3] = -1e30  # head 0: every score is minus infinity
+    q.view(rows, nh, hd)[:, 1:, 3] = 0
+    token_seq, positions = i32([0] * rows), i32(range(L - rows, L))
+
+    def run(ids):
+        out = torch.full((rows, nh * hd), 9.0, device=DEV)
+        ops.attn_paged(q, nh * hd, out, kc, vc, token_seq, positions, indptr, ids, None, rows, nh, nkv, hd, ps, 1.0, None)
+        return out.view(rows, nh, hd)
+
+    out = run(pages)
+    assert out[:, 0].isnan().all() and out[:, 1:].isfinite().all()
+    assert (run(torch.full_like(pages, -1)) == 0).all()  # no key at all
+    target = 133
+    kc[int(pages[target // ps]), 0, target % ps, 3] = 0
+    torch.testing.assert_close(run(pages)[:, 0].cpu(), V[0][target, 0].expand(rows, hd), rtol=1e-6, atol=0)

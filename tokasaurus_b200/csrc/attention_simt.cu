@@ -149,6 +149,7 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
     const int* table = page_ids + page_indptr[s];
     int lo[NQ], hi[NQ];  // the keys each of this warp's pairs sees: lo .. hi
     float M[NQ], L[NQ], O[NQ][DPL];
+    unsigned seen = 0;  // pairs that see a key, though its score may be minus infinity
 #pragma unroll
     for (int a = 0; a < NQ; a++) {
       const int pr = warp * NQ + a, r = pr / heads_a_block;
@@ -282,7 +283,16 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
       }
 #pragma unroll
       for (int a = 0; a < NQ; a++) {
-        if (l[a] == 0.f) continue;  // no key of this segment
+        if (l[a] == 0.f) {  // no key of this segment, or none that counts
+          bool any = false;
+#pragma unroll
+          for (int t = 0; t < TILES; t++) {
+            const int key = base + t * TILE + lane;
+            any |= key >= lo[a] && key <= hi[a] && offs[t * TILE + lane] >= 0;
+          }
+          seen |= __any_sync(0xffffffffu, any) ? 1u << a : 0u;
+          continue;
+        }
         float keep, take;
         merge_factors(M[a], L[a], m[a], l[a], keep, take);
 #pragma unroll
@@ -293,7 +303,7 @@ attn_rows_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
     for (int a = 0; a < NQ; a++) {
       if (hi[a] < 0) continue;
       const int pr = warp * NQ + a, r = pr / heads_a_block, h = pr - r * heads_a_block;
-      const float inv = L[a] == 0.f ? 0.f : 1.f / L[a];
+      const float inv = L[a] == 0.f && !(seen >> a & 1) ? 0.f : 1.f / L[a];  // (all scores minus infinity: 0 / 0)
       T* orow = out + (size_t)(r0 + r) * out_stride + (size_t)(h0 + h) * HD;
 #pragma unroll
       for (int i = 0; i < DPL; i++)
@@ -366,6 +376,7 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
     }
     constexpr int MINE = (NQ * HD + FEW_THREADS - 1) / FEW_THREADS;  // output elements a thread merges
     float M[MINE], L[MINE], O[MINE];
+    unsigned seen = 0;
 #pragma unroll
     for (int i = 0; i < MINE; i++) M[i] = -FLT_MAX, L[i] = 0.f, O[i] = 0.f;
 
@@ -429,8 +440,14 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
 #pragma unroll
         for (int i = 0; i < DPL; i++)
           if (lane + 32 * i < HD) part[team][member][lane + 32 * i] = o[i];
+        bool any = false;
+        if (l == 0.f) {
+#pragma unroll
+          for (int u = 0; u < TILES; u++) any |= offs[team][u * TILE + lane] >= 0;
+          any = __any_sync(0xffffffffu, any);
+        }
         if (lane == 0) {
-          seg_m[team][member] = m;
+          seg_m[team][member] = any ? -INFINITY : m;  // keys there are, but none that counts
           seg_l[team][member] = l;
         }
       }
@@ -441,7 +458,10 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
         if (h >= heads) continue;
         for (int u = 0; u < TEAMS; u++) {
           const float l = seg_l[u][h];
-          if (l == 0.f) continue;  // no key of this segment
+          if (l == 0.f) {  // no key of this segment, or none that counts
+            if (seg_m[u][h] == -INFINITY) seen |= 1u << i;
+            continue;
+          }
           float keep, take;
           merge_factors(M[i], L[i], seg_m[u][h], l, keep, take);
           O[i] = fmaf(O[i], keep, part[u][h][d] * take);
@@ -452,7 +472,7 @@ attn_few_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int 
     for (int i = 0; i < MINE; i++) {
       const int e = tid + i * FEW_THREADS, h = e / HD, d = e - h * HD;
       if (h >= heads) continue;
-      const float inv = L[i] == 0.f ? 0.f : 1.f / L[i];
+      const float inv = L[i] == 0.f && !(seen >> i & 1) ? 0.f : 1.f / L[i];  // (all scores minus infinity: 0 / 0)
       out[(size_t)row * out_stride + (size_t)(h0 + h) * HD + d] = from_float<T>(O[i] * inv);
     }
     if (!lone) return;
