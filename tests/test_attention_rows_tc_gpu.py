@@ -156,3 +156,25 @@ def test_the_step_takes_it():
     check(out.view(p.T, 8, 64), want, torch.ones(p.T, dtype=torch.bool, device=DEV), 2.5)
     assert ops.sink_rows_tc_modules(64, 64, maps=2) == ops.sink_rows_tc_modules(64, 64, distance=True) == ()
     assert ops.sink_rows_tc_modules(64, 64, keep_first=4) == ops.sink_rows_tc_modules(48, 64) == ops.sink_rows_tc_modules(64, 256) == ()
+
+
+@pytest.mark.parametrize("dim", [64, 48])  # on this kernel, on the mma.sync one
+def test_a_gate_with_more_rows_than_tokens(dim):
+    """The gate's logits as a column slice of a taller and wider tensor: ``attn_sink_tc`` takes the first rows."""
+    from tokasaurus_b200.kernels import ops
+
+    p = Problem(2 * dim, 2, 16, [300, 64, 90], [172, 64, 1], 5)
+    q = torch.randn(p.T, 8 * dim, generator=p.g).bfloat16().to(DEV)
+    wide = torch.randn(p.T + 19, 20, generator=p.g).to(DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(gate):
+        out = torch.empty(p.T, 8 * dim, dtype=torch.bfloat16, device=DEV)
+        ops.attn_sink_tc(q, out, p.cache, **p.tables, n_seqs=3, sinks=None, n_heads=8, n_kv_heads=2, dim=dim, vdim=dim, page_size=16,
+                         scale=0.125, softcap=None, window=100, status=status, gate=gate)
+        return out
+
+    assert torch.equal(run(wide[:, 7:15]), run(wide[:p.T, 7:15].contiguous()))
+    for bad in (wide[:p.T - 1, 7:15], wide[:, 7:14], wide[:, 7:15].double(), wide.T[7:15, :p.T].T[:, :8].T.contiguous().T):
+        with pytest.raises(ops.KernelError):
+            run(bad)

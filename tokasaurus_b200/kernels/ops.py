@@ -1674,20 +1674,20 @@ def attn_rows_tc(module: tuple, q: torch.Tensor, out: torch.Tensor, out_head: in
                  out_scale: float = 1.0) -> None:
     """Attention of the requests that bring several tokens over cached rows [pages, kv heads, page size, row]; ``module``: an
     element of ``rows_tc_modules``.  q [T, heads * kd]; head h's values go to columns h * out_head .. of out's rows."""
-    _need_cuda(q, out, cache, seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids, sinks, status, head_scale, head_bias, gate)
+    _need_cuda(q, out, cache, seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids, sinks, status, head_scale, head_bias)
     d = module[1]
     T = q.shape[0]
     _need(q.dtype == out.dtype == cache.dtype == torch.bfloat16 and q.is_contiguous() and q.shape[1] == n_heads * d["TKB_KD"],
           "attn_rows_tc: bfloat16, q [T, heads * key size]")
     _need(cache.is_contiguous() and tuple(cache.shape[1:]) == (n_kv_heads, page_size, d["TKB_ROW"]), "attn_rows_tc: cache rows")
-    _need(out.dim() == 2 and out.shape[0] == T and out.stride(1) == 1 and out.shape[1] >= (n_heads - 1) * out_head + d["TKB_VD"]
-          and (gate is None or (gate.dtype == torch.float32 and tuple(gate.shape) == (T, n_heads))), "attn_rows_tc: out and gate")
+    _need(out.dim() == 2 and out.shape[0] == T and out.stride(1) == 1 and out.shape[1] >= (n_heads - 1) * out_head + d["TKB_VD"],
+          "attn_rows_tc: out")
+    gate_args = _sink_gate(gate, T, n_heads, 1, "attn_rows_tc")
     _check(_fn(_libs.get(module[0], **d), "tkb_attn_rows_tc")(
         _ptr(q), _ptr(out), _ptr(cache), c_int(cache.shape[0]), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len),
         _ptr(page_indptr), _ptr(page_ids), c_int(n_seqs), c_int(T), c_int(n_heads), c_int(n_kv_heads), c_int(page_size),
         c_float(scale), c_float(softcap), c_int(window or 0), c_int(chunk), _ptr(sinks), _ptr(head_scale), _ptr(head_bias),
-        c_int(1 if sigmoid else 0), _ptr(gate), c_int(_row_stride(gate) if gate is not None else 0), c_float(out_scale),
-        ctypes.c_longlong(_row_stride(out)), c_int(out_head), _ptr(status), _stream()), "attn_rows_tc")
+        c_int(1 if sigmoid else 0), *gate_args, c_float(out_scale), ctypes.c_longlong(_row_stride(out)), c_int(out_head), _ptr(status), _stream()), "attn_rows_tc")
 
 
 # ---------------------------------------------------------------------------------------------
