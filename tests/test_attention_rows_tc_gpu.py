@@ -178,3 +178,25 @@ def test_a_gate_with_more_rows_than_tokens(dim):
     for bad in (wide[:p.T - 1, 7:15], wide[:, 7:14], wide[:, 7:15].double(), wide.T[7:15, :p.T].T[:, :8].T.contiguous().T):
         with pytest.raises(ops.KernelError):
             run(bad)
+
+
+def test_more_tiles_than_a_grid_has_rows():
+    """128 heads a kv head are a block a token: a step of more tokens than 65,535, which the mma.sync kernel took."""
+    from tokasaurus_b200.kernels import ops
+
+    T, heads, row, ps, window = 66000, 128, 128, 16, 40
+    (module,) = ops.rows_tc_modules(row, row, 0, 64, False)
+    g = torch.Generator(DEV).manual_seed(1)
+    pages = -(-T // ps)
+    cache = torch.randn(pages, 1, ps, row, generator=g, device=DEV).bfloat16()
+    q = torch.randn(T, heads * row, generator=g, device=DEV, dtype=torch.bfloat16)
+    out = torch.full((T, heads * 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.attn_rows_tc(module, q, out, 64, cache, i32([0]), i32([T]), i32([T]), i32([0, pages]), i32(range(pages)), n_seqs=1,
+                     n_heads=heads, n_kv_heads=1, page_size=ps, scale=0.1, window=window, status=status)
+    assert int(status) == 0
+    flat = cache.view(-1, row)
+    for t in (0, 17, 40000, 65535, 65536, T - 1):
+        rows = flat[max(0, t - window + 1):t + 1].double()
+        w = torch.softmax(q[t].view(heads, row).double() @ rows.T * 0.1, -1)
+        check(out[t].view(1, heads, 64), (w @ rows[:, :64])[None], torch.ones(1, dtype=torch.bool, device=DEV), 4.5)

@@ -280,7 +280,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
   // the last tiles first, for all kv heads: without a window a portion's last queries see the most keys.  Tiles are counted
   // over the step's requests that bring more than one token.
   if (warp == 0) {
-    const int want = (int)gridDim.y - 1 - (int)blockIdx.y;
+    const int want = (int)((gridDim.x - 1 - blockIdx.x) / a.nkv);
     int found = -1, tile = 0;
     for (int s0 = 0, base = 0; s0 < a.n_seqs && found < 0; s0 += 32) {
       const int len = s0 + lane < a.n_seqs ? a.seq_q_len[s0 + lane] : 0;
@@ -321,7 +321,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_consta
   unsigned char* sQ = base;
   unsigned char* ring = sQ + Q_BYTES;
   unsigned char* sP = ring + STAGES * TILE_BYTES;  // a tile a half
-  const int kvh = blockIdx.x, head0 = kvh * group;
+  const int kvh = blockIdx.x % a.nkv, head0 = kvh * group;
   const int q_len = a.seq_q_len[s], kv_len = a.seq_kv_len[s];
   const int tok0 = where[1] * tq, toks = min(tq, q_len - tok0);
   const int pos0 = kv_len - q_len + tok0;                                 // position of the block's first token
@@ -576,8 +576,8 @@ TKB_EXPORT int tkb_attn_rows_tc(const void* q, void* out, const void* cache, int
   if (((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)cache & 15)) return -2;
   if (!TKB_CAP && (softcap > 0.f || sinks || head_scale || head_bias || gate || sigmoid)) return -2;
   const int tq = BM / (nh / nkv);
-  const long long tiles = n_tokens / tq + (long long)n_seqs;  // no step of this shape has more
-  if (tiles > 65535) return -3;
+  const long long blocks = (n_tokens / tq + (long long)n_seqs) * nkv;  // no step of this shape has more
+  if (blocks >= 1ll << 31) return -3;
   static SharedMemoryRequest shared_memory;
   if (const int rc = shared_memory({{(const void*)attn_rows_tc_kernel, SMEM_BYTES}})) return rc;
   CUtensorMap map;
@@ -593,5 +593,5 @@ TKB_EXPORT int tkb_attn_rows_tc(const void* q, void* out, const void* cache, int
   const Args a = {(const bf16*)q, (bf16*)out, (const bf16*)cache, seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids,
                   sinks, head_scale, head_bias, gate, status, out_stride, n_seqs, nh, nkv, out_head, ps, window, chunk, n_pages,
                   tma_rows, gate_stride, sigmoid, scale, softcap, out_scale};
-  return launch_pdl(attn_rows_tc_kernel, dim3(nkv, (unsigned)tiles), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)st, map, a);
+  return launch_pdl(attn_rows_tc_kernel, dim3((unsigned)blocks), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)st, map, a);
 }
