@@ -265,3 +265,44 @@ def test_chunks_far_from_one(form, heads, groups, size, monkeypatch):
         want = want.double() / up
         err = lambda x: float((x.double() - want).norm() / want.norm())  # noqa: E731
         assert got.isfinite().all() and err(got) <= 1.5 * err(walk) + 16 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("lens,chunks", [([128] * 5, None), ([100, 191, 150], None), ([100, 200, 1, 321], 4 + 6)])
+@pytest.mark.parametrize("layer", ["decayed", "forget"])
+def test_a_step_s_layer_launches_what_its_requests_need(lens, chunks, layer, monkeypatch):
+    """A layer of an eager step: no chunk kernel and no scratch without a long request, and scratch for the long ones alone."""
+    from tokasaurus_b200.cache import CacheManager
+    from tokasaurus_b200.engine.batch import Stager, StepContext, StepEntry, build_host_batch
+    from tokasaurus_b200.engine.runtime import Runtime
+    from tokasaurus_b200.kernels import ops
+    from tokasaurus_b200 import parts as P
+
+    H, W = 2, 256
+    if layer == "decayed":
+        part = P.DecayedLinearAttention(W, H, 128, 128, [0.9, 0.99], 1e-5, "q", "k", "v", "g", "norm", "o")
+    else:
+        part = P.GatedLinearRecurrence(W, H, 128, 128, 1e-5, "q", "k", "f_bias", "lower", "v", "norm", "o")
+    g = torch.Generator().manual_seed(1)
+    rt = Runtime.make(DEV, "bfloat16")
+    part.bind({s.name: (torch.rand(s.shape, generator=g) * 0.5 if s.role == "vector" else torch.randn(s.shape, generator=g) / 16).to(
+        DEV, torch.float32 if s.role == "vector" else torch.bfloat16) for s in part.weight_specs()}, rt)
+    cm = CacheManager({0: part.cache_need()}, 16, 4, len(lens), dtype=rt.dtype, device=rt.device)
+    for i, n in enumerate(lens):
+        cm.admit(i)
+        cm.ensure_capacity(i, n)
+    ctx = StepContext(build_host_batch([StepEntry(i, [0] * n, 0, [n - 1]) for i, n in enumerate(lens)], cm), cm, rt.device, Stager(rt.device))
+    h = torch.randn(sum(lens), W, generator=g).bfloat16().to(DEV)
+    seen, real = [], ops._decay_chunks
+
+    def spy(*args):
+        out = real(*args)
+        seen.append(out[1].shape[0])
+        return out
+
+    monkeypatch.setattr(ops, "_decay_chunks", spy)
+    part.forward(ctx, h, cm.layer_cache(0))
+    assert seen == ([] if chunks is None else [chunks])
+    seen.clear()
+    ctx.plan_caps = {}  # as while a step graph is recorded: what any step of the shape can need
+    part.forward(ctx, h, cm.layer_cache(0))
+    assert len(seen) == 1 and seen[0] >= (chunks or 0)

@@ -104,6 +104,12 @@ class StepContext:
         self.last_token = cache_manager.last_token
         self.status = stager.status
 
+    @property
+    def lengths(self) -> np.ndarray | None:
+        """How many tokens each request brings, for work whose launches and scratch go by it; None in a step graph, which is
+        replayed for requests of other lengths."""
+        return None if self.plan_caps is not None else self.host.seq_q_len
+
     def layer_cache(self, entry: int, writable: bool = True):
         return self.cache_manager.layer_cache(entry, writable)
 

@@ -13,6 +13,7 @@ import math
 import threading
 from ctypes import c_float, c_int, c_void_p
 
+import numpy as np
 import torch
 
 from tokasaurus_b200.kernels import build
@@ -878,11 +879,12 @@ def recurrence_defines(dim: int, vdim: int) -> dict:
 def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tensor, low: torch.Tensor,
                      norm_w: torch.Tensor, out: torch.Tensor, seq_slot: torch.Tensor, seq_q_start: torch.Tensor,
                      seq_q_len: torch.Tensor, n_seqs: int, heads: int, dim: int, vdim: int, eps: float,
-                     write_state: bool = True, split_heads: bool = True) -> None:
+                     write_state: bool = True, split_heads: bool = True, lengths=None) -> None:
     """The recurrence S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T, o_t = S_t^T q_t over each request's tokens, then an
     RMS norm of every head's o.  qfv: float32 [T, heads*dim (q) + heads*dim (f) + heads*vdim (v)] raw projections;
     state: float32 [slots, heads, vdim, dim] (S transposed); out: [T, heads*vdim].  ``split_heads``: a step with more
-    tokens than requests may spread a head's columns over several blocks (raw outputs through a float32 buffer)."""
+    tokens than requests may spread a head's columns over several blocks (raw outputs through a float32 buffer).  ``lengths``: as in
+    ``decay_walk``."""
     _need_cuda(qfv, state, f_bias, low, norm_w, out, seq_slot, seq_q_start, seq_q_len)
     T = qfv.shape[0]
     _need(qfv.dtype == torch.float32 and qfv.stride(1) == 1 and qfv.shape[1] == heads * (2 * dim + vdim),
@@ -895,8 +897,9 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
     f = _fn(_libs.get("recurrence.cu", **recurrence_defines(dim, vdim)), f"tkb_gated_recurrence_{_suffix(out.dtype)}")
     raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=qfv.device) if (split_heads and T > n_seqs) else None
     # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the gates and the walk over what is left
-    by_chunks = (raw is not None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and bool(decay_chunk_modules(dim, vdim))
-                 and qfv.stride(0) % 4 == 0 and qfv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0)
+    n_chunks = 0
+    if raw is not None and decay_chunk_modules(dim, vdim) and qfv.stride(0) % 4 == 0 and qfv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
+        n_chunks = decay_chunk_count(T, n_seqs, lengths)
 
     def run(phase: int, marks: tuple) -> None:
         _check(f(_ptr(qfv), c_int(qfv.stride(0)), _ptr(state), _ptr(f_bias), _ptr(low), _ptr(norm_w), _ptr(out),
@@ -904,12 +907,12 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
                  c_int(vdim), c_float(eps), c_int(1 if write_state else 0), _ptr(raw), *marks, c_int(phase), _stream()),
                "gated_recurrence")
 
-    if not by_chunks:
+    if not n_chunks:
         return run(0, _NO_MARKS)
     run(1, _NO_MARKS)
     decay = qfv[:, heads * dim:2 * heads * dim]
     chunks = _decay_chunks(qfv[:, :heads * dim], None, qfv[:, 2 * heads * dim:], 1, None, None, decay, None, state.view(state.shape[0], -1),
-                           raw, seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state)
+                           raw, seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state, n_chunks)
     run(2, _marks(chunks))
 
 
@@ -1402,6 +1405,21 @@ DECAY_CHUNK = 64
 DECAY_CHUNKS_FROM = 192
 
 
+def decay_chunk_count(n_tokens: int, n_seqs: int, lengths=None) -> int:
+    """Chunks of a step's long requests, 0 if it has none: what the chunk kernels' grids and scratch are sized by.  ``lengths``: the
+    requests' tokens, where the host knows them and may go by them; else the most that a step of this shape can have (requests without
+    a token among them; a step of as many tokens as requests decodes)."""
+    if n_tokens < DECAY_CHUNKS_FROM:
+        return 0
+    if lengths is not None:
+        n = np.asarray(lengths)
+        _need(n.shape == (n_seqs,), "a length for every request")
+        return int(((n + DECAY_CHUNK - 1) // DECAY_CHUNK)[n >= DECAY_CHUNKS_FROM].sum())
+    if n_tokens <= n_seqs:
+        return 0
+    return n_tokens // DECAY_CHUNK + min(n_seqs, n_tokens // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
+
+
 def decay_chunk_modules(dim: int, vdim: int) -> tuple:
     """The kernel module for long requests, if heads of this size have one."""
     return (("decay_chunks.cu", None),) if dim == 128 and vdim in (64, 128) else ()
@@ -1456,12 +1474,10 @@ def ssm_prep(proj: torch.Tensor, xbc_off: int, channels: int, conv_w: torch.Tens
 
 
 def _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
-                  heads, dim, vdim, write_state) -> tuple[torch.Tensor, torch.Tensor]:
+                  heads, dim, vdim, write_state, chunks) -> tuple[torch.Tensor, torch.Tensor]:
     """The recurrence of ``decay_walk`` for the requests that bring at least ``DECAY_CHUNKS_FROM`` tokens, in chunks (the caller
     has checked the operands).  ``k`` None: 1 - decay_vec.  Returns what the walk that follows needs to do over again what was not
     finite: the chunks' marks and the states they started from."""
-    T = q.shape[0]
-    chunks = T // DECAY_CHUNK + min(n_seqs, T // DECAY_CHUNKS_FROM)  # every request's last one may be cut short
     states = torch.empty((chunks, heads, vdim, dim), dtype=torch.float32, device=q.device)
     gains = torch.empty((chunks, heads, dim if decay_vec is not None else 1), dtype=torch.float32, device=q.device)
     bad = torch.empty((chunks, heads), dtype=torch.int32, device=q.device)
@@ -1486,14 +1502,16 @@ def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: 
                decay_head: torch.Tensor | None, skip: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor,
                seq_slot: torch.Tensor, seq_q_start: torch.Tensor, seq_q_len: torch.Tensor, n_seqs: int, heads: int,
                dim: int, vdim: int, write_state: bool = True, decay_vec: torch.Tensor | None = None,
-               ones_out: torch.Tensor | None = None) -> None:
+               ones_out: torch.Tensor | None = None, lengths=None) -> None:
     """S_t = a_t S_(t-1) + (c_t k_t) v_t^T, o_t = S_t^T q_t + skip * v_t over each request's tokens.  q, k [T, . * dim]
     and v [T, heads * vdim] are float32 (column slices allowed); head h reads q and k number h // heads_per_qk.
     ``dt_dec`` [T, 2 heads] = (c, a) per token, or ``decay_head`` [heads] with
     c = 1, or ``decay_vec`` float32 [T, heads * dim] (a column slice allowed): a decay for every key channel,
     S_t = diag(f_t) S_(t-1) + k_t v_t^T.  state float32 [slots, n], S^T of the heads first: [heads, vdim, dim]; out
     float32 [T, heads * vdim].  ``ones_out`` float32 [T, heads] (not with ``decay_vec``): a head's state holds one more
-    column, [heads, vdim + 1, dim], whose value is 1 at every token; its S^T q goes there."""
+    column, [heads, vdim + 1, dim], whose value is 1 at every token; its S^T q goes there.  ``lengths``: seq_q_len as numbers on
+    the host, where the call is made for these and no other requests (not while a step graph is recorded): the launches and the
+    scratch for long requests then go by them."""
     _need_cuda(q, k, v, dt_dec, decay_head, skip, state, out, seq_slot, seq_q_start, seq_q_len, decay_vec, ones_out)
     vall = vdim + (1 if ones_out is not None else 0)
     T = q.shape[0]
@@ -1514,15 +1532,17 @@ def decay_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads_per_qk: 
     _need(ones_out is None or (decay_vec is None and ones_out.dtype == torch.float32 and ones_out.is_contiguous()
                                and tuple(ones_out.shape) == (T, heads)), "decay_walk: ones_out float32 [T, heads]")
     _need(out.dtype == torch.float32 and out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "decay_walk: out float32 [T, heads * vdim]")
-    chunks = None
+    chunks, n_chunks = None, 0
     rows = [q, k, v] + ([decay_vec] if decay_vec is not None else [])
-    if (ones_out is None and T - n_seqs + 1 >= DECAY_CHUNKS_FROM and decay_chunk_modules(dim, vdim)
+    if (ones_out is None and decay_chunk_modules(dim, vdim)
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in rows)
             and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0):
+        n_chunks = decay_chunk_count(T, n_seqs, lengths)
+    if n_chunks:
         # requests that bring many tokens; the walk below then leaves them alone, unless their numbers are not finite.  Which
         # requests these are is read on the device: a step graph is replayed for other lengths.
         chunks = _decay_chunks(q, k, v, heads_per_qk, dt_dec, decay_head, decay_vec, skip, state, out, seq_slot, seq_q_start, seq_q_len,
-                               n_seqs, heads, dim, vdim, write_state)
+                               n_seqs, heads, dim, vdim, write_state, n_chunks)
     defines = _walk_defines(dim, vdim, n_seqs * heads * vall, T == n_seqs, q.device)
     _check(_fn(_libs.get("decay_recurrence.cu", **defines), "tkb_decay_walk")(
         _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), c_int(heads_per_qk), _ptr(decay_vec),

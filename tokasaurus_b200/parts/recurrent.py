@@ -56,7 +56,8 @@ class GatedLinearRecurrence(Mixer):
         qfv = ops.linear(h, self.w_qfv, out_dtype=torch.float32)
         o = torch.empty((h.shape[0], self.n_heads * self.vdim), dtype=h.dtype, device=h.device)
         ops.gated_recurrence(qfv, cache.state, self.f_bias, self.lower, self.norm_w, o, ctx.seq_slot, ctx.seq_q_start,
-                             ctx.seq_q_len, ctx.n_seqs, self.n_heads, self.dim, self.vdim, self.norm_eps, cache.writable)
+                             ctx.seq_q_len, ctx.n_seqs, self.n_heads, self.dim, self.vdim, self.norm_eps, cache.writable,
+                             lengths=getattr(ctx, "lengths", None))
         if out_rows is not None:
             cut = torch.empty((out_rows.numel(), o.shape[1]), dtype=o.dtype, device=o.device)
             ops.gather_rows(o, out_rows, cut)
@@ -116,7 +117,7 @@ class DecayedLinearAttention(Mixer):
         ops.silu_cols(proj, 2 * H * d + H * e, self.defines)  # q, k and v, in place
         raw = torch.empty((T, H * e), dtype=torch.float32, device=h.device)
         ops.decay_walk(q, k, v, 1, None, self.decay_t, None, cache.state, raw, ctx.seq_slot, ctx.seq_q_start,
-                       ctx.seq_q_len, ctx.n_seqs, H, d, e, cache.writable)
+                       ctx.seq_q_len, ctx.n_seqs, H, d, e, cache.writable, lengths=getattr(ctx, "lengths", None))
         if out_rows is not None:
             raw, g = _rows(raw, out_rows), _rows(g.contiguous(), out_rows)
         o = torch.empty(raw.shape, dtype=h.dtype, device=h.device)
@@ -190,7 +191,7 @@ class GatedLinearAttention(Mixer):
                       self.defines)
         raw = torch.empty((T, H * e), dtype=torch.float32, device=h.device)
         ops.decay_walk(q, k, v, 1, None, None, None, cache.state, raw, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len,
-                       ctx.n_seqs, H, d, e, cache.writable, decay_vec=f)
+                       ctx.n_seqs, H, d, e, cache.writable, decay_vec=f, lengths=getattr(ctx, "lengths", None))
         if out_rows is not None:
             raw, g = _rows(raw, out_rows), _rows(g.contiguous(), out_rows)
         o = torch.empty(raw.shape, dtype=h.dtype, device=h.device)
@@ -258,7 +259,7 @@ class Retention(Mixer):
                          ctx.token_seq, 1.0, self.k_scale, self.defines)
         raw = torch.empty((T, H * e), dtype=torch.float32, device=h.device)
         ops.decay_walk(q, k, v, 1, None, self.decay_t, None, cache.state, raw, ctx.seq_slot, ctx.seq_q_start,
-                       ctx.seq_q_len, ctx.n_seqs, H, d, e, cache.writable)
+                       ctx.seq_q_len, ctx.n_seqs, H, d, e, cache.writable, lengths=getattr(ctx, "lengths", None))
         if out_rows is not None:
             raw, g = _rows(raw, out_rows), _rows(g.contiguous(), out_rows)
         o = torch.empty(raw.shape, dtype=h.dtype, device=h.device)
