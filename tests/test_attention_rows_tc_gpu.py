@@ -200,3 +200,38 @@ def test_more_tiles_than_a_grid_has_rows():
         rows = flat[max(0, t - window + 1):t + 1].double()
         w = torch.softmax(q[t].view(heads, row).double() @ rows.T * 0.1, -1)
         check(out[t].view(1, heads, 64), (w @ rows[:, :64])[None], torch.ones(1, dtype=torch.bool, device=DEV), 4.5)
+
+
+@pytest.mark.parametrize("ps", [16, 12])  # pages that come as TMA boxes, pages that are gathered
+@pytest.mark.parametrize("form", ["latent", "key_value"])
+def test_pages_given_back_and_pages_beyond_the_pool(ps, form):
+    """Pages behind the window (id -1) are not looked at; an id beyond the pool sets the status bit, its keys' values count for nothing,
+    and no other request sees anything of it."""
+    from tokasaurus_b200.kernels import ops
+
+    kd, v0, vd, nkv, heads, window = (256, 0, 192, 1, 16, 100) if form == "latent" else (64, 64, 64, 3, 12, 100)
+    row = 256 if form == "latent" else 128
+    (module,) = ops.rows_tc_modules(row, kd, v0, vd, form != "latent")
+    p = Problem(row, nkv, ps, [400, 333, 90], [70, 129, 90], ps)
+    q = torch.randn(p.T, heads * kd, generator=p.g).bfloat16().to(DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(ids):
+        out = torch.full((p.T, heads * vd), 7.0, dtype=torch.bfloat16, device=DEV)
+        ops.attn_rows_tc(module, q, out, vd, p.cache, **{**p.tables, "page_ids": ids}, n_seqs=3, n_heads=heads, n_kv_heads=nkv,
+                         page_size=ps, scale=kd ** -0.5, window=window, status=status)
+        return out
+
+    whole = run(p.tables["page_ids"])
+    check(whole.view(p.T, heads, vd), p.want(q, kd, v0, vd, heads, kd ** -0.5, window), torch.ones(p.T, dtype=torch.bool, device=DEV), 4.5)
+    ids = p.tables["page_ids"].clone()
+    first = (400 - 70 - window + 1) // ps  # the first page that request 0's portion sees
+    ids[:first] = -1
+    assert torch.equal(run(ids), whole) and int(status) == 0
+    at = int(p.tables["page_indptr"][1]) + 250 // ps
+    ids[at] = p.cache.shape[0] + 5
+    out = run(ids)
+    assert int(status) == 2  # a page id outside the pool
+    mine = slice(p.start[1], p.start[1] + 129)
+    assert torch.equal(out[: p.start[1]], whole[: p.start[1]]) and torch.equal(out[p.start[2]:], whole[p.start[2]:])
+    assert out[mine].isfinite().all() and not torch.equal(out[mine], whole[mine])
