@@ -381,9 +381,18 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
   if (by_16 && smem_split <= 200 * 1024 && threads <= SPLIT_THREADS_MAX) {
     if (smem_split > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split);
-    rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
-                    (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
-                    cols_per_block, raw_out, marks);
+    // behind the chunk kernels an ordinary launch: blocks that come onto the SMs while those still hold some of them would be placed
+    // where room happens to be, several to an SM (four prompts of 700 tokens in all, the layer: 258 us, 246 so)
+    if (phase == 2) {
+      gated_recurrence_split_kernel<<<dim3(n_seqs, heads, split), dim3(threads), smem_split, st>>>(
+          (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state, cols_per_block,
+          raw_out, marks);
+      rc = launch_status();
+    } else {
+      rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
+                      (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
+                      cols_per_block, raw_out, marks);
+    }
   } else {
     rc = launch_pdl(gated_recurrence_kernel<T, true>, dim3(n_seqs, heads, split), dim3(threads), smem, st,
                     (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start, seq_q_len,
