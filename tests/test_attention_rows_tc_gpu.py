@@ -141,6 +141,22 @@ def test_key_value_rows(dim, vdim, heads, nkv, window, chunk, ps, form):
     assert (out.view(p.T, heads, vdim)[~several] == 7).all()
 
 
+def test_what_it_refuses():
+    """A sink beside sigmoid weights would scale the result, and vectors of other sizes would be read out of range."""
+    from tokasaurus_b200.kernels import ops
+
+    p = Problem(128, 2, 16, [90, 64], [30, 64], 5)
+    q = torch.randn(p.T, 8 * 64, generator=p.g).bfloat16().to(DEV)
+    out, status = torch.empty_like(q), torch.zeros(1, dtype=torch.int32, device=DEV)
+    (module,) = ops.sink_rows_tc_modules(64, 64)
+    vec = lambda n, t=torch.float32: torch.zeros(n, dtype=t, device=DEV)  # noqa: E731
+    for opt in (dict(sigmoid=True, sinks=vec(8)), dict(sinks=vec(7)), dict(head_scale=vec(8, torch.float64)), dict(head_bias=vec(4)),
+                dict(gate=torch.zeros(p.T - 1, 8, device=DEV))):
+        with pytest.raises(ops.KernelError):
+            ops.attn_rows_tc(module, q, out, 64, p.cache, **p.tables, n_seqs=2, n_heads=8, n_kv_heads=2, page_size=16, scale=0.1,
+                             window=None, status=status, **opt)
+
+
 def test_the_step_takes_it():
     """``attn_sink_tc``: portions on this kernel, single tokens on theirs; forms that it does not have stay where they were."""
     from tokasaurus_b200.kernels import ops

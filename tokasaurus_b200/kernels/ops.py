@@ -1702,6 +1702,8 @@ def attn_rows_tc(module: tuple, q: torch.Tensor, out: torch.Tensor, out_head: in
     _need(cache.is_contiguous() and tuple(cache.shape[1:]) == (n_kv_heads, page_size, d["TKB_ROW"]), "attn_rows_tc: cache rows")
     _need(out.dim() == 2 and out.shape[0] == T and out.stride(1) == 1 and out.shape[1] >= (n_heads - 1) * out_head + d["TKB_VD"],
           "attn_rows_tc: out")
+    _need(not (sigmoid and sinks is not None), "attn_rows_tc: the sigmoid form has no sink")
+    _head_vectors(n_heads, "attn_rows_tc", sinks, head_scale, head_bias)
     gate_args = _sink_gate(gate, T, n_heads, 1, "attn_rows_tc")
     _check(_fn(_libs.get(module[0], **d), "tkb_attn_rows_tc")(
         _ptr(q), _ptr(out), _ptr(cache), c_int(cache.shape[0]), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len),
