@@ -11,8 +11,8 @@
 //   chunk_outputs  a block a (chunk, head): o_t = (q_t decayed from the chunk's start) S_start + sum_s A[t][s] v_s with
 //                  A[t][s] = q_t . (decay from s to t) c_s k_s for s <= t.
 // What is not finite, and what overflows on the way, is the walk's (decay_chunks.cuh).
-// No factor exceeds the decays' own products: one number a head is kept as a sum of logarithms in 64 bits, whose differences
-// are exact enough; a number a channel is kept as running products inside blocks of 16 tokens: A's blocks beside the diagonal
+// No factor exceeds the decays' own products: one number a head is kept as a sum of logarithms, made in 64 bits and kept as two
+// floats, whose differences are exact enough; a number a channel is kept as running products inside blocks of 16 tokens: A's blocks beside the diagonal
 // take q decayed from its block's start, k decayed to its block's end and the product of the blocks between, and A's diagonal
 // blocks are summed on the FP32 pipes with the product running along.  So nothing overflows, and what underflows is zero.
 //

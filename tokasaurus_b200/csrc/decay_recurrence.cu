@@ -29,9 +29,9 @@
 // heads of 128): a warp alone issues an instruction every four cycles (each waits for the one before), so the time
 // goes down with the number of warps, and that is the state's size over what a thread holds.  Tokens come in chunks of
 // 16 by cp.async, one chunk ahead; the lanes' shares of a chunk's outputs wait in shared memory and are added up after
-// the chunk.  Activations of q, k and v are applied beforehand, once.  Heads of 128 x 64 and 128 x 128 are walked only for
-// requests that bring fewer than 192 tokens; longer ones go in chunks whose inner products are matrix products
-// (decay_chunks.cu).
+// the chunk.  Activations of q, k and v are applied beforehand, once.  Heads of 128 x 64 and 128 x 128: requests that bring 192
+// tokens or more go in chunks whose inner products are matrix products (decay_chunks.cu), unless rows, strides or state are not whole
+// 16-byte pieces or the state has a column of ones; the walk does what is left of them where something is not finite.
 //
 // Compile with -DTKB_DR_LANES=<threads that share a column: the power of two from 8 to 32 nearest above dim / 4> and
 // -DTKB_DR_DPT=<dims a lane: 4 * ceil(dim / (4 * lanes))>.

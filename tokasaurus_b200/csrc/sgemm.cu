@@ -169,7 +169,8 @@ __device__ __forceinline__ void fetch8(const float* __restrict__ p, int left, fl
 // lane's feature, whose weights are the row w, and of the token in row i of A.  G tokens at a time share a reading of the
 // weights, REDO_K numbers of which are on their way together.  Tokens that are finite in all of a warp's features are passed by,
 // and so are tokens with a NaN among their numbers: every result of theirs is NaN, and is there.
-// (One element after the other, a number of each row at a time, 500 rows of NaN took 69 ms where a clean product takes 0.26.)
+// (One element after the other, a number of each row at a time, 500 rows of NaN x 2,048 x 8,192 took 31 ms; measured on B200 now 215
+// us, a clean product 148, and 660 us with one row that has an infinity.)
 template <bool VEC, int G, int REDO_K>
 __device__ __forceinline__ void redo_chains(float (&acc)[G], const float* __restrict__ A, int lda, int rows, const float* __restrict__ w,
                                             int K) {

@@ -768,7 +768,7 @@ def linear_few_rows_gated(a: torch.Tensor, w_interleaved: torch.Tensor, status: 
 
 
 def linear(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """a[M, K] @ w[N, K]^T.  float32: this engine's FP32 kernel (no tf32).  bfloat16: the library
+    """a[M, K] @ w[N, K]^T.  float32: this engine's true 32-bit product (``sgemm_tn``; no tf32).  bfloat16: the library
     matrix product (cuBLAS through torch), float32 accumulation, output bfloat16 or float32."""
     _need_cuda(a, w)
     M = a.shape[0]
