@@ -18,8 +18,8 @@ __device__ __forceinline__ uint32_t cut_pack(float a, float b) {
 }
 // Two neighbouring numbers.
 __device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-  a *= CUT_SCALE;
-  b *= CUT_SCALE;
+  asm("{\n.reg .b64 x, s;\nmov.b64 x, {%0, %1};\nmov.b64 s, {%2, %2};\nmul.rn.f32x2 x, x, s;\nmov.b64 {%0, %1}, x;\n}"
+      : "+f"(a), "+f"(b) : "f"(CUT_SCALE));  // both at once
   h = cut_pack(a, b);
   const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
   m = cut_pack(ra, rb);

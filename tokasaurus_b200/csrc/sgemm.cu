@@ -383,18 +383,33 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     }
   } else {
     // ---------------- fetch, cut, store: pieces of 8 numbers, eight threads a row of the chunk
-    // (a piece's place and where it goes are worked out where they are wanted: what is kept across the loop is short of registers)
+    // A piece's place is kept across the loop, or (128 token columns, short of registers) worked out where it is wanted: 500 rows x
+    // 16,384 x 2,048 266 us kept, with spills, and 255 so; 64 rows 50 kept, 52 so.
+    constexpr bool KEPT = NT < 128;
+    const float* src[KEPT ? TASKS : 1];
     float4 x[AHEAD][TASKS][2];
     const int seg = tid & 7, k0 = c_begin * CHUNK + seg * 8, r0 = (tid - 32) >> 3;
     constexpr int ROWS = CONVERTERS / 8;  // rows between a thread's pieces
+    if constexpr (KEPT)
+#pragma unroll
+      for (int i = 0; i < TASKS; i++) {
+        const int r = r0 + i * ROWS;
+        src[i] = nullptr;
+        if (r < 128 && n0 + r < N) src[i] = W + (size_t)(n0 + r) * ldw + k0;
+        if (r >= 128 && r < 128 + NT && m0 + r - 128 < M) src[i] = A + (size_t)(m0 + r - 128) * lda + k0;
+      }
     auto fetch = [&](int c, int into) {
       const int k = k0 + c * CHUNK, left = c < n_chunks ? K - k : 0;
 #pragma unroll
       for (int i = 0; i < TASKS; i++) {
-        const int r = r0 + i * ROWS;
-        const bool is_w = r < 128, there = is_w ? n0 + r < N : r < 128 + NT && m0 + r - 128 < M;
-        const float* p = (is_w ? W + (size_t)(n0 + r) * ldw : A + (size_t)(m0 + r - 128) * lda) + k;
-        fetch8<VEC>(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
+        if constexpr (KEPT) {
+          fetch8<VEC>(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
+        } else {
+          const int r = r0 + i * ROWS;
+          const bool is_w = r < 128, there = is_w ? n0 + r < N : r < 128 + NT && m0 + r - 128 < M;
+          const float* p = (is_w ? W + (size_t)(n0 + r) * ldw : A + (size_t)(m0 + r - 128) * lda) + k;
+          fetch8<VEC>(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
+        }
       }
     };
 #pragma unroll
