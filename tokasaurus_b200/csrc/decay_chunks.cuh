@@ -28,14 +28,16 @@ __device__ __forceinline__ int decay_first_chunk(const int* __restrict__ seq_q_l
 struct ChunkMarks {
   const int* bad;       // [chunks][heads]
   const float* states;  // [chunks][heads][vdim * dim]: the state every chunk started from
-  int least;            // requests of so many tokens went in chunks (INT_MAX: none)
+  int least;            // requests of so many tokens go in chunks (INT_MAX: none)
+  bool rest_only;       // the shorter requests have been walked already
 };
 // The walk's part of request `seq` (n tokens from row `start` on): nothing (false), all of it (`from` null), or what comes behind
-// the first marked chunk's start (`from`: the state there).  By every warp of the block alike.
+// the first marked chunk's start (`from`: the state there).  By every warp of the block alike.  `bad` null: a walk ahead of the chunks.
 __device__ __forceinline__ bool walk_part(const ChunkMarks& m, const int* __restrict__ seq_q_len, int seq, int head, int heads,
                                           size_t state_size, int& start, int& n, const float*& from) {
   from = nullptr;
-  if (n < m.least) return n > 0;
+  if (n < m.least) return n > 0 && !m.rest_only;
+  if (m.bad == nullptr) return false;
   const int lane = threadIdx.x & 31, chunks = decay_chunks_of(n, m.least), first = decay_first_chunk(seq_q_len, seq, m.least);
   for (int c0 = 0; c0 < chunks; c0 += 32) {
     const bool bad = c0 + lane < chunks && m.bad[(size_t)(first + c0 + lane) * heads + head] != 0;

@@ -433,7 +433,7 @@ TKB_EXPORT int tkb_decay_walk(const float* q, int q_stride, const float* k, int 
                               int vdim, int write_state, float* ones_out, const int* bad, const float* states, int least,
                               void* st) {
   if (bad != nullptr && (states == nullptr || least < 1 || ones_out != nullptr)) return -2;
-  const ChunkMarks marks = {bad, states, bad != nullptr ? least : INT_MAX};
+  const ChunkMarks marks = {bad, states, bad != nullptr ? least : INT_MAX, false};
   if (fvec != nullptr && (dt_dec != nullptr || qk_div != 1 || ones_out != nullptr)) return -2;
   return walk_launch(q, q_stride, k, k_stride, qk_div, fvec, f_stride, v, v_stride, dt_dec, decay_head, skip, state, slot_stride, out,
                      seq_slot, seq_q_start, seq_q_len, n_seqs, n_tokens, heads, dim, vdim, write_state, ones_out, marks, (cudaStream_t)st);

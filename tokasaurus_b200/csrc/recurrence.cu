@@ -374,31 +374,22 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
   if (phase != 2)
     rc = launch_pdl(recurrence_gates_kernel, dim3(n_tokens), dim3(heads * dim >= 1024 ? 256 : 128), 0, st, qfv, row_stride, f_bias,
                     low, heads * dim);
-  if (rc != 0 || phase == 1) return rc;
+  if (rc != 0) return rc;
   const bool by_16 = dim % 4 == 0 && vdim % 4 == 0 && row_stride % 4 == 0 && (((uintptr_t)qfv) & 15) == 0;
   constexpr int SPLIT_SP = (DPT % 4 == 0) ? DPT + (((DPT / 4) % 2 == 0) ? 4 : 0) : DPT;  // as in the kernel
   const size_t smem_split = (size_t)CHUNK * (2 * (2 * LANES * SPLIT_SP + cols_per_block) + cols_per_block) * sizeof(float);
   if (by_16 && smem_split <= 200 * 1024 && threads <= SPLIT_THREADS_MAX) {
     if (smem_split > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split);
-    // behind the chunk kernels an ordinary launch: blocks that come onto the SMs while those still hold some of them would be placed
-    // where room happens to be, several to an SM (four prompts of 700 tokens in all, the layer: 258 us, 246 so)
-    if (phase == 2) {
-      gated_recurrence_split_kernel<<<dim3(n_seqs, heads, split), dim3(threads), smem_split, st>>>(
-          (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state, cols_per_block,
-          raw_out, marks);
-      rc = launch_status();
-    } else {
-      rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
-                      (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
-                      cols_per_block, raw_out, marks);
-    }
+    rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
+                    (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
+                    cols_per_block, raw_out, marks);
   } else {
     rc = launch_pdl(gated_recurrence_kernel<T, true>, dim3(n_seqs, heads, split), dim3(threads), smem, st,
                     (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start, seq_q_len,
                     heads, dim, vdim, eps, write_state, cols_per_block, raw_out, marks);
   }
-  if (rc != 0) return rc;
+  if (rc != 0 || phase == 1) return rc;
   return launch_pdl(head_rmsnorm_kernel<T>, dim3((rows + 7) / 8), dim3(256), 0, st, (const float*)raw_out, norm_w, (T*)out,
                     rows, vdim, eps);
 }
@@ -408,8 +399,9 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
 // qfv: float32 [tokens, row_stride]; state: float32 [slots, heads, vdim, dim]; out: [tokens, heads * vdim];
 // raw: float32 [tokens, heads * vdim] scratch for the split form, or null (every block then owns a whole head).
 // The split form turns the q and f columns of qfv into gates in place.  phase 0: everything.  Where
-// decay_chunks.cu does the requests with at least `least` tokens (the split form, raw given), it runs between phase 1, the gates, and
-// phase 2, the walk over what it left (bad, states: ChunkMarks) and the norm.
+// decay_chunks.cu does the requests with at least `least` tokens (the split form, raw given), it runs between phase 1, the gates and the
+// walk over the other requests, and phase 2, the walk over what it left (bad, states: ChunkMarks) and the norm.  (One walk behind the
+// chunks cost 13 us where requests of 184 tokens stood beside one of 263: it no longer starts while the gates' kernel ends.)
 TKB_EXPORT int tkb_gated_recurrence_f32(float* qfv, int row_stride, float* state, const float* f_bias,
                                         const float* low, const float* norm_w, void* out, const int* seq_slot,
                                         const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
@@ -417,7 +409,7 @@ TKB_EXPORT int tkb_gated_recurrence_f32(float* qfv, int row_stride, float* state
                                         const float* states, int least, int phase, void* st) {
   return launch<float>(qfv, row_stride, state, f_bias, low, norm_w, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
                        n_tokens, heads, dim, vdim, eps, write_state, raw,
-                       {bad, states, bad != nullptr ? least : INT_MAX}, phase, (cudaStream_t)st);
+                       {bad, states, phase != 0 ? least : INT_MAX, phase == 2}, phase, (cudaStream_t)st);
 }
 TKB_EXPORT int tkb_gated_recurrence_bf16(float* qfv, int row_stride, float* state, const float* f_bias,
                                          const float* low, const float* norm_w, void* out, const int* seq_slot,
@@ -426,7 +418,7 @@ TKB_EXPORT int tkb_gated_recurrence_bf16(float* qfv, int row_stride, float* stat
                                         const float* states, int least, int phase, void* st) {
   return launch<__nv_bfloat16>(qfv, row_stride, state, f_bias, low, norm_w, out, seq_slot, seq_q_start, seq_q_len, n_seqs,
                                n_tokens, heads, dim, vdim, eps, write_state, raw,
-                               {bad, states, bad != nullptr ? least : INT_MAX}, phase, (cudaStream_t)st);
+                               {bad, states, phase != 0 ? least : INT_MAX, phase == 2}, phase, (cudaStream_t)st);
 }
 TKB_EXPORT int tkb_gated_recurrence_dpt() { return DPT; }
 TKB_EXPORT int tkb_gated_recurrence_cpt() { return CPT; }

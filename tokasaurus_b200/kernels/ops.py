@@ -896,7 +896,7 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
     _need(out.is_contiguous() and tuple(out.shape) == (T, heads * vdim), "gated_recurrence: out [T, heads * vdim]")
     f = _fn(_libs.get("recurrence.cu", **recurrence_defines(dim, vdim)), f"tkb_gated_recurrence_{_suffix(out.dtype)}")
     raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=qfv.device) if (split_heads and T > n_seqs) else None
-    # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the gates and the walk over what is left
+    # requests that bring many tokens go in chunks (csrc/decay_chunks.cu), between the walk over the others and a look at what is left
     n_chunks = 0
     if raw is not None and decay_chunk_modules(dim, vdim) and qfv.stride(0) % 4 == 0 and qfv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
         n_chunks = decay_chunk_count(T, n_seqs, lengths)
@@ -909,7 +909,7 @@ def gated_recurrence(qfv: torch.Tensor, state: torch.Tensor, f_bias: torch.Tenso
 
     if not n_chunks:
         return run(0, _NO_MARKS)
-    run(1, _NO_MARKS)
+    run(1, (c_void_p(0), c_void_p(0), c_int(DECAY_CHUNKS_FROM)))
     decay = qfv[:, heads * dim:2 * heads * dim]
     chunks = _decay_chunks(qfv[:, :heads * dim], None, qfv[:, 2 * heads * dim:], 1, None, None, decay, None, state.view(state.shape[0], -1),
                            raw, seq_slot, seq_q_start, seq_q_len, n_seqs, heads, dim, vdim, write_state, n_chunks)
