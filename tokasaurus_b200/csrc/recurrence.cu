@@ -187,6 +187,9 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
 
+// MARKS: what decay_chunks.cu left of its requests; else the requests below marks.least tokens (a build of its own: 52 registers in
+// place of 60, which is a third block an SM where a head is three blocks, and a step of 16 heads and 8 requests all resident at once).
+template <bool MARKS>
 __global__ void __launch_bounds__(SPLIT_THREADS_MAX)
 gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, float* __restrict__ state,
                               const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
@@ -207,7 +210,7 @@ gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, flo
   const int s = blockIdx.x, head = blockIdx.y;
   int n = seq_q_len[s], start = seq_q_start[s];
   const float* from = nullptr;
-  if (!walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from)) return;
+  if (MARKS ? !walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from) : n <= 0 || n >= marks.least) return;
   const int tid = threadIdx.x, lane = tid & (LANES - 1);
   const int cols_per_pass = blockDim.x / LANES;
   const int col_begin = blockIdx.z * cols_per_block;
@@ -215,7 +218,7 @@ gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, flo
   const int ncols = col_end - col_begin;
   const int col0 = tid / LANES;  // within the block's columns
   float* st = state + ((size_t)seq_slot[s] * heads + head) * (size_t)vdim * dim;
-  if (from == nullptr) from = st;
+  if (!MARKS) from = st;
   float S[CPT][DPT];
 #pragma unroll
   for (int c = 0; c < CPT; c++) {
@@ -378,10 +381,11 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
   const bool by_16 = dim % 4 == 0 && vdim % 4 == 0 && row_stride % 4 == 0 && (((uintptr_t)qfv) & 15) == 0;
   constexpr int SPLIT_SP = (DPT % 4 == 0) ? DPT + (((DPT / 4) % 2 == 0) ? 4 : 0) : DPT;  // as in the kernel
   const size_t smem_split = (size_t)CHUNK * (2 * (2 * LANES * SPLIT_SP + cols_per_block) + cols_per_block) * sizeof(float);
+  auto split_kernel = phase == 2 ? gated_recurrence_split_kernel<true> : gated_recurrence_split_kernel<false>;
   if (by_16 && smem_split <= 200 * 1024 && threads <= SPLIT_THREADS_MAX) {
     if (smem_split > 48 * 1024)
-      cudaFuncSetAttribute(gated_recurrence_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split);
-    rc = launch_pdl(gated_recurrence_split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
+      cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_split);
+    rc = launch_pdl(split_kernel, dim3(n_seqs, heads, split), dim3(threads), smem_split, st,
                     (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
                     cols_per_block, raw_out, marks);
   } else {
@@ -400,8 +404,7 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
 // raw: float32 [tokens, heads * vdim] scratch for the split form, or null (every block then owns a whole head).
 // The split form turns the q and f columns of qfv into gates in place.  phase 0: everything.  Where
 // decay_chunks.cu does the requests with at least `least` tokens (the split form, raw given), it runs between phase 1, the gates and the
-// walk over the other requests, and phase 2, the walk over what it left (bad, states: ChunkMarks) and the norm.  (One walk behind the
-// chunks cost 13 us where requests of 184 tokens stood beside one of 263: it no longer starts while the gates' kernel ends.)
+// walk over the other requests, and phase 2, the walk over what it left (bad, states: ChunkMarks) and the norm.
 TKB_EXPORT int tkb_gated_recurrence_f32(float* qfv, int row_stride, float* state, const float* f_bias,
                                         const float* low, const float* norm_w, void* out, const int* seq_slot,
                                         const int* seq_q_start, const int* seq_q_len, int n_seqs, int n_tokens,
