@@ -52,7 +52,8 @@ __global__ void recurrence_gates_kernel(float* __restrict__ qfv, int row_stride,
   }
 }
 
-template <typename T, bool PREGATED>
+// MARKS (with PREGATED): as in the kernel below.
+template <typename T, bool PREGATED, bool MARKS>
 __global__ void __launch_bounds__(1024)
 gated_recurrence_kernel(const float* __restrict__ qfv, int row_stride, float* __restrict__ state,
                         const float* __restrict__ f_bias, const float* __restrict__ low,
@@ -69,14 +70,15 @@ gated_recurrence_kernel(const float* __restrict__ qfv, int row_stride, float* __
   const int s = blockIdx.x, head = blockIdx.y;
   int n = seq_q_len[s], start = seq_q_start[s];
   const float* from = nullptr;
-  if (PREGATED ? !walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from) : n <= 0) return;
+  if (MARKS ? !walk_part(marks, seq_q_len, s, head, heads, (size_t)vdim * dim, start, n, from)
+            : n <= 0 || (PREGATED && n >= marks.least)) return;
   const int tid = threadIdx.x, lane = tid & (LANES - 1);
   const int cols_per_pass = blockDim.x / LANES;
   const int col_begin = blockIdx.z * cols_per_block;
   const int col_end = min(vdim, col_begin + cols_per_block);
   const int col0 = col_begin + tid / LANES;
   float* st = state + ((size_t)seq_slot[s] * heads + head) * (size_t)vdim * dim;
-  if (from == nullptr) from = st;
+  if (!MARKS) from = st;
 
   float S[CPT][DPT];
 #pragma unroll
@@ -187,8 +189,8 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
 
-// MARKS: what decay_chunks.cu left of its requests; else the requests below marks.least tokens (a build of its own: 52 registers in
-// place of 60, which is a third block an SM where a head is three blocks, and a step of 16 heads and 8 requests all resident at once).
+// MARKS: what decay_chunks.cu left of its requests; else the requests below marks.least tokens.  (A build of its own, so that the walk
+// keeps its registers: how many of its few long-lived blocks an SM takes goes by them.)
 template <bool MARKS>
 __global__ void __launch_bounds__(SPLIT_THREADS_MAX)
 gated_recurrence_split_kernel(const float* __restrict__ qfv, int row_stride, float* __restrict__ state,
@@ -363,14 +365,15 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
   const size_t smem = (size_t)CHUNK * (2 * dim + 2 * vdim) * sizeof(float);
   if (smem > 200 * 1024) return -2;
   if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(gated_recurrence_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(gated_recurrence_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gated_recurrence_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gated_recurrence_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gated_recurrence_kernel<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
   const int rows = n_tokens * heads;
   if (phase != 0 && raw == nullptr) return -2;
   float* raw_out = split > 1 || phase != 0 ? raw : nullptr;
   if (raw_out == nullptr)
-    return launch_pdl(gated_recurrence_kernel<T, false>, dim3(n_seqs, heads, 1), dim3(threads), smem, st,
+    return launch_pdl(gated_recurrence_kernel<T, false, false>, dim3(n_seqs, heads, 1), dim3(threads), smem, st,
                       (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start,
                       seq_q_len, heads, dim, vdim, eps, write_state, cols_per_block, raw_out, marks);
   int rc = 0;
@@ -389,7 +392,7 @@ int launch(float* qfv, int row_stride, float* state, const float* f_bias, const 
                     (const float*)qfv, row_stride, state, seq_slot, seq_q_start, seq_q_len, heads, dim, vdim, write_state,
                     cols_per_block, raw_out, marks);
   } else {
-    rc = launch_pdl(gated_recurrence_kernel<T, true>, dim3(n_seqs, heads, split), dim3(threads), smem, st,
+    rc = launch_pdl(phase == 2 ? gated_recurrence_kernel<T, true, true> : gated_recurrence_kernel<T, true, false>, dim3(n_seqs, heads, split), dim3(threads), smem, st,
                     (const float*)qfv, row_stride, state, f_bias, low, norm_w, (T*)out, seq_slot, seq_q_start, seq_q_len,
                     heads, dim, vdim, eps, write_state, cols_per_block, raw_out, marks);
   }
