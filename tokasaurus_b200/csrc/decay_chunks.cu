@@ -21,8 +21,9 @@
 // (mma.sync m16n8k16) cut their sums off instead of rounding them, so a chain of the six for 16 terms starts from zero, the
 // small ones first, and its result is added to the float32 sum with an ordinary addition.
 //
-// What bounds it: instruction issue and, with one block an SM in chunk_outputs, the loads that open a block; then the states'
-// way through the L2 (64 KB a chunk and head, four times).  Operands are cut once a block and not once a warp that reads
+// What bounds it: latency.  One block of 16 warps an SM (registers and shared memory) waits for the loads that open it and for chains
+// of six mma.sync: ncu shows the tensor pipe at 23 to 39 % and issue at 23 to 36 %; then the states' way through the L2 (64 KB a
+// chunk and head, four times).  Operands are cut once a block and not once a warp that reads
 // them (cut from the fragments into tf32 halves, the kernels took 132 us where they take 108 now).  Chunks of 64: half the
 // states' traffic of 32, and the products inside a chunk are still a third of the work.
 // Measured on B200: 2,048 tokens, 16 heads of 128 x 128: one decay a head 108 us (the walk 300), a decay a channel 137 us (358);
