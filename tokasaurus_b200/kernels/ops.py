@@ -454,14 +454,17 @@ def attn_decode_mma(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
                     n_dec: torch.Tensor, dec_cap: int, out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
                     page_size: int, scale: float, window: int | None,
                     out_row_of: torch.Tensor | None = None, item_entry: torch.Tensor | None = None,
-                    tma: bool = True, status: torch.Tensor | None = None) -> None:
+                    tma: bool = True, status: torch.Tensor | None = None, item_order: torch.Tensor | None = None) -> None:
     """bfloat16 split-key attention for requests that bring one token: ``items`` are (request row,
     first key, number of keys) triples, computed into float32 partial results and merged into
     ``out`` [T, n_heads*head_dim] at each request's token row (or at row ``out_row_of[request]``).
     ``n_items``/``n_dec`` are device counters; the launch grids are sized by ``items_cap``/``dec_cap``.
-    ``tma``: some work item is longer than three tiles (the kernel variant that fetches tiles by TMA pays)."""
+    ``tma``: some work item is longer than three tiles (the kernel variant that fetches tiles by TMA pays).
+    ``item_order``: (an item's three numbers, its place in ``items``) in the order in which the items' blocks start (with
+    ``item_entry``; None: as they are listed)."""
     _need_cuda(qkv, kcache, vcache, seq_q_start, seq_kv_len, page_indptr, page_ids, items, n_items, dec_seqs,
-               dec_item_start, n_dec, out, status)
+               dec_item_start, n_dec, out, status, item_order)
+    _need(item_order is None or item_order.numel() >= 4 * items_cap, "attn_decode_mma: item_order")
     check_head_dim(head_dim)
     _need(qkv.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16,
           "attn_decode_mma: bfloat16 only")
@@ -479,7 +482,7 @@ def attn_decode_mma(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
             _ptr(seq_q_start), _ptr(seq_kv_len), _ptr(page_indptr), _ptr(page_ids), _ptr(items), _ptr(n_items),
             c_int(items_cap), _ptr(part_o), _ptr(part_ml), c_int(n_heads), c_int(n_kv_heads), c_int(page_size),
             c_float(scale), c_int(window or 0), c_int(0), _ptr(None), c_int(0), c_int(0), c_int(kcache.shape[0]),
-            c_int(1 if tma else 0), _ptr(status), _ptr(counters), _ptr(item_entry), _ptr(dec_item_start),
+            c_int(1 if tma else 0), _ptr(status), _ptr(counters), _ptr(item_order), _ptr(item_entry), _ptr(dec_item_start),
             _ptr(out_row_of if out_row_of is not None else seq_q_start), _ptr(out), c_int(out.shape[1]), _ptr(None),
             _ptr(None), c_float(0.0), _stream()), "attn_decode_merged")
         return
@@ -502,13 +505,14 @@ def attn_decode_rope_mma(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.
                          window: int | None, inv_freq: torch.Tensor | None, rotary_dim: int,
                          write_cache: bool, status: torch.Tensor, item_entry: torch.Tensor | None = None,
                          tma: bool = True, bias: torch.Tensor | None = None, qk_norm: torch.Tensor | None = None,
-                         norm_eps: float = 0.0) -> None:
+                         norm_eps: float = 0.0, item_order: torch.Tensor | None = None) -> None:
     """``attn_decode_mma`` with rotary encoding and the cache write folded in: ``qkv`` holds the step's
     un-rotated q|k|v rows of requests that bring one token each, as bfloat16 [T, C] or as the float32 slices
     [slices, T, C] of a K-split product (``linear_smallm``); C = (n_heads + 2 n_kv_heads) * head_dim."""
     _need_cuda(qkv, kcache, vcache, seq_q_start, seq_kv_len, page_indptr, page_ids, items, n_items, dec_seqs,
-               dec_item_start, n_dec, out, inv_freq, status, bias, qk_norm)
+               dec_item_start, n_dec, out, inv_freq, status, bias, qk_norm, item_order)
     check_head_dim(head_dim)
+    _need(item_order is None or item_order.numel() >= 4 * items_cap, "attn_decode_rope_mma: item_order")
     C = (n_heads + 2 * n_kv_heads) * head_dim
     _check_qkv_stage(bias, qk_norm, C, head_dim)
     _need(kcache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "attn_decode_rope_mma: bfloat16 only")
@@ -536,7 +540,7 @@ def attn_decode_rope_mma(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.
             _ptr(n_items), c_int(items_cap), _ptr(part_o), _ptr(part_ml), c_int(n_heads), c_int(n_kv_heads),
             c_int(page_size), c_float(scale), c_int(window or 0), c_int(1), _ptr(inv_freq),
             c_int(rotary_dim), c_int(1 if write_cache else 0), c_int(kcache.shape[0]), c_int(1 if tma else 0),
-            _ptr(status), _ptr(counters),
+            _ptr(status), _ptr(counters), _ptr(item_order),
             _ptr(item_entry), _ptr(dec_item_start), _ptr(seq_q_start), _ptr(out), c_int(out.shape[1]), _ptr(bias),
             _ptr(qk_norm), c_float(norm_eps), _stream()), "attn_decode_merged")
         return
