@@ -131,3 +131,17 @@ def test_split_product_far_from_one(M, N, small, large):
         # as for numbers around one, and half a unit of the smallest number for a result that is one
         bound = 64 * 2.0 ** -24 * (x.abs().double() @ y.abs().double().T) + 2.0 ** -149
         assert ((out.double() - want).abs() <= bound).all()
+
+
+# rows that take 16-byte loads go to the kernel that brings the weights by TMA, others to the one that loads them itself; tokens are cut
+# ahead from 65 rows on; few and many blocks a slice, K slices in one block and in several
+@pytest.mark.parametrize("M", [3, 16, 31, 64, 65, 128, 300, 513])
+@pytest.mark.parametrize("N,K", [(129, 132), (3072, 1028), (2048, 2052), (300, 4100)])
+def test_both_split_kernels_give_the_same_bits(M, N, K):
+    g = torch.Generator().manual_seed(M + N)
+    a0, w0 = torch.randn(M, K + 1, generator=g).to(DEV), torch.randn(N, K + 1, generator=g).to(DEV)
+    a, w = a0[:, 1:], w0[:, 1:]  # (rows start where no 16-byte load may)
+    want = product(a, w)
+    out = torch.full((M, N + 5), 7.0, device=DEV)
+    product(a.contiguous(), w.contiguous(), out[:, :N])
+    assert torch.equal(out[:, :N], want) and (out[:, N:] == 7).all()

@@ -16,14 +16,20 @@ __device__ __forceinline__ uint32_t cut_pack(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
+// Two numbers' differences at once.
+__device__ __forceinline__ void cut_minus(float& a, float& b, uint32_t x, uint32_t y) {
+  asm("{\n.reg .b64 p, q;\nmov.b64 p, {%0, %1};\nmov.b64 q, {%2, %3};\nsub.rn.f32x2 p, p, q;\nmov.b64 {%0, %1}, p;\n}"
+      : "+f"(a), "+f"(b) : "r"(x), "r"(y));
+}
 // Two neighbouring numbers.
 __device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
   asm("{\n.reg .b64 x, s;\nmov.b64 x, {%0, %1};\nmov.b64 s, {%2, %2};\nmul.rn.f32x2 x, x, s;\nmov.b64 {%0, %1}, x;\n}"
       : "+f"(a), "+f"(b) : "f"(CUT_SCALE));  // both at once
   h = cut_pack(a, b);
-  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-  m = cut_pack(ra, rb);
-  l = cut_pack(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+  cut_minus(a, b, h << 16, h & 0xffff0000u);
+  m = cut_pack(a, b);
+  cut_minus(a, b, m << 16, m & 0xffff0000u);
+  l = cut_pack(a, b);
 }
 // Eight numbers -> three 16-byte pieces.
 __device__ __forceinline__ void cut8(const float4& x, const float4& y, uint4& h, uint4& m, uint4& l) {

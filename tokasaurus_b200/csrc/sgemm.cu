@@ -15,14 +15,16 @@
 //   bits the result is closer than an FMA chain's (normal numbers, K = 2,048 and 8,192: relative error 1.4e-7 and 1.5e-7).
 //   An element that does not come out finite (an infinity, a NaN or a number from 2^104 on among its inputs: 0 times infinity in a
 //   cut form is not what it is uncut; or a sum from 2^80 on) is done once more as the FMA chain, by the warp that has it (redo).
-//   What bounds it: with many rows the tensor instructions (six products: a sixth of their rate is the bound) and their
-//   operands' way through shared memory, with few the weights' way from memory.  A block is 15 warps that fetch, cut and
-//   store (the next chunks on their way into registers meanwhile) and one that issues the tensor instructions; all 16 read
-//   the sums.  The weights are on the 128-row side, 16 to 128 tokens on the other.  K is cut into slices by N and K alone,
-//   as many as fill the GPU when there are few rows; then each slice is a block's and a second kernel adds them in order.
-//   With enough row tiles to fill the GPU a block does all slices and adds them in the same order.
-//   Measured on B200 (the whole product): 4 rows x 16,384 x 2,048 633 us on the FP32 pipes, 44 us here
-//   (3.1 TB/s of weights); 500 rows the same 1,390 us, 250 us here (134 TFLOP/s of float32 products; the FP32 pipes have 74).
+//   K is cut into slices by N and K alone, as many as fill the GPU when there are few rows; then each slice is a block's and a
+//   second kernel adds them in order.  Where that ends sooner (slice_scratch) a block does all slices and adds them in the same order.
+//   Two kernels with the same bits: sgemm_tma_kernel where both operands' rows take 16-byte loads, sgemm_split_kernel (15 warps that
+//   fetch, cut and store, the next chunks on their way into registers meanwhile, and one that issues the tensor instructions) else.
+//   What bounds sgemm_tma_kernel: with many rows the tensor instructions (six products: a sixth of their rate is the bound; two
+//   thirds of a block's time they run, the rest goes on the sums' way out, for which there is no second buffer, and on blocks' starts),
+//   with few the warps that cut (clocks of a chunk of 64 k's: 1,250 of 1,900; at 40 GB/s an SM the weights take 1,550).
+//   Measured on B200 (the whole product; sgemm_split_kernel for all / sgemm_tma_kernel): 4 rows x 16,384 x 2,048 42.3 / 34.1 us (3.9
+//   TB/s of weights), x 2,048 x 8,192 25.2 / 20.9; 60 rows 49.1 / 46.2; 500 rows 255 / 190 us (177 TFLOP/s of float32 products),
+//   x 2,048 x 8,192 139 / 116.
 #include "per_device.h"
 #include "cut3.cuh"
 #include "tcgen05.cuh"
@@ -149,20 +151,14 @@ template <> __device__ __forceinline__ void tmem_read<32>(uint32_t a, float (&v)
 }
 
 // Eight numbers from p on, of which `left` are there (p null: none).
-template <bool VEC>
 __device__ __forceinline__ void fetch8(const float* __restrict__ p, int left, float4& x0, float4& x1) {
   x0 = x1 = make_float4(0.f, 0.f, 0.f, 0.f);
   if (p == nullptr) return;
-  if (VEC) {  // (K is a multiple of 4: a piece of four is there or not)
-    if (left > 0) x0 = __ldg(reinterpret_cast<const float4*>(p));
-    if (left > 4) x1 = __ldg(reinterpret_cast<const float4*>(p + 4));
-  } else {
-    float v[8];
+  float v[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) v[u] = u < left ? __ldg(p + u) : 0.f;
-    x0 = make_float4(v[0], v[1], v[2], v[3]);
-    x1 = make_float4(v[4], v[5], v[6], v[7]);
-  }
+  for (int u = 0; u < 8; u++) v[u] = u < left ? __ldg(p + u) : 0.f;
+  x0 = make_float4(v[0], v[1], v[2], v[3]);
+  x1 = make_float4(v[4], v[5], v[6], v[7]);
 }
 
 // Results that did not come out finite, once more as FMA chains over K in index order.  A warp: o[i * ldo] (i below `tokens`) of the
@@ -227,9 +223,9 @@ __device__ __forceinline__ void redo(float* o, int ldo, int tokens, bool there, 
 // their registers.
 template <int NT, bool VEC>
 __device__ __noinline__ void redo_tile(const float* __restrict__ A, const float* __restrict__ W, float* C, int M, int N, int K, int lda,
-                                       int ldw, int ldc) {
-  constexpr int CPT = SCfg<NT>::CPT;
-  const int n = blockIdx.x * 128 + (threadIdx.x & 127), m = blockIdx.y * NT + (threadIdx.x >> 7) * CPT;
+                                       int ldw, int ldc, int n0, int m0) {
+  constexpr int CPT = NT / 4;
+  const int n = n0 + (threadIdx.x & 127), m = m0 + (threadIdx.x >> 7) * CPT;
   redo<8, 32>(C + (size_t)m * ldc + n, ldc, min(CPT, M - m), n < N, A + (size_t)m * lda, lda, W + (size_t)min(n, N - 1) * ldw, K, VEC);
 }
 // What a block leaves in the place of its results when one of its waits ran out (a NaN of its own: no arithmetic makes it).
@@ -246,7 +242,7 @@ __device__ __noinline__ void redo_row(const float* __restrict__ part, const floa
 }
 
 // out: C when a block does all slices (`slices_here`), else the slices' partial results [slice][M][N].
-template <int NT, bool VEC>
+template <int NT>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N, int K,
                    int lda, int ldw, int ldc, int per_slice, int slices_here, int partial, int* __restrict__ status) {
@@ -403,12 +399,12 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
 #pragma unroll
       for (int i = 0; i < TASKS; i++) {
         if constexpr (KEPT) {
-          fetch8<VEC>(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
+          fetch8(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
         } else {
           const int r = r0 + i * ROWS;
           const bool is_w = r < 128, there = is_w ? n0 + r < N : r < 128 + NT && m0 + r - 128 < M;
           const float* p = (is_w ? W + (size_t)(n0 + r) * ldw : A + (size_t)(m0 + r - 128) * lda) + k;
-          fetch8<VEC>(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
+          fetch8(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
         }
       }
     };
@@ -449,11 +445,329 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
   tcgen05_fence_before();
   __syncthreads();
   if (tid == 0 && failed && status != nullptr) atomicOr(status, TKB_STATUS_WAIT_TIMEOUT);
-  if (!partial && !failed && odd) redo_tile<NT, VEC>(A, W, out, M, N, K, lda, ldw, ldc);
+  if (!partial && !failed && odd) redo_tile<NT, false>(A, W, out, M, N, K, lda, ldw, ldc, n0, m0);
   if (warp == 0) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Z::TMEM) : "memory");
   }
+}
+
+// ------------------------------------------------------------------- the split product with the weights by TMA
+// The same products in the same order, so the same bits, for operands that take 16-byte loads; sgemm_split_kernel does the others.
+// The weights come as they are (float32) into a ring of 32 KB stages, so that what is on its way does not wait for registers, and
+// their pieces go from the threads into tensor memory, from where the instructions take them: the instructions then read
+// only the tokens' pieces from shared memory, whose bandwidth was what 24 instructions of 128 x 16 and 128 x 128 a chunk spent most
+// time on.  A warp owns 32 of the 128 weight rows (a quarter of the lanes) and 16 of a chunk's 64 k's, and cuts a share of the tokens'
+// numbers, which it fetches itself a chunk ahead.  A block's column tiles are neighbours in the grid: they share the weights in the L2.
+// 16 warps cut and read the sums, one issues the instructions, one the copies.
+constexpr int TMA_THREADS = 608;
+constexpr int WORKERS = 16;            // warps that cut
+constexpr int RAW_BYTES = 128 * CHUNK * 4;
+
+template <int NT> struct TCfg {
+  static constexpr int PLANE = NT * 128;                         // a plane of the tokens' pieces
+  static constexpr int STAGES = NT <= 16 ? 4 : NT <= 32 ? 3 : 2; // of pieces: tokens in shared memory, weights in tensor memory
+  static constexpr int RAWS = NT <= 16 ? 6 : NT <= 64 ? 5 : 3;
+  static constexpr int SMEM = RAWS * RAW_BYTES + STAGES * 3 * PLANE + 1024;
+  static constexpr int BUFS = NT <= 64 ? 2 : 1;                  // of sums; one: the small sums are read first, and handed back
+  static constexpr int TMEM_W = 2 * NT * BUFS;                   // first column of the weights' pieces: 32 columns a plane
+  static constexpr int CPT = NT / 4;
+  static constexpr bool PRECUT = NT > 64;                        // the tokens' pieces are there (sgemm_cut_kernel) and come by TMA
+  static constexpr int NA = NT / 8;                              // else: numbers of the tokens that a thread cuts
+};
+static_assert(TCfg<16>::SMEM <= 227 * 1024 && TCfg<32>::SMEM <= 227 * 1024 && TCfg<64>::SMEM <= 227 * 1024 && TCfg<128>::SMEM <= 227 * 1024, "");
+static_assert(TCfg<128>::TMEM_W + 2 * 96 <= 512 && TCfg<64>::TMEM_W + 2 * 96 <= 512 && TCfg<16>::TMEM_W + 4 * 96 <= 512, "");
+
+// D += A B with A in tensor memory (row = lane, two neighbouring k's a column)
+__device__ __forceinline__ void umma_a_tmem(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_put4(uint32_t addr, const uint4& x) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+}
+__device__ __forceinline__ void prefetch_box(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
+template <int NT>
+__global__ void __launch_bounds__(TMA_THREADS, 1)
+sgemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const float* __restrict__ A, const float* __restrict__ W,
+                 float* __restrict__ out, int M, int N, int K, int lda, int ldw, int ldc, int col_tiles, int per_slice,
+                 int slices_here, int partial, int* __restrict__ status) {
+  using Z = TCfg<NT>;
+  constexpr int CPT = Z::CPT, STAGES = Z::STAGES, RAWS = Z::RAWS, BUFS = Z::BUFS, NA = Z::NA;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t raw_full[RAWS], raw_empty[RAWS], full_bar[STAGES], empty_bar[STAGES], acc_full[BUFS], small_empty[BUFS],
+      big_empty[BUFS], tok_full[STAGES];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int failed, odd;  // a wait ran out; some result is not finite
+  unsigned char* raws = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* planes = raws + RAWS * RAW_BYTES;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tile = blockIdx.x / col_tiles, n0 = tile * 128, m0 = (blockIdx.x - tile * col_tiles) * NT;
+  const int chunks_all = (K + CHUNK - 1) / CHUNK;
+  const int c_begin = blockIdx.z * per_slice;  // (one slice a block when there are several blocks in z)
+  const int n_chunks = min(chunks_all, c_begin + per_slice * slices_here) - c_begin;
+  trigger_dependents();
+  if (tid == 0) {
+    for (int s = 0; s < RAWS; s++) mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], WORKERS);
+    for (int s = 0; s < STAGES; s++) mbar_init(&full_bar[s], WORKERS), mbar_init(&empty_bar[s], 1), mbar_init(&tok_full[s], 1);
+    for (int s = 0; s < BUFS; s++) mbar_init(&acc_full[s], 1), mbar_init(&small_empty[s], WORKERS), mbar_init(&big_empty[s], WORKERS);
+    failed = odd = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == WORKERS + 1 && lane < 2)  // into the L2 only while the kernel ahead runs: whoever wrote the weights may be in flight
+    for (int c = 0; c < RAWS && c < n_chunks; c++) prefetch_box(&map_w, (c_begin + c) * CHUNK + 32 * lane, n0);
+  grid_dependency_wait();
+  if (warp == WORKERS) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = tmem_slot;
+  // a group of chunks ends with the slice or after GROUP chunks; `at`: the chunk's place in its slice
+  auto ends_slice = [&](int c, int at) { return at + 1 == per_slice || c + 1 == n_chunks; };
+  auto ends_group = [&](int c, int at) { return at % GROUP == GROUP - 1 || ends_slice(c, at); };
+  const int n = n0 + (warp & 3) * 32 + lane, col0 = (warp >> 2) * CPT;
+  float* o = (partial ? out + (size_t)blockIdx.z * M * N : out) + n;
+  const int ldo = partial ? N : ldc;
+  bool ok = true;
+
+  if (warp == WORKERS + 1) {
+    // ---------------- the weights' way in
+    int c = 0;
+    for (; c < n_chunks; c++) {
+      const int s = c % RAWS;
+      if (failed || (c >= RAWS && !mbar_wait_idle(&raw_empty[s], ((c / RAWS) - 1) & 1))) { ok = false; break; }
+      if (lane == 0) mbar_expect_tx(&raw_full[s], RAW_BYTES);
+      __syncwarp();
+      if (lane < 2) tma_load_2d(raws + s * RAW_BYTES + lane * (RAW_BYTES / 2), &map_w, &raw_full[s], (c_begin + c) * CHUNK + 32 * lane, n0);
+    }
+    if (!ok)  // nothing of this block's is on its way when it leaves
+      for (int i = max(0, c - RAWS); i < c; i++) mbar_wait_idle(&raw_full[i % RAWS], (i / RAWS) & 1);
+  } else if (warp == WORKERS + 2) {
+    // ---------------- the tokens' pieces, where they have been cut ahead
+    if constexpr (Z::PRECUT) {
+      int c = 0;
+      for (; c < n_chunks; c++) {
+        const int s = c % STAGES;
+        if (failed || (c >= STAGES && !mbar_wait_idle(&empty_bar[s], ((c / STAGES) - 1) & 1))) { ok = false; break; }
+        if (lane == 0) mbar_expect_tx(&tok_full[s], 3 * Z::PLANE);
+        __syncwarp();
+        if (lane < 3) tma_load_2d(planes + (s * 3 + lane) * Z::PLANE, &map_a, &tok_full[s], (c_begin + c) * CHUNK, lane * M + m0);
+      }
+      if (!ok)
+        for (int i = max(0, c - STAGES); i < c; i++) mbar_wait_idle(&tok_full[i % STAGES], (i / STAGES) & 1);
+    }
+  } else if (warp == WORKERS) {
+    // ---------------- tensor instructions
+    constexpr uint32_t idesc = make_idesc(128, NT);
+    const uint64_t desc0 = make_desc(smem_u32(planes));
+    int group = 0, at = 0;
+    bool fresh = true;
+    for (int c = 0; c < n_chunks; c++) {
+      const int s = c % STAGES, buf = group % BUFS;
+      const bool reused = fresh && group >= BUFS;
+      if (reused && !mbar_wait(&small_empty[buf], ((group / BUFS) - 1) & 1)) { ok = false; break; }
+      if (!mbar_wait(&full_bar[s], (c / STAGES) & 1)) { ok = false; break; }
+      if (Z::PRECUT && !mbar_wait(&tok_full[s], (c / STAGES) & 1)) { ok = false; break; }
+      tcgen05_fence_after();
+      const uint32_t big = tmem + buf * 2 * NT, small = big + NT, first = fresh ? 0u : 1u, w = tmem + Z::TMEM_W + s * 96;
+      const uint64_t a = desc0 + (uint64_t)(s * (3 * Z::PLANE >> 4));
+      auto mma = [&](uint32_t d, int wp, int ap, int k, uint32_t more) {
+        umma_a_tmem(d, w + wp * 32 + 8 * k, a + (ap * (Z::PLANE >> 4) + 2 * k), idesc, more);
+      };
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(small, 1, 1, k, k == 0 ? first : 1u);
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(small, 0, 2, k, 1u);
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(small, 2, 0, k, 1u);
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(small, 0, 1, k, 1u);
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(small, 1, 0, k, 1u);
+      if (reused) {
+        if (!mbar_wait(&big_empty[buf], ((group / BUFS) - 1) & 1)) { ok = false; break; }
+        tcgen05_fence_after();
+      }
+#pragma unroll
+      for (int k = 0; k < CHUNK / UMMA_K; k++) mma(big, 0, 0, k, k == 0 ? first : 1u);
+      commit_warp(&empty_bar[s]);
+      fresh = false;
+      if (ends_group(c, at)) {
+        commit_warp(&acc_full[buf]);
+        group++;
+        fresh = true;
+      }
+      if (++at == per_slice) at = 0;
+    }
+  } else {
+    // ---------------- reading the sums of a group: features across the lanes of a warp, tokens across its registers.  A slice's
+    // sums go to memory when the slice ends; a block that does several adds each to what it left there itself.
+    float acc[CPT];
+#pragma unroll
+    for (int i = 0; i < CPT; i++) acc[i] = 0.f;
+    const uint32_t quarter = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t sums = tmem + quarter + col0;
+    int drained = 0;
+    bool first_slice = true;
+    constexpr int RD = CPT < 16 ? CPT : NT == 64 ? 8 : 16;
+    auto add = [&](uint32_t from) {
+#pragma unroll
+      for (int i0 = 0; i0 < CPT; i0 += RD) {
+        float v[RD];
+        tmem_read<RD>(from + i0, v);
+#pragma unroll
+        for (int i = 0; i < RD; i++) acc[i0 + i] = fmaf(v[i], CUT_BACK, acc[i0 + i]);
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+    };
+    auto drain = [&](bool slice_ends, bool last) {  // the oldest group not yet read; false if its sums never come
+      const int buf = drained % BUFS;
+      if (!mbar_wait(&acc_full[buf], (drained / BUFS) & 1)) return false;
+      tcgen05_fence_after();
+      add(sums + buf * 2 * NT + NT);
+      if (lane == 0) mbar_arrive(&small_empty[buf]);
+      add(sums + buf * 2 * NT);
+      if (lane == 0) mbar_arrive(&big_empty[buf]);
+      drained++;
+      if (slice_ends) {
+#pragma unroll
+        for (int i0 = 0; i0 < CPT; i0 += RD) {  // what is there comes together: a load behind each store took 5 us a slice
+          float was[RD];
+#pragma unroll
+          for (int i = 0; i < RD; i++)
+            was[i] = !first_slice && n < N && m0 + col0 + i0 + i < M ? o[(size_t)(m0 + col0 + i0 + i) * ldo] : 0.f;
+#pragma unroll
+          for (int i = 0; i < RD; i++) {
+            const int m = m0 + col0 + i0 + i;
+            if (n < N && m < M) {
+              const float x = first_slice ? acc[i0 + i] : was[i] + acc[i0 + i];
+              o[(size_t)m * ldo] = x;
+              if (last && !isfinite(x)) odd = 1;
+            }
+            acc[i0 + i] = 0.f;
+          }
+        }
+        first_slice = false;
+      }
+      return true;
+    };
+    // ---------------- the tokens' numbers: NA neighbouring ones of a row
+    constexpr int PER = Z::PRECUT ? 2 : NA, TPR = CHUNK / PER;  // threads a row
+    const int ar = tid / TPR, ak = (tid % TPR) * PER;
+    float xa[PER];
+    auto fetch = [&](int c) {
+      const int k = (c_begin + c) * CHUNK + ak;
+      const bool there = c < n_chunks && m0 + ar < M;
+      const float* p = A + (size_t)(m0 + ar) * lda + k;
+      if constexpr (PER == 2) {
+        const float2 x = there && k < K ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f);
+        xa[0] = x.x, xa[1] = x.y;
+      } else {
+#pragma unroll
+        for (int u = 0; u < PER; u += 4) {
+          const float4 x = there && k + u < K ? __ldg(reinterpret_cast<const float4*>(p + u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          xa[u] = x.x, xa[u + 1] = x.y, xa[u + 2] = x.z, xa[u + 3] = x.w;
+        }
+      }
+    };
+    const int wr = (warp & 3) * 32 + lane, kq = warp >> 2;  // the thread's weight row, and its 16 of the 64 k's
+    const unsigned char* raw_row = raws + (kq >> 1) * (RAW_BYTES / 2) + wr * 128;
+    bool waiting = false, waiting_ends = false;  // a group to be read, and whether its slice ends with it
+    int at = 0;                                  // the chunk's place in its slice
+    if constexpr (!Z::PRECUT) fetch(0);
+#pragma unroll 1
+    for (int c = 0; c < n_chunks; c++) {
+      const int s = c % STAGES, rs = c % RAWS;
+      if (failed || !mbar_wait(&raw_full[rs], (c / RAWS) & 1)) { ok = false; break; }
+      float4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        x[u] = *reinterpret_cast<const float4*>(raw_row + rs * RAW_BYTES + ((((kq & 1) * 4 + u) ^ (wr & 7)) << 4));
+      if (c >= STAGES && !mbar_wait(&empty_bar[s], ((c / STAGES) - 1) & 1)) { ok = false; break; }
+      tcgen05_fence_after();
+      const uint32_t wt = tmem + quarter + Z::TMEM_W + s * 96 + kq * 8;
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        uint4 h, m, l;
+        cut8(x[2 * u], x[2 * u + 1], h, m, l);
+        tmem_put4(wt + 4 * u, h);
+        tmem_put4(wt + 32 + 4 * u, m);
+        tmem_put4(wt + 64 + 4 * u, l);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&raw_empty[rs]);
+      if constexpr (!Z::PRECUT) {
+        unsigned char* dst = planes + s * 3 * Z::PLANE + ar * 128 + (((ak >> 3) ^ (ar & 7)) << 4) + (ak & 7) * 2;
+        uint32_t h[PER / 2], m[PER / 2], l[PER / 2];
+#pragma unroll
+        for (int u = 0; u < PER / 2; u++) cut2(xa[2 * u], xa[2 * u + 1], h[u], m[u], l[u]);
+        auto put = [&](unsigned char* p, const uint32_t (&x)[PER / 2]) {
+          if constexpr (PER == 8) *reinterpret_cast<uint4*>(p) = make_uint4(x[0], x[1], x[2], x[3]);
+          else if constexpr (PER == 4) *reinterpret_cast<uint2*>(p) = make_uint2(x[0], x[1]);
+          else *reinterpret_cast<uint32_t*>(p) = x[0];
+        };
+        put(dst, h);
+        put(dst + Z::PLANE, m);
+        put(dst + 2 * Z::PLANE, l);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[s]);
+      if constexpr (!Z::PRECUT) fetch(c + 1);
+      // a group is read behind the storing of the chunk that follows it
+      if (waiting && !drain(waiting_ends, false)) { ok = false; break; }
+      waiting = ends_group(c, at);
+      waiting_ends = ends_slice(c, at);
+      if (++at == per_slice) at = 0;
+    }
+    if (ok) ok = drain(true, true);
+    if (!ok)  // a wait ran out: nothing that could be taken for a result stays behind
+      for (int i = 0; i < CPT; i++)
+        if (n < N && m0 + col0 + i < M) o[(size_t)(m0 + col0 + i) * ldo] = __int_as_float(LOST);
+  }
+  if (!ok) failed = 1;
+  tcgen05_fence_before();
+  __syncthreads();
+  if (tid == 0 && failed && status != nullptr) atomicOr(status, TKB_STATUS_WAIT_TIMEOUT);
+  if (!partial && !failed && odd && warp < WORKERS) redo_tile<NT, true>(A, W, out, M, N, K, lda, ldw, ldc, n0, m0);
+  if (warp == WORKERS) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// The tokens' numbers cut ahead: planes [3][M][ld] of bfloat16, ld = K rounded up to 8.  From 65 rows on: a block of sgemm_tma_kernel
+// has 128 of them and would cut as many numbers of theirs as of the weights, again in every row tile (500 rows x 16,384 x 2,048: 211 us cut there,
+// 190 with this kernel).
+__global__ void __launch_bounds__(256) sgemm_cut_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, int M, int K, int lda, int ld) {
+  trigger_dependents();
+  grid_dependency_wait();
+  const size_t id = (size_t)blockIdx.x * 256 + threadIdx.x;
+  const int pieces = ld / 8;
+  const size_t r = id / pieces;
+  if (r >= (size_t)M) return;
+  const int k = (int)(id - r * pieces) * 8;
+  const float* p = A + r * lda + k;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 x = __ldg(reinterpret_cast<const float4*>(p)), y = k + 4 < K ? __ldg(reinterpret_cast<const float4*>(p + 4)) : zero;
+  uint4 h, m, l;
+  cut8(x, y, h, m, l);
+  __nv_bfloat16* o = planes + r * ld + k;
+  const size_t plane = (size_t)M * ld;
+  *reinterpret_cast<uint4*>(o) = h;
+  *reinterpret_cast<uint4*>(o + plane) = m;
+  *reinterpret_cast<uint4*>(o + 2 * plane) = l;
 }
 
 // C = the slices' results, added in order.
@@ -486,23 +800,48 @@ int chunks_a_slice(int N, int K) {
   return (chunks + s - 1) / s;
 }
 
-template <int NT, bool VEC>
-int split_launch(const float* A, const float* W, float* C, float* part, int M, int N, int K, int lda, int ldw, int ldc,
+// float32 [rows, K] with row stride ld: boxes of 128 rows x 32 numbers, 128-byte swizzle
+int make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld) {
+  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {32, 128}, estr[2] = {1, 1};
+  const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
+}
+
+// vec: both operands' rows take 16-byte loads
+template <int NT>
+int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, float* part, int M, int N, int K, int lda, int ldw, int ldc, bool vec,
                  int* status, cudaStream_t st) {
   static SharedMemoryRequest shared_memory;
-  int rc = shared_memory({{(const void*)sgemm_split_kernel<NT, VEC>, SCfg<NT>::SMEM}});
+  int rc = shared_memory({{(const void*)sgemm_split_kernel<NT>, SCfg<NT>::SMEM}, {(const void*)sgemm_tma_kernel<NT>, TCfg<NT>::SMEM}});
   if (rc) return rc;
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
-  const dim3 block(SPLIT_THREADS);
   const int tiles = (N + 127) / 128, rows = (M + NT - 1) / NT;
-  if (part == nullptr)
-    return launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, 1), block, (size_t)SCfg<NT>::SMEM, st, A, W, C, M, N, K,
-                      lda, ldw, ldc, per, slices, 0, status);
-  rc = launch_pdl(sgemm_split_kernel<NT, VEC>, dim3(tiles, rows, slices), block, (size_t)SCfg<NT>::SMEM, st, A, W, part, M,
-                      N, K, lda, ldw, ldc, per, 1, 1, status);
-  if (rc) return rc;
+  const int here = part == nullptr ? slices : 1, partial = part != nullptr;
+  float* out = partial ? part : C;
+  if (vec && (long long)tiles * rows < (1ll << 31)) {
+    CUtensorMap map, map_a;
+    memset(&map_a, 0, sizeof(map_a));
+    rc = get_encode();
+    if (rc == 0) rc = make_map_f32(&map, W, N, K, ldw);
+    if constexpr (TCfg<NT>::PRECUT) {
+      const int ld = (K + 7) / 8 * 8;
+      if (rc == 0) rc = make_map(&map_a, cut, 3 * M, K, ld, NT);
+      const long long blocks = ((long long)M * (ld / 8) + 255) / 256;
+      if (rc == 0) rc = launch_pdl(sgemm_cut_kernel, dim3((unsigned)blocks), dim3(256), 0, st, A, cut, M, K, lda, ld);
+    }
+    if (rc) return rc;
+    rc = launch_pdl(sgemm_tma_kernel<NT>, dim3(tiles * rows, 1, slices / here), dim3(TMA_THREADS), (size_t)TCfg<NT>::SMEM, st, map, map_a, A, W,
+                    out, M, N, K, lda, ldw, ldc, rows, per, here, partial, status);
+  } else {
+    rc = launch_pdl(sgemm_split_kernel<NT>, dim3(tiles, rows, slices / here), dim3(SPLIT_THREADS), (size_t)SCfg<NT>::SMEM, st, A, W, out,
+                    M, N, K, lda, ldw, ldc, per, here, partial, status);
+  }
+  if (rc || !partial) return rc;
   return launch_pdl(sgemm_add_slices_kernel, dim3((N + 255) / 256, M), dim3(256), 0, st, (const float*)part, A, W, C, M, N, K,
-                    lda, ldw, ldc, slices, (int)VEC);
+                    lda, ldw, ldc, slices, (int)vec);
 }
 
 // Token columns of an instruction: the fewest that hold all rows, at most 128.
@@ -510,14 +849,25 @@ int token_columns(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 1
 
 }  // namespace
 
-// Float32 values of scratch that tkb_sgemm_tn_f32 wants for these sizes (0: none): the K slices' partial results, when one
-// block a slice is what fills the GPU.  With row tiles for three quarters of the SMs a block does all slices itself.
+// Scratch, in float32 values: the tokens' pieces where they are cut ahead, then the K slices' partial results, when one block a
+// slice ends sooner than blocks that do all of K (500 rows x 3,072 x 2,048: 69 us in slices, 60 in 96 blocks; 300 rows 51 and 58;
+// 700 rows x 2,048 x 2,048 83 and 63).  The results' bits do not depend on it.
+static long long cut_scratch(int M, int K) { return token_columns(M) > 64 ? (3ll * M * ((K + 7) / 8 * 8) + 7) / 8 * 4 : 0; }
+static long long slice_scratch(int M, int N, int K) {
+  const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
+  const long long blocks = (long long)((N + 127) / 128) * ((M + token_columns(M) - 1) / token_columns(M)), sms = tkb::sm_count();
+  auto waves = [&](long long b) { return (b + sms - 1) / sms; };
+  // in chunks (1.3 us): a block's start and end are worth five, a slice added to those before it three, the adding kernel three
+  // and its traffic
+  const long long all = waves(blocks) * (chunks + 3 * slices + 5);
+  const long long sliced = waves(blocks * slices) * (per + 5) + 3 + (long long)slices * M * N / 800000;
+  if (slices == 1 || all <= sliced || M > 65535) return 0;
+  return (long long)slices * M * N;
+}
+// Float32 values of scratch that tkb_sgemm_tn_f32 wants for these sizes (0: none).
 TKB_EXPORT long long tkb_sgemm_tn_scratch(int M, int N, int K) {
   if (M <= 0 || N < SPLIT_MIN || K < SPLIT_MIN) return 0;
-  const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
-  const long long blocks = (long long)((N + 127) / 128) * ((M + token_columns(M) - 1) / token_columns(M));
-  if (slices == 1 || blocks * 4 >= 3ll * tkb::sm_count() || M > 65535) return 0;
-  return (long long)slices * M * N;
+  return cut_scratch(M, K) + slice_scratch(M, N, K);
 }
 
 // scratch: as many float32 values as tkb_sgemm_tn_scratch says, or null where it says 0.  status: the device status word that
@@ -531,10 +881,10 @@ TKB_EXPORT int tkb_sgemm_tn_f32(const float* A, const float* W, float* C, float*
     if ((scratch != nullptr) != (tkb_sgemm_tn_scratch(M, N, K) > 0)) return -4;
     const int nt = token_columns(M);
     if ((M + nt - 1) / nt > 65535) return -3;
-    const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
-#define TKB_GO(NT)                                                                                                  \
-  return vec ? split_launch<NT, true>(A, W, C, scratch, M, N, K, lda, ldw, ldc, status, st)                                  \
-             : split_launch<NT, false>(A, W, C, scratch, M, N, K, lda, ldw, ldc, status, st);
+    const bool vec = 3ll * M < (1ll << 31) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+    __nv_bfloat16* cut = reinterpret_cast<__nv_bfloat16*>(scratch);
+    float* part = slice_scratch(M, N, K) ? scratch + cut_scratch(M, K) : nullptr;
+#define TKB_GO(NT) return split_launch<NT>(A, W, C, cut, part, M, N, K, lda, ldw, ldc, vec, status, st);
     if (nt == 16) { TKB_GO(16) }
     if (nt == 32) { TKB_GO(32) }
     if (nt == 64) { TKB_GO(64) }
