@@ -1,0 +1,66 @@
+"""Prompt portions on tcgen05 whose heads are shared out among units of a block: every number of key tiles for every number of units
+that take them in turn, odd groups of heads, windows, and scores that are not finite."""
+
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, i32, make_paged, run_mma_attention
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tokasaurus_b200.kernels import ops
+
+    return ops
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nh,nkv,ps,window", [(3, 1, 16, None), (4, 2, 5, None), (5, 1, 8, 100)])
+@pytest.mark.parametrize("single", [False, True])
+def test_numbers_of_key_tiles(ops, hd, nh, nkv, ps, window, single):
+    """Portions that end 1 to 12 tiles of 64 keys behind their requests' beginnings: fewer tiles than units, as many, more, and
+    rounds of the ring of tiles."""
+    lens_kv = [2, 63, 65, 128, 129, 193, 257, 320, 383, 450, 513, 641, 767]
+    lens_q = [2, 63, 3, 128, 100, 2, 65, 64, 5, 130, 2, 2, 66]
+    got, want = run_mma_attention(ops, lens_q, lens_kv, nh, nkv, hd, ps, window, seed=hd + nh, tc=True, single_heads=single)
+    assert not torch.isnan(got).any()
+    torch.testing.assert_close(got, want, rtol=1.6e-2, atol=1.2e-2)  # the bound of the other tests of these kernels
+    again, _ = run_mma_attention(ops, lens_q, lens_kv, nh, nkv, hd, ps, window, seed=hd + nh, tc=True, single_heads=single)
+    assert torch.equal(got, again)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("value", [math.nan, math.inf])
+def test_scores_that_are_not_finite(ops, hd, single, value):
+    """A row of q that holds a NaN or an infinity is NaN, and nothing of it reaches other rows or heads."""
+    import numpy as np
+    from types import SimpleNamespace
+
+    from tokasaurus_b200.parts.attention import plan_attention
+
+    nh, nkv, ps, L, n = 3, 1, 16, 400, 150
+    kc, vc, indptr, pages, _, _ = make_paged(torch.bfloat16, 1, [L], nkv, hd, ps, 30, seed=2)
+    plan = plan_attention(SimpleNamespace(seq_q_len=np.asarray([n], dtype=np.int32), seq_kv_len=np.asarray([L], dtype=np.int32)), None,
+                          query_tile=128)
+    c = i32(plan["counts"])
+
+    def run(qkv):
+        out, status = torch.zeros(n, nh * hd, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.attn_prefill_tc(qkv.to(DEV), out, kc, vc, i32([0]), i32([n]), i32([L]), indptr, pages, i32(plan["tiles"]), c[2:3],
+                            int(plan["counts"][2]), nh, nkv, hd, ps, hd ** -0.5, None, status, single_heads=single)
+        assert int(status) == 0
+        return out.view(n, nh, hd)
+
+    qkv = torch.randn(n, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    want = run(qkv)
+    qkv[77, hd + 3] = value
+    got = run(qkv)
+    assert got[77, 1].isnan().all()
+    keep = torch.ones(n, nh, dtype=torch.bool)
+    keep[77, 1] = False
+    assert torch.equal(got[keep.to(DEV)], want[keep.to(DEV)])

@@ -1,33 +1,38 @@
 // Causal attention for prompt portions on the fifth-generation tensor cores (head size 64, bfloat16).
 //
 // A block owns 128 consecutive query tokens of TWO query heads that share a kv head (one head where the group
-// size is odd and no partner is left) and walks the keys they may see in tiles of 128.  The K and V tiles are
-// gathered once for both heads.  For each head:
-//     S = Q . K^T      tcgen05.mma 128 x 128 x 16, four per tile, Q and K tiles K-major in shared memory,
+// size is odd and no partner is left, or where pairs would leave SMs without a block) and walks the keys they may see
+// in tiles of 64, which are brought once for both heads.  Four UNITS share the work: each has 128 rows of one head, every
+// second tile (two heads) or every fourth (one head), and scores, reference, sum and output of its own; a head's units are put
+// together at the end.  For each unit and tile:
+//     S = Q . K^T      tcgen05.mma 128 x 64 x 16, four per tile, Q and K tiles K-major in shared memory,
 //                      S (float32) in tensor memory
-//     softmax          a warpgroup per head, one thread per query row (a lane of tensor memory): two passes of
-//                      tcgen05.ld over S (row maximum, then exp2 and row sum), no shuffles; P (bfloat16) goes to
-//                      shared memory in the 128-byte-swizzled K-major layout
-//     O += P . V       tcgen05.mma 128 x 64 x 16, eight per tile, accumulating in tensor memory over ALL tiles; V
-//                      stays as the cache holds it ([key][head size]), described to the tensor core as an
+//     softmax          a warpgroup per unit, one thread per query row (a lane of tensor memory): the row's 64 scores come into
+//                      registers once, row maximum, then exp2 and row sum, no shuffles; P (bfloat16) goes back to tensor memory,
+//                      over the row's own scores
+//     O += P . V       tcgen05.mma 128 x 64 x 16 with P from tensor memory, four per tile, accumulating in tensor memory over ALL
+//                      the unit's tiles; V stays as the cache holds it ([key][head size]), described to the tensor core as an
 //                      MN-major operand
 // The exponentials of a row use a reference that stays put while the row's scores stay below reference + 16
 // (probabilities up to 2^16 are no problem for bfloat16 or for float32 sums).  When a row tops that, its warp
-// waits for the P . V products issued so far, reads its 32 lanes of O, scales the rows concerned and writes
-// them back (tcgen05.st): rare after the first tiles, so the loop has no pass over O and a thread keeps no
-// output in registers (104 registers a thread; folding an O tile into registers every key tile took 158 and
-// measured 2 % slower).  The row sum l follows the same reference; O / l at the end does not depend on it.
-// Roles: warps 0-3 and 4-7 softmax and output of the two heads; warp 8 brings K tiles and warp 9 V tiles, two
-// buffers each: a tile whose 128 keys all exist comes by TMA, one box per page through the block table (page
-// sizes that are powers of two from 8 up); the request's last, partial tile and other page sizes are gathered
-// with cp.async, zero-filling keys beyond the request.  Warps 10 and 11 issue the MMAs, one lane each, one
-// warp per head: the tensor core is fed by single threads, and two instruction streams feed it twice as fast.
-// Warp 10 also allocates tensor memory.  The second head starts half a tile behind the first, so that one
-// head's exponentials run while the other scans for its row maxima.  P is double buffered: after a thread has
-// handed P_j over it never waits for P_j . V; the tensor core computes Q . K_{j+1}^T first, then P_j . V, while
-// the thread starts on S_{j+1}.  The softmax warps (one a scheduler and head) are the bound: trading ex2 for a
-// polynomial on the FMA pipe, or pairs of float32 operations for the packed f32x2 forms, measured no faster.
-// One block per SM (225 KiB of shared memory, 384 columns of tensor memory in use).  Tensor memory is taken only
+// reads its 32 lanes of O, scales the rows concerned and writes them back (tcgen05.st): rare after the first tiles, so the
+// loop has no pass over O.  (S_j is complete only after P_(j-1) . V: one thread issues both, in that order.)
+// What bounds it: exponentials and the chain a unit goes through for each of its tiles (scores into registers, maximum, exponentials, P,
+// the wait for the unit's slowest warp, the issue of eight instructions, S), about 3,000 clocks with four units at once; of 128
+// keys of two heads the exponentials alone take 1,540 (three quarters on the special-function unit, a quarter as a polynomial).
+// Neither the products nor the scan for the maximum: a quarter of the instructions left out, or the scan, changed nothing.
+// Four units and not two: with one warp a scheduler and head (the form before, tiles of 128 keys, P through shared memory) 128 keys took
+// 3,490 clocks, in which waits for S and the exponentials hardly overlapped; taking turns at the exponentials, skewing the heads and a
+// polynomial for some of them changed nothing there.
+// Measured (32 heads on 8 kv heads, the form before / now): one prompt of 2,048 tokens 44.7 / 41.9 us, of 8,192 477 / 400 us (688 TFLOP/s of
+// causal flops), 2,048 tokens behind 2,048 others 107 / 93, 512 behind 2,048 (one head a block) 38 / 29; 24 heads on 8, 2,048
+// tokens 48.5 / 39.7.
+// Roles: warps 0-15 softmax and output of the four units, one warp of each also issues its unit's MMAs (warps of their own took 440
+// clocks longer a tile: their instructions, polls among them, share the schedulers with four busy warps each); warp 16 brings K
+// tiles and warp 17 V tiles into a ring: a tile whose 64 keys all exist comes by TMA, one box per page through the block table
+// (page sizes that are powers of two from 8 up); the request's last, partial tile and other page sizes are gathered with
+// cp.async, zero-filling keys beyond the request.  Warp 16 also allocates tensor memory.
+// One block per SM (all 512 columns of tensor memory).  Tensor memory is taken only
 // after the kernel ahead in the stream has finished.  Every wait on an mbarrier is bounded; after the limit
 // the block sets TKB_STATUS_WAIT_TIMEOUT and leaves.
 #include "tcgen05.cuh"
@@ -38,14 +43,18 @@ namespace {
 
 constexpr int HD = 64;
 constexpr int BQ = 128;   // queries per block
-constexpr int BKV = 128;  // keys per tile
-constexpr int THREADS = 384;
+constexpr int BKV = 64;   // keys per tile
+constexpr int UNITS = 4;
+constexpr int STAGES = 10; // tiles of K and V on their way or in use
+static_assert(STAGES >= UNITS, "a unit's next tile is at most one round of the ring further");
+constexpr int SOFTMAX_WARPS = 4 * UNITS;
+constexpr int THREADS = (SOFTMAX_WARPS + 2) * 32;
 constexpr int Q_BYTES = BQ * HD * 2;    // 16 KiB
-constexpr int KV_BYTES = BKV * HD * 2;  // 16 KiB
-constexpr int P_BYTES = BQ * BKV * 2;   // 32 KiB: two [128 x 64] atoms
-constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * KV_BYTES + 2 * KV_BYTES + 4 * P_BYTES + 1024;
-constexpr uint32_t TMEM_COLS = 512;     // S of head 0, S of head 1 (128 columns each), O of each head (64 of 128)
-constexpr uint32_t TMEM_S = 0, TMEM_O = 256;
+constexpr int KV_BYTES = BKV * HD * 2;  // 8 KiB
+constexpr int O_BYTES = BQ * HD * 4;    // a unit's output on its way to the head's first unit
+constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * STAGES * KV_BYTES + 1024;
+static_assert((UNITS - 1) * O_BYTES <= 2 * STAGES * KV_BYTES, "the outputs go through the ring's memory");
+constexpr uint32_t TMEM_COLS = 512;     // a unit's S, then P in its first half (64 columns), and O (64)
 constexpr float NEG_BIG = -1.0e30f;
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
@@ -82,6 +91,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+  tmem_wait();
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 constexpr float REF_SLACK = 16.f;  // a row's reference moves when a score tops it by more than this (log2)
@@ -97,15 +115,15 @@ __device__ __forceinline__ uint64_t make_desc_mn(uint32_t smem_addr) {
   return d;
 }
 
-// One 128-key tile of K or V of one kv head into a swizzled [128 x 64] tile; keys outside [key_lo, key_hi) are
-// zero.  A warp's lane takes rows lane, lane+32, lane+64, lane+96: the four page lookups go out together.
+// One 64-key tile of K or V of one kv head into a swizzled [64 x 64] tile; keys outside [key_lo, key_hi) are
+// zero.  A warp's lane takes rows lane and lane + 32: the two page lookups go out together.
 __device__ __forceinline__ void gather_tile(uint32_t dst, const bf16* __restrict__ cache, const int* __restrict__ table,
                                             int kvh, int nkv, int ps, int ps_shift, int key_base, int key_lo, int key_hi,
                                             int lane, int num_pages, bool& bad_page) {
-  size_t off[4];
-  bool valid[4];
+  size_t off[2];
+  bool valid[2];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < 2; i++) {
     const int key = key_base + lane + 32 * i;
     valid[i] = key >= key_lo && key < key_hi;
     off[i] = 0;
@@ -118,93 +136,111 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const bf16* __restrict
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < 2; i++) {
     const int r = lane + 32 * i;
 #pragma unroll
     for (int c = 0; c < 8; c++) cp_async16(dst + r * 128 + ((c ^ (r & 7)) << 4), cache + off[i] + c * 8, valid[i]);
   }
 }
 
-// Row maximum of one thread's 128 scores in tensor memory.  The loops over column blocks stay rolled on purpose:
-// the softmax warps run this code once per key tile, and unrolled it no longer fits the instruction cache.
-template <bool MASKED>
-__device__ __forceinline__ float row_max(uint32_t s_addr, int lo, uint32_t span) {
-  float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-#pragma unroll 1
-  for (int c0 = 0; c0 < BKV; c0 += 64) {
-    uint32_t a[32], b[32];
-    tmem_ld32_issue(s_addr + c0, a);
-    tmem_ld32_issue(s_addr + c0 + 32, b);
-    tmem_wait();
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      float x0 = __uint_as_float(a[i]), x1 = __uint_as_float(a[i + 1]);
-      float y0 = __uint_as_float(b[i]), y1 = __uint_as_float(b[i + 1]);
-      if (MASKED) {
-        const int c = c0 + i - lo;
-        if ((uint32_t)c > span) x0 = -INFINITY;
-        if ((uint32_t)(c + 1) > span) x1 = -INFINITY;
-        if ((uint32_t)(c + 32) > span) y0 = -INFINITY;
-        if ((uint32_t)(c + 33) > span) y1 = -INFINITY;
-      }
-      m0 = fmaxf(m0, x0);
-      m1 = fmaxf(m1, x1);
-      m2 = fmaxf(m2, y0);
-      m3 = fmaxf(m3, y1);
-    }
-  }
-  return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
 }
-
-// 32 columns of one row: p = 2^(s * scale - m) as bfloat16 into the row's place of the swizzled P tile; returns
-// the sum of the even columns and adds that of the odd ones to `odd`.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// The largest of one thread's 64 scores; MASKED: those outside columns [lo, lo + span] become -infinity first.
 template <bool MASKED>
-__device__ __forceinline__ float exp_32_columns(const uint32_t (&v)[32], unsigned char* prow, int r, int c0, int lo,
-                                                uint32_t span, float scale, float neg_m, float& odd) {
-  float s0 = 0.f, s1 = 0.f;
-  uint32_t pk[16];
+__device__ __forceinline__ float row_max(uint32_t (&a)[32], uint32_t (&b)[32], int lo, uint32_t span) {
+  float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
-    float x0 = __uint_as_float(v[i]), x1 = __uint_as_float(v[i + 1]);
     if (MASKED) {
-      const int c = c0 + i - lo;
-      if ((uint32_t)c > span) x0 = -INFINITY;
-      if ((uint32_t)(c + 1) > span) x1 = -INFINITY;
+      const int c = i - lo;
+      if ((uint32_t)c > span) a[i] = 0xff800000u;
+      if ((uint32_t)(c + 1) > span) a[i + 1] = 0xff800000u;
+      if ((uint32_t)(c + 32) > span) b[i] = 0xff800000u;
+      if ((uint32_t)(c + 33) > span) b[i + 1] = 0xff800000u;
     }
-    const float p0 = fast_exp2(fmaf(x0, scale, neg_m)), p1 = fast_exp2(fmaf(x1, scale, neg_m));
-    s0 += p0;
-    s1 += p1;
+    m0 = max3(m0, __uint_as_float(a[i]), __uint_as_float(a[i + 1]));
+    m1 = max3(m1, __uint_as_float(b[i]), __uint_as_float(b[i + 1]));
+  }
+  return max_nan(m0, m1);
+}
+__device__ __forceinline__ uint64_t twice(float x) {
+  uint64_t y;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(a) : "l"(b), "l"(c));
+  return a;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
+  return a;
+}
+// 2^x of two numbers up to 2^6 on the FMA pipe: x = n + f with n the nearest integer, 2^f by a polynomial of degree 4 fitted to 2^f on
+// [-1/2, 1/2] by least squares, weighted until the largest relative error was the smallest (2.6e-6).  Below -126: 2^-126.
+__device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
+  float x0, x1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(x));
+  x0 = fmaxf(x0, -126.f);
+  x1 = fmaxf(x1, -126.f);
+  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(x0), "f"(x1));
+  constexpr float ROUND = 12582912.f;  // 1.5 * 2^23: the sum's last bits are n
+  const uint64_t t = add2(x, twice(ROUND));
+  uint64_t f = add2(t, twice(-ROUND));
+  asm("sub.rn.f32x2 %0, %1, %0;" : "+l"(f) : "l"(x));
+  uint64_t p = fma2(f, twice(0.009570101276040077f), twice(0.05591785907745361f));
+  p = fma2(p, f, twice(0.240247443318367f));
+  p = fma2(p, f, twice(0.6931217908859253f));
+  p = fma2(p, f, twice(0.9999992847442627f));
+  int n0, n1, b0, b1;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(n0), "=r"(n1) : "l"(t));
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(b0), "=r"(b1) : "l"(p));
+  p0 = __int_as_float(b0 + (n0 << 23));
+  p1 = __int_as_float(b1 + (n1 << 23));
+}
+// Of 16 pairs so many take the polynomial and not the special-function unit (one prompt of 8,192 tokens, 32 heads: none 422 us, 2
+// 416, 4 401, 6 430, 8 460).
+constexpr int POLY = 4;
+// p = 2^(s * scale - m) of 32 scores, as bfloat16 pairs; adds them to `sum`.  Scaling and adding take two at a time.
+__device__ __forceinline__ void row_exp(const uint32_t (&v)[32], uint32_t* pk, uint64_t scale, uint64_t neg_m, uint64_t& sum) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 2) {
+    uint64_t x;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(v[i]), "r"(v[i + 1]));
+    x = fma2(x, scale, neg_m);
+    float p0, p1;
+    if (((i >> 1) * POLY) % 16 < POLY) {
+      exp2_poly(x, p0, p1);
+    } else {
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(x));
+      p0 = fast_exp2(p0);
+      p1 = fast_exp2(p1);
+    }
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(p0), "f"(p1));
+    sum = add2(sum, x);
     pk[i >> 1] = pack_bf16(p0, p1);
   }
-  // 32 keys = four 16-byte chunks of this row in atom c0 / 64
-  unsigned char* dst = prow + (c0 >> 6) * (BQ * 128);
-  const int cbase = (c0 & 63) >> 3;
-#pragma unroll
-  for (int cc = 0; cc < 4; cc++)
-    *reinterpret_cast<uint4*>(dst + (((cbase + cc) ^ (r & 7)) << 4)) =
-        make_uint4(pk[4 * cc], pk[4 * cc + 1], pk[4 * cc + 2], pk[4 * cc + 3]);
-  odd += s1;
-  return s0;
 }
-
-// p = 2^(s * scale - m) of one row: bfloat16 into the row's place of the swizzled P tile; returns the row sum.
-template <bool MASKED>
-__device__ __forceinline__ float row_exp(uint32_t s_addr, unsigned char* prow, int r, int lo, uint32_t span, float scale,
-                                         float neg_m) {
-  float s0 = 0.f, s1 = 0.f;
-  // 32 columns at a time; the load of the next 32 is on its way while these are worked on
-  uint32_t v[32], w[32];
-  tmem_ld32_issue(s_addr, v);
-#pragma unroll 1
-  for (int c0 = 0; c0 < BKV; c0 += 64) {
-    tmem_wait();
-    tmem_ld32_issue(s_addr + c0 + 32, w);
-    s0 += exp_32_columns<MASKED>(v, prow, r, c0, lo, span, scale, neg_m, s1);
-    tmem_wait();
-    if (c0 + 64 < BKV) tmem_ld32_issue(s_addr + c0 + 64, v);
-    s0 += exp_32_columns<MASKED>(w, prow, r, c0 + 32, lo, span, scale, neg_m, s1);
-  }
-  return s0 + s1;
+// D += A B with A in tensor memory (row = lane, two neighbouring k's a column), by a whole warp
+__device__ __forceinline__ void umma_a_tmem(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ bool mbar_done(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return done;
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -217,54 +253,62 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        const int* __restrict__ n_tiles_ptr, int nh, int nkv, int ps, float scale_log2, int window,
                        int* __restrict__ status, int num_pages, int single) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done[2][2], skew;
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], s_full[UNITS], p_full[UNITS], o_done[UNITS], over, merged[2];
+  __shared__ float unit_m[UNITS][BQ], unit_l[UNITS][BQ];
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
   trigger_dependents();
   grid_dependency_wait();
-  if ((int)blockIdx.y >= *n_tiles_ptr) return;
+  // Blocks of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
+  // tiles' order the last blocks of two heads started when the SMs were nearly through).
+  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
+  const int group = nh / nkv, per_tile = nkv * (single ? group : group >> 1);
+  const unsigned id = blockIdx.y * gridDim.x + blockIdx.x, n_pairs = gridDim.y * per_tile;
+  const bool paired = id < n_pairs;
+  const int tile = paired ? id / per_tile : (id - n_pairs) / nkv;
+  if (tile >= *n_tiles_ptr) return;
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  unsigned char* sQ = base;                 // two heads
-  unsigned char* sK = sQ + 2 * Q_BYTES;     // two buffers
-  unsigned char* sV = sK + 2 * KV_BYTES;    // two buffers
-  unsigned char* sP = sV + 2 * KV_BYTES;    // two heads x two buffers
+  unsigned char* sQ = base;                        // two heads
+  unsigned char* sK = sQ + 2 * Q_BYTES;            // ring
+  unsigned char* sV = sK + STAGES * KV_BYTES;      // ring
+  float* sO = reinterpret_cast<float*>(sK);        // [unit][column][row], once the ring is no longer used
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  const int s = tiles[2 * blockIdx.y], qt0 = tiles[2 * blockIdx.y + 1];
-  const int group = nh / nkv;
-  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
-  const int pairs = single ? group : (group + 1) >> 1;
-  const int kvh = blockIdx.x / pairs;
-  const int pair = blockIdx.x - kvh * pairs;
-  const int head0 = kvh * group + (single ? pair : 2 * pair);
-  const int n_heads_here = (!single && 2 * pair + 1 < group) ? 2 : 1;
+  const int s = tiles[2 * tile], qt0 = tiles[2 * tile + 1];
+  const int in_tile = paired ? id - tile * per_tile : id - n_pairs - tile * nkv;
+  const int kvh = paired ? in_tile / (single ? group : group >> 1) : in_tile;
+  const int head0 = paired ? in_tile * (single ? 1 : 2) + (single ? 0 : kvh * (group & 1)) : (kvh + 1) * group - 1;
+  const int n_heads_here = paired && !single ? 2 : 1;
+  const int streams = UNITS / n_heads_here;  // unit u: head u / streams, tiles u % streams, u % streams + streams, ...
   const int q_len = seq_q_len[s], kv_len = seq_kv_len[s];
   const int rows_live = min(BQ, q_len - qt0);
   const int pos0 = kv_len - q_len + qt0;
-  // the first tile starts on a multiple of 128 keys, so that whole tiles are whole pages
+  // the first tile starts on a multiple of 64 keys, so that whole tiles are whole pages
   int k_begin = 0;
   if (window > 0 && pos0 - window + 1 > 0) k_begin = (pos0 - window + 1) & ~(BKV - 1);
   const int k_end = pos0 + rows_live;  // one past the last key any row of the tile sees
   const int n_kv_tiles = (k_end - k_begin + BKV - 1) / BKV;
+  const int live_streams = min(streams, n_kv_tiles);
+  auto tiles_of = [&](int stream) { return (n_kv_tiles - stream + streams - 1) / streams; };  // (0 from live_streams on)
   const int* table = page_ids + page_indptr[s];
   const int t0 = seq_q_start[s] + qt0;
 
   if (tid == 0) {
-    for (int i = 0; i < 2; i++) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], n_heads_here);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], n_heads_here);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&pv_done[i][0], 1);
-      mbar_init(&pv_done[i][1], 1);
+    for (int i = 0; i < STAGES; i++) {
+      mbar_init(&full[i], 2);
+      mbar_init(&empty[i], n_heads_here);
     }
-    mbar_init(&skew, 128);
+    for (int i = 0; i < UNITS; i++) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&o_done[i], 1);
+    }
+    for (int i = 0; i < 2; i++) mbar_init(&merged[i], max(1, 4 * (live_streams - 1)));
+    mbar_init(&over, 4 * live_streams * n_heads_here);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 10) {
+  if (warp == SOFTMAX_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -285,21 +329,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const uint32_t tmem = tmem_slot;
   const int ps_shift = (ps & (ps - 1)) == 0 ? 31 - __clz(ps) : -1;
 
-  if (warp == 8 || warp == 9) {
-    // ---------------- loaders: warp 8 K tiles, warp 9 V tiles, two buffers each
-    const bool is_v = warp == 9;
+  if (warp >= SOFTMAX_WARPS) {
+    // ---------------- loaders: K tiles and V tiles
+    const bool is_v = warp == SOFTMAX_WARPS + 1;
     const bf16* cache = is_v ? vcache : kcache;
     const CUtensorMap* map = is_v ? &map_v : &map_k;
     unsigned char* ring = is_v ? sV : sK;
-    uint64_t* full = is_v ? v_full : k_full;
-    uint64_t* empty = is_v ? v_empty : k_empty;
     bool ok = true, bad_page = false;
     for (int j = 0; j < n_kv_tiles; j++) {
-      const int b = j & 1;
+      const int b = j % STAGES;
       const int key_base = k_begin + j * BKV;
-      if (j >= 2 && !mbar_wait_idle(&empty[b], ((j >> 1) - 1) & 1)) { ok = false; break; }
+      if (j >= STAGES && !mbar_wait_idle(&empty[b], ((j / STAGES) - 1) & 1)) { ok = false; break; }
       if (tma_rows > 0 && key_base + BKV <= kv_len) {
-        // every key of the tile exists: one box per page (or per 128 slots of a larger page)
+        // every key of the tile exists: one box per page (or per 64 slots of a larger page)
         if (lane == 0) mbar_expect_tx(&full[b], KV_BYTES);
         __syncwarp();
         if (lane * tma_rows < BKV) {
@@ -318,121 +360,174 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
     if (!ok) failed = 1;
     report_bad_page(bad_page, status);
-  } else if (warp >= 10) {
-    const int hh = warp - 10;
-    if (lane == 0 && hh < n_heads_here) {
-      // ---------------- MMA issuer of head hh: QK_0; then for every tile: (wait P_j) QK_{j+1}, P_j . V
-      // All operand descriptors are made once; a k step adds its byte offset (in 16-byte units) to the address field.
-      const uint32_t idesc_qk = make_idesc(BQ, BKV);
-      const uint32_t idesc_pv = make_idesc(BQ, HD) | (1u << 16);  // B operand MN-major
-      const uint64_t desc_q = make_desc(smem_u32(sQ + hh * Q_BYTES));
-      const uint64_t desc_k0 = make_desc(smem_u32(sK)), desc_v0 = make_desc_mn(smem_u32(sV));
-      const uint64_t desc_p0 = make_desc(smem_u32(sP + (hh * 2) * P_BYTES));
-      bool ok = true;
-      auto issue_qk = [&](int j) {
-        const int kb = j & 1;
-        if (!mbar_wait_idle(&k_full[kb], (j >> 1) & 1)) return false;
-        tcgen05_fence_after();
-        const uint64_t dk = desc_k0 + (uint64_t)(kb * (KV_BYTES / 16));
-#pragma unroll
-        for (int k = 0; k < HD / UMMA_K; k++)
-          umma(tmem + TMEM_S + hh * 128, desc_q + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_qk, k > 0 ? 1u : 0u);
-        tcgen05_commit(&k_empty[kb]);
-        tcgen05_commit(&s_full[hh]);
-        return true;
-      };
-      ok = issue_qk(0);
-      for (int j = 0; j < n_kv_tiles && ok; j++) {
-        const int vb = j & 1;
-        if (!mbar_wait_idle(&p_full[hh], j & 1)) { ok = false; break; }
-        if (j + 1 < n_kv_tiles && !issue_qk(j + 1)) { ok = false; break; }
-        if (!mbar_wait_idle(&v_full[vb], (j >> 1) & 1)) { ok = false; break; }
-        tcgen05_fence_after();
-        const uint64_t dp = desc_p0 + (uint64_t)(vb * (P_BYTES / 16)), dv = desc_v0 + (uint64_t)(vb * (KV_BYTES / 16));
-#pragma unroll
-        for (int k = 0; k < BKV / UMMA_K; k++)
-          umma(tmem + TMEM_O + hh * 128, dp + (uint64_t)((k >> 2) * (BQ * 128 / 16) + (k & 3) * 2),
-                  dv + (uint64_t)(k * (2048 / 16)), idesc_pv, (k > 0 || j > 0) ? 1u : 0u);
-        tcgen05_commit(&v_empty[vb]);
-        tcgen05_commit(&pv_done[hh][vb]);
-      }
-      if (!ok) failed = 1;
-    }
-  } else if ((warp >> 2) < n_heads_here) {
+  } else if ((warp >> 2) % streams < live_streams) {
     // ---------------- softmax and output: thread = query row = lane of tensor memory
-    const int hh = warp >> 2;
-    const int r = tid & 127;
+    const int u = warp >> 2, hh = u / streams, stream = u - hh * streams;
+    const int r = tid & 127, n = tiles_of(stream);
     const int pos = pos0 + r;
     const int lim_hi = pos < k_end - 1 ? pos : k_end - 1;
     const int lim_lo = window > 0 ? max(pos - window + 1, 0) : 0;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t s_addr = lane_addr + TMEM_S + hh * 128, o_addr = lane_addr + TMEM_O + hh * 128;
+    const uint32_t s_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + u * 128, o_addr = s_addr + 64;
+    const uint64_t scale2 = twice(scale_log2);
     float m = NEG_BIG, l = 0.f;  // reference of the row's exponentials (and so of O and l); row sum
     bool ok = true;
-    // the second head starts when the first has handed over its first P
-    if (hh == 1 && !mbar_wait(&skew, 0)) ok = false;
-    for (int j = 0; j < n_kv_tiles && ok; j++) {
-      const int key0 = k_begin + j * BKV;
-      if (!mbar_wait(&s_full[hh], j & 1)) { ok = false; break; }
+    // One of the unit's warps (one a scheduler) also issues its MMAs: S_0; then, with P_j of all four there, O += P_j . V_j and
+    // S_(j+1), which takes the place of S_j and P_j (the instructions of one thread run in order)
+    const bool issuer = (warp & 3) == u;
+    constexpr uint32_t idesc_qk = make_idesc(BQ, BKV);
+    constexpr uint32_t idesc_pv = make_idesc(BQ, HD) | (1u << 16);  // B operand MN-major
+    const uint32_t unit = tmem + u * 128;
+    int ring = stream;       // the ring's place of tile j, and its phase
+    uint32_t phase = 0;
+    auto next_ring = [&]() { return ring + streams >= STAGES ? ring + streams - STAGES : ring + streams; };
+    auto next_phase = [&]() { return ring + streams >= STAGES ? phase ^ 1 : phase; };
+    auto issue_qk = [&]() {
+      const uint64_t q0 = make_desc(smem_u32(sQ + hh * Q_BYTES)), k0 = make_desc(smem_u32(sK + ring * KV_BYTES));
+#pragma unroll
+      for (int k = 0; k < HD / UMMA_K; k++) umma_warp(unit, q0 + (uint64_t)(k * 2), k0 + (uint64_t)(k * 2), idesc_qk, k > 0 ? 1u : 0u);
+      commit_warp(&s_full[u]);
+    };
+    if (issuer) {
+      ok = mbar_wait(&full[ring], phase);
       tcgen05_fence_after();
-      const bool whole = key0 + BKV - 1 <= pos0 && key0 + BKV <= k_end && (window <= 0 || key0 >= pos0 + BQ - window);
-      const int lo = lim_hi >= lim_lo ? lim_lo - key0 : (1 << 30);
-      const uint32_t span = lim_hi >= lim_lo ? (uint32_t)(lim_hi - lim_lo) : 0u;
-      const float tile_max = (whole ? row_max<false>(s_addr, lo, span) : row_max<true>(s_addr, lo, span)) * scale_log2;
-      const bool moves = tile_max - m > REF_SLACK;
+      __syncwarp();
+      if (ok) issue_qk();
+    }
+    // Tiles [whole_from, whole_to) of the unit are seen whole by every row of the block and need no mask; in the others columns
+    // [lo, lo + span] are visible.
+    const int first = k_begin + stream * BKV, step = streams * BKV;
+    const int whole_to = min(pos0 + 1, k_end) - BKV - first < 0 ? 0 : (min(pos0 + 1, k_end) - BKV - first) / step + 1;
+    const int whole_from = window <= 0 || first >= pos0 + BQ - window ? 0 : (pos0 + BQ - window - first + step - 1) / step;
+    const uint32_t span = lim_hi >= lim_lo ? (uint32_t)(lim_hi - lim_lo) : 0u;
+    for (int j = 0; j < n && ok; j++) {
+      if (!mbar_wait(&s_full[u], j & 1)) { ok = false; break; }
+      tcgen05_fence_after();
+      uint32_t a[32], b[32];
+      tmem_ld32_issue(s_addr, a);
+      tmem_ld32_issue(s_addr + 32, b);
+      tmem_wait();
+      float tile_max;
+      if (j >= whole_from && j < whole_to) {
+        tile_max = row_max<false>(a, b, 0, 0);
+      } else {
+        tile_max = row_max<true>(a, b, lim_hi >= lim_lo ? lim_lo - first - j * step : 1 << 30, span);
+      }
+      tile_max *= scale_log2;
+      // (a row with a score that is infinite or no number is NaN from here on: the polynomial would make numbers of those)
+      const bool moves = !(tile_max - m <= REF_SLACK);
+      tile_max += moves ? tile_max - tile_max : 0.f;
       if (j == 0) {
         if (moves) m = tile_max;
       } else if (__any_sync(0xffffffffu, moves)) {
-        if (!mbar_wait(&pv_done[hh][(j - 1) & 1], ((j - 1) >> 1) & 1)) { ok = false; break; }
-        tcgen05_fence_after();
-        const float m_new = moves ? fmaxf(m, tile_max) : m;
+        // rows of this warp move their reference: O and l of those rows are scaled to the new one
+        const float m_new = moves ? max_nan(m, tile_max) : m;
         const float alpha = fast_exp2(m - m_new);
+#pragma unroll 1
+        for (int c0 = 0; c0 < HD; c0 += 8) {
+          uint32_t v[8];
+          tmem_ld8(o_addr + c0, v);
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+          tmem_st8(o_addr + c0, v);
+        }
+        l *= alpha;
+        m = m_new;
+      }
+      // the tile of S_(j+1), on its way for long
+      if (issuer && j + 1 < n && !mbar_wait(&full[next_ring()], next_phase())) { ok = false; break; }
+      uint32_t pk[32];
+      uint64_t sums = 0;
+      row_exp(a, pk, scale2, twice(-m), sums);
+      row_exp(b, pk + 16, scale2, twice(-m), sums);
+      tmem_st32(s_addr, pk);
+      float s0, s1;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sums));
+      l += s0 + s1;
+      tmem_wait_st();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[u]);
+      if (issuer) {
+        const uint64_t v0 = make_desc_mn(smem_u32(sV + ring * KV_BYTES));
+        uint64_t* done = &empty[ring];
+        const int next = next_ring();
+        phase = next_phase();
+        ring = next;
+        if (!mbar_wait(&p_full[u], j & 1)) { ok = false; break; }
+        tcgen05_fence_after();
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < BKV / UMMA_K; k++)  // 16 keys a step: 8 columns of P, two 8-key groups of V
+          umma_a_tmem(unit + 64, unit + k * 8, v0 + (uint64_t)(k * (2048 / 16)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+        if (j + 1 < n) issue_qk();
+        else commit_warp(&o_done[u]);
+        commit_warp(done);
+      }
+    }
+    if (ok) ok = mbar_wait(&o_done[u], 0);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&over);  // (every tile that was asked for has been used by then)
+    if (ok && stream > 0) ok = mbar_wait(&over, 0);
+    if (ok) {
+      tcgen05_fence_after();
+      if (stream > 0) {
+        // the head's first unit puts the others' outputs to its own
+        unit_m[u][r] = m;
+        unit_l[u][r] = l;
+        float* dst = sO + (size_t)(u - hh - 1) * (BQ * HD) + r;  // (the first units hand nothing over)
 #pragma unroll 1
         for (int c0 = 0; c0 < HD; c0 += 32) {
           uint32_t v[32];
           tmem_ld32_issue(o_addr + c0, v);
           tmem_wait();
 #pragma unroll
-          for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-          tmem_st32(o_addr + c0, v);
+          for (int i = 0; i < 32; i++) dst[(c0 + i) * BQ] = __uint_as_float(v[i]);
         }
-        tmem_wait_st();
-        l *= alpha;
-        m = m_new;
-      }
-      if (j >= 2 && !mbar_wait(&pv_done[hh][j & 1], ((j - 2) >> 1) & 1)) { ok = false; break; }
-      unsigned char* prow = sP + (hh * 2 + (j & 1)) * P_BYTES + r * 128;
-      l += whole ? row_exp<false>(s_addr, prow, r, lo, span, scale_log2, -m) : row_exp<true>(s_addr, prow, r, lo, span, scale_log2, -m);
-      tcgen05_fence_before();
-      fence_proxy_async();
-      mbar_arrive(&p_full[hh]);
-      if (j == 0 && hh == 0) mbar_arrive(&skew);
-    }
-    if (ok) ok = mbar_wait(&pv_done[hh][(n_kv_tiles - 1) & 1], ((n_kv_tiles - 1) >> 1) & 1);
-    if (!ok) failed = 1;
-    if (ok) {
-      tcgen05_fence_after();
-      uint32_t a[32], b[32];
-      tmem_ld32_issue(o_addr, a);
-      tmem_ld32_issue(o_addr + 32, b);
-      tmem_wait();
-      if (r < rows_live) {
-        const float inv = 1.f / l;
-        bf16* dst = out + (size_t)(t0 + r) * out_stride + (size_t)(head0 + hh) * HD;
-        auto two = [&](const uint32_t (&v)[32], int i) {
-          return pack_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv);
-        };
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&merged[hh]);
+      } else {
+        if (live_streams > 1) ok = mbar_wait(&merged[hh], 0);
+        float top = m, w[UNITS];
+        for (int i = 1; i < live_streams; i++) top = fmaxf(top, unit_m[u + i][r]);
+        w[0] = fast_exp2(m - top);
+        float sum = l * w[0];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-          *reinterpret_cast<uint4*>(dst + c * 8) = make_uint4(two(a, 8 * c), two(a, 8 * c + 2), two(a, 8 * c + 4), two(a, 8 * c + 6));
-          *reinterpret_cast<uint4*>(dst + 32 + c * 8) = make_uint4(two(b, 8 * c), two(b, 8 * c + 2), two(b, 8 * c + 4), two(b, 8 * c + 6));
+        for (int i = 1; i < UNITS; i++) {
+          w[i] = i < live_streams ? fast_exp2(unit_m[u + i][r] - top) : 0.f;
+          if (i < live_streams) sum += unit_l[u + i][r] * w[i];
+        }
+        const float inv = 1.f / sum;
+        bf16* dst = out + (size_t)(t0 + r) * out_stride + (size_t)(head0 + hh) * HD;
+        const float* other = sO + (size_t)(u - hh) * (BQ * HD) + r;
+#pragma unroll 1
+        for (int c0 = 0; c0 < HD && ok; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32_issue(o_addr + c0, v);
+          tmem_wait();
+          float x[32];
+#pragma unroll
+          for (int i = 0; i < 32; i++) x[i] = __uint_as_float(v[i]) * w[0];
+#pragma unroll
+          for (int k = 1; k < UNITS; k++) {
+            if (k >= live_streams) break;
+#pragma unroll
+            for (int i = 0; i < 32; i++) x[i] = fmaf(other[(size_t)(k - 1) * (BQ * HD) + (c0 + i) * BQ], w[k], x[i]);
+          }
+          if (r < rows_live) {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+              *reinterpret_cast<uint4*>(dst + c0 + c * 8) =
+                  make_uint4(pack_bf16(x[8 * c] * inv, x[8 * c + 1] * inv), pack_bf16(x[8 * c + 2] * inv, x[8 * c + 3] * inv),
+                             pack_bf16(x[8 * c + 4] * inv, x[8 * c + 5] * inv), pack_bf16(x[8 * c + 6] * inv, x[8 * c + 7] * inv));
+          }
         }
       }
     }
+    if (!ok) failed = 1;
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 10) {
+  if (warp == SOFTMAX_WARPS) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }

@@ -1,8 +1,11 @@
 // Causal attention for prompt portions on the fifth-generation tensor cores with the output accumulated in tensor
 // memory (head sizes 64 and 128, bfloat16; compile with -DTKB_HD).
 //
-// A block owns 128 consecutive query tokens of TWO query heads that share a kv head (one head where the group
-// size is odd and no partner is left) and walks the keys they may see in tiles of 64.  For each head:
+// A block owns 128 consecutive query tokens of TWO query heads that share a kv head (one head where the group size is odd and no
+// partner is left, or where pairs would leave SMs without a block) and walks the keys they may see in tiles of 64.  Two UNITS
+// share the work: the two heads, or the even and the odd tiles of one head, each with a reference, sum and output of its own that
+// are put together at the end (one head in one unit left the other half of the block idle: 24 heads on 8 kv heads, 2,048 tokens behind
+// 2,048 others 126 us, 111 with two units and the blocks of two heads first).  For each unit:
 //     S = Q . K^T      tcgen05.mma 128 x 64 x 16, HD / 16 per tile, two S tiles in tensor memory (the product of
 //                      tile j+2 starts as soon as the softmax threads are through with S_j)
 //     softmax          a warpgroup per head, one thread per query row (a lane of tensor memory): row maximum, then
@@ -193,12 +196,20 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         int* __restrict__ status, int num_pages, int single) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t k_full[KV_STAGES], k_empty[KV_STAGES], v_full[KV_STAGES], v_empty[KV_STAGES],
-      s_full[2][2], p_full[2], pv_done[2][2];
+      s_full[2][2], p_full[2], pv_done[2][2], over, merged;
+  __shared__ float other_m[BQ], other_l[BQ];
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
   trigger_dependents();
   grid_dependency_wait();
-  if ((int)blockIdx.y >= *n_tiles_ptr) return;
+  // Blocks of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
+  // tiles' order the last blocks of two heads started when the SMs were nearly through).
+  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
+  const int group = nh / nkv, per_tile = nkv * (single ? group : group >> 1);
+  const unsigned id = blockIdx.y * gridDim.x + blockIdx.x, n_pairs = gridDim.y * per_tile;
+  const bool paired = id < n_pairs;
+  const int tile = paired ? id / per_tile : (id - n_pairs) / nkv;
+  if (tile >= *n_tiles_ptr) return;
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sQ = base;                         // two heads
   unsigned char* sK = sQ + 2 * Q_BYTES;             // ring
@@ -206,14 +217,12 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   unsigned char* sP = sV + KV_STAGES * KV_BYTES;    // two heads x two buffers
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  const int s = tiles[2 * blockIdx.y], qt0 = tiles[2 * blockIdx.y + 1];
-  const int group = nh / nkv;
-  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
-  const int pairs = single ? group : (group + 1) >> 1;
-  const int kvh = blockIdx.x / pairs;
-  const int pair = blockIdx.x - kvh * pairs;
-  const int head0 = kvh * group + (single ? pair : 2 * pair);
-  const int n_heads_here = (!single && 2 * pair + 1 < group) ? 2 : 1;
+  const int s = tiles[2 * tile], qt0 = tiles[2 * tile + 1];
+  const int in_tile = paired ? id - tile * per_tile : id - n_pairs - tile * nkv;
+  const int kvh = paired ? in_tile / (single ? group : group >> 1) : in_tile;
+  const int head0 = paired ? in_tile * (single ? 1 : 2) + (single ? 0 : kvh * (group & 1)) : (kvh + 1) * group - 1;
+  const int n_heads_here = paired && !single ? 2 : 1;
+  const int streams = 3 - n_heads_here;  // unit u: head u, or tiles u, u + 2, ... of the only head
   const int q_len = seq_q_len[s], kv_len = seq_kv_len[s];
   const int rows_live = min(BQ, q_len - qt0);
   const int pos0 = kv_len - q_len + qt0;
@@ -221,6 +230,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   if (window > 0 && pos0 - window + 1 > 0) k_begin = (pos0 - window + 1) & ~(BKV - 1);
   const int k_end = pos0 + rows_live;  // one past the last key any row of the tile sees
   const int n_kv_tiles = (k_end - k_begin + BKV - 1) / BKV;
+  const int live_units = min(2, n_heads_here * n_kv_tiles);
   const int* table = page_ids + page_indptr[s];
   const int t0 = seq_q_start[s] + qt0;
 
@@ -238,6 +248,8 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         mbar_init(&pv_done[i][b], 1);
       }
     }
+    mbar_init(&over, 4 * live_units);
+    mbar_init(&merged, 4);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -299,19 +311,20 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if (!ok) failed = 1;
     report_bad_page(bad_page, status);
   } else if (warp >= 10) {
-    const int hh = warp - 10;
-    if (lane == 0 && hh < n_heads_here) {
-      // ---------------- MMA issuer of head hh: S_0 and S_1; then for every tile: (wait P_j, which also frees its S
+    const int hh = warp - 10, head = streams == 2 ? 0 : hh, stream = streams == 2 ? hh : 0;
+    const int n_mine = (n_kv_tiles - stream + streams - 1) / streams;
+    if (lane == 0 && hh < live_units) {
+      // ---------------- MMA issuer of unit hh: S_0 and S_1; then for every tile: (wait P_j, which also frees its S
       // tile) Q . K_{j+2}^T, O += P_j . V_j
       const uint32_t idesc_qk = make_idesc(BQ, BKV);
       const uint32_t idesc_pv = make_idesc(BQ, HD) | (1u << 16);  // B operand MN-major
-      const uint64_t desc_q = make_desc(smem_u32(sQ + hh * Q_BYTES));
+      const uint64_t desc_q = make_desc(smem_u32(sQ + head * Q_BYTES));
       const uint64_t desc_k0 = make_desc(smem_u32(sK)), desc_v0 = make_desc_mn(smem_u32(sV));
       const uint64_t desc_p0 = make_desc(smem_u32(sP + (hh * 2) * P_BYTES));
       bool ok = true;
       auto issue_qk = [&](int j) {
-        const int kb = j % KV_STAGES;
-        if (!mbar_wait(&k_full[kb], (j / KV_STAGES) & 1)) return false;
+        const int t = stream + j * streams, kb = t % KV_STAGES;
+        if (!mbar_wait(&k_full[kb], (t / KV_STAGES) & 1)) return false;
         tcgen05_fence_after();
         const uint64_t dk = desc_k0 + (uint64_t)(kb * (KV_BYTES / 16));
 #pragma unroll
@@ -323,12 +336,12 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         return true;
       };
       ok = issue_qk(0);
-      if (ok && n_kv_tiles > 1) ok = issue_qk(1);
-      for (int j = 0; j < n_kv_tiles && ok; j++) {
-        const int vb = j % KV_STAGES, pb = j & 1;
+      if (ok && n_mine > 1) ok = issue_qk(1);
+      for (int j = 0; j < n_mine && ok; j++) {
+        const int t = stream + j * streams, vb = t % KV_STAGES, pb = j & 1;
         if (!mbar_wait(&p_full[hh], j & 1)) { ok = false; break; }
-        if (j + 2 < n_kv_tiles && !issue_qk(j + 2)) { ok = false; break; }
-        if (!mbar_wait(&v_full[vb], (j / KV_STAGES) & 1)) { ok = false; break; }
+        if (j + 2 < n_mine && !issue_qk(j + 2)) { ok = false; break; }
+        if (!mbar_wait(&v_full[vb], (t / KV_STAGES) & 1)) { ok = false; break; }
         tcgen05_fence_after();
         const uint64_t dp = desc_p0 + (uint64_t)(pb * (P_BYTES / 16)), dv = desc_v0 + (uint64_t)(vb * (KV_BYTES / 16));
 #pragma unroll
@@ -340,9 +353,10 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       }
       if (!ok) failed = 1;
     }
-  } else if ((warp >> 2) < n_heads_here) {
+  } else if ((warp >> 2) < live_units) {
     // ---------------- softmax and output: thread = query row = lane of tensor memory
-    const int hh = warp >> 2;
+    const int hh = warp >> 2, head = streams == 2 ? 0 : hh, stream = streams == 2 ? hh : 0;
+    const int n_mine = (n_kv_tiles - stream + streams - 1) / streams;
     const int r = tid & 127;
     const int pos = pos0 + r;
     const int lim_hi = pos < k_end - 1 ? pos : k_end - 1;
@@ -351,8 +365,8 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const uint32_t s_addr = lane_addr + TMEM_S + hh * 128, o_addr = lane_addr + TMEM_O + hh * 128;
     float ref = NEG_BIG, l = 0.f;  // reference of the exponentials (and so of O and l); row sum
     bool ok = true;
-    for (int j = 0; j < n_kv_tiles; j++) {
-      const int key0 = k_begin + j * BKV;
+    for (int j = 0; j < n_mine; j++) {
+      const int key0 = k_begin + (stream + j * streams) * BKV;
       if (!mbar_wait(&s_full[hh][j & 1], (j >> 1) & 1)) { ok = false; break; }
       tcgen05_fence_after();
       const uint32_t sj = s_addr + (j & 1) * BKV;
@@ -396,17 +410,44 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       if (j >= 1 && !mbar_wait(&p_full[hh], (j - 1) & 1)) { ok = false; break; }
       mbar_arrive(&p_full[hh]);
     }
-    if (ok) ok = mbar_wait(&pv_done[hh][(n_kv_tiles - 1) & 1], ((n_kv_tiles - 1) >> 1) & 1);
-    if (!ok) failed = 1;
-    if (ok) {
+    if (ok) ok = mbar_wait(&pv_done[hh][(n_mine - 1) & 1], ((n_mine - 1) >> 1) & 1);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&over);
+    float* sO = reinterpret_cast<float*>(sP);  // [column][row], once no product reads a P any more
+    static_assert(4 * P_BYTES >= BQ * HD * 4, "the second unit's output goes through the P tiles' memory");
+    if (ok && stream > 0) {
+      // the first unit puts this one's output to its own
+      ok = mbar_wait(&over, 0);
       tcgen05_fence_after();
-      const float inv = 1.f / l;
-      bf16* dst = out + (size_t)(t0 + r) * out_stride + (size_t)(head0 + hh) * HD;
+      other_m[r] = ref;
+      other_l[r] = l;
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD; c0 += 32) {
+      for (int c0 = 0; c0 < HD && ok; c0 += 32) {
         uint32_t v[32];
         tmem_ld32_issue(o_addr + c0, v);
         tmem_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i++) sO[(c0 + i) * BQ + r] = __uint_as_float(v[i]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&merged);
+    } else if (ok) {
+      tcgen05_fence_after();
+      const bool two = streams == 2 && live_units == 2;
+      if (two) ok = mbar_wait(&merged, 0);
+      const float top = two ? fmaxf(ref, other_m[r]) : ref;
+      const float mine = two ? fast_exp2(ref - top) : 1.f, theirs = two ? fast_exp2(other_m[r] - top) : 0.f;
+      const float inv = 1.f / (two ? l * mine + other_l[r] * theirs : l);
+      bf16* dst = out + (size_t)(t0 + r) * out_stride + (size_t)(head0 + head) * HD;
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD && ok; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32_issue(o_addr + c0, v);
+        tmem_wait();
+        if (two) {
+#pragma unroll
+          for (int i = 0; i < 32; i++) v[i] = __float_as_uint(fmaf(sO[(c0 + i) * BQ + r], theirs, __uint_as_float(v[i]) * mine));
+        }
         if (r < rows_live) {
 #pragma unroll
           for (int c = 0; c < 4; c++)
@@ -418,6 +459,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
       }
     }
+    if (!ok) failed = 1;
   }
   tcgen05_fence_before();
   __syncthreads();
