@@ -459,8 +459,7 @@ namespace {
 // walked all of a row's columns one load after the other took the same 0.2 ms for 8 tokens as for 2,048), the tokens'
 // low-rank rows lie in shared memory rank-major, so that GT / 4 16-byte reads bring one rank's values of all GT tokens
 // to the whole warp (one 4-byte read a token and rank made shared memory the bound at thousands of tokens).  The sum
-// over the rank runs in order, whatever the tiling.  GT = 8 at every step size: with 32 tokens a block (a quarter of
-// the second factor's traffic out of the L2) 2,048 tokens took 73 us against 49 us.
+// over the rank runs in order, whatever the tiling.
 template <int GT>
 __global__ void __launch_bounds__(256)
 gla_gates_kernel(float* __restrict__ proj, int stride, int low_off, int rank, const float* __restrict__ a2t,
@@ -530,6 +529,104 @@ gla_gates_kernel(float* __restrict__ proj, int stride, int low_off, int rank, co
   }
 }
 
+// The same for 64 tokens and more: a block 64 tokens x 128 columns, 32 ranks of both factors at a time in shared memory, a thread
+// 4 tokens x 8 columns (12 values read for 32 FMAs).  Every sum is the other kernel's chain: bias, then the ranks in order.  A block of 8
+// tokens reads the whole second factor for them: 197 MB out of the L2 for 3,001 tokens of 2,048 columns, rank 64: 60 us, 41 here (sums
+// 16, decays 8, the rest memory).  Where the tiles are fewer than the SMs the other kernel is the faster one (64 tokens of 2,048
+// columns: a layer 62 us, 66 with tiles).
+constexpr int GT_TOKENS = 64, GT_COLS = 128, GT_RANKS = 32;
+__global__ void __launch_bounds__(256)
+gla_gates_tile_kernel(float* __restrict__ proj, int stride, int low_off, int rank, const float* __restrict__ a2t,
+                      const float* __restrict__ bias, float inv_tau, int C, float* __restrict__ f, int q_off, int q_cols,
+                      float q_scale, int n_tokens) {
+  __shared__ __align__(16) float low[GT_RANKS][GT_TOKENS + 4], w[GT_RANKS][GT_COLS];
+  trigger_dependents();
+  grid_dependency_wait();
+  const int tid = threadIdx.x, t0 = blockIdx.x * GT_TOKENS, c0 = blockIdx.y * GT_COLS;
+  const int nt = min(GT_TOKENS, n_tokens - t0);
+  const int tt = (tid >> 4) * 4, tc = (tid & 15) * 4;  // this thread's tokens; its columns tc.. and 64 + tc..
+  float z[4][8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const int c = c0 + (j >> 2) * 64 + tc + (j & 3);
+    const float b = bias && c < C ? bias[c] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) z[i][j] = b;
+  }
+  for (int r0 = 0; r0 < rank; r0 += GT_RANKS) {
+    const int nr = min(GT_RANKS, rank - r0);
+    float x[GT_TOKENS * GT_RANKS / 256], y[GT_RANKS * GT_COLS / 256];
+#pragma unroll
+    for (int i = 0; i < GT_TOKENS * GT_RANKS / 256; i++) {
+      const int t = (tid >> 5) + 8 * i, r = tid & 31;
+      x[i] = t < nt && r < nr ? proj[(size_t)(t0 + t) * stride + low_off + r0 + r] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < GT_RANKS * GT_COLS / 256; i++) {
+      const int r = (tid >> 7) + 2 * i, c = c0 + (tid & 127);
+      y[i] = r < nr && c < C ? a2t[(size_t)(r0 + r) * C + c] : 0.f;
+    }
+    __syncthreads();  // the ranks before have been read
+#pragma unroll
+    for (int i = 0; i < GT_TOKENS * GT_RANKS / 256; i++) low[tid & 31][(tid >> 5) + 8 * i] = x[i];
+#pragma unroll
+    for (int i = 0; i < GT_RANKS * GT_COLS / 256; i++) w[(tid >> 7) + 2 * i][tid & 127] = y[i];
+    __syncthreads();
+    for (int r = 0; r < nr; r++) {
+      const float4 l = *reinterpret_cast<const float4*>(&low[r][tt]);
+      const float4 a = *reinterpret_cast<const float4*>(&w[r][tc]), b = *reinterpret_cast<const float4*>(&w[r][64 + tc]);
+      const float lv[4] = {l.x, l.y, l.z, l.w}, wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) z[i][j] = fmaf(wv[j], lv[i], z[i][j]);
+    }
+  }
+  const bool vec = (C & 3) == 0 && ((uintptr_t)f & 15) == 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    if (tt + i >= nt) break;
+    float* row = f + (size_t)(t0 + tt + i) * C;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int c = c0 + h * 64 + tc;
+      float g[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float x = z[i][4 * h + j];
+        g[j] = expf((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * inv_tau);
+      }
+      if (vec && c < C) {
+        *reinterpret_cast<float4*>(row + c) = make_float4(g[0], g[1], g[2], g[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (c + j < C) row[c + j] = g[j];
+      }
+    }
+  }
+  if (q_scale != 1.f) {
+    const bool vec_q = ((stride | q_off | q_cols) & 3) == 0 && ((uintptr_t)proj & 15) == 0;
+    for (int j = c0 + (tid & 31) * 4; j < q_cols; j += gridDim.y * GT_COLS) {
+      float* at = proj + (size_t)(t0 + (tid >> 5)) * stride + q_off + j;
+      const size_t step = (size_t)8 * stride;
+      if (vec_q) {
+        float4 v[GT_TOKENS / 8];  // all on their way together
+#pragma unroll
+        for (int i = 0; i < GT_TOKENS / 8; i++)
+          if ((tid >> 5) + 8 * i < nt) v[i] = *reinterpret_cast<const float4*>(at + i * step);
+#pragma unroll
+        for (int i = 0; i < GT_TOKENS / 8; i++)
+          if ((tid >> 5) + 8 * i < nt)
+            *reinterpret_cast<float4*>(at + i * step) = make_float4(v[i].x * q_scale, v[i].y * q_scale, v[i].z * q_scale, v[i].w * q_scale);
+      } else {
+        for (int i = 0; i < GT_TOKENS / 8; i++)
+          for (int u = 0; u < 4 && j + u < q_cols && (tid >> 5) + 8 * i < nt; u++) at[i * step + u] *= q_scale;
+      }
+    }
+  }
+}
+
 // Rotation by position of the q and k heads of float32 rows, in place: the first rot_dims channels of a head, channel i
 // paired with i + rot_dims / 2 (pairs == 0) or channel 2i with 2i + 1 (pairs != 0); (u, v) -> (u cos a - v sin a,
 // v cos a + u sin a), a = position * freq[i].  The angle, sine and cosine are float64 (the float32 product of a
@@ -580,6 +677,10 @@ TKB_EXPORT int tkb_gla_gates(float* proj, int stride, int low_off, int rank, con
   if (n_tokens <= 0) return 0;
   if (rank <= 0 || C <= 0 || (size_t)8 * rank * sizeof(float) > 48 * 1024) return -2;
   if ((C + 255) / 256 > 65535) return -2;
+  const long long tiles = (long long)((n_tokens + GT_TOKENS - 1) / GT_TOKENS) * ((C + GT_COLS - 1) / GT_COLS);
+  if (tiles >= sm_count() && (C + GT_COLS - 1) / GT_COLS <= 65535)
+    return launch_pdl(gla_gates_tile_kernel, dim3((n_tokens + GT_TOKENS - 1) / GT_TOKENS, (C + GT_COLS - 1) / GT_COLS), dim3(256), 0,
+                      (cudaStream_t)st, proj, stride, low_off, rank, a2t, bias, inv_tau, C, f, q_off, q_cols, q_scale, n_tokens);
   return launch_pdl(gla_gates_kernel<8>, dim3((n_tokens + 7) / 8, (C + 255) / 256), dim3(256),
                     (size_t)8 * rank * sizeof(float), (cudaStream_t)st, proj, stride, low_off, rank, a2t, bias, inv_tau, C,
                     f, q_off, q_cols, q_scale, n_tokens);
