@@ -72,6 +72,7 @@ class StepContext:
         self.n_seqs = int(host.seq_slot.shape[0])
         # every request brings exactly one token (a decode step): kernels that fuse across a token's row may run
         self.single_token_step = self.n_tokens == self.n_seqs and bool((host.seq_q_len == 1).all())
+        self.some_single_token = bool((host.seq_q_len == 1).any())
         self.all_rows_wanted = (
             host.logit_rows.shape[0] == self.n_tokens
             and bool(np.array_equal(host.logit_rows, np.arange(self.n_tokens, dtype=np.int32)))
@@ -109,6 +110,11 @@ class StepContext:
         """How many tokens each request brings, for work whose launches and scratch go by it; None in a step graph, which is
         replayed for requests of other lengths."""
         return None if self.plan_caps is not None else self.host.seq_q_len
+
+    @property
+    def may_hold_single_tokens(self) -> bool:
+        """Whether a request of the step (of any step a step graph is replayed for) may bring one token only."""
+        return self.plan_caps is not None or self.some_single_token
 
     def layer_cache(self, entry: int, writable: bool = True):
         return self.cache_manager.layer_cache(entry, writable)

@@ -272,7 +272,8 @@ class SinkAttention(Mixer):
             attn = out if out is not None else torch.empty((T, H * M * e), dtype=out_dtype, device=dev)
             ops.attn_sink_tc(q, attn, cache.k, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, tables.indptr,
                              tables.page_ids, ctx.n_seqs, self.sinks, H, G, d, e, cache.page_size, self.scale, self.softcap,
-                             self.window, ctx.status, portions=not ctx.single_token_step, **options)
+                             self.window, ctx.status, portions=not ctx.single_token_step,
+                             singles=ctx.may_hold_single_tokens, **options)
             if out_rows is not None:
                 cut = torch.empty((out_rows.numel(), H * M * e), dtype=out_dtype, device=dev)
                 ops.gather_rows(attn, out_rows, cut)
