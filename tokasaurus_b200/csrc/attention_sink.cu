@@ -344,6 +344,124 @@ sink_attn_prep_vec_kernel(const float* __restrict__ qkv, int stride, const float
     }
   }
 }
+// The same for many tokens: a block has four of them, and its warps take 128 columns at a time of all four, so that a column's bias
+// and norm weight are read once; the next 128 columns are on their way while one lot is worked on.  Bound by memory and by the
+// rotation's angles; with a block a token each vector waited for its own row, bias and weight in turn.  Measured (rows, biases and unit norms
+// as a layer has them, a block a token / this): 32 + 8 + 8 heads of 64, 4,096 tokens 29.7 / 18.9 us, 2,048 17.3 / 13.3, 600 13.8 / 13.6;
+// 8 + 2 + 2 heads, 4,096 tokens 18.9 / 9.7; 32 + 8 + 8 heads of 128, 4,096 tokens 44.4 / 36.4, 2,048 20.0 / 18.9, 1,300 14.8 / 15.9.
+// 64 registers, for four blocks an SM: with three, 2,048 tokens' blocks do not start together (those of 128: 22.5 us).  Eight tokens
+// a block: 23.6 us for the first.
+constexpr int PREP_TOKENS = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(256, 4)
+sink_attn_prep_rows_kernel(const float* __restrict__ qkv, int stride, const float* __restrict__ bias, int norm, float eps,
+                           T* __restrict__ q_out, T* __restrict__ cache, const int* __restrict__ positions,
+                           const int* __restrict__ token_seq, const int* __restrict__ page_indptr,
+                           const int* __restrict__ page_ids, int n_tokens, int nh, int nkv, int page_size, int num_pages, int write_cache,
+                           int* __restrict__ status, const float* __restrict__ norm_w, const double* __restrict__ freq,
+                           int rot_dims, int values_are_keys, int own_kv) {
+  constexpr int N = PREP_TOKENS, LANES = QK / 4;  // lanes that share a vector
+  __shared__ float2 rot_cs[N][QK / 2];            // cosine and sine of each token's angles
+  __shared__ int live[N];                         // a token of this step
+  __shared__ long long at[N];                     // its row in the cache's first head; -1: none
+  trigger_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t0 = blockIdx.x * N, n = min(N, n_tokens - t0);
+  const int nk = own_kv ? nkv : 0, n_qk = (nh + nk) * LANES;            // 16-byte pieces of q and k, and of v behind them
+  const int n_all = n_qk + (write_cache ? nk * VD / 4 : 0);
+  const int voff = values_are_keys ? nh * QK : (nh + nk) * QK;          // (the keys as projected are the values)
+  const int half = freq != nullptr ? rot_dims / 2 : 0;
+  auto column = [&](int i) { return i < n_qk ? 4 * i : voff + 4 * (i - n_qk); };
+  float4 v[N], next[N], b, next_b = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto fetch = [&](int i) {
+    if (i >= n_all) return;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (k < n) next[k] = *reinterpret_cast<const float4*>(qkv + (size_t)(t0 + k) * stride + column(i));
+    if (bias) next_b = *reinterpret_cast<const float4*>(bias + column(i));
+  };
+  fetch(warp * 32 + lane);
+  if (threadIdx.x < N) {
+    const int k = threadIdx.x, s = k < n ? token_seq[t0 + k] : -1;
+    long long row = -1;
+    if (s >= 0 && write_cache && own_kv) {
+      const int p = positions[t0 + k], page = checked_page(page_ids[page_indptr[s] + p / page_size], num_pages, status);
+      if (page >= 0) row = (long long)page * nkv * page_size + p % page_size;
+    }
+    live[k] = s >= 0;
+    at[k] = row;
+  }
+  for (int i = threadIdx.x; i < N * half; i += 256) {
+    const int k = i / half, j = i % half;
+    if (k < n && token_seq[t0 + k] >= 0) {
+      double sn, c;
+      sincos((double)positions[t0 + k] * freq[j], &sn, &c);
+      rot_cs[k][j] = make_float2((float)c, (float)sn);
+    }
+  }
+  __syncthreads();
+  auto store = [](T* to, const float4& x) {
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(to) = x;
+    } else {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+      *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+  };
+  for (int i0 = warp * 32; i0 < n_all; i0 += 256) {
+    const int i = i0 + lane;
+    const bool is_qk = i < n_qk, in = i < n_all;
+    const int hh = is_qk ? i / LANES : (i - n_qk) / (VD / 4), e = (is_qk ? i % LANES : (i - n_qk) % (VD / 4)) * 4;  // vector, first number
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = next[k];
+    b = next_b;
+    fetch(i + 256);
+    if (bias) {
+#pragma unroll
+      for (int k = 0; k < N; k++) v[k].x += b.x, v[k].y += b.y, v[k].z += b.z, v[k].w += b.w;
+    }
+    if (norm && i0 < n_qk) {
+      float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (norm_w && is_qk) w = *reinterpret_cast<const float4*>(norm_w + (hh < nh ? 0 : QK) + e);
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        float ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, v[k].w * v[k].w)));
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);  // (a vector's lanes are all of q and k or none)
+        const float r = rsqrtf(ss / (float)QK + eps);
+        if (is_qk) v[k].x = v[k].x * r * w.x, v[k].y = v[k].y * r * w.y, v[k].z = v[k].z * r * w.z, v[k].w = v[k].w * r * w.w;
+      }
+    }
+    const int j = e / 2;  // the first pair's number
+    if (is_qk && j < half) {
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        const float2 c0 = rot_cs[k][j];
+        const float a = v[k].x, b = v[k].y;
+        v[k].x = a * c0.x - b * c0.y;
+        v[k].y = b * c0.x + a * c0.y;
+        if (j + 1 < half) {
+          const float2 c1 = rot_cs[k][j + 1];
+          const float a1 = v[k].z, b1 = v[k].w;
+          v[k].z = a1 * c1.x - b1 * c1.y;
+          v[k].w = b1 * c1.x + a1 * c1.y;
+        }
+      }
+    }
+    if (is_qk && hh < nh) {
+#pragma unroll
+      for (int k = 0; k < N; k++)
+        if (live[k]) store(q_out + ((size_t)(t0 + k) * nh + hh) * QK + e, v[k]);
+    } else if (in) {
+      const size_t head = is_qk ? (size_t)(hh - nh) * page_size : (size_t)hh * page_size;
+#pragma unroll
+      for (int k = 0; k < N; k++)
+        if (at[k] >= 0) store(cache + (at[k] + head) * ROW + (is_qk ? 0 : KW) + e, v[k]);
+    }
+  }
+}
 #endif
 
 // A short causal convolution a channel between the projections and what sink_attn_prep does:
@@ -710,7 +828,14 @@ int prep_launch(const float* qkv, int stride, const float* bias, int norm, float
   if (norm < 0 || norm > 2) return -2;
 #ifdef TKB_SINK_PREP_VEC
   auto al16 = [](const void* p) { return p == nullptr || ((uintptr_t)p & 15) == 0; };
-  if (norm != 2 && (freq == nullptr || rot_pairs) && stride % 4 == 0 && al16(qkv) && al16(bias) && al16(norm_w) && al16(q_out) && al16(cache))
+  const bool vec = norm != 2 && (freq == nullptr || rot_pairs) && stride % 4 == 0 && al16(qkv) && al16(bias) && al16(norm_w) && al16(q_out) && al16(cache);
+  // From four tokens an SM on; rows of more than 4,096 columns keep a warp busy for long, and need more blocks.
+  const int columns = (nh + (own_kv ? nkv : 0)) * QK + (own_kv ? nkv * VD : 0);
+  if (vec && n_tokens >= (columns <= 4096 ? 592 : 2048))
+    return launch_pdl(sink_attn_prep_rows_kernel<T>, dim3((n_tokens + PREP_TOKENS - 1) / PREP_TOKENS), dim3(256), 0, st, qkv, stride, bias, norm, eps, (T*)q_out,
+                      (T*)cache, positions, token_seq, page_indptr, page_ids, n_tokens, nh, nkv, page_size, num_pages, write_cache,
+                      status, norm_w, freq, rot_dims, values_are_keys, own_kv);
+  if (vec)
     return launch_pdl(sink_attn_prep_vec_kernel<T>, dim3(n_tokens), dim3(256), 0, st, qkv, stride, bias, norm, eps, (T*)q_out,
                       (T*)cache, positions, token_seq, page_indptr, page_ids, nh, nkv, page_size, num_pages, write_cache, status,
                       norm_w, freq, rot_dims, values_are_keys, own_kv);
