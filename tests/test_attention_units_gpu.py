@@ -64,3 +64,58 @@ def test_scores_that_are_not_finite(ops, hd, single, value):
     keep = torch.ones(n, nh, dtype=torch.bool)
     keep[77, 1] = False
     assert torch.equal(got[keep.to(DEV)], want[keep.to(DEV)])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("L,n", [(150, 150), (400, 150), (20, 20)])
+def test_scores_of_minus_infinity(ops, hd, single, L, n):
+    """A score of minus infinity is a weight of zero: beside finite scores the row is what it is without that key, a row that sees
+    no other score is 0 / 0, and the values of keys behind a row's own position do not reach it, however large they are."""
+    import numpy as np
+    from types import SimpleNamespace
+
+    from tokasaurus_b200.parts.attention import plan_attention
+
+    nh, nkv, ps = 3, 1, 1
+    kc, vc, indptr, pages, k, v = make_paged(torch.bfloat16, 1, [L], nkv, hd, ps, L + 3, seed=4)
+    table = pages[:L].long()
+    kc[table, 0, 0, 5] = kc[table, 0, 0, 5].abs() + 0.5  # component 5 of every key is positive
+    plan = plan_attention(SimpleNamespace(seq_q_len=np.asarray([n], dtype=np.int32), seq_kv_len=np.asarray([L], dtype=np.int32)), None,
+                          query_tile=128)
+    c = i32(plan["counts"])
+
+    def run(qkv, kc, vc):
+        out, status = torch.zeros(n, nh * hd, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.attn_prefill_tc(qkv.to(DEV), out, kc, vc, i32([0]), i32([n]), i32([L]), indptr, pages, i32(plan["tiles"]), c[2:3],
+                            int(plan["counts"][2]), nh, nkv, hd, ps, hd ** -0.5, None, status, single_heads=single)
+        assert int(status) == 0
+        return out.view(n, nh, hd)
+
+    qkv = torch.randn(n, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    qkv[:, 5: nh * hd: hd] = qkv[:, 5: nh * hd: hd].abs() + 0.5
+    want = run(qkv, kc, vc)
+    # every score of these rows is minus infinity
+    rows = [0, 7, n - 1]
+    bad = qkv.clone()
+    bad[rows, hd + 5] = -math.inf
+    got = run(bad, kc, vc)
+    assert got[rows, 1].isnan().all()
+    keep = torch.ones(n, nh, dtype=torch.bool)
+    keep[rows, 1] = False
+    assert torch.equal(got[keep.to(DEV)], want[keep.to(DEV)])
+    # one key of minus infinity: rows that see it and others are as without it (float64 sums; the bound of the other tests)
+    key = max(0, L - n) + 3
+    gone = kc.clone()
+    gone[table[key], 0, 0, 5] = -math.inf
+    got = run(qkv, gone, vc)
+    q = qkv[:, : nh * hd].view(n, nh, hd).double().to(DEV)
+    s = torch.einsum("nhd,kd->nhk", q, kc[table, 0, 0].double()) * hd ** -0.5
+    pos = torch.arange(L - n, L, device=DEV)
+    hidden = (torch.arange(L, device=DEV)[None] > pos[:, None]) | (torch.arange(L, device=DEV)[None] == key)
+    ref = torch.softmax(s.masked_fill(hidden[:, None], -math.inf), dim=2) @ vc[table, 0, 0].double()
+    torch.testing.assert_close(got.double(), ref, rtol=1.6e-2, atol=1.2e-2)
+    # the last token's value, which only its own row sees
+    large = vc.clone()
+    large[table[L - 1], 0, 0] = 3.0e38
+    assert torch.equal(run(qkv, kc, large)[: n - 1], want[: n - 1])

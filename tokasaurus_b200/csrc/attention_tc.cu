@@ -185,21 +185,22 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return a;
 }
 // 2^x of two numbers up to 2^6 on the FMA pipe: x = n + f with n the nearest integer, 2^f by a polynomial of degree 4 fitted to 2^f on
-// [-1/2, 1/2] by least squares, weighted until the largest relative error was the smallest (2.6e-6).  Below -126: 2^-126.
+// [-1/2, 1/2] by least squares, weighted until the largest relative error was the smallest (2.8e-6).  Its constant term is one, so that
+// numbers of -127 and below (-infinity among them: masked columns) are zero as they are from ex2: the exponent's bits come out empty.
 __device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
   float x0, x1;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(x));
-  x0 = fmaxf(x0, -126.f);
-  x1 = fmaxf(x1, -126.f);
+  x0 = fmaxf(x0, -127.f);
+  x1 = fmaxf(x1, -127.f);
   asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(x0), "f"(x1));
   constexpr float ROUND = 12582912.f;  // 1.5 * 2^23: the sum's last bits are n
   const uint64_t t = add2(x, twice(ROUND));
   uint64_t f = add2(t, twice(-ROUND));
   asm("sub.rn.f32x2 %0, %1, %0;" : "+l"(f) : "l"(x));
-  uint64_t p = fma2(f, twice(0.009570101276040077f), twice(0.05591785907745361f));
-  p = fma2(p, f, twice(0.240247443318367f));
-  p = fma2(p, f, twice(0.6931217908859253f));
-  p = fma2(p, f, twice(0.9999992847442627f));
+  uint64_t p = fma2(f, twice(0.009582852944731712f), twice(0.05590642616152763f));
+  p = fma2(p, f, twice(0.24024099111557007f));
+  p = fma2(p, f, twice(0.6931242346763611f));
+  p = fma2(p, f, twice(1.f));
   int n0, n1, b0, b1;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(n0), "=r"(n1) : "l"(t));
   asm("mov.b64 {%0, %1}, %2;" : "=r"(b0), "=r"(b1) : "l"(p));
@@ -413,7 +414,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         tile_max = row_max<true>(a, b, lim_hi >= lim_lo ? lim_lo - first - j * step : 1 << 30, span);
       }
       tile_max *= scale_log2;
-      // (a row with a score that is infinite or no number is NaN from here on: the polynomial would make numbers of those)
+      // (a row with a score of infinity or no number is NaN from here on: the polynomial would make numbers of those.  A score of
+      // -infinity is a weight of zero; a row that has no other is 0 / 0)
       const bool moves = !(tile_max - m <= REF_SLACK);
       tile_max += moves ? tile_max - tile_max : 0.f;
       if (j == 0) {
