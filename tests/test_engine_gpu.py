@@ -426,6 +426,40 @@ def test_warm_up_records_the_decode_graphs(tiny_model_dirs):
     assert len(eng.graphs.graphs) == made
 
 
+def test_warm_up_serves_steps_of_one_wave_and_of_more(tiny_model_dirs, monkeypatch):
+    """Whether a step's work items are started longest first is no part of a graph: after ``warm_up`` decoding records nothing
+    more while requests end and the steps of one padded batch size go from more than a wave of items to one."""
+    from tokasaurus_b200.engine.graphs import DecodeGraphs
+
+    lens, ends = (5, 17, 32, 40, 9, 25, 60, 100), (6, 20, 9, 14, 30, 17, 25, 11)
+    prompts = [cuttings.random_tokens(n, 256, 3 * n) for n in lens]
+    seen = []
+    prepare = DecodeGraphs.prepare
+
+    def watched(self, *a):
+        got = prepare(self, *a)
+        seen.extend((got["bp"], int(p["counts"][8])) for p in got["plans"].values())
+        return got
+
+    monkeypatch.setattr(DecodeGraphs, "prepare", watched)
+
+    def tokens(warm, **kw):
+        eng = make_engine(tiny_model_dirs[0], dtype="bfloat16", graph_max_tokens=0, max_seqs_per_forward=8, kv_cache_num_tokens=8 * 4096, **kw)
+        for m in eng.runner.model.planners().values():
+            m.block_slots = 12  # of two blocks an item: five and six short requests are one wave, seven and eight more
+        made = eng.warm_up() if warm else 0
+        seen.clear()
+        ids = [eng.add_request(p, None, n, True) for p, n in zip(prompts, ends)]
+        done = {o.id: o.completion_ids for o in eng.run_until_done()}
+        return [done[i] for i in ids], made, eng
+
+    want, _, _ = tokens(False, use_cudagraphs=False)
+    assert not seen
+    got, made, eng = tokens(True, cudagraph_step=8, cudagraph_max_size=8)
+    assert {(8, 0), (8, 1)} <= set(seen)
+    assert got == want and made == len(eng.graphs.graphs)
+
+
 @pytest.mark.parametrize("sizes", ["1b", "8b"])
 def test_llama_layer_sizes_bfloat16_against_float32(sizes):
     """Two layers of the sizes the benchmark runs (hidden 2,048, 32 heads of 64 on 8 kv heads, inner 8,192,

@@ -85,3 +85,42 @@ def test_order_gives_the_same_bits(hd, nh, nkv, ps, tma, fused):
     assert int(status) == 0 and not want[0].isnan().any()
     for a, b in zip(want, got):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 32, 8), (128, 24, 8), (80, 34, 2)])
+def test_a_grid_larger_than_the_items_serves_both_orders(hd, nh, nkv, fused):
+    """The launch of a step graph: more places than items, and a word on the device that says whether this step is ordered."""
+    from test_kernels_gpu import i32, make_paged
+
+    from tokasaurus_b200.kernels import ops
+
+    ps, lens_kv = 16, [1030, 1, 65, 700, 256, 64, 333]
+    B, blocks = len(lens_kv), nkv * ((nh // nkv + 15) // 16)
+    kc, vc, indptr, pages, _, _ = make_paged(torch.bfloat16, B, lens_kv, nkv, hd, ps, sum(-(-n // ps) for n in lens_kv) + 3, seed=hd)
+    plan = plan_of(lens_kv, None, blocks, 8 * blocks)
+    n_items = int(plan["counts"][0])
+    cap = n_items + 9
+    grown = lambda x, n: i32(np.concatenate([x[:n], np.zeros(n // n_items * cap - n, dtype=np.int32)]))  # noqa: E731
+    items, entry = grown(plan["items"], 3 * n_items), grown(plan["item_entry"], n_items)
+    qkv = torch.randn(B, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(hd)).to(torch.bfloat16).to(DEV)
+    c, status = i32(plan["counts"]), torch.zeros(1, dtype=torch.int32, device=DEV)
+    rot = hd if hd % 4 == 0 else 0
+    inv = RotaryEncoding(rot, 10000.0).inv_freq().to(DEV)
+
+    def run(order, n):
+        k, v, out = kc.clone(), vc.clone(), torch.full((B, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+        args = (qkv, k, v, i32(list(range(B))), i32(lens_kv), indptr, pages, items, i32([n]), cap, i32(plan["dec_seqs"]),
+                i32(plan["dec_item_start"]), c[1:2], B, out, nh, nkv, hd, ps, 1 / math.sqrt(hd), None)
+        if fused:
+            ops.attn_decode_rope_mma(*args, inv, rot, True, status, item_entry=entry, item_order=order)
+        else:
+            ops.attn_decode_mma(*args, item_entry=entry, status=status, item_order=order)
+        return out.view(torch.int16), k.view(torch.int16), v.view(torch.int16)
+
+    want = run(None, n_items)
+    assert int(status) == 0 and not want[0].view(torch.bfloat16).isnan().any()
+    order = grown(plan["item_order"], 4 * n_items)
+    for got in (run(order, n_items), run(torch.zeros_like(order), n_items | ops.ITEMS_LISTED), run(None, n_items | ops.ITEMS_LISTED)):
+        assert all(torch.equal(a, b) for a, b in zip(want, got))

@@ -276,12 +276,13 @@ __device__ __forceinline__ float2 merge_splits(const float* __restrict__ part_o,
 
 // ------------------------------------------------------------------------------------------------
 // Decode: a block a work item (request row, split) and kv head * head_tiles + head tile.  Steps whose items all fit the
-// GPU at once: blockIdx.x = item, blockIdx.y = head block.  Steps of more items than that come with `item_order`, the
-// longest first, and the blocks of one item are neighbours in the grid (x), so that every kv head comes to the items in
-// that order; with the items of one head after those of another the last heads' longest items started when the other
-// heads were nearly through.  A layer's attention and products, heads of 128, 64 requests of 1,000 to 8,192 keys: 324 us,
-// 302 with an item's heads side by side, 225 with the longest first as well.  A step in one wave loses by either: batch 8
+// GPU at once: blockIdx.x = item, blockIdx.y = head block.  Steps of more items than that are ordered: their blocks go through `item_order`, the longest item first, and the blocks of one item are neighbours in the grid, so that every kv
+// head comes to the items in that order; with the items of one head after those of another the last heads' longest items started
+// when the other heads were nearly through.  A layer's attention and products, heads of 128, 64 requests of 1,000 to 8,192 keys:
+// 324 us, 302 with an item's heads side by side, 225 with the longest first as well.  A step in one wave loses by either: batch 8
 // at 2,048 keys 788 us, 793 side by side, 801 sorted too (the requests' last, short items then end together).
+// Which of the two a step is, is read on the device, as a graph of decode steps is replayed for both: ITEMS_LISTED beside the
+// number of items says that `item_order` is not to be gone by.
 // FUSED: q points at the un-rotated q|k|v rows of the step [tokens, (nh + 2 nkv) * HD]; the kernel rotates
 // q on the fly, and the block that owns the split holding the token's own position rotates this kv
 // head's k, writes it and v into the cache page, and only then reads its tiles.
@@ -294,14 +295,16 @@ struct KvMapsParam {
 template <>
 struct KvMapsParam<false> {};
 
-template <bool FUSED, bool TMA, bool ORDERED>
+constexpr int ITEMS_LISTED = 1 << 30;
+
+template <bool FUSED, bool TMA>
 __global__ void __launch_bounds__(128)
 attn_decode_mma_kernel(const __grid_constant__ KvMapsParam<TMA> maps, int tma_rows,
                        const bf16* __restrict__ q, int q_stride, bf16* __restrict__ kcache,
                        bf16* __restrict__ vcache, const int* __restrict__ seq_q_start,
                        const int* __restrict__ seq_kv_len, const int* __restrict__ page_indptr,
                        const int* __restrict__ page_ids, const int* __restrict__ items,
-                       const int* __restrict__ n_items_ptr, float* __restrict__ part_o, float* __restrict__ part_ml,
+                       const int* __restrict__ n_items_ptr, const int* __restrict__ item_order, float* __restrict__ part_o, float* __restrict__ part_ml,
                        int nh, int nkv, int ps, float scale_log2, int window, int head_tiles,
                        const float* __restrict__ inv_freq, int rot, int write_cache, int num_pages,
                        int* __restrict__ status, const float* __restrict__ qkv_parts, int n_parts,
@@ -314,13 +317,24 @@ attn_decode_mma_kernel(const __grid_constant__ KvMapsParam<TMA> maps, int tma_ro
   trigger_dependents();
   // What the host wrote for this step (work items, lengths, block tables) is there before any kernel of the
   // step starts, so the block works out its geometry while the kernel ahead (the q|k|v product) still runs.
-  const int place = ORDERED ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.x;
-  const unsigned hb = ORDERED ? blockIdx.x : blockIdx.y;
-  if (place >= *n_items_ptr) return;
-  // work item: request row, first key (counted from the first visible key), keys; ORDERED: and its place among the items
-  const int* rec = items + (ORDERED ? 4 : 3) * place;
-  const int item = ORDERED ? rec[3] : place;
-  const int s = rec[0];
+  // work item: request row, first key (counted from the first visible key), keys; `item_order` has its place among the items too.
+  // The record that an unordered block takes comes with the number of items, not behind it (0.25 us a layer).
+  int word, s, first, keys, item = blockIdx.x;
+  asm volatile("ld.global.nc.s32 %0, [%4];\nld.global.nc.s32 %1, [%5];\nld.global.nc.s32 %2, [%5 + 4];\nld.global.nc.s32 %3, [%5 + 8];"
+               : "=&r"(word), "=&r"(s), "=&r"(first), "=&r"(keys) : "l"(n_items_ptr), "l"(items + 3 * blockIdx.x));
+  const int n_items = word & (ITEMS_LISTED - 1);
+  unsigned hb = blockIdx.y;
+  if (item_order != nullptr && !(word & ITEMS_LISTED)) {
+    const unsigned id = blockIdx.y * gridDim.x + blockIdx.x, place = id / gridDim.y;
+    if (place >= n_items) return;
+    hb = id - place * gridDim.y;
+    s = item_order[4 * place];
+    first = item_order[4 * place + 1];
+    keys = item_order[4 * place + 2];
+    item = item_order[4 * place + 3];
+  } else if (item >= n_items) {
+    return;
+  }
   const int kvh = hb / head_tiles, ht = hb - kvh * head_tiles;
   const int group = nh / nkv;
   const int g0 = ht * 16;
@@ -330,8 +344,8 @@ attn_decode_mma_kernel(const __grid_constant__ KvMapsParam<TMA> maps, int tma_ro
   const int p = kv_len - 1;
   int lo = 0;
   if (window > 0 && p - window + 1 > 0) lo = p - window + 1;
-  const int k_begin = lo + rec[1];
-  const int k_end = min(kv_len, k_begin + rec[2]);
+  const int k_begin = lo + first;
+  const int k_end = min(kv_len, k_begin + keys);
   const int* table = page_ids + page_indptr[s];
   const int t = seq_q_start[s];
   const bf16* qrow = q + (size_t)t * q_stride + (size_t)(kvh * group + g0) * HD;
@@ -683,7 +697,7 @@ attn_decode_mma_kernel(const __grid_constant__ KvMapsParam<TMA> maps, int tma_ro
   __threadfence();  // this block's partial results are visible before its arrival is counted
   __syncthreads();
   if (tid == 0) {
-    int* c = counters + (size_t)e * (ORDERED ? gridDim.x : gridDim.y) + hb;
+    int* c = counters + (size_t)e * gridDim.y + hb;
     const int prev = atomicAdd(c, 1);
     s_last = prev == i1 - i0 - 1;
     if (s_last) *c = 0;  // every block of this group has arrived: leave the counter ready for the next launch
@@ -890,14 +904,10 @@ static int ensure_smem_attr() {
     if (e == cudaSuccess && DEC_SMEM_B > 48 * 1024)
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM_B);
   };
-  allow(attn_decode_mma_kernel<false, false, false>);
-  allow(attn_decode_mma_kernel<true, false, false>);
-  allow(attn_decode_mma_kernel<false, true, false>);
-  allow(attn_decode_mma_kernel<true, true, false>);
-  allow(attn_decode_mma_kernel<false, false, true>);
-  allow(attn_decode_mma_kernel<true, false, true>);
-  allow(attn_decode_mma_kernel<false, true, true>);
-  allow(attn_decode_mma_kernel<true, true, true>);
+  allow(attn_decode_mma_kernel<false, false>);
+  allow(attn_decode_mma_kernel<true, false>);
+  allow(attn_decode_mma_kernel<false, true>);
+  allow(attn_decode_mma_kernel<true, true>);
   if (e != cudaSuccess) return (int)e;
   g_attr_set = true;
   return 0;
@@ -946,24 +956,19 @@ static int kv_maps(KvMaps& m, const void* kcache, const void* vcache, long long 
 }
 
 // Launch of the split-key kernel: the instantiation with TMA tiles if `tma` and there are descriptors
-template <bool FUSED, bool TMA, bool ORDERED, typename... Rest>
+template <bool FUSED, bool TMA, typename... Rest>
 static int launch_decode_as(dim3 grid, cudaStream_t st, const KvMaps& maps, Rest... rest) {
   KvMapsParam<TMA> param;
   if constexpr (TMA) {
     param.k = maps.k;
     param.v = maps.v;
   }
-  return launch_pdl(attn_decode_mma_kernel<FUSED, TMA, ORDERED>, grid, dim3(128), (size_t)DEC_SMEM_B, st, param, maps.rows, rest...);
+  return launch_pdl(attn_decode_mma_kernel<FUSED, TMA>, grid, dim3(128), (size_t)DEC_SMEM_B, st, param, maps.rows, rest...);
 }
-template <bool FUSED, bool ORDERED, typename... Rest>
-static int launch_decode(bool tma, int items, int head_blocks, void* st, const KvMaps& maps, Rest... rest) {
-  dim3 grid(items, head_blocks);
-  if (ORDERED) {  // the head blocks of an item beside each other, then the items
-    const int y = items < 32768 ? items : 32768;
-    grid = dim3(head_blocks, y, (items + y - 1) / y);
-  }
-  if (tma && maps.rows > 0) return launch_decode_as<FUSED, true, ORDERED>(grid, (cudaStream_t)st, maps, rest...);
-  return launch_decode_as<FUSED, false, ORDERED>(grid, (cudaStream_t)st, maps, rest...);
+template <bool FUSED, typename... Rest>
+static int launch_decode(bool tma, dim3 grid, void* st, const KvMaps& maps, Rest... rest) {
+  if (tma && maps.rows > 0) return launch_decode_as<FUSED, true>(grid, (cudaStream_t)st, maps, rest...);
+  return launch_decode_as<FUSED, false>(grid, (cudaStream_t)st, maps, rest...);
 }
 
 }  // namespace
@@ -989,10 +994,12 @@ TKB_EXPORT int tkb_attn_decode_mma_bf16(const void* q, int q_stride, const void*
   const int group = nh / nkv;
   const int head_tiles = (group + 15) / 16;
   if ((long long)nkv * head_tiles > 65535) return -3;
+  dim3 grid(items_cap, nkv * head_tiles);
   KvMaps maps;
   memset(&maps, 0, sizeof(maps));  // every tile is gathered (num_pages <= 0: the caller does not know the pool's size)
-  return launch_decode<false, false>(false, items_cap, nkv * head_tiles, st, maps, (const bf16*)q, q_stride, (bf16*)kcache, (bf16*)vcache, seq_q_start,
-                              seq_kv_len, page_indptr, page_ids, items, n_items_ptr, part_o, part_ml, nh, nkv, ps,
+  return launch_decode<false>(false, grid, st, maps, (const bf16*)q, q_stride, (bf16*)kcache, (bf16*)vcache, seq_q_start,
+                              seq_kv_len, page_indptr, page_ids, items, n_items_ptr, (const int*)nullptr,
+                              part_o, part_ml, nh, nkv, ps,
                               scale * 1.4426950408889634f, window, head_tiles, (const float*)nullptr, 0, 0, num_pages,
                               status, (const float*)nullptr, 0, 0LL, (int*)nullptr, (const int*)nullptr,
                               (const int*)nullptr, (const int*)nullptr, (bf16*)nullptr, 0, (const float*)nullptr,
@@ -1022,11 +1029,13 @@ TKB_EXPORT int tkb_attn_decode_rope_mma_bf16(const void* qkv, int q_stride, cons
   const int group = nh / nkv;
   const int head_tiles = (group + 15) / 16;
   if ((long long)nkv * head_tiles > 65535) return -3;
+  dim3 grid(items_cap, nkv * head_tiles);
   KvMaps maps;
   rc = kv_maps(maps, kcache, vcache, num_pages, nkv, ps);
   if (rc) return rc;
-  return launch_decode<true, false>(tma != 0, items_cap, nkv * head_tiles, st, maps, (const bf16*)qkv, q_stride, (bf16*)kcache, (bf16*)vcache, seq_q_start,
-                             seq_kv_len, page_indptr, page_ids, items, n_items_ptr, part_o, part_ml, nh, nkv, ps,
+  return launch_decode<true>(tma != 0, grid, st, maps, (const bf16*)qkv, q_stride, (bf16*)kcache, (bf16*)vcache, seq_q_start,
+                             seq_kv_len, page_indptr, page_ids, items, n_items_ptr, (const int*)nullptr,
+                             part_o, part_ml, nh, nkv, ps,
                              scale * 1.4426950408889634f, window, head_tiles, inv_freq, rot, write_cache, num_pages,
                              status, qkv_parts, n_parts, part_stride, (int*)nullptr, (const int*)nullptr,
                              (const int*)nullptr, (const int*)nullptr, (bf16*)nullptr, 0, qkv_bias, qk_norm_w, norm_eps);
@@ -1035,8 +1044,10 @@ TKB_EXPORT int tkb_attn_decode_rope_mma_bf16(const void* qkv, int q_stride, cons
 // Split-key attention with the merge of the splits inside the same kernel (the last block to finish a request's
 // group of heads adds the splits up).  qkv/q_stride as in tkb_attn_decode_mma_bf16 when fused == 0 (rotated q),
 // as in tkb_attn_decode_rope_mma_bf16 when fused != 0.  counters: int32 [dec_cap * head blocks] that are zero
-// before the first launch and are left zero by every launch; item_order: int32 [n_items_cap * 4] (an item's three numbers and
-// its place in `items`) in the order in which the blocks start (null: as they are listed); item_entry[i]: index of item i's request in the decode list; dec_item_start: CSR over that list; out_row_of[request row]: row of `out` to write.
+// before the first launch and are left zero by every launch; item_order: int32 [n_items_cap * 4] (an item's three numbers and its
+// place in `items`) in the order in which the blocks start, or null; n_items_ptr: bit 30 of it says not to go by that order;
+// item_entry[i]: index of item i's request in the decode list; dec_item_start: CSR over that list; out_row_of[request row]: row of
+// `out` to write.
 TKB_EXPORT int tkb_attn_decode_merged_bf16(const void* qkv, int q_stride, const float* qkv_parts, int n_parts,
                                            long long part_stride, void* kcache, void* vcache, const int* seq_q_start,
                                            const int* seq_kv_len, const int* page_indptr, const int* page_ids,
@@ -1059,18 +1070,18 @@ TKB_EXPORT int tkb_attn_decode_merged_bf16(const void* qkv, int q_stride, const 
   KvMaps maps;
   rc = kv_maps(maps, kcache, vcache, num_pages, nkv, ps);
   if (rc) return rc;
-  auto launch = [&](auto run) {
-    return run(tma != 0, items_cap, nkv * head_tiles, st, maps, (const bf16*)qkv, q_stride, (bf16*)kcache, (bf16*)vcache,
-               seq_q_start, seq_kv_len, page_indptr, page_ids, item_order != nullptr ? item_order : items, n_items_ptr, part_o, part_ml, nh, nkv,
-               ps, sl2, window, head_tiles, fused ? inv_freq : nullptr, fused ? rot : 0, fused ? write_cache : 0, num_pages, status,
-               fused ? qkv_parts : nullptr, fused ? n_parts : 0, fused ? part_stride : 0LL, counters,
-               item_entry, dec_item_start, out_row_of, (bf16*)out, out_stride,
-               fused ? qkv_bias : nullptr, fused ? qk_norm_w : nullptr, fused ? norm_eps : 0.f);
-  };
-  if (fused && item_order != nullptr) return launch([](auto... a) { return launch_decode<true, true>(a...); });
-  if (fused) return launch([](auto... a) { return launch_decode<true, false>(a...); });
-  if (item_order != nullptr) return launch([](auto... a) { return launch_decode<false, true>(a...); });
-  return launch([](auto... a) { return launch_decode<false, false>(a...); });
+  dim3 grid(items_cap, nkv * head_tiles);
+  if (fused)
+    return launch_decode<true>(tma != 0, grid, st, maps, (const bf16*)qkv, q_stride, (bf16*)kcache, (bf16*)vcache,
+                               seq_q_start, seq_kv_len, page_indptr, page_ids, items, n_items_ptr, item_order,
+                               part_o, part_ml, nh, nkv, ps, sl2, window, head_tiles, inv_freq, rot, write_cache, num_pages,
+                               status, qkv_parts, n_parts, part_stride, counters, item_entry, dec_item_start, out_row_of,
+                               (bf16*)out, out_stride, qkv_bias, qk_norm_w, norm_eps);
+  return launch_decode<false>(tma != 0, grid, st, maps, (const bf16*)qkv, q_stride, (bf16*)kcache, (bf16*)vcache,
+                              seq_q_start, seq_kv_len, page_indptr, page_ids, items, n_items_ptr, item_order,
+                              part_o, part_ml, nh, nkv, ps, sl2, window, head_tiles, (const float*)nullptr, 0, 0, num_pages,
+                              status, (const float*)nullptr, 0, 0LL, counters, item_entry, dec_item_start, out_row_of,
+                              (bf16*)out, out_stride, (const float*)nullptr, (const float*)nullptr, 0.f);
 }
 
 TKB_EXPORT int tkb_attn_decode_merge_bf16(const float* part_o, const float* part_ml, const int* dec_seqs,

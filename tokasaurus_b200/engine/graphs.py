@@ -110,7 +110,7 @@ class DecodeGraphs:
                 return None
             caps[key] = c
         key = ("general", tp, sp, tuple(page_caps),
-               tuple(sorted((str(k), tuple(sorted(c.items())), *(int(n) for n in raw[k]["counts"][5:])) for k, c in caps.items())))
+               tuple(sorted((str(k), tuple(sorted(c.items())), *(int(n) for n in raw[k]["counts"][5:8])) for k, c in caps.items())))
         plans = {k: planners[k].pad_plan(p, caps[k]) for k, p in raw.items()}
         last = [int(ip[-1]) for ip in host.table_indptr]
         padded = HostBatch(
@@ -151,7 +151,7 @@ class DecodeGraphs:
             cap = bound["items"] if bound is not None and items <= bound["items"] else _pow2_at_least(items, 8)
             caps[key] = dict(items=cap, dec=bp, tiles=0)
         # the kernels a graph holds are chosen at recording: whatever of a plan decides between variants is in the key
-        key = (bp, tuple(page_caps), tuple(sorted((str(k), c["items"], *(int(n) for n in raw[k]["counts"][5:])) for k, c in caps.items())))
+        key = (bp, tuple(page_caps), tuple(sorted((str(k), c["items"], *(int(n) for n in raw[k]["counts"][5:8])) for k, c in caps.items())))
         plans = {k: planners[k].pad_plan(p, caps[k]) for k, p in raw.items()}
         ex = dict(temperature=_pad(extra["temperature"], bp), stream_key=_pad(extra["stream_key"], bp),
                   sample_pos=_pad(extra["sample_pos"], bp), row_slot=_pad(extra["row_slot"], bp, -1))

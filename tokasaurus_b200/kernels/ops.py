@@ -429,6 +429,7 @@ def attn_paged(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: torch.
              _ptr(status), _stream()), "attn_paged")
 
 
+ITEMS_LISTED = 1 << 30  # beside the number of work items on the device: the step's items are not started by ``item_order``
 _COUNTERS: dict = {}
 _COUNTER_INTS = 1 << 20
 
@@ -461,7 +462,7 @@ def attn_decode_mma(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
     ``n_items``/``n_dec`` are device counters; the launch grids are sized by ``items_cap``/``dec_cap``.
     ``tma``: some work item is longer than three tiles (the kernel variant that fetches tiles by TMA pays).
     ``item_order``: (an item's three numbers, its place in ``items``) in the order in which the items' blocks start (with
-    ``item_entry``; None: as they are listed)."""
+    ``item_entry``; None, or ``ITEMS_LISTED`` set beside the number in ``n_items``: as they are listed)."""
     _need_cuda(qkv, kcache, vcache, seq_q_start, seq_kv_len, page_indptr, page_ids, items, n_items, dec_seqs,
                dec_item_start, n_dec, out, status, item_order)
     _need(item_order is None or item_order.numel() >= 4 * items_cap, "attn_decode_mma: item_order")

@@ -120,7 +120,9 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
     item_first = (np.arange(n_items) - np.repeat(dec_start[:-1], n_splits)) * item_size
     items = np.stack([item_seq, item_first, item_size], axis=1).reshape(-1)
     item_entry = np.repeat(np.arange(dec_seqs.shape[0]), n_splits)  # index of each item's request in dec_seqs
-    # items of more than a wave are started longest first (counts[8]): a long one that starts last is what the others wait for
+    # items of more than a wave are started longest first (counts[8]): a long one that starts last is what the others wait for.
+    # The kernel reads it on the device (counts[9]: the number of items, with ops.ITEMS_LISTED where they go as they are
+    # listed), since a step graph is replayed for both
     ordered = int(n_items * blocks_per_item > slots)
     item_order = np.zeros((0,), dtype=np.int64)
     if ordered:
@@ -169,7 +171,7 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
     # counts[7]: so few query tiles that blocks of two heads would leave SMs idle: one head a block
     few_tiles = int(0 < n_tiles <= head_blocks)
     counts = np.asarray([n_items, dec_seqs.shape[0], n_tiles, n_row_items, n_rows, long_items, long_row_items,
-                         few_tiles, ordered], dtype=np.int32)
+                         few_tiles, ordered, n_items | (0 if ordered else ops.ITEMS_LISTED)], dtype=np.int32)
 
     def padded(x, n):
         a = np.zeros(max(n, x.shape[0], 1), dtype=np.int32)
@@ -177,7 +179,7 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
         return a
 
     return dict(counts=counts, items=padded(items, 3 * cap.get("items", 0)),
-                item_entry=padded(item_entry, cap.get("items", 0)), item_order=padded(item_order, 4 * cap.get("items", 0) * ordered),
+                item_entry=padded(item_entry, cap.get("items", 0)), item_order=padded(item_order, 4 * cap.get("items", 0)),
                 dec_seqs=padded(dec_seqs, cap.get("dec", 0)), dec_item_start=padded(dec_start, cap.get("dec", 0) + 1),
                 tiles=padded(tiles, 2 * cap.get("tiles", 0)), **extra)
 
@@ -229,7 +231,7 @@ class AttentionPlanning:
         out = dict(plan)
         out["items"] = padded(plan["items"], 3 * capacity.get("items", 0))
         out["item_entry"] = padded(plan["item_entry"], capacity.get("items", 0))
-        out["item_order"] = padded(plan["item_order"], 4 * capacity.get("items", 0) * int(plan["counts"][8]))
+        out["item_order"] = padded(plan["item_order"], 4 * capacity.get("items", 0))
         out["dec_seqs"] = padded(plan["dec_seqs"], capacity.get("dec", 0))
         out["dec_item_start"] = padded(plan["dec_item_start"], capacity.get("dec", 0) + 1)
         out["tiles"] = padded(plan["tiles"], 2 * capacity.get("tiles", 0))
@@ -332,11 +334,12 @@ class PagedAttention(AttentionPlanning, Mixer):
                 caps = ctx.plan_caps.get(self.plan_key()) if ctx.plan_caps else None
                 c = plan["counts"]
                 ops.attn_decode_rope_mma(parts, cache.k, cache.v, ctx.seq_q_start, ctx.seq_kv_len, tables.indptr,
-                                         tables.page_ids, plan["items"], c[0:1], caps["items"] if caps else int(counts[0]),
+                                         tables.page_ids, plan["items"], c[9:10], caps["items"] if caps else int(counts[0]),
                                          plan["dec_seqs"], plan["dec_item_start"], c[1:2],
                                          caps["dec"] if caps else int(counts[1]), attn, nh, nkv, hd, cache.page_size,
                                          self.scale, self.window, self.inv_freq, rot, cache.writable,
-                                         ctx.status, item_entry=plan["item_entry"], item_order=plan["item_order"] if counts[8] else None, tma=bool(counts[5]),
+                                         ctx.status, item_entry=plan["item_entry"], tma=bool(counts[5]),
+                                         item_order=plan["item_order"] if caps or counts[8] else None,
                                          bias=self.qkv_bias, qk_norm=self.qk_norm, norm_eps=self.norm_eps)
                 return few(attn, self.w_o)
             qkv = torch.empty((T, nh * hd), dtype=h.dtype, device=h.device)  # q only; k and v go straight to the cache
@@ -383,9 +386,10 @@ class PagedAttention(AttentionPlanning, Mixer):
         c = plan["counts"]
         if dec_cap:
             ops.attn_decode_mma(qkv, cache.k, cache.v, ctx.seq_q_start, ctx.seq_kv_len, tables.indptr, tables.page_ids,
-                                plan["items"], c[0:1], items_cap, plan["dec_seqs"], plan["dec_item_start"], c[1:2],
+                                plan["items"], c[9:10], items_cap, plan["dec_seqs"], plan["dec_item_start"], c[1:2],
                                 dec_cap, attn, nh, nkv, hd, cache.page_size, self.scale, self.window,
-                                item_entry=plan["item_entry"], tma=bool(counts[5]), status=ctx.status, item_order=plan["item_order"] if counts[8] else None)
+                                item_entry=plan["item_entry"], tma=bool(counts[5]), status=ctx.status,
+                                item_order=plan["item_order"] if caps or counts[8] else None)
         if tiles_cap and self._query_tile() == QUERY_TILE_TC:
             ops.attn_prefill_tc(qkv, attn, cache.k, cache.v, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
                                 tables.indptr, tables.page_ids, plan["tiles"], c[2:3], tiles_cap, nh, nkv, hd,

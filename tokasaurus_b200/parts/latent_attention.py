@@ -218,10 +218,10 @@ class LatentAttention(AttentionPlanning, Mixer):
         rows = cache.k  # keys and values at once
         if dec_cap:
             ops.attn_decode_mma(q2, rows, rows, ctx.seq_q_start, ctx.seq_kv_len, tables.indptr, tables.page_ids,
-                                plan["items"], c[0:1], items_cap, plan["dec_seqs"], plan["dec_item_start"], c[1:2],
+                                plan["items"], c[9:10], items_cap, plan["dec_seqs"], plan["dec_item_start"], c[1:2],
                                 dec_cap, attn, H, 1, Dk, cache.page_size, self.scale, self.window,
                                 item_entry=plan["item_entry"], tma=bool(counts[5]), status=ctx.status,
-                                item_order=plan["item_order"] if counts[8] else None)
+                                item_order=plan["item_order"] if caps or counts[8] else None)
         if tiles_cap and self._rows_tc():
             ops.attn_rows_tc(self._rows_tc()[0], q2, attn, Dk, rows, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, tables.indptr,
                              tables.page_ids, ctx.n_seqs, H, 1, cache.page_size, self.scale, self.window, ctx.status)
