@@ -460,6 +460,32 @@ def test_warm_up_serves_steps_of_one_wave_and_of_more(tiny_model_dirs, monkeypat
     assert got == want and made == len(eng.graphs.graphs)
 
 
+@pytest.mark.parametrize("graph_max_tokens", [0, 1024])
+def test_wanted_rows_go_by_their_order(tiny_model_dirs, monkeypatch, graph_max_tokens):
+    """The last layer's one query a wanted row: its items of more than a wave are started longest first, with the same tokens."""
+    from tokasaurus_b200.kernels import ops
+
+    prompts = [cuttings.random_tokens(n, 256, 3 * n) for n in (100, 17, 110, 40, 90, 25, 60, 5)]
+    launch, seen = ops.attn_decode_mma, []
+
+    def watched(*a, item_order=None, **kw):
+        if kw.get("out_row_of") is not None:
+            seen.append((int(a[7].numel()), item_order is not None))
+            item_order = None if drop else item_order
+        return launch(*a, item_order=item_order, **kw)
+
+    monkeypatch.setattr(ops, "attn_decode_mma", watched)
+    outs = []
+    for drop in (True, False):
+        eng = make_engine(tiny_model_dirs[0], dtype="bfloat16", max_seqs_per_forward=8, kv_cache_num_tokens=4096, graph_max_tokens=graph_max_tokens)
+        for m in eng.runner.model.planners().values():
+            m.block_slots = 4
+        seen.clear()
+        outs.append([o.completion_ids for o in eng.generate(prompts, max_num_tokens=6, ignore_eos=True)])
+        assert any(given for _, given in seen)
+    assert outs[0] == outs[1]
+
+
 @pytest.mark.parametrize("sizes", ["1b", "8b"])
 def test_llama_layer_sizes_bfloat16_against_float32(sizes):
     """Two layers of the sizes the benchmark runs (hidden 2,048, 32 heads of 64 on 8 kv heads, inner 8,192,

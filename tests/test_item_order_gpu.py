@@ -46,6 +46,30 @@ def test_unequal_requests_end_sooner_cut_at_the_nearest_share():
     assert slots // 8 < len(items) <= slots // 8 + 32
 
 
+@pytest.mark.parametrize("slots,ordered", [(64, True), (4096, False)])
+def test_order_of_the_wanted_rows(slots, ordered):
+    """The wanted rows' items of more than a wave have an order of their own, also padded to a graph's sizes."""
+    from tokasaurus_b200.kernels import ops
+    from tokasaurus_b200.parts.attention import AttentionPlanning
+
+    lens_q, lens_kv = [5, 1, 300, 7, 64], [700, 40, 3000, 7, 1200]
+    ends = np.cumsum(lens_q) - 1
+    positions = np.concatenate([np.arange(n - q, n) for q, n in zip(lens_q, lens_kv)])
+    host = SimpleNamespace(seq_q_len=np.asarray(lens_q, dtype=np.int32), seq_kv_len=np.asarray(lens_kv, dtype=np.int32),
+                           logit_rows=ends.astype(np.int32), token_ids=positions, positions=positions,
+                           token_seq=np.repeat(np.arange(5), lens_q), table_indptr=[np.arange(6)])
+    plan = plan_attention(host, None, blocks_per_item=8, slots=slots)
+    n, word = int(plan["counts"][3]), int(plan["counts"][10])
+    assert word == n | (0 if ordered else ops.ITEMS_LISTED) and ordered == (8 * n > slots)
+    grown = AttentionPlanning.pad_plan(None, plan, dict(items=50, dec=9, tiles=20, row_items=n + 7, rows=6))
+    assert grown["row_item_order"].shape[0] == 4 * (n + 7)
+    if ordered:
+        items, order = plan["row_items"][: 3 * n].reshape(-1, 3), grown["row_item_order"][: 4 * n].reshape(-1, 4)
+        assert sorted(order[:, 3].tolist()) == list(range(n)) and (items[order[:, 3]] == order[:, :3]).all()
+        keys = np.minimum(order[:, 2], np.asarray(lens_kv)[order[:, 0]] - order[:, 1])
+        assert (keys > 0).all() and (np.diff(keys) <= 0).all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("hd,nh,nkv,ps", [(64, 32, 8, 16), (128, 24, 8, 16), (48, 6, 3, 4), (80, 34, 2, 16), (256, 4, 1, 16)])
 @pytest.mark.parametrize("tma", [True, False])

@@ -99,6 +99,12 @@ def _slowest_slot(span, n, size, slots: int) -> float:
     return most
 
 
+def _longest_first(row, first, size, span) -> np.ndarray:
+    """(row, first key, keys, place in the list) of every work item, those with the most keys first."""
+    order = np.argsort(-np.minimum(size, span - first), kind="stable")
+    return np.stack([row, first, size, np.arange(row.shape[0])], axis=1)[order].reshape(-1)
+
+
 def plan_attention(host, window: int | None, capacity: dict | None = None, blocks_per_item: int = 8,
                    query_tile: int = QUERY_TILE, slots: int = DECODE_BLOCK_SLOTS,
                    head_blocks: int = 0) -> dict[str, np.ndarray]:
@@ -124,10 +130,7 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
     # The kernel reads it on the device (counts[9]: the number of items, with ops.ITEMS_LISTED where they go as they are
     # listed), since a step graph is replayed for both
     ordered = int(n_items * blocks_per_item > slots)
-    item_order = np.zeros((0,), dtype=np.int64)
-    if ordered:
-        by_keys = np.argsort(-np.minimum(item_size, np.repeat(span, n_splits) - item_first), kind="stable")
-        item_order = np.stack([item_seq, item_first, item_size, np.arange(n_items)], axis=1)[by_keys].reshape(-1)
+    item_order = _longest_first(item_seq, item_first, item_size, np.repeat(span, n_splits)) if ordered else np.zeros((0,), dtype=np.int64)
     pre_seqs = np.nonzero(q_len > 1)[0]
     n_tiles_seq = -(-q_len[pre_seqs] // query_tile)
     tile_start = np.concatenate([[0], np.cumsum(n_tiles_seq)])
@@ -142,7 +145,7 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
     # wanted rows, when they are only some of the step's rows: each is one query over the keys up to its
     # own position, which is what the split-key kernel computes for a request that brings one token
     extra = {}
-    n_row_items = n_rows = 0
+    n_row_items = n_rows = rows_ordered = 0
     rows = getattr(host, "logit_rows", None)
     if rows is not None and capacity is None and 0 < rows.shape[0] and not (
             rows.shape[0] == host.token_ids.shape[0] and np.array_equal(rows, np.arange(rows.shape[0]))):
@@ -155,8 +158,10 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
         r_item = np.repeat(np.arange(n_rows), r_splits)
         r_isize = np.repeat(r_size, r_splits)
         r_first = (np.arange(n_row_items) - np.repeat(r_start[:-1], r_splits)) * r_isize
+        rows_ordered = int(n_row_items * blocks_per_item > slots)  # (counts[10], as counts[9])
         i32 = lambda a: np.ascontiguousarray(a, dtype=np.int32)  # noqa: E731
-        extra = dict(row_items=i32(np.stack([r_item, r_first, r_isize], axis=1).reshape(-1)), row_item_start=i32(r_start),
+        extra = dict(row_item_order=i32(_longest_first(r_item, r_first, r_isize, np.repeat(r_span, r_splits)) if rows_ordered else [0]),
+                     row_items=i32(np.stack([r_item, r_first, r_isize], axis=1).reshape(-1)), row_item_start=i32(r_start),
                      row_item_entry=i32(r_item),
                      row_token=i32(rows), row_kv_len=i32(r_kv),
                      row_index=i32(np.arange(n_rows)))
@@ -171,7 +176,8 @@ def plan_attention(host, window: int | None, capacity: dict | None = None, block
     # counts[7]: so few query tiles that blocks of two heads would leave SMs idle: one head a block
     few_tiles = int(0 < n_tiles <= head_blocks)
     counts = np.asarray([n_items, dec_seqs.shape[0], n_tiles, n_row_items, n_rows, long_items, long_row_items,
-                         few_tiles, ordered, n_items | (0 if ordered else ops.ITEMS_LISTED)], dtype=np.int32)
+                         few_tiles, ordered, n_items | (0 if ordered else ops.ITEMS_LISTED),
+                         n_row_items | (0 if rows_ordered else ops.ITEMS_LISTED)], dtype=np.int32)
 
     def padded(x, n):
         a = np.zeros(max(n, x.shape[0], 1), dtype=np.int32)
@@ -239,6 +245,7 @@ class AttentionPlanning:
             ri, rows = capacity.get("row_items", 0), capacity.get("rows", 0)
             out["row_items"] = padded(plan["row_items"], 3 * ri)
             out["row_item_entry"] = padded(plan["row_item_entry"], ri)
+            out["row_item_order"] = padded(plan["row_item_order"], 4 * ri)
             out["row_item_start"] = padded(plan["row_item_start"], rows + 1)
             for name in plan:
                 if name in ("row_token", "row_kv_len", "row_index") or name.startswith("row_indptr_g"):
@@ -364,10 +371,11 @@ class PagedAttention(AttentionPlanning, Mixer):
             c = plan["counts"]
             ops.attn_decode_mma(qkv, cache.k, cache.v, plan["row_token"], plan["row_kv_len"],
                                 plan[f"row_indptr_g{cache.group}"],
-                                tables.page_ids, plan["row_items"], c[3:4], n_items, plan["row_index"],
+                                tables.page_ids, plan["row_items"], c[10:11], n_items, plan["row_index"],
                                 plan["row_item_start"], c[4:5], n_rows, attn, nh, nkv, hd, cache.page_size,
                                 self.scale, self.window, out_row_of=plan["row_index"],
-                                item_entry=plan["row_item_entry"], tma=bool(counts[6]), status=ctx.status)
+                                item_entry=plan["row_item_entry"], tma=bool(counts[6]), status=ctx.status,
+                                item_order=plan["row_item_order"] if caps or not counts[10] & ops.ITEMS_LISTED else None)
             return project(attn, self.w_o)
         if plan is None or out_rows is not None:
             # float32, or only some rows are wanted: the FP32-pipe kernel
