@@ -105,3 +105,20 @@ def test_few_query_tiles_ask_for_one_head_a_block():
     assert counts([1, 1, 300], 148 // 32)[7] == 1  # decoding requests make no tiles
     assert counts([1, 1], 148 // 32)[7] == 0       # no tiles at all
     assert counts([512], 0)[7] == 0                # a planner that was given no device
+
+
+def test_a_finer_cut_goes_into_a_second_wave_only_for_a_gain():
+    """Unequal requests cut at the nearest share make a few items more than a wave: worth it where the estimate is well below the other
+    cut's (32 requests of 512 to 4,096 keys), not where it is next to the same (16 of 173 to 1,384, which measured 41 and 50 us)."""
+    def items(spans, slots=37):
+        n, size = split_keys_evenly(np.asarray(spans, dtype=np.int64), 8, 8 * slots)
+        assert ((n - 1) * size < spans).all() and (n * size >= spans).all()
+        return int(n.sum())
+
+    def contexts(requests, most):
+        return np.asarray([int(most * (0.125 + 0.875 * ((i * 29) % 64) / 63.0)) for i in range(requests)])
+
+    assert items(contexts(32, 4096)) > 37
+    for requests, most in ((16, 1387), (30, 1200), (12, 976), (41, 785)):
+        assert items(contexts(requests, most)) <= max(37, requests), (requests, most)
+    assert 31 < items(np.asarray([5819 - 97 * i for i in range(16)])) <= 37  # within a wave: finer where the slots allow it
