@@ -19,14 +19,14 @@
 // loop has no pass over O.  (S_j is complete only after P_(j-1) . V: one thread issues both, in that order.)
 // What bounds it: exponentials and the chain a unit goes through for each of its tiles (scores into registers, maximum, exponentials, P,
 // the wait for the unit's slowest warp, the issue of eight instructions, S), about 3,000 clocks with four units at once; of 128
-// keys of two heads the exponentials alone take 1,540 (three quarters on the special-function unit, a quarter as a polynomial).
+// keys of two heads the exponentials alone take about 1,540 (most on the special-function unit, some as a polynomial).
 // Neither the products nor the scan for the maximum: a quarter of the instructions left out, or the scan, changed nothing.
 // Four units and not two: with one warp a scheduler and head (the form before, tiles of 128 keys, P through shared memory) 128 keys took
 // 3,490 clocks, in which waits for S and the exponentials hardly overlapped; taking turns at the exponentials, skewing the heads and a
 // polynomial for some of them changed nothing there.
-// Measured (32 heads on 8 kv heads, the form before / now): one prompt of 2,048 tokens 44.7 / 41.9 us, of 8,192 477 / 400 us (688 TFLOP/s of
-// causal flops), 2,048 tokens behind 2,048 others 107 / 93, 512 behind 2,048 (one head a block) 38 / 29; 24 heads on 8, 2,048
-// tokens 48.5 / 39.7.
+// Measured (32 heads on 8 kv heads, the form before / now): one prompt of 2,048 tokens 43.8 / 42.5 us, of 8,192 477 / 412 us (668 TFLOP/s of
+// causal flops), 2,048 tokens behind 2,048 others 108 / 95, 512 behind 2,048 (one head a block) 37 / 28; 12 heads on 4, 8,192
+// tokens 226 / 178.
 // Roles: warps 0-15 softmax and output of the four units, one warp of each also issues its unit's MMAs (warps of their own took 440
 // clocks longer a tile: their instructions, polls among them, share the schedulers with four busy warps each); warp 16 brings K
 // tiles and warp 17 V tiles into a ring: a tile whose 64 keys all exist comes by TMA, one box per page through the block table
@@ -184,8 +184,9 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
   return a;
 }
-// 2^x of two numbers up to 2^6 on the FMA pipe: x = n + f with n the nearest integer, 2^f by a polynomial of degree 4 fitted to 2^f on
-// [-1/2, 1/2] by least squares, weighted until the largest relative error was the smallest (2.8e-6).  Its constant term is one, so that
+// 2^x of two numbers up to 2^6 on the FMA pipe: x = n + f with n the nearest integer, 2^f by a polynomial of degree 5 fitted to 2^f on
+// [-1/2, 1/2] by least squares, weighted until the largest relative error was the smallest (9e-8; 1.7e-7 with float32's roundings, which
+// is ex2's).  Its constant term is one, so that
 // numbers of -127 and below (-infinity among them: masked columns) are zero as they are from ex2: the exponent's bits come out empty.
 __device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
   float x0, x1;
@@ -197,9 +198,10 @@ __device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
   const uint64_t t = add2(x, twice(ROUND));
   uint64_t f = add2(t, twice(-ROUND));
   asm("sub.rn.f32x2 %0, %1, %0;" : "+l"(f) : "l"(x));
-  uint64_t p = fma2(f, twice(0.009582852944731712f), twice(0.05590642616152763f));
-  p = fma2(p, f, twice(0.24024099111557007f));
-  p = fma2(p, f, twice(0.6931242346763611f));
+  uint64_t p = fma2(f, twice(0.001326472731307149f), twice(0.009671512991189957f));
+  p = fma2(p, f, twice(0.05550733581185341f));
+  p = fma2(p, f, twice(0.24022242426872253f));
+  p = fma2(p, f, twice(0.6931470036506653f));
   p = fma2(p, f, twice(1.f));
   int n0, n1, b0, b1;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(n0), "=r"(n1) : "l"(t));
@@ -207,9 +209,9 @@ __device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
   p0 = __int_as_float(b0 + (n0 << 23));
   p1 = __int_as_float(b1 + (n1 << 23));
 }
-// Of 16 pairs so many take the polynomial and not the special-function unit (one prompt of 8,192 tokens, 32 heads: none 422 us, 2
-// 416, 4 401, 6 430, 8 460).
-constexpr int POLY = 4;
+// Of 16 pairs so many take the polynomial and not the special-function unit (32 heads, us, 2 / 3 / 4: one prompt of 8,192 tokens 418 /
+// 412 / 437, 2,048 tokens behind 2,048 others 95.6 / 95.0 / 99.3, one prompt of 2,048 42.8 / 42.5 / 43.0, of 700 18.5 / 18.3 / 17.5).
+constexpr int POLY = 3;
 // p = 2^(s * scale - m) of 32 scores, as bfloat16 pairs; adds them to `sum`.  Scaling and adding take two at a time.
 __device__ __forceinline__ void row_exp(const uint32_t (&v)[32], uint32_t* pk, uint64_t scale, uint64_t neg_m, uint64_t& sum) {
 #pragma unroll
