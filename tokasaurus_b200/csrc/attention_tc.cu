@@ -3,8 +3,8 @@
 // A block owns 128 consecutive query tokens of TWO query heads that share a kv head (one head where the group
 // size is odd and no partner is left, or where pairs would leave SMs without a block) and walks the keys they may see
 // in tiles of 64, which are brought once for both heads.  Four UNITS share the work: each has 128 rows of one head, every
-// second tile (two heads) or every fourth (one head), and scores, reference, sum and output of its own; a head's units are put
-// together at the end.  For each unit and tile:
+// second tile (two heads) or every fourth (one head; where there are few, all of them or every second), and scores, reference, sum
+// and output of its own; a head's units are put together at the end.  For each unit and tile:
 //     S = Q . K^T      tcgen05.mma 128 x 64 x 16, four per tile, Q and K tiles K-major in shared memory,
 //                      S (float32) in tensor memory
 //     softmax          a warpgroup per unit, one thread per query row (a lane of tensor memory): the row's 64 scores come into
@@ -24,7 +24,7 @@
 // Four units and not two: with one warp a scheduler and head (the form before, tiles of 128 keys, P through shared memory) 128 keys took
 // 3,490 clocks, in which waits for S and the exponentials hardly overlapped; taking turns at the exponentials, skewing the heads and a
 // polynomial for some of them changed nothing there.
-// Measured (32 heads on 8 kv heads, the form before / now): one prompt of 2,048 tokens 43.8 / 42.5 us, of 8,192 477 / 412 us (668 TFLOP/s of
+// Measured (32 heads on 8 kv heads, the form before / now): one prompt of 2,048 tokens 43.9 / 42.2 us, of 8,192 475 / 412 us (668 TFLOP/s of
 // causal flops), 2,048 tokens behind 2,048 others 108 / 95, 512 behind 2,048 (one head a block) 37 / 28; 12 heads on 4, 8,192
 // tokens 226 / 178.
 // Roles: warps 0-15 softmax and output of the four units, one warp of each also issues its unit's MMAs (warps of their own took 440
@@ -209,10 +209,11 @@ __device__ __forceinline__ void exp2_poly(uint64_t x, float& p0, float& p1) {
   p0 = __int_as_float(b0 + (n0 << 23));
   p1 = __int_as_float(b1 + (n1 << 23));
 }
-// Of 16 pairs so many take the polynomial and not the special-function unit (32 heads, us, 2 / 3 / 4: one prompt of 8,192 tokens 418 /
-// 412 / 437, 2,048 tokens behind 2,048 others 95.6 / 95.0 / 99.3, one prompt of 2,048 42.8 / 42.5 / 43.0, of 700 18.5 / 18.3 / 17.5).
-constexpr int POLY = 3;
-// p = 2^(s * scale - m) of 32 scores, as bfloat16 pairs; adds them to `sum`.  Scaling and adding take two at a time.
+// p = 2^(s * scale - m) of 32 scores, as bfloat16 pairs; adds them to `sum`.  Scaling and adding take two at a time.  Of the 16 pairs
+// POLY take the polynomial and not the special-function unit.  A row's two halves with two and four of them (32 heads, us, beside two,
+// three, four in both): one prompt of 8,192 tokens 412 (418, 414, 435), 2,048 tokens behind 2,048 others 94.8 (95.6, 95.7, 98.8), one
+// prompt of 2,048 42.2 (42.8, 42.7, 42.7).
+template <int POLY>
 __device__ __forceinline__ void row_exp(const uint32_t (&v)[32], uint32_t* pk, uint64_t scale, uint64_t neg_m, uint64_t& sum) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
@@ -262,13 +263,31 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   __shared__ int failed;
   trigger_dependents();
   grid_dependency_wait();
-  // Blocks of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
+  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block).  In odd groups of heads the blocks
+  // of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
   // tiles' order the last blocks of two heads started when the SMs were nearly through).
-  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
-  const int group = nh / nkv, per_tile = nkv * (single ? group : group >> 1);
-  const unsigned id = blockIdx.y * gridDim.x + blockIdx.x, n_pairs = gridDim.y * per_tile;
-  const bool paired = id < n_pairs;
-  const int tile = paired ? id / per_tile : (id - n_pairs) / nkv;
+  const int group = nh / nkv;
+  int tile = blockIdx.y, kvh, head0, n_heads_here = single ? 1 : 2;
+  if (single || !(group & 1)) {
+    kvh = blockIdx.x / (single ? group : group >> 1);
+    head0 = blockIdx.x * n_heads_here;
+  } else {
+    const int per_tile = nkv * (group >> 1);
+    unsigned id = blockIdx.y * gridDim.x + blockIdx.x;
+    const unsigned n_pairs = gridDim.y * per_tile;
+    if (id < n_pairs) {
+      tile = id / per_tile;
+      id -= tile * per_tile;
+      kvh = id / (group >> 1);
+      head0 = 2 * id + kvh;
+    } else {
+      id -= n_pairs;
+      tile = id / nkv;
+      kvh = id - tile * nkv;
+      head0 = (kvh + 1) * group - 1;
+      n_heads_here = 1;
+    }
+  }
   if (tile >= *n_tiles_ptr) return;
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sQ = base;                        // two heads
@@ -278,11 +297,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   const int s = tiles[2 * tile], qt0 = tiles[2 * tile + 1];
-  const int in_tile = paired ? id - tile * per_tile : id - n_pairs - tile * nkv;
-  const int kvh = paired ? in_tile / (single ? group : group >> 1) : in_tile;
-  const int head0 = paired ? in_tile * (single ? 1 : 2) + (single ? 0 : kvh * (group & 1)) : (kvh + 1) * group - 1;
-  const int n_heads_here = paired && !single ? 2 : 1;
-  const int streams = UNITS / n_heads_here;  // unit u: head u / streams, tiles u % streams, u % streams + streams, ...
   const int q_len = seq_q_len[s], kv_len = seq_kv_len[s];
   const int rows_live = min(BQ, q_len - qt0);
   const int pos0 = kv_len - q_len + qt0;
@@ -291,8 +305,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (window > 0 && pos0 - window + 1 > 0) k_begin = (pos0 - window + 1) & ~(BKV - 1);
   const int k_end = pos0 + rows_live;  // one past the last key any row of the tile sees
   const int n_kv_tiles = (k_end - k_begin + BKV - 1) / BKV;
+  // Unit u: head u >> split, tiles u & (streams - 1), that + streams, ...  Putting units together costs 1.4 us, a key tile 0.4 us: a lone
+  // head's tiles go to two units up to nine of them (512 tokens of 32 heads 12.1 us with four, 11.3 with two; 600 keys 12.6 and 13.0),
+  // those of two heads to one unit a head up to two (30 prompts of 100 tokens 36.3 and 34.9).
+  const int split = n_heads_here == 2 ? (n_kv_tiles > 2 ? 1 : 0) : n_kv_tiles > 9 ? 2 : 1, streams = 1 << split;
   const int live_streams = min(streams, n_kv_tiles);
-  auto tiles_of = [&](int stream) { return (n_kv_tiles - stream + streams - 1) / streams; };  // (0 from live_streams on)
+  auto tiles_of = [&](int stream) { return (n_kv_tiles - stream + streams - 1) >> split; };  // (0 from live_streams on)
   const int* table = page_ids + page_indptr[s];
   const int t0 = seq_q_start[s] + qt0;
 
@@ -363,9 +381,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
     if (!ok) failed = 1;
     report_bad_page(bad_page, status);
-  } else if ((warp >> 2) % streams < live_streams) {
+  } else if ((warp >> 2) < n_heads_here << split && ((warp >> 2) & (streams - 1)) < live_streams) {
     // ---------------- softmax and output: thread = query row = lane of tensor memory
-    const int u = warp >> 2, hh = u / streams, stream = u - hh * streams;
+    const int u = warp >> 2, hh = u >> split, stream = u & (streams - 1);
     const int r = tid & 127, n = tiles_of(stream);
     const int pos = pos0 + r;
     const int lim_hi = pos < k_end - 1 ? pos : k_end - 1;
@@ -399,8 +417,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     // Tiles [whole_from, whole_to) of the unit are seen whole by every row of the block and need no mask; in the others columns
     // [lo, lo + span] are visible.
     const int first = k_begin + stream * BKV, step = streams * BKV;
-    const int whole_to = min(pos0 + 1, k_end) - BKV - first < 0 ? 0 : (min(pos0 + 1, k_end) - BKV - first) / step + 1;
-    const int whole_from = window <= 0 || first >= pos0 + BQ - window ? 0 : (pos0 + BQ - window - first + step - 1) / step;
+    const int whole_to = min(pos0 + 1, k_end) - BKV - first < 0 ? 0 : ((min(pos0 + 1, k_end) - BKV - first) >> (6 + split)) + 1;
+    const int whole_from = window <= 0 || first >= pos0 + BQ - window ? 0 : (pos0 + BQ - window - first + step - 1) >> (6 + split);
+    static_assert(BKV == 64, "shifts");
     const uint32_t span = lim_hi >= lim_lo ? (uint32_t)(lim_hi - lim_lo) : 0u;
     for (int j = 0; j < n && ok; j++) {
       if (!mbar_wait(&s_full[u], j & 1)) { ok = false; break; }
@@ -441,8 +460,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       if (issuer && j + 1 < n && !mbar_wait(&full[next_ring()], next_phase())) { ok = false; break; }
       uint32_t pk[32];
       uint64_t sums = 0;
-      row_exp(a, pk, scale2, twice(-m), sums);
-      row_exp(b, pk + 16, scale2, twice(-m), sums);
+      row_exp<2>(a, pk, scale2, twice(-m), sums);
+      row_exp<4>(b, pk + 16, scale2, twice(-m), sums);
       tmem_st32(s_addr, pk);
       float s0, s1;
       asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sums));
