@@ -119,3 +119,13 @@ def test_scores_of_minus_infinity(ops, hd, single, L, n):
     large = vc.clone()
     large[table[L - 1], 0, 0] = 3.0e38
     assert torch.equal(run(qkv, kc, large)[: n - 1], want[: n - 1])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nh,nkv,ps,window,single", [(3, 1, 16, None, False), (4, 2, 5, None, True), (5, 1, 8, 1350, False), (1, 1, 16, None, False)])
+def test_lone_heads_with_many_key_tiles(ops, hd, nh, nkv, ps, window, single):
+    """Around the number of key tiles from which a lone head's go to two units (heads of 128), odd and even numbers of them."""
+    lens_kv = [1344, 1345, 1408, 1409, 1530, 2047]
+    lens_q = [2, 130, 3, 2, 70, 5]
+    got, want = run_mma_attention(ops, lens_q, lens_kv, nh, nkv, hd, ps, window, seed=hd + nh, tc=True, single_heads=single)
+    torch.testing.assert_close(got, want, rtol=1.6e-2, atol=1.2e-2)  # the bound of the other tests of these kernels

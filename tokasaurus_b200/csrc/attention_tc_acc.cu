@@ -3,9 +3,9 @@
 //
 // A block owns 128 consecutive query tokens of TWO query heads that share a kv head (one head where the group size is odd and no
 // partner is left, or where pairs would leave SMs without a block) and walks the keys they may see in tiles of 64.  Two UNITS
-// share the work: the two heads, or the even and the odd tiles of one head, each with a reference, sum and output of its own that
-// are put together at the end (one head in one unit left the other half of the block idle: 24 heads on 8 kv heads, 2,048 tokens behind
-// 2,048 others 126 us, 111 with two units and the blocks of two heads first).  For each unit:
+// share the work: the two heads, or, with LONE_TILES key tiles and more, the even and the odd tiles of one head, each with a reference,
+// sum and output of its own that are put together at the end (one head in one unit left the other half of the block idle: 24 heads on 8 kv
+// heads, 2,048 tokens behind 2,048 others 126 us, 111 with two units and the blocks of two heads first).  For each unit:
 //     S = Q . K^T      tcgen05.mma 128 x 64 x 16, HD / 16 per tile, two S tiles in tensor memory (the product of
 //                      tile j+2 starts as soon as the softmax threads are through with S_j)
 //     softmax          a warpgroup per head, one thread per query row (a lane of tensor memory): row maximum, then
@@ -33,6 +33,10 @@ static_assert(TKB_HD == 64 || TKB_HD == 128, "head size 64 or 128");
 using namespace tkb5;
 
 namespace {
+
+// Key tiles from which a lone head's go to two units: what putting two together costs is won back late (24 heads of 128 on 8, us, one
+// unit / two: 64 tokens at 364 keys 11.6 / 13.2, at 1,264 24.4 / 24.6, at 1,664 29.6 / 28.9, 128 at 2,128 39.0 / 37.0).
+constexpr int LONE_TILES = 22;
 
 constexpr int HD = TKB_HD;
 constexpr int ATOMS = HD / 64;           // 64-column (128-byte) blocks of a row of head size
@@ -185,6 +189,8 @@ __device__ __forceinline__ float row_exp(uint32_t s_addr, unsigned char* prow, i
   return s0 + s1;
 }
 
+// LONE: some block has one head (the build without is that of two heads a block throughout)
+template <bool LONE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int tma_rows,
                         const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out, int out_stride,
@@ -202,13 +208,31 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   __shared__ int failed;
   trigger_dependents();
   grid_dependency_wait();
-  // Blocks of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
+  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block).  In odd groups of heads the blocks
+  // of two heads for all query tiles come first, then the ones of the heads without a partner, which take half as long (in the
   // tiles' order the last blocks of two heads started when the SMs were nearly through).
-  // `single`: one head a block (the host asks for it when pairs would leave SMs without a block)
-  const int group = nh / nkv, per_tile = nkv * (single ? group : group >> 1);
-  const unsigned id = blockIdx.y * gridDim.x + blockIdx.x, n_pairs = gridDim.y * per_tile;
-  const bool paired = id < n_pairs;
-  const int tile = paired ? id / per_tile : (id - n_pairs) / nkv;
+  const int group = nh / nkv;
+  int tile = blockIdx.y, kvh, head0, n_heads_here = LONE && single ? 1 : 2;
+  if (!LONE || single || !(group & 1)) {
+    kvh = blockIdx.x / (single ? group : group >> 1);
+    head0 = blockIdx.x * n_heads_here;
+  } else {
+    const int per_tile = nkv * (group >> 1);
+    unsigned id = blockIdx.y * gridDim.x + blockIdx.x;
+    const unsigned n_pairs = gridDim.y * per_tile;
+    if (id < n_pairs) {
+      tile = id / per_tile;
+      id -= tile * per_tile;
+      kvh = id / (group >> 1);
+      head0 = 2 * id + kvh;
+    } else {
+      id -= n_pairs;
+      tile = id / nkv;
+      kvh = id - tile * nkv;
+      head0 = (kvh + 1) * group - 1;
+      n_heads_here = 1;
+    }
+  }
   if (tile >= *n_tiles_ptr) return;
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sQ = base;                         // two heads
@@ -218,11 +242,6 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   const int s = tiles[2 * tile], qt0 = tiles[2 * tile + 1];
-  const int in_tile = paired ? id - tile * per_tile : id - n_pairs - tile * nkv;
-  const int kvh = paired ? in_tile / (single ? group : group >> 1) : in_tile;
-  const int head0 = paired ? in_tile * (single ? 1 : 2) + (single ? 0 : kvh * (group & 1)) : (kvh + 1) * group - 1;
-  const int n_heads_here = paired && !single ? 2 : 1;
-  const int streams = 3 - n_heads_here;  // unit u: head u, or tiles u, u + 2, ... of the only head
   const int q_len = seq_q_len[s], kv_len = seq_kv_len[s];
   const int rows_live = min(BQ, q_len - qt0);
   const int pos0 = kv_len - q_len + qt0;
@@ -230,7 +249,9 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   if (window > 0 && pos0 - window + 1 > 0) k_begin = (pos0 - window + 1) & ~(BKV - 1);
   const int k_end = pos0 + rows_live;  // one past the last key any row of the tile sees
   const int n_kv_tiles = (k_end - k_begin + BKV - 1) / BKV;
-  const int live_units = min(2, n_heads_here * n_kv_tiles);
+  // Unit u: head u, or (split: a lone head from LONE_TILES on) tiles u, u + 2, ... of the only head
+  const int split = LONE && n_heads_here == 1 && n_kv_tiles >= LONE_TILES ? 1 : 0, streams = 1 << split;
+  const int live_units = split ? 2 : n_heads_here;
   const int* table = page_ids + page_indptr[s];
   const int t0 = seq_q_start[s] + qt0;
 
@@ -248,7 +269,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         mbar_init(&pv_done[i][b], 1);
       }
     }
-    mbar_init(&over, 4 * live_units);
+    mbar_init(&over, 8);
     mbar_init(&merged, 4);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -311,8 +332,8 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if (!ok) failed = 1;
     report_bad_page(bad_page, status);
   } else if (warp >= 10) {
-    const int hh = warp - 10, head = streams == 2 ? 0 : hh, stream = streams == 2 ? hh : 0;
-    const int n_mine = (n_kv_tiles - stream + streams - 1) / streams;
+    const int hh = warp - 10, head = split ? 0 : hh, stream = split ? hh : 0;
+    const int n_mine = (n_kv_tiles - stream + streams - 1) >> split;
     if (lane == 0 && hh < live_units) {
       // ---------------- MMA issuer of unit hh: S_0 and S_1; then for every tile: (wait P_j, which also frees its S
       // tile) Q . K_{j+2}^T, O += P_j . V_j
@@ -323,7 +344,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       const uint64_t desc_p0 = make_desc(smem_u32(sP + (hh * 2) * P_BYTES));
       bool ok = true;
       auto issue_qk = [&](int j) {
-        const int t = stream + j * streams, kb = t % KV_STAGES;
+        const int t = stream + (j << split), kb = t % KV_STAGES;
         if (!mbar_wait(&k_full[kb], (t / KV_STAGES) & 1)) return false;
         tcgen05_fence_after();
         const uint64_t dk = desc_k0 + (uint64_t)(kb * (KV_BYTES / 16));
@@ -338,7 +359,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       ok = issue_qk(0);
       if (ok && n_mine > 1) ok = issue_qk(1);
       for (int j = 0; j < n_mine && ok; j++) {
-        const int t = stream + j * streams, vb = t % KV_STAGES, pb = j & 1;
+        const int t = stream + (j << split), vb = t % KV_STAGES, pb = j & 1;
         if (!mbar_wait(&p_full[hh], j & 1)) { ok = false; break; }
         if (j + 2 < n_mine && !issue_qk(j + 2)) { ok = false; break; }
         if (!mbar_wait(&v_full[vb], (t / KV_STAGES) & 1)) { ok = false; break; }
@@ -355,8 +376,8 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     }
   } else if ((warp >> 2) < live_units) {
     // ---------------- softmax and output: thread = query row = lane of tensor memory
-    const int hh = warp >> 2, head = streams == 2 ? 0 : hh, stream = streams == 2 ? hh : 0;
-    const int n_mine = (n_kv_tiles - stream + streams - 1) / streams;
+    const int hh = warp >> 2, head = split ? 0 : hh, stream = split ? hh : 0;
+    const int n_mine = (n_kv_tiles - stream + streams - 1) >> split;
     const int r = tid & 127;
     const int pos = pos0 + r;
     const int lim_hi = pos < k_end - 1 ? pos : k_end - 1;
@@ -366,7 +387,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     float ref = NEG_BIG, l = 0.f;  // reference of the exponentials (and so of O and l); row sum
     bool ok = true;
     for (int j = 0; j < n_mine; j++) {
-      const int key0 = k_begin + (stream + j * streams) * BKV;
+      const int key0 = k_begin + (stream + (j << split)) * BKV;
       if (!mbar_wait(&s_full[hh][j & 1], (j >> 1) & 1)) { ok = false; break; }
       tcgen05_fence_after();
       const uint32_t sj = s_addr + (j & 1) * BKV;
@@ -411,8 +432,10 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       mbar_arrive(&p_full[hh]);
     }
     if (ok) ok = mbar_wait(&pv_done[hh][(n_mine - 1) & 1], ((n_mine - 1) >> 1) & 1);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&over);
+    if (split) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&over);
+    }
     float* sO = reinterpret_cast<float*>(sP);  // [column][row], once no product reads a P any more
     static_assert(4 * P_BYTES >= BQ * HD * 4, "the second unit's output goes through the P tiles' memory");
     if (ok && stream > 0) {
@@ -433,7 +456,7 @@ attn_prefill_acc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       if (lane == 0) mbar_arrive(&merged);
     } else if (ok) {
       tcgen05_fence_after();
-      const bool two = streams == 2 && live_units == 2;
+      const bool two = split != 0;
       if (two) ok = mbar_wait(&merged, 0);
       const float top = two ? fmaxf(ref, other_m[r]) : ref;
       const float mine = two ? fast_exp2(ref - top) : 1.f, theirs = two ? fast_exp2(other_m[r] - top) : 0.f;
@@ -485,7 +508,8 @@ TKB_EXPORT int tkb_attn_prefill_acc_bf16(const void* q, int q_stride, void* out,
   if (tiles_cap > 65535) return -3;
   static bool attr_done = false;
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_acc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_acc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_acc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
@@ -504,7 +528,8 @@ TKB_EXPORT int tkb_attn_prefill_acc_bf16(const void* q, int q_stride, void* out,
   }
   const int pairs = single ? nh / nkv : (nh / nkv + 1) / 2;
   dim3 grid(nkv * pairs, tiles_cap);  // the head pairs of one query tile are neighbours: long tiles start first
-  return launch_pdl(attn_prefill_acc_kernel, grid, dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)st, map_k, map_v,
+  const bool lone = single || (nh / nkv) % 2 != 0;
+  return launch_pdl(lone ? attn_prefill_acc_kernel<true> : attn_prefill_acc_kernel<false>, grid, dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)st, map_k, map_v,
                     tma_rows, (const bf16*)q, q_stride, (bf16*)out, out_stride, (const bf16*)kcache, (const bf16*)vcache,
                     seq_q_start, seq_q_len, seq_kv_len, page_indptr, page_ids, tiles, n_tiles_ptr, nh, nkv, ps,
                     scale * 1.4426950408889634f, window, status, n_pages, single ? 1 : 0);
