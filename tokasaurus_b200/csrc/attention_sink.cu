@@ -427,9 +427,20 @@ sink_attn_prep_rows_kernel(const float* __restrict__ qkv, int stride, const floa
       if (norm_w && is_qk) w = *reinterpret_cast<const float4*>(norm_w + (hh < nh ? 0 : QK) + e);
 #pragma unroll
       for (int k = 0; k < N; k++) {
-        float ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, v[k].w * v[k].w)));
+        // the additions of sink_attn_prep_vec_kernel, in which every lane of a warp has QK / 32 of a vector's numbers (a vector's
+        // lanes are all of q and k or none)
+        float ss;
+        if constexpr (QK == 128) {
+          ss = fmaf(v[k].w, v[k].w, fmaf(v[k].z, v[k].z, fmaf(v[k].y, v[k].y, v[k].x * v[k].x)));
 #pragma unroll
-        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);  // (a vector's lanes are all of q and k or none)
+          for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        } else {
+          float s1 = fmaf(v[k].w, v[k].w, v[k].z * v[k].z);
+          ss = fmaf(v[k].y, v[k].y, v[k].x * v[k].x);
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o), s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+          ss += s1;
+        }
         const float r = rsqrtf(ss / (float)QK + eps);
         if (is_qk) v[k].x = v[k].x * r * w.x, v[k].y = v[k].y * r * w.y, v[k].z = v[k].z * r * w.z, v[k].w = v[k].w * r * w.w;
       }
