@@ -840,9 +840,13 @@ int prep_launch(const float* qkv, int stride, const float* bias, int norm, float
 #ifdef TKB_SINK_PREP_VEC
   auto al16 = [](const void* p) { return p == nullptr || ((uintptr_t)p & 15) == 0; };
   const bool vec = norm != 2 && (freq == nullptr || rot_pairs) && stride % 4 == 0 && al16(qkv) && al16(bias) && al16(norm_w) && al16(q_out) && al16(cache);
-  // From four tokens an SM on; rows of more than 4,096 columns keep a warp busy for long, and need more blocks.
+  // Narrow rows from four tokens an SM on, wide ones, which keep a warp busy for long, where there are blocks for them.  Us, a block a
+  // token / four tokens a block (bias and weighted norms): heads of 64, 768 columns 600 tokens 3.8 / 3.7; 1,536 columns 600 4.3 / 5.1,
+  // 800 7.0 / 5.5; 3,072 columns 600 5.8 / 7.3, 800 8.8 / 8.1; heads of 128, 3,072 columns 600 4.8 / 7.8, 1,300 8.7 / 9.1, 1,600 10.7 / 9.3;
+  // more than 4,096 columns from 2,048 on.
   const int columns = (nh + (own_kv ? nkv : 0)) * QK + (own_kv ? nkv * VD : 0);
-  if (vec && n_tokens >= (columns <= 4096 ? 592 : 2048))
+  const int tokens_from = columns > 4096 ? 2048 : QK > 64 ? 1536 : columns > 1024 ? 740 : 592;
+  if (vec && n_tokens >= tokens_from)
     return launch_pdl(sink_attn_prep_rows_kernel<T>, dim3((n_tokens + PREP_TOKENS - 1) / PREP_TOKENS), dim3(256), 0, st, qkv, stride, bias, norm, eps, (T*)q_out,
                       (T*)cache, positions, token_seq, page_indptr, page_ids, n_tokens, nh, nkv, page_size, num_pages, write_cache,
                       status, norm_w, freq, rot_dims, values_are_keys, own_kv);
