@@ -532,8 +532,8 @@ gla_gates_kernel(float* __restrict__ proj, int stride, int low_off, int rank, co
 // The same for 64 tokens and more: a block 64 tokens x 128 columns, 32 ranks of both factors at a time in shared memory, a thread
 // 4 tokens x 8 columns (12 values read for 32 FMAs).  Every sum is the other kernel's chain: bias, then the ranks in order.  A block of 8
 // tokens reads the whole second factor for them: 197 MB out of the L2 for 3,001 tokens of 2,048 columns, rank 64: 60 us, 41 here (sums
-// 16, decays 8, the rest memory).  Where the tiles are fewer than the SMs the other kernel is the faster one (64 tokens of 2,048
-// columns: a layer 62 us, 66 with tiles).
+// 16, decays 8, the rest memory).  Where the tiles are few the other kernel is the faster one (64 tokens of 2,048 columns: a layer
+// 62 us, 66 with tiles).
 constexpr int GT_TOKENS = 64, GT_COLS = 128, GT_RANKS = 32;
 __global__ void __launch_bounds__(256)
 gla_gates_tile_kernel(float* __restrict__ proj, int stride, int low_off, int rank, const float* __restrict__ a2t,
@@ -678,7 +678,10 @@ TKB_EXPORT int tkb_gla_gates(float* proj, int stride, int low_off, int rank, con
   if (rank <= 0 || C <= 0 || (size_t)8 * rank * sizeof(float) > 48 * 1024) return -2;
   if ((C + 255) / 256 > 65535) return -2;
   const long long tiles = (long long)((n_tokens + GT_TOKENS - 1) / GT_TOKENS) * ((C + GT_COLS - 1) / GT_COLS);
-  if (tiles >= sm_count() && (C + GT_COLS - 1) / GT_COLS <= 65535)
+  // Tiles from where there are 1.75 an SM (four beyond a rank of 64): a block of either kernel is a chain, and one tile's is the longer
+  // one.  Rank 64, us, 8 tokens a block / tiles: 160 tiles (600 tokens of 2,048 columns) 15.3 / 20.2, 256 20.4 / 20.9, 264 22.7 / 21.0, 320
+  // 25.2 / 21.3; 4,800 tokens of 130 columns (150) 10.0 / 17.2; rank 128: 256 34 / 41, 512 60.6 / 61.2, 752 87 / 74.
+  if ((rank <= 64 ? 4 * tiles >= 7ll * sm_count() : tiles >= 4ll * sm_count()) && (C + GT_COLS - 1) / GT_COLS <= 65535)
     return launch_pdl(gla_gates_tile_kernel, dim3((n_tokens + GT_TOKENS - 1) / GT_TOKENS, (C + GT_COLS - 1) / GT_COLS), dim3(256), 0,
                       (cudaStream_t)st, proj, stride, low_off, rank, a2t, bias, inv_tau, C, f, q_off, q_cols, q_scale, n_tokens);
   return launch_pdl(gla_gates_kernel<8>, dim3((n_tokens + 7) / 8, (C + 255) / 256), dim3(256),
