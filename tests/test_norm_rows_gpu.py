@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
 
 
-@pytest.mark.parametrize("rows,H", [(592, 1024), (593, 1028), (595, 2044), (597, 2048), (599, 2052), (601, 3000), (1030, 4096), (594, 4092)])
+@pytest.mark.parametrize("rows,H", [(592, 1024), (593, 1028), (595, 2044), (597, 2048), (599, 2052), (601, 3000), (1030, 4096), (594, 4092),
+                                    (887, 1024), (889, 1028), (891, 1536), (1479, 2048), (1483, 2044), (1776, 2048), (1777, 1540)])
 @pytest.mark.parametrize("form", ["none", "bfloat16", "slice"])
 def test_add_rmsnorm_of_many_rows(rows, H, form):
     from tokasaurus_b200.kernels import ops

@@ -310,7 +310,7 @@ static int add_rmsnorm_bulk_launch(float* x, Slices sl, size_t bulk_bytes, const
 // a row (one to 2,048 numbers, two beyond), a lane up to 16 pieces of four numbers, all on their way together; nothing but the
 // lanes' sums crosses a barrier.  Bound by memory.  With a block a row (two pieces a thread, two barriers) and so, us: 2,048 rows of
 // 2,048 with an update in bfloat16 11.5 and 10.0, as a float32 slice 14.4 and 11.5; 4,001 rows 24.4 and 19.1 (6.0 TB/s); 2,080 rows of
-// 3,072 16.7 and 13.3; from 592 rows (four an SM) on, below there are too few warps (600 rows of 1,024 3.6 either way).
+// 3,072 16.7 and 13.3; below 592 rows (four an SM) there are too few warps (600 rows of 1,024 3.6 either way).
 template <typename T, int MODE, int WPR>
 __global__ void __launch_bounds__(128, 3)
 add_rmsnorm_warp_kernel(float* __restrict__ x, const void* __restrict__ update, const float* __restrict__ w, T* __restrict__ out,
@@ -386,8 +386,13 @@ static int add_rmsnorm_launch(float* x, const void* delta, Slices sl, const floa
   }
   // few rows: many threads a row, they hide the latency; many rows: several rows an SM in flight do
   int threads = H >= 8192 || (H >= 2048 && rows < 592) ? 512 : (H >= 512 ? 256 : 128);
-  if (sizeof(T) == 2 && rows >= 592 && (H & 3) == 0 && H >= 1024 && H <= 4096 && (sl.p == nullptr || (sl.n == 1 && sl.p2 == nullptr))) {
-    const int mode = sl.p != nullptr ? 2 : (delta != nullptr ? 1 : 0), wpr = H <= 2048 ? 1 : 2;
+  const int row_mode = sl.p != nullptr ? 2 : (delta != nullptr ? 1 : 0), wpr = H <= 2048 ? 1 : 2;
+  // A float32 slice gains from 592 rows on (600 rows of 2,048 5.6 -> 4.4 us), and so do rows of two warps.  Rows of one warp without
+  // one need more of them: 700 rows of 2,048 with an update in bfloat16 3.7 us a block a row, 4.8 a warp a row (1,000: 5.0 and 5.2, 1,500:
+  // 6.0 and 5.5), without an update 2.4 and 3.0 (1,500: 3.4 and 3.7, 2,048: 4.4 and 3.6); of 1,024 3.1 and 3.5 (1,000: 4.0 and 3.8).
+  const int rows_from = row_mode == 2 || wpr == 2 ? 592 : H <= 1536 ? 888 : row_mode == 1 ? 1480 : 1776;
+  if (sizeof(T) == 2 && rows >= rows_from && (H & 3) == 0 && H >= 1024 && H <= 4096 && (sl.p == nullptr || (sl.n == 1 && sl.p2 == nullptr))) {
+    const int mode = row_mode;
     const dim3 grid((rows + 4 / wpr - 1) / (4 / wpr));
     const void* update = mode == 2 ? (const void*)sl.p : delta;
 #define TKB_NORM_ROWS(MODE, WPR) \
