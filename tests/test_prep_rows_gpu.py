@@ -23,7 +23,7 @@ DT = {"bfloat16": torch.bfloat16, "float32": torch.float32}
     (739, 16, 4, 64, 64, True, 2, 64, False, True, True),
     (743, 16, 4, 64, 64, True, 2, 64, False, True, True),
     (1537, 6, 2, 128, 64, False, 1, 64, False, True, True),
-    (1601, 24, 8, 64, 128, False, 1, 42, True, True, True),
+    (1601, 24, 8, 64, 64, False, 1, 42, True, True, True),
 ])
 def test_prep_of_many_tokens_is_that_of_few(dtype, tokens, heads, kv, dim, vdim, bias, norm, rot, vk, own, write):
     from tokasaurus_b200.kernels import ops

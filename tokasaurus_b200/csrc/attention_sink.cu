@@ -451,13 +451,13 @@ sink_attn_prep_rows_kernel(const float* __restrict__ qkv, int stride, const floa
       for (int k = 0; k < N; k++) {
         const float2 c0 = rot_cs[k][j];
         const float a = v[k].x, b = v[k].y;
-        v[k].x = a * c0.x - b * c0.y;
-        v[k].y = b * c0.x + a * c0.y;
+        v[k].x = fmaf(a, c0.x, -(b * c0.y));
+        v[k].y = fmaf(b, c0.x, a * c0.y);
         if (j + 1 < half) {
           const float2 c1 = rot_cs[k][j + 1];
           const float a1 = v[k].z, b1 = v[k].w;
-          v[k].z = a1 * c1.x - b1 * c1.y;
-          v[k].w = b1 * c1.x + a1 * c1.y;
+          v[k].z = fmaf(a1, c1.x, -(b1 * c1.y));
+          v[k].w = fmaf(b1, c1.x, a1 * c1.y);
         }
       }
     }
