@@ -810,6 +810,9 @@ int make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld) {
   return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
 }
 
+// Numbers from one row of the pieces that are cut ahead to the next
+long long cut_ld(int K) { return (K + 7) / 8 * 8; }
+
 // vec: both operands' rows take 16-byte loads
 template <int NT>
 int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, float* part, int M, int N, int K, int lda, int ldw, int ldc, bool vec,
@@ -827,7 +830,7 @@ int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, f
     rc = get_encode();
     if (rc == 0) rc = make_map_f32(&map, W, N, K, ldw);
     if constexpr (TCfg<NT>::PRECUT) {
-      const int ld = (K + 7) / 8 * 8;
+      const int ld = (int)cut_ld(K);
       if (rc == 0) rc = make_map(&map_a, cut, 3 * M, K, ld, NT);
       const long long blocks = ((long long)M * (ld / 8) + 255) / 256;
       if (rc == 0) rc = launch_pdl(sgemm_cut_kernel, dim3((unsigned)blocks), dim3(256), 0, st, A, cut, M, K, lda, ld);
@@ -849,10 +852,27 @@ int token_columns(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 1
 
 }  // namespace
 
+// Whether both operands' rows take 16-byte loads (sgemm_tma_kernel).
+static bool operands_vec(const float* A, const float* W, int M, int K, int lda, int ldw) {
+  return 3ll * M < (1ll << 31) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+}
+// Rows whose pieces are cut ahead at a time.  Pieces take 6 bytes a number, and nothing beside torch's allocator accounts for them:
+// calls of more than CUT_BYTES of them (8,192 rows of 8,192 numbers would take 403 MB) go in blocks of rows, of as many row tiles up
+// to that bound, and from half of it on, as leave the fewest SMs idle in the last wave.  A row tile has 128 rows whatever the bound.
+constexpr long long CUT_BYTES = 128ll << 20;
+static int cut_rows(int M, int N, int K) {
+  const long long tiles = (N + 127) / 128, sms = tkb::sm_count(), fit = CUT_BYTES / (128 * 6 * cut_ld(K)), most = fit > 1 ? fit : 1;
+  if (token_columns(M) <= 64 || M <= most * 128) return M;
+  auto idle = [&](long long r) { return (double)((r * tiles + sms - 1) / sms * sms) / (double)(r * tiles); };
+  long long best = most;
+  for (long long r = most - 1; r >= 1 && 2 * r >= most; r--)
+    if (idle(r) < idle(best)) best = r;
+  return (int)best * 128;
+}
 // Scratch, in float32 values: the tokens' pieces where they are cut ahead, then the K slices' partial results, when one block a
 // slice ends sooner than blocks that do all of K (500 rows x 3,072 x 2,048: 69 us in slices, 60 in 96 blocks; 300 rows 51 and 58;
 // 700 rows x 2,048 x 2,048 83 and 63).  The results' bits do not depend on it.
-static long long cut_scratch(int M, int K) { return token_columns(M) > 64 ? (3ll * M * ((K + 7) / 8 * 8) + 7) / 8 * 4 : 0; }
+static long long cut_scratch(int M, int K, bool vec) { return vec && token_columns(M) > 64 ? (3ll * M * cut_ld(K) + 7) / 8 * 4 : 0; }
 static long long slice_scratch(int M, int N, int K) {
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
   const long long blocks = (long long)((N + 127) / 128) * ((M + token_columns(M) - 1) / token_columns(M)), sms = tkb::sm_count();
@@ -864,10 +884,12 @@ static long long slice_scratch(int M, int N, int K) {
   if (slices == 1 || all <= sliced || M > 65535) return 0;
   return (long long)slices * M * N;
 }
-// Float32 values of scratch that tkb_sgemm_tn_f32 wants for these sizes (0: none).
-TKB_EXPORT long long tkb_sgemm_tn_scratch(int M, int N, int K) {
+// Float32 values of scratch that tkb_sgemm_tn_f32 wants for this call (0: none).
+TKB_EXPORT long long tkb_sgemm_tn_scratch(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
   if (M <= 0 || N < SPLIT_MIN || K < SPLIT_MIN) return 0;
-  return cut_scratch(M, K) + slice_scratch(M, N, K);
+  const bool vec = operands_vec(A, W, M, K, lda, ldw);
+  const int rows = vec ? cut_rows(M, N, K) : M;
+  return cut_scratch(rows, K, vec) + slice_scratch(rows, N, K);
 }
 
 // scratch: as many float32 values as tkb_sgemm_tn_scratch says, or null where it says 0.  status: the device status word that
@@ -878,13 +900,20 @@ TKB_EXPORT int tkb_sgemm_tn_f32(const float* A, const float* W, float* C, float*
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return -2;
   if (N >= SPLIT_MIN && K >= SPLIT_MIN) {
-    if ((scratch != nullptr) != (tkb_sgemm_tn_scratch(M, N, K) > 0)) return -4;
+    if ((scratch != nullptr) != (tkb_sgemm_tn_scratch(A, W, M, N, K, lda, ldw) > 0)) return -4;
     const int nt = token_columns(M);
     if ((M + nt - 1) / nt > 65535) return -3;
-    const bool vec = 3ll * M < (1ll << 31) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+    const bool vec = operands_vec(A, W, M, K, lda, ldw);
+    const int rows = vec ? cut_rows(M, N, K) : M;
     __nv_bfloat16* cut = reinterpret_cast<__nv_bfloat16*>(scratch);
-    float* part = slice_scratch(M, N, K) ? scratch + cut_scratch(M, K) : nullptr;
-#define TKB_GO(NT) return split_launch<NT>(A, W, C, cut, part, M, N, K, lda, ldw, ldc, vec, status, st);
+    float* part = slice_scratch(rows, N, K) ? scratch + cut_scratch(rows, K, vec) : nullptr;
+    for (int m = 0; m + rows < M; m += rows) {  // (more than a block of rows: 128 token columns)
+      const int rc = split_launch<128>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, rows, N, K, lda, ldw, ldc, vec, status, st);
+      if (rc) return rc;
+    }
+    const int m = (M - 1) / rows * rows;
+#define TKB_GO(NT) \
+  return split_launch<NT>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, M - m, N, K, lda, ldw, ldc, vec, status, st);
     if (nt == 16) { TKB_GO(16) }
     if (nt == 32) { TKB_GO(32) }
     if (nt == 64) { TKB_GO(64) }

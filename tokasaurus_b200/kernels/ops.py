@@ -388,7 +388,7 @@ class reporting_to:
 
 def _sgemm_scratch(lib: ctypes.CDLL):
     f = _fn(lib, "tkb_sgemm_tn_scratch")
-    f.restype, f.argtypes = ctypes.c_longlong, (c_int, c_int, c_int)
+    f.restype, f.argtypes = ctypes.c_longlong, (c_void_p, c_void_p) + (c_int,) * 5
     return f
 
 
@@ -401,11 +401,12 @@ def sgemm_tn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _need(a.dtype == w.dtype == out.dtype == torch.float32, "sgemm_tn: float32 only")
     _need(a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1, "sgemm_tn: rows must be contiguous")
     lib = _libs.get("sgemm.cu")
-    n_scratch = _sgemm_scratch(lib)(M, N, K)
+    lda, ldw = a.stride(0) if M > 1 else K, w.stride(0) if N > 1 else K
+    n_scratch = _sgemm_scratch(lib)(_ptr(a), _ptr(w), M, N, K, lda, ldw)
     scratch = torch.empty((n_scratch,), dtype=torch.float32, device=a.device) if n_scratch else None
     f = _fn(lib, "tkb_sgemm_tn_f32")
-    _check(f(_ptr(a), _ptr(w), _ptr(out), _ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(a.stride(0) if M > 1 else K),
-             c_int(w.stride(0) if N > 1 else K), c_int(out.stride(0) if M > 1 else N), _ptr(getattr(_step, "status", None)), _stream()),
+    _check(f(_ptr(a), _ptr(w), _ptr(out), _ptr(scratch), c_int(M), c_int(N), c_int(K), c_int(lda),
+             c_int(ldw), c_int(out.stride(0) if M > 1 else N), _ptr(getattr(_step, "status", None)), _stream()),
            "sgemm_tn")
 
 
