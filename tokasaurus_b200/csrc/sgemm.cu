@@ -17,8 +17,9 @@
 //   cut form is not what it is uncut; or a sum from 2^80 on) is done once more as the FMA chain, by the warp that has it (redo).
 //   K is cut into slices by N and K alone, as many as fill the GPU when there are few rows; then each slice is a block's and a
 //   second kernel adds them in order.  Where that ends sooner (slice_scratch) a block does all slices and adds them in the same order.
-//   Two kernels with the same bits: sgemm_tma_kernel where both operands' rows take 16-byte loads, sgemm_split_kernel (15 warps that
-//   fetch, cut and store, the next chunks on their way into registers meanwhile, and one that issues the tensor instructions) else.
+//   Two kernels with the same bits: sgemm_tma_kernel where both operands' rows take 16-byte loads (and goes_by_tma says so),
+//   sgemm_split_kernel (15 warps that fetch, cut and store, the next chunks on their way into registers meanwhile, and one that issues
+//   the tensor instructions) else.
 //   What bounds sgemm_tma_kernel: with many rows the tensor instructions (six products: a sixth of their rate is the bound; two
 //   thirds of a block's time they run, the rest goes on the sums' way out, for which there is no second buffer, and on blocks' starts),
 //   with few the warps that cut (clocks of a chunk of 64 k's: 1,250 of 1,900; at 40 GB/s an SM the weights take 1,550).
@@ -150,15 +151,22 @@ template <> __device__ __forceinline__ void tmem_read<32>(uint32_t a, float (&v)
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Eight numbers from p on, of which `left` are there (p null: none).
+// Eight numbers from p on, of which `left` are there (p null: none).  VEC: in 16-byte loads (K is a multiple of 4: a piece of four is
+// there or not).
+template <bool VEC>
 __device__ __forceinline__ void fetch8(const float* __restrict__ p, int left, float4& x0, float4& x1) {
   x0 = x1 = make_float4(0.f, 0.f, 0.f, 0.f);
   if (p == nullptr) return;
-  float v[8];
+  if (VEC) {
+    if (left > 0) x0 = __ldg(reinterpret_cast<const float4*>(p));
+    if (left > 4) x1 = __ldg(reinterpret_cast<const float4*>(p + 4));
+  } else {
+    float v[8];
 #pragma unroll
-  for (int u = 0; u < 8; u++) v[u] = u < left ? __ldg(p + u) : 0.f;
-  x0 = make_float4(v[0], v[1], v[2], v[3]);
-  x1 = make_float4(v[4], v[5], v[6], v[7]);
+    for (int u = 0; u < 8; u++) v[u] = u < left ? __ldg(p + u) : 0.f;
+    x0 = make_float4(v[0], v[1], v[2], v[3]);
+    x1 = make_float4(v[4], v[5], v[6], v[7]);
+  }
 }
 
 // Results that did not come out finite, once more as FMA chains over K in index order.  A warp: o[i * ldo] (i below `tokens`) of the
@@ -242,7 +250,7 @@ __device__ __noinline__ void redo_row(const float* __restrict__ part, const floa
 }
 
 // out: C when a block does all slices (`slices_here`), else the slices' partial results [slice][M][N].
-template <int NT>
+template <int NT, bool VEC>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N, int K,
                    int lda, int ldw, int ldc, int per_slice, int slices_here, int partial, int* __restrict__ status) {
@@ -399,12 +407,12 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
 #pragma unroll
       for (int i = 0; i < TASKS; i++) {
         if constexpr (KEPT) {
-          fetch8(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
+          fetch8<VEC>(src[i] == nullptr ? nullptr : src[i] + (size_t)c * CHUNK, left, x[into][i][0], x[into][i][1]);
         } else {
           const int r = r0 + i * ROWS;
           const bool is_w = r < 128, there = is_w ? n0 + r < N : r < 128 + NT && m0 + r - 128 < M;
           const float* p = (is_w ? W + (size_t)(n0 + r) * ldw : A + (size_t)(m0 + r - 128) * lda) + k;
-          fetch8(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
+          fetch8<VEC>(there ? p : nullptr, left, x[into][i][0], x[into][i][1]);
         }
       }
     };
@@ -423,7 +431,7 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
           const int r = r0 + i * ROWS, dst = r * 128 + ((seg ^ (r & 7)) << 4);
           if (r >= 128 + NT) continue;
           uint4 h, m, l;
-          cut8(x[u][i][0], x[u][i][1], h, m, l);
+          cut8<NT != 128>(x[u][i][0], x[u][i][1], h, m, l);
           *reinterpret_cast<uint4*>(st + dst) = h;
           *reinterpret_cast<uint4*>(st + dst + Z::PLANE) = m;
           *reinterpret_cast<uint4*>(st + dst + 2 * Z::PLANE) = l;
@@ -445,7 +453,7 @@ sgemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
   tcgen05_fence_before();
   __syncthreads();
   if (tid == 0 && failed && status != nullptr) atomicOr(status, TKB_STATUS_WAIT_TIMEOUT);
-  if (!partial && !failed && odd) redo_tile<NT, false>(A, W, out, M, N, K, lda, ldw, ldc, n0, m0);
+  if (!partial && !failed && odd) redo_tile<NT, VEC>(A, W, out, M, N, K, lda, ldw, ldc, n0, m0);
   if (warp == 0) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Z::TMEM) : "memory");
@@ -813,18 +821,19 @@ int make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld) {
 // Numbers from one row of the pieces that are cut ahead to the next
 long long cut_ld(int K) { return (K + 7) / 8 * 8; }
 
-// vec: both operands' rows take 16-byte loads
+// vec: both operands' rows take 16-byte loads; tma: sgemm_tma_kernel's call
 template <int NT>
 int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, float* part, int M, int N, int K, int lda, int ldw, int ldc, bool vec,
-                 int* status, cudaStream_t st) {
+                 bool tma, int* status, cudaStream_t st) {
   static SharedMemoryRequest shared_memory;
-  int rc = shared_memory({{(const void*)sgemm_split_kernel<NT>, SCfg<NT>::SMEM}, {(const void*)sgemm_tma_kernel<NT>, TCfg<NT>::SMEM}});
+  int rc = shared_memory({{(const void*)sgemm_split_kernel<NT, false>, SCfg<NT>::SMEM}, {(const void*)sgemm_split_kernel<NT, NT == 128>, SCfg<NT>::SMEM},
+                      {(const void*)sgemm_tma_kernel<NT>, TCfg<NT>::SMEM}});
   if (rc) return rc;
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
   const int tiles = (N + 127) / 128, rows = (M + NT - 1) / NT;
   const int here = part == nullptr ? slices : 1, partial = part != nullptr;
   float* out = partial ? part : C;
-  if (vec && (long long)tiles * rows < (1ll << 31)) {
+  if (tma && (long long)tiles * rows < (1ll << 31)) {
     CUtensorMap map, map_a;
     memset(&map_a, 0, sizeof(map_a));
     rc = get_encode();
@@ -839,7 +848,9 @@ int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, f
     rc = launch_pdl(sgemm_tma_kernel<NT>, dim3(tiles * rows, 1, slices / here), dim3(TMA_THREADS), (size_t)TCfg<NT>::SMEM, st, map, map_a, A, W,
                     out, M, N, K, lda, ldw, ldc, rows, per, here, partial, status);
   } else {
-    rc = launch_pdl(sgemm_split_kernel<NT>, dim3(tiles, rows, slices / here), dim3(SPLIT_THREADS), (size_t)SCfg<NT>::SMEM, st, A, W, out,
+    // (with 16-byte loads only where sgemm_tma_kernel leaves such calls to it: 128 token columns)
+    auto kernel = vec && NT == 128 ? sgemm_split_kernel<NT, NT == 128> : sgemm_split_kernel<NT, false>;
+    rc = launch_pdl(kernel, dim3(tiles, rows, slices / here), dim3(SPLIT_THREADS), (size_t)SCfg<NT>::SMEM, st, A, W, out,
                     M, N, K, lda, ldw, ldc, per, here, partial, status);
   }
   if (rc || !partial) return rc;
@@ -869,27 +880,40 @@ static int cut_rows(int M, int N, int K) {
     if (idle(r) < idle(best)) best = r;
   return (int)best * 128;
 }
+// Whether a call is sgemm_tma_kernel's.  Not with more than 64 rows where cutting the tokens' numbers ahead, a pass over memory of its
+// own, saves little cutting: few column tiles share what is cut, and few blocks there are to be had.  Us, sgemm_split_kernel /
+// sgemm_tma_kernel: 300 rows x 256 x 4,096 22.5 / 24.0, 1,000 x 512 x 512 13.6 / 14.9, 200 x 1,024 x 1,024 12.6 / 14.6, 1,500 x 130 x 16,384
+// 159 / 173, 100 x 2,048 x 2,048 16.1 / 17.3; 1,000 rows x 1,024 x 1,024 47 / 46, 1,500 68 / 42, 129 x 2,048 x 2,048 30 / 28.
+static bool goes_by_tma(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
+  if (!operands_vec(A, W, M, K, lda, ldw)) return false;
+  if (token_columns(M) <= 64) return true;
+  const long long tiles = (N + 127) / 128, rows = (M + 127) / 128;
+  return !(tiles <= 8 && tiles * rows <= 64) && !(rows == 1 && (long long)N * K <= 1 << 22);
+}
 // Scratch, in float32 values: the tokens' pieces where they are cut ahead, then the K slices' partial results, when one block a
 // slice ends sooner than blocks that do all of K (500 rows x 3,072 x 2,048: 69 us in slices, 60 in 96 blocks; 300 rows 51 and 58;
 // 700 rows x 2,048 x 2,048 83 and 63).  The results' bits do not depend on it.
-static long long cut_scratch(int M, int K, bool vec) { return vec && token_columns(M) > 64 ? (3ll * M * cut_ld(K) + 7) / 8 * 4 : 0; }
-static long long slice_scratch(int M, int N, int K) {
+static long long cut_scratch(int M, int K, bool tma) { return tma && token_columns(M) > 64 ? (3ll * M * cut_ld(K) + 7) / 8 * 4 : 0; }
+static long long slice_scratch(int M, int N, int K, bool tma) {
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
   const long long blocks = (long long)((N + 127) / 128) * ((M + token_columns(M) - 1) / token_columns(M)), sms = tkb::sm_count();
+  if (slices == 1 || M > 65535) return 0;
   auto waves = [&](long long b) { return (b + sms - 1) / sms; };
   // in chunks (1.3 us): a block's start and end are worth five, a slice added to those before it three, the adding kernel three
   // and its traffic
   const long long all = waves(blocks) * (chunks + 3 * slices + 5);
   const long long sliced = waves(blocks * slices) * (per + 5) + 3 + (long long)slices * M * N / 800000;
-  if (slices == 1 || all <= sliced || M > 65535) return 0;
+  // sgemm_split_kernel, which adds a slice to those before it number by number: whole sums with row tiles for three quarters of the
+  // SMs (1,500 rows x 1,024 x 2,050, 96 blocks: 122 us in slices, 156 whole)
+  if (tma ? all <= sliced : blocks * 4 >= 3 * sms) return 0;
   return (long long)slices * M * N;
 }
 // Float32 values of scratch that tkb_sgemm_tn_f32 wants for this call (0: none).
 TKB_EXPORT long long tkb_sgemm_tn_scratch(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
   if (M <= 0 || N < SPLIT_MIN || K < SPLIT_MIN) return 0;
-  const bool vec = operands_vec(A, W, M, K, lda, ldw);
-  const int rows = vec ? cut_rows(M, N, K) : M;
-  return cut_scratch(rows, K, vec) + slice_scratch(rows, N, K);
+  const bool tma = goes_by_tma(A, W, M, N, K, lda, ldw);
+  const int rows = tma ? cut_rows(M, N, K) : M;
+  return cut_scratch(rows, K, tma) + slice_scratch(rows, N, K, tma);
 }
 
 // scratch: as many float32 values as tkb_sgemm_tn_scratch says, or null where it says 0.  status: the device status word that
@@ -903,17 +927,17 @@ TKB_EXPORT int tkb_sgemm_tn_f32(const float* A, const float* W, float* C, float*
     if ((scratch != nullptr) != (tkb_sgemm_tn_scratch(A, W, M, N, K, lda, ldw) > 0)) return -4;
     const int nt = token_columns(M);
     if ((M + nt - 1) / nt > 65535) return -3;
-    const bool vec = operands_vec(A, W, M, K, lda, ldw);
-    const int rows = vec ? cut_rows(M, N, K) : M;
+    const bool vec = operands_vec(A, W, M, K, lda, ldw), tma = goes_by_tma(A, W, M, N, K, lda, ldw);
+    const int rows = tma ? cut_rows(M, N, K) : M;
     __nv_bfloat16* cut = reinterpret_cast<__nv_bfloat16*>(scratch);
-    float* part = slice_scratch(rows, N, K) ? scratch + cut_scratch(rows, K, vec) : nullptr;
+    float* part = slice_scratch(rows, N, K, tma) ? scratch + cut_scratch(rows, K, tma) : nullptr;
     for (int m = 0; m + rows < M; m += rows) {  // (more than a block of rows: 128 token columns)
-      const int rc = split_launch<128>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, rows, N, K, lda, ldw, ldc, vec, status, st);
+      const int rc = split_launch<128>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, rows, N, K, lda, ldw, ldc, vec, tma, status, st);
       if (rc) return rc;
     }
     const int m = (M - 1) / rows * rows;
 #define TKB_GO(NT) \
-  return split_launch<NT>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, M - m, N, K, lda, ldw, ldc, vec, status, st);
+  return split_launch<NT>(A + (size_t)m * lda, W, C + (size_t)m * ldc, cut, part, M - m, N, K, lda, ldw, ldc, vec, tma, status, st);
     if (nt == 16) { TKB_GO(16) }
     if (nt == 32) { TKB_GO(32) }
     if (nt == 64) { TKB_GO(64) }
