@@ -148,19 +148,19 @@ def test_both_split_kernels_give_the_same_bits(M, N, K):
 
 
 def test_pieces_cut_ahead_are_bounded():
-    """Large calls go in blocks of rows, so that the pieces cut ahead take 128 MB at most; the bits are those of smaller calls, and
+    """Large calls go in blocks of rows, so that the pieces cut ahead take 256 MB at most; the bits are those of smaller calls, and
     operands without 16-byte loads, whose kernel cuts itself, ask for none."""
     from tokasaurus_b200.kernels import ops
 
     lib = ops._libs.get("sgemm.cu")
     sizes = lambda a, w: (ops._ptr(a), ops._ptr(w), a.shape[0], w.shape[0], a.shape[1], a.stride(0), w.stride(0))  # noqa: E731
     w = torch.empty(20000, 8192, device=DEV)  # enough column tiles for whole sums in a block
-    assert 0 < 4 * ops._sgemm_scratch(lib)(*sizes(torch.empty(8192, 8192, device=DEV), w)) <= 128 << 20
+    assert 0 < 4 * ops._sgemm_scratch(lib)(*sizes(torch.empty(8192, 8192, device=DEV), w)) <= 256 << 20
     odd = torch.empty(8192, 8193, device=DEV)[:, :8192]
     assert ops._sgemm_scratch(lib)(*sizes(odd, w)) == 0
     g = torch.Generator().manual_seed(9)
     K = 16384
-    for M, N in ((2900, 256), (1500, 2100)):  # two and three blocks of rows; sums in slices and whole
+    for M, N in ((2900, 1100), (2700, 2100)):  # two blocks of rows; sums in slices and whole
         a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
         out = torch.full((M + 1, N), 7.0, device=DEV)
         ops.sgemm_tn(a, w, out[:M])

@@ -870,7 +870,7 @@ static bool operands_vec(const float* A, const float* W, int M, int K, int lda, 
 // Rows whose pieces are cut ahead at a time.  Pieces take 6 bytes a number, and nothing beside torch's allocator accounts for them:
 // calls of more than CUT_BYTES of them (8,192 rows of 8,192 numbers would take 403 MB) go in blocks of rows, of as many row tiles up
 // to that bound, and from half of it on, as leave the fewest SMs idle in the last wave.  A row tile has 128 rows whatever the bound.
-constexpr long long CUT_BYTES = 128ll << 20;
+constexpr long long CUT_BYTES = 256ll << 20;
 static int cut_rows(int M, int N, int K) {
   const long long tiles = (N + 127) / 128, sms = tkb::sm_count(), fit = CUT_BYTES / (128 * 6 * cut_ld(K)), most = fit > 1 ? fit : 1;
   if (token_columns(M) <= 64 || M <= most * 128) return M;
