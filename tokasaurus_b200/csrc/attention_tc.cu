@@ -240,12 +240,6 @@ __device__ __forceinline__ void umma_a_tmem(uint32_t d, uint32_t a, uint64_t bde
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
       ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ bool mbar_done(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return done;
-}
 
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int tma_rows,

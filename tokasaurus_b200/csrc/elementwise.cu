@@ -386,25 +386,26 @@ static int add_rmsnorm_launch(float* x, const void* delta, Slices sl, const floa
   }
   // few rows: many threads a row, they hide the latency; many rows: several rows an SM in flight do
   int threads = H >= 8192 || (H >= 2048 && rows < 592) ? 512 : (H >= 512 ? 256 : 128);
-  const int row_mode = sl.p != nullptr ? 2 : (delta != nullptr ? 1 : 0), wpr = H <= 2048 ? 1 : 2;
-  // A float32 slice gains from 592 rows on (600 rows of 2,048 5.6 -> 4.4 us), and so do rows of two warps.  Rows of one warp without
-  // one need more of them: 700 rows of 2,048 with an update in bfloat16 3.7 us a block a row, 4.8 a warp a row (1,000: 5.0 and 5.2, 1,500:
-  // 6.0 and 5.5), without an update 2.4 and 3.0 (1,500: 3.4 and 3.7, 2,048: 4.4 and 3.6); of 1,024 3.1 and 3.5 (1,000: 4.0 and 3.8).
-  const int rows_from = row_mode == 2 || wpr == 2 ? 592 : H <= 1536 ? 888 : row_mode == 1 ? 1480 : 1776;
-  if (sizeof(T) == 2 && rows >= rows_from && (H & 3) == 0 && H >= 1024 && H <= 4096 && (sl.p == nullptr || (sl.n == 1 && sl.p2 == nullptr))) {
-    const int mode = row_mode;
-    const dim3 grid((rows + 4 / wpr - 1) / (4 / wpr));
-    const void* update = mode == 2 ? (const void*)sl.p : delta;
+  if constexpr (sizeof(T) == 2) {
+    const int mode = sl.p != nullptr ? 2 : (delta != nullptr ? 1 : 0), wpr = H <= 2048 ? 1 : 2;
+    // A float32 slice gains from 592 rows on (600 rows of 2,048 5.6 -> 4.4 us), and so do rows of two warps.  Rows of one warp without
+    // one need more of them: 700 rows of 2,048 with an update in bfloat16 3.7 us a block a row, 4.8 a warp a row (1,000: 5.0 and 5.2, 1,500:
+    // 6.0 and 5.5), without an update 2.4 and 3.0 (1,500: 3.4 and 3.7, 2,048: 4.4 and 3.6); of 1,024 3.1 and 3.5 (1,000: 4.0 and 3.8).
+    const int rows_from = mode == 2 || wpr == 2 ? 592 : H <= 1536 ? 888 : mode == 1 ? 1480 : 1776;
+    if (rows >= rows_from && (H & 3) == 0 && H >= 1024 && H <= 4096 && (sl.p == nullptr || (sl.n == 1 && sl.p2 == nullptr))) {
+      const dim3 grid((rows + 4 / wpr - 1) / (4 / wpr));
+      const void* update = mode == 2 ? (const void*)sl.p : delta;
 #define TKB_NORM_ROWS(MODE, WPR) \
   if (mode == MODE && wpr == WPR) \
     return launch_pdl(add_rmsnorm_warp_kernel<T, MODE, WPR>, grid, dim3(128), 0, st, x, update, w, (T*)out, eps, rows, H);
-    TKB_NORM_ROWS(0, 1)
-    TKB_NORM_ROWS(1, 1)
-    TKB_NORM_ROWS(2, 1)
-    TKB_NORM_ROWS(0, 2)
-    TKB_NORM_ROWS(1, 2)
-    TKB_NORM_ROWS(2, 2)
+      TKB_NORM_ROWS(0, 1)
+      TKB_NORM_ROWS(1, 1)
+      TKB_NORM_ROWS(2, 1)
+      TKB_NORM_ROWS(0, 2)
+      TKB_NORM_ROWS(1, 2)
+      TKB_NORM_ROWS(2, 2)
 #undef TKB_NORM_ROWS
+    }
   }
 #define TKB_NORM(MODE, MAXT)                                                                                        \
   return launch_pdl(add_rmsnorm_kernel<T, MODE, MAXT>, dim3(rows), dim3(threads), 0, st, x, (const T*)delta, sl, w, \
