@@ -861,17 +861,15 @@ int split_launch(const float* A, const float* W, float* C, __nv_bfloat16* cut, f
 // Token columns of an instruction: the fewest that hold all rows, at most 128.
 int token_columns(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
-}  // namespace
-
 // Whether both operands' rows take 16-byte loads (sgemm_tma_kernel).
-static bool operands_vec(const float* A, const float* W, int M, int K, int lda, int ldw) {
+bool operands_vec(const float* A, const float* W, int M, int K, int lda, int ldw) {
   return 3ll * M < (1ll << 31) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
 }
 // Rows whose pieces are cut ahead at a time.  Pieces take 6 bytes a number, and nothing beside torch's allocator accounts for them:
 // calls of more than CUT_BYTES of them (8,192 rows of 8,192 numbers would take 403 MB) go in blocks of rows, of as many row tiles up
 // to that bound, and from half of it on, as leave the fewest SMs idle in the last wave.  A row tile has 128 rows whatever the bound.
 constexpr long long CUT_BYTES = 256ll << 20;
-static int cut_rows(int M, int N, int K) {
+int cut_rows(int M, int N, int K) {
   const long long tiles = (N + 127) / 128, sms = tkb::sm_count(), fit = CUT_BYTES / (128 * 6 * cut_ld(K)), most = fit > 1 ? fit : 1;
   if (token_columns(M) <= 64 || M <= most * 128) return M;
   auto idle = [&](long long r) { return (double)((r * tiles + sms - 1) / sms * sms) / (double)(r * tiles); };
@@ -884,7 +882,7 @@ static int cut_rows(int M, int N, int K) {
 // own, saves little cutting: few column tiles share what is cut, and few blocks there are to be had.  Us, sgemm_split_kernel /
 // sgemm_tma_kernel: 300 rows x 256 x 4,096 22.5 / 24.0, 1,000 x 512 x 512 13.6 / 14.9, 200 x 1,024 x 1,024 12.6 / 14.6, 1,500 x 130 x 16,384
 // 159 / 173, 100 x 2,048 x 2,048 16.1 / 17.3; 1,000 rows x 1,024 x 1,024 47 / 46, 1,500 68 / 42, 129 x 2,048 x 2,048 30 / 28.
-static bool goes_by_tma(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
+bool goes_by_tma(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
   if (!operands_vec(A, W, M, K, lda, ldw)) return false;
   if (token_columns(M) <= 64) return true;
   const long long tiles = (N + 127) / 128, rows = (M + 127) / 128;
@@ -893,8 +891,8 @@ static bool goes_by_tma(const float* A, const float* W, int M, int N, int K, int
 // Scratch, in float32 values: the tokens' pieces where they are cut ahead, then the K slices' partial results, when one block a
 // slice ends sooner than blocks that do all of K (500 rows x 3,072 x 2,048: 69 us in slices, 60 in 96 blocks; 300 rows 51 and 58;
 // 700 rows x 2,048 x 2,048 83 and 63).  The results' bits do not depend on it.
-static long long cut_scratch(int M, int K, bool tma) { return tma && token_columns(M) > 64 ? (3ll * M * cut_ld(K) + 7) / 8 * 4 : 0; }
-static long long slice_scratch(int M, int N, int K, bool tma) {
+long long cut_scratch(int M, int K, bool tma) { return tma && token_columns(M) > 64 ? (3ll * M * cut_ld(K) + 7) / 8 * 4 : 0; }
+long long slice_scratch(int M, int N, int K, bool tma) {
   const int chunks = (K + CHUNK - 1) / CHUNK, per = chunks_a_slice(N, K), slices = (chunks + per - 1) / per;
   const long long blocks = (long long)((N + 127) / 128) * ((M + token_columns(M) - 1) / token_columns(M)), sms = tkb::sm_count();
   if (slices == 1 || M > 65535) return 0;
@@ -908,6 +906,8 @@ static long long slice_scratch(int M, int N, int K, bool tma) {
   if (tma ? all <= sliced : blocks * 4 >= 3 * sms) return 0;
   return (long long)slices * M * N;
 }
+}  // namespace
+
 // Float32 values of scratch that tkb_sgemm_tn_f32 wants for this call (0: none).
 TKB_EXPORT long long tkb_sgemm_tn_scratch(const float* A, const float* W, int M, int N, int K, int lda, int ldw) {
   if (M <= 0 || N < SPLIT_MIN || K < SPLIT_MIN) return 0;
